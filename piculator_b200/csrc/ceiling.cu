@@ -45,9 +45,9 @@ __global__ void __launch_bounds__(256) butterfly_ceiling_kernel(uint64_t* out, c
 }
 
 // The same radix-8 DIF groups with the FP64 butterflies of the FP64 form
-// (fp64mod.cuh, twiddles w with the companion formed per use): signed
-// residues below p in and out of every group, the sums reduced at the
-// group's last level, mod the first FP64 prime.
+// (fp64mod.cuh): signed residues up to 2 p in and out of every group, the
+// sums of outputs 0 and 4 reduced at the group's last level, mod the first
+// FP64 prime.
 __global__ void __launch_bounds__(256) butterfly_ceiling_dbl_kernel(uint64_t* out, const uint64_t* tw, double p,
                                                                     int iters)
 {
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256) butterfly_ceiling_dbl_kernel(uint64_t* ou
                 const int ti = (l == 0 ? 0 : (l == 1 ? 4 : 6)) + (m & (hm - 1));
                 const double sm = __dadd_rn(x[m], x[m + hm]), d = __dadd_rn(x[m], -x[m + hm]);
                 x[m + hm] = dmul_w(d, w[ti], p, pinv);
-                x[m] = l == 2 ? dreduce(sm, p, pinv) : sm;
+                x[m] = l == 2 && (m & 3) == 0 ? dreduce(sm, p, pinv) : sm;
             }
         }
     }

@@ -774,13 +774,20 @@ __device__ __forceinline__ void fbfly_unit_dit(uint64_t& a, uint64_t& b, const L
 
 // Arithmetic of the fast passes.  ArithInt: lazy Shoup butterflies on 64-bit
 // residues (lazy primes).  ArithDbl: FP64 butterflies (FP64 primes, values
-// stored as the bits of doubles; twiddles w form their companion per use,
-// so a product lands below p).  `LAST` marks the last level of a register
-// round: the FP64 forward butterflies reduce their sums there, so every
-// round starts and ends with |x| <= p; inside a round of B levels the values
-// stay below 2^B p (16 p for radix-16, under 2^51 for primes below 2^47).
+// stored as the bits of doubles; a product with a twiddle lands below p).
+// An FP64 forward sum grows only along the path that has met no product since
+// the round began, so reduce_sum / reduce_unit name the few outputs of a
+// round's last level that need a reduction (three FP64 instructions each).
+// Radix-2 .. radix-8 rounds take and return |x| <= 2 p: inside a radix-8 round
+// the values stay below 2^3 2 p = 16 p, and of its sums only outputs 0 (16 p)
+// and 4 (4 p) are reduced, the others are sums of two products.  Radix-16
+// rounds take and return |x| <= p, all sums reduced, again 16 p inside;
+// 16 p < 2^51 for primes below 2^47.
+// With the shorter product of dmul_w this took a product of 1,048,573 by
+// 400,009 words from 186.4 to 179.8 us, one of 2^24-word operands from 4.03
+// to 3.97 ms (the passes are bound by shared-memory traffic, not by FP64).
 // FP64 inverse butterflies add at most p per level and never reduce: a pass
-// of L levels over inputs below X ends below 2 X + (L - 1) p (15 p for a
+// of L levels over inputs below X ends below 2 X + (L - 1) p (16 p for a
 // 13-level row pass over the merges' T1 +- T2, below 1.5 p).
 struct ArithInt {
     using T = uint64_t;
@@ -789,10 +796,12 @@ struct ArithInt {
     static __device__ __forceinline__ Ctx ctx(const PrimeDev& P) { return lazy_prime(P); }
     static __device__ __forceinline__ T ld(uint64_t v) { return v; }
     static __device__ __forceinline__ uint64_t st(T v) { return v; }
-    template <bool LAST>
+    template <bool RED>
     static __device__ __forceinline__ void dif(T& a, T& b, const ulonglong2 t, const Ctx& L) { fbfly_dif(a, b, t, L); }
-    template <bool LAST>
+    template <bool RED>
     static __device__ __forceinline__ void dif_unit(T& a, T& b, const Ctx& L) { fbfly_unit_dif(a, b, L); }
+    static constexpr bool reduce_sum(int, int) { return false; }  // its butterflies keep [0, 4p) by themselves
+    static constexpr bool reduce_unit(int, int) { return false; }
     static __device__ __forceinline__ void dit(T& a, T& b, const ulonglong2 t, const Ctx& L) { fbfly_dit(a, b, t, L); }
     static __device__ __forceinline__ void dit_unit(T& a, T& b, const Ctx& L) { fbfly_unit_dit(a, b, L); }
     // v * w (pass twiddle) into [0, 4p) from any 64-bit v
@@ -816,19 +825,23 @@ struct ArithDbl {
     static __device__ __forceinline__ Ctx ctx(const PrimeDev& P) { return Ctx{P.pd, P.pinv}; }
     static __device__ __forceinline__ T ld(uint64_t v) { return dbits(v); }
     static __device__ __forceinline__ uint64_t st(T v) { return dstore(v); }
-    template <bool LAST>
+    // last level of a radix-2^B round: whether the sum at even output m, or
+    // with unit twiddles both outputs at m and m + 1, must be reduced
+    static constexpr bool reduce_sum(int B, int m) { return B == 4 || (m & 3) == 0; }
+    static constexpr bool reduce_unit(int B, int m) { return reduce_sum(B, m); }
+    template <bool RED>
     static __device__ __forceinline__ void dif(T& a, T& b, const Tw t, const Ctx& L)
     {
         const double s = __dadd_rn(a, b), d = __dadd_rn(a, -b);
         b = dmul_w(d, t, L.p, L.pinv);
-        a = LAST ? dreduce(s, L.p, L.pinv) : s;
+        a = RED ? dreduce(s, L.p, L.pinv) : s;
     }
-    template <bool LAST>
+    template <bool RED>
     static __device__ __forceinline__ void dif_unit(T& a, T& b, const Ctx& L)
     {
         const double s = __dadd_rn(a, b), d = __dadd_rn(a, -b);
-        a = LAST ? dreduce(s, L.p, L.pinv) : s;
-        b = LAST ? dreduce(d, L.p, L.pinv) : d;
+        a = RED ? dreduce(s, L.p, L.pinv) : s;
+        b = RED ? dreduce(d, L.p, L.pinv) : d;
     }
     static __device__ __forceinline__ void dit(T& a, T& b, const Tw t, const Ctx& L)
     {
@@ -864,7 +877,10 @@ __device__ __forceinline__ void group_fast(typename A::T (&x)[1 << B], int j, co
             const int hm = 1 << (B - 1 - l);
             if (l == B - 1 && LST == 0) {
 #pragma unroll
-                for (int m = 0; m < (1 << B); m += 2) A::template dif_unit<true>(x[m], x[m + 1], L);
+                for (int m = 0; m < (1 << B); m += 2) {
+                    if (A::reduce_unit(B, m)) A::template dif_unit<true>(x[m], x[m + 1], L);
+                    else A::template dif_unit<false>(x[m], x[m + 1], L);
+                }
                 continue;
             }
 #pragma unroll
@@ -872,7 +888,7 @@ __device__ __forceinline__ void group_fast(typename A::T (&x)[1 << B], int j, co
                 if (m & hm) continue;
                 const int u = m & (hm - 1);
                 const typename A::Tw t = __ldg(tw + ((1 << (B - l + LST - 1)) - 1) + j + (u << LST));
-                if (l == B - 1) A::template dif<true>(x[m], x[m + hm], t, L);
+                if (l == B - 1 && A::reduce_sum(B, m)) A::template dif<true>(x[m], x[m + hm], t, L);
                 else A::template dif<false>(x[m], x[m + hm], t, L);
             }
         }

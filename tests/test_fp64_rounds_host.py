@@ -1,0 +1,22 @@
+"""The FP64 form's forward register rounds (tests/host/fp64_round_check.c):
+with only the named outputs reduced, values stay in the FP64 quotient's range
+and every output within what the next round accepts, exactly congruent."""
+from __future__ import annotations
+
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.mark.skipif(shutil.which("gcc") is None, reason="gcc not available")
+@pytest.mark.parametrize("bits", [1, 2, 3, 4])
+def test_forward_round_ranges(tmp_path, bits):
+    exe = tmp_path / "fp64_round_check"
+    subprocess.run(["gcc", "-O2", "-ffp-contract=off", "-o", str(exe),
+                    os.path.join(HERE, "host", "fp64_round_check.c"), "-lm"], check=True)
+    out = subprocess.run([str(exe), str(bits), "200000"], capture_output=True, text=True)
+    assert out.returncode == 0 and out.stdout.startswith("bad=0"), out.stdout + out.stderr
