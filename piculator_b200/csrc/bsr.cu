@@ -916,59 +916,6 @@ __global__ void __launch_bounds__(256) merge_pointwise_kernel(uint64_t* __restri
     *reinterpret_cast<ulonglong2*>(R + L) = make_ulonglong2(mont_mul_c(rl.x, rr.x, M.p, c), mont_mul_c(rl.y, rr.y, M.p, c));
 }
 
-// The same on FP64-form residues (signed doubles, fp64mod.cuh): forward
-// outputs |x| <= p give products |y| <= 0.75 p (the quotient of a product
-// below p^2 is off by far less than 1/4), and T1 +- T2 stays below 1.5 p,
-// inside what the FP64 inverse accepts.
-struct DblMod3 {
-    double p[3], pinv[3];
-};
-
-__global__ void __launch_bounds__(256) merge_pointwise_d_kernel(uint64_t* __restrict__ P, uint64_t* __restrict__ Q,
-                                                                uint64_t* __restrict__ R, uint32_t npar, int k,
-                                                                size_t stride, uint32_t jbpr, DblMod3 M,
-                                                                const uint8_t* __restrict__ sgn)
-{
-    const uint32_t row = blockIdx.x / jbpr, jb = blockIdx.x - row * jbpr;
-    const uint32_t q = row / npar, i = row - q * npar;
-    const size_t j = ((size_t)jb * blockDim.x + threadIdx.x) * 2;
-    if (j >= ((size_t)1 << k)) return;
-    const double p = q == 0 ? M.p[0] : (q == 1 ? M.p[1] : M.p[2]);
-    const double pinv = q == 0 ? M.pinv[0] : (q == 1 ? M.pinv[1] : M.pinv[2]);
-    const size_t base = (size_t)q * 2 * npar;
-    const size_t L = (base + 2 * (size_t)i) * stride + j, Rr = L + stride;
-    const double2 pl = *reinterpret_cast<const double2*>(P + L), pr = *reinterpret_cast<const double2*>(P + Rr);
-    const double2 ql = *reinterpret_cast<const double2*>(Q + L), qr = *reinterpret_cast<const double2*>(Q + Rr);
-    const double2 rl = *reinterpret_cast<const double2*>(R + L), rr = *reinterpret_cast<const double2*>(R + Rr);
-    const double2 t1 = make_double2(dmul_mod(pl.x, qr.x, p, pinv), dmul_mod(pl.y, qr.y, p, pinv));
-    const double2 t2 = make_double2(dmul_mod(pr.x, rl.x, p, pinv), dmul_mod(pr.y, rl.y, p, pinv));
-    if (sgn != nullptr) {
-        const bool same = (sgn[2 * i] != 0) == (sgn[2 * i + 1] != 0);
-        *reinterpret_cast<double2*>(P + L) = same ? make_double2(__dadd_rn(t1.x, t2.x), __dadd_rn(t1.y, t2.y))
-                                                  : make_double2(__dadd_rn(t1.x, -t2.x), __dadd_rn(t1.y, -t2.y));
-    } else {
-        *reinterpret_cast<double2*>(P + L) = t1;
-        *reinterpret_cast<double2*>(P + Rr) = t2;
-    }
-    *reinterpret_cast<double2*>(Q + L) = make_double2(dmul_mod(ql.x, qr.x, p, pinv), dmul_mod(ql.y, qr.y, p, pinv));
-    *reinterpret_cast<double2*>(R + L) = make_double2(dmul_mod(rl.x, rr.x, p, pinv), dmul_mod(rl.y, rr.y, p, pinv));
-}
-
-static void launch_merge_pointwise_d(uint64_t* P, uint64_t* Q, uint64_t* R, size_t npar, int k, size_t stride,
-                                     const uint8_t* sgn, cudaStream_t s)
-{
-    PIC_REQUIRE(k >= 1 && stride % 2 == 0 && npar <= 0x7fffffffu / 3, PIC_ERR_INVALID, "pointwise merge shape");
-    const uint32_t jbpr = (uint32_t)((((size_t)1 << k) + 511) / 512);
-    const size_t blocks = 3 * npar * (size_t)jbpr;
-    PIC_REQUIRE(blocks <= 0x7fffffffu, PIC_ERR_INVALID, "pointwise merge grid too large");
-    DblMod3 M;
-    for (int q = 0; q < 3; q++) {
-        M.p[q] = (double)kDblPrimes[q];
-        M.pinv[q] = 1.0 / M.p[q];
-    }
-    merge_pointwise_d_kernel<<<(unsigned)blocks, 256, 0, s>>>(P, Q, R, (uint32_t)npar, k, stride, jbpr, M, sgn);
-}
-
 // Launch over 3 primes x npar parents x 2^k points (stride even, 2^k >= 2).
 static void launch_merge_pointwise(uint64_t* P, uint64_t* Q, uint64_t* R, size_t npar, int k, size_t stride,
                                    const Mod64& m0, const Mod64& m1, const Mod64& m2, const uint8_t* sgn,
@@ -1466,79 +1413,56 @@ static void ntt_products(const Level& ch, size_t p0, size_t np, const MergeShape
         const Slots* arrays[3] = {&ch.P, &ch.Q, &ch.R};
         uint64_t* mains[3] = {PB, QB, RB};
         uint64_t* tails[3] = {PT, QT, RT};
-        for (int a = 0; a < 3; a++) {
+        auto source = [&](int a, size_t first) {
             SplitSrc src;
             src.words = arrays[a]->w.get();
             src.len = arrays[a]->len.get();
             src.cap = arrays[a]->cap;
             src.c0 = c0;
-            src.first = 0;
-            fb.data = mains[a];
-            fb.src = src;
-            ntt_forward_dif(fb, k, s);
-            if (sh.wrap) {
-                src.first = sh.t0;
-                tb.data = tails[a];
-                tb.src = src;
-                ntt_forward_dif(tb, sh.kt, s);
-            }
-        }
-        fb.src = SplitSrc{};
-        tb.src = SplitSrc{};
-        {
-            ProfScope ps(KC_NTT_POINTWISE, 3.0 * 3 * np * (double)(N + T) * 80.0 / 8.0, s);
-            if (dbl) {
-                launch_merge_pointwise_d(PB, QB, RB, np, k, ST, o.csign, s);
-                if (sh.wrap) launch_merge_pointwise_d(PT, QT, RT, np, sh.kt, T, o.csign, s);
-            } else {
-                launch_merge_pointwise(PB, QB, RB, np, k, ST, m0, m1, m2, o.csign, s);
-                if (sh.wrap) launch_merge_pointwise(PT, QT, RT, np, sh.kt, T, m0, m1, m2, o.csign, s);
-            }
-            PIC_CHECK_LAUNCH();
-            count_launch(sh.wrap ? 2 : 1);
-        }
-        // inverses: P holds T1, T2 for every parent (all items), or only the
+            src.first = first;
+            return src;
+        };
+        // results: P holds T1, T2 for every parent (all items), or only the
         // combined item 2i; Q, R the even items
         const bool comb = o.csign != nullptr;
-        {
-            NttBatch eb = fb;
-            eb.stride = 2 * ST;
-            eb.count = (int)(3 * np);
-            eb.per_prime = (int)np;
-            if (comb) {
-                eb.data = PB;
-                ntt_inverse_dit(eb, k, s);
+        auto results = [&](NttBatch b, size_t stride, bool all) {
+            b.src = SplitSrc{};
+            if (all) return b;
+            b.stride = 2 * stride;
+            b.count = (int)(3 * np);
+            b.per_prime = (int)np;
+            return b;
+        };
+        // six forward transforms, the products and the inverse transforms at
+        // length 2^kk over the arrays `arr3` (item stride `stride`)
+        auto transform = [&](NttBatch b, uint64_t* const* arr3, int kk, size_t stride, size_t first) {
+            const int rows = merge_row_bits(kk);
+            for (int a = 0; a < 3; a++) {
+                b.data = arr3[a];
+                b.src = source(a, first);
+                if (!dbl) ntt_forward_dif(b, kk, s);
+                else if (rows < kk) ntt_forward_cols(b, kk, rows, s);
+            }
+            if (dbl) {
+                MergeMiddle mm{arr3[0], arr3[1], arr3[2], source(0, first), source(1, first), source(2, first),
+                               stride, np, o.csign, needR};
+                ntt_merge_middle(mm, kk, s);
             } else {
-                NttBatch ib = fb;
-                ib.data = PB;
-                ntt_inverse_dit(ib, k, s);
+                ProfScope ps(KC_NTT_POINTWISE, 3.0 * np * (double)((size_t)1 << kk) * 80.0, s);
+                launch_merge_pointwise(arr3[0], arr3[1], arr3[2], np, kk, stride, m0, m1, m2, o.csign, s);
+                PIC_CHECK_LAUNCH();
+                count_launch();
             }
-            eb.data = QB;
-            ntt_inverse_dit(eb, k, s);
-            if (needR) {
-                eb.data = RB;
-                ntt_inverse_dit(eb, k, s);
+            for (int a = 0; a < (needR ? 3 : 2); a++) {
+                NttBatch r = results(b, stride, a == 0 && !comb);
+                r.data = arr3[a];
+                if (!dbl) ntt_inverse_dit(r, kk, s);
+                else if (rows < kk) ntt_inverse_cols(r, kk, rows, s);
             }
-        }
+        };
+        transform(fb, mains, k, ST, 0);
         if (sh.wrap) {
-            NttBatch eb = tb;
-            eb.stride = 2 * T;
-            eb.count = (int)(3 * np);
-            eb.per_prime = (int)np;
-            if (comb) {
-                eb.data = PT;
-                ntt_inverse_dit(eb, sh.kt, s);
-            } else {
-                NttBatch ib = tb;
-                ib.data = PT;
-                ntt_inverse_dit(ib, sh.kt, s);
-            }
-            eb.data = QT;
-            ntt_inverse_dit(eb, sh.kt, s);
-            if (needR) {
-                eb.data = RT;
-                ntt_inverse_dit(eb, sh.kt, s);
-            }
+            transform(tb, tails, sh.kt, T, sh.t0);
             ProfScope ps(KC_NTT_POINTWISE, 3.0 * 4 * np * (double)sh.W * 24.0, s);
             const size_t W = sh.W;
             auto fix = [&](uint64_t* y, const uint64_t* tail, size_t nitems, size_t item_mul) {

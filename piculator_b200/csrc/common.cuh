@@ -132,7 +132,7 @@ void read_words(uint32_t* host, const uint32_t* dev, size_t count, cudaStream_t 
 // bytes it must move; pic_profile_end reduces them per kernel class.
 enum KernelClass {
     KC_NTT_COLS = 0, KC_NTT_ROWS, KC_NTT_POINTWISE, KC_SPLIT, KC_CRT, KC_CARRY, KC_LINEAR, KC_SCHOOL,
-    KC_FFT_COLS, KC_FFT_ROWS, KC_BSR, KC_OTHER, KC_COUNT
+    KC_FFT_COLS, KC_FFT_ROWS, KC_BSR, KC_OTHER, KC_NTT_MIDDLE, KC_COUNT
 };
 const char* kernel_class_name(int c);
 bool profiling();

@@ -1,0 +1,348 @@
+// Fused middle passes of the FP64 product form (see ntt.cuh).
+//
+// A product needs, after the column passes, the forward row pass of each
+// operand, a pointwise product and the inverse row pass of each result.  Rows
+// are contiguous and the three steps keep a row's points in place, so one CTA
+// takes the same row of every operand through all of them in shared memory:
+// the row passes' own HBM traffic (16 B a point and pass) and the pointwise
+// kernel's (80 B per parent point of a merge) become one read of the operands
+// and one write of the results, 72 B per parent point of a merge instead of 224.
+// The last forward round, the pointwise product and the first inverse round
+// work on the same groups of points, so they run in registers without an
+// exchange between them.  A thread takes the same group of every operand, so a
+// round's twiddles are loaded once for all of them.
+//
+// Merges of a pi computation at 1e9 digits (binary splitting, one B200): a
+// level of 2^17-point transforms 64.4 -> 54.5 ms, of 2^12 points 55.8 -> 38.6,
+// the whole computation 1.73 -> 1.49 s, against the same passes launched
+// apart.  What is left in the kernel is FP64 work (about 430 instructions per
+// parent point and prime: 6 forward and 3 inverse rows of 11 levels) with two
+// CTAs of 256 threads per SM, the rows' 96 KB of shared memory being the limit.
+#include <algorithm>
+
+#include "common.cuh"
+#include "passes.cuh"
+
+namespace pic {
+
+using Dbl = ArithDbl;
+
+// The twiddles of one group (see group_fast): level l, butterfly u at
+// (2^B - 2^(B-l)) + u.  The unit level of LST 0 is not loaded.
+template <int B, int LST>
+struct GroupTw {
+    double w[(1 << B) - 1];
+    __device__ __forceinline__ void load(const double* __restrict__ tw, int j)
+    {
+#pragma unroll
+        for (int l = 0; l < B; l++) {
+            if (l == B - 1 && LST == 0) continue;
+#pragma unroll
+            for (int u = 0; u < (1 << (B - 1 - l)); u++)
+                w[(1 << B) - (1 << (B - l)) + u] = __ldg(tw + ((1 << (B - l + LST - 1)) - 1) + j + (u << LST));
+        }
+    }
+    __device__ __forceinline__ double at(int l, int u) const { return w[(1 << B) - (1 << (B - l)) + u]; }
+};
+
+template <int B, int LST>
+__device__ __forceinline__ void fwd_group(double (&x)[1 << B], const GroupTw<B, LST>& t, const Dbl::Ctx& L)
+{
+#pragma unroll
+    for (int l = 0; l < B; l++) {
+        const int hm = 1 << (B - 1 - l);
+#pragma unroll
+        for (int m = 0; m < (1 << B); m++) {
+            if (m & hm) continue;
+            if (l == B - 1 && LST == 0) {
+                if (Dbl::reduce_unit(B, m)) Dbl::dif_unit<true>(x[m], x[m + hm], L);
+                else Dbl::dif_unit<false>(x[m], x[m + hm], L);
+            } else {
+                if (l == B - 1 && Dbl::reduce_sum(B, m)) Dbl::dif<true>(x[m], x[m + hm], t.at(l, m & (hm - 1)), L);
+                else Dbl::dif<false>(x[m], x[m + hm], t.at(l, m & (hm - 1)), L);
+            }
+        }
+    }
+}
+
+template <int B, int LST>
+__device__ __forceinline__ void inv_group(double (&x)[1 << B], const GroupTw<B, LST>& t, const Dbl::Ctx& L)
+{
+#pragma unroll
+    for (int l = B - 1; l >= 0; l--) {
+        const int hm = 1 << (B - 1 - l);
+#pragma unroll
+        for (int m = 0; m < (1 << B); m++) {
+            if (m & hm) continue;
+            if (l == B - 1 && LST == 0) Dbl::dit_unit(x[m], x[m + hm], L);
+            else Dbl::dit(x[m], x[m + hm], t.at(l, m & (hm - 1)), L);
+        }
+    }
+}
+
+// Shared-memory place of a row's element e: bits 4, 5, 6 of e are XORed into
+// bits 0, (1 and 2), 3.  The map is linear, so the place of base + (m << LST)
+// (disjoint bits) is place(base) ^ place(m << LST), the latter a constant.
+// Half a warp's 16 elements then fall in 16 different bank pairs in every round
+// of 11-bit rows (strides 2^8, 2^5, 2^2, 1).
+__host__ __device__ constexpr int place(int e)
+{
+    return e ^ ((e >> 4) & 1) ^ (((e >> 5) & 1) * 6) ^ (((e >> 6) & 1) << 3);
+}
+
+// Rounds of a 2^LR row: radix 8, the remainder last (smallest stride).
+template <int LR, int R>
+using Round = typename RoundPlan<LR, 3>::template At<R>;
+
+// A CTA's shape: 2^LT rows of 2^LR points of each operand, one thread per
+// radix-8 group of one operand.
+template <int LR, int LT>
+struct MiddleShape {
+    static constexpr int TOT = 1 << (LR + LT);  // points of one operand in the CTA
+    static constexpr int NT = TOT >> 3;
+    static constexpr int NR = RoundPlan<LR, 3>::NR;
+};
+
+// Forward rounds 0 .. NR - 2 of every operand: in(a, t, e) reads operand a's
+// element e of the CTA's row t.
+template <int LR, int LT, int NOP, int R, class In>
+__device__ __forceinline__ void forward_rounds(double* __restrict__ s, const Dbl::Ctx& L,
+                                               const double* __restrict__ tw, int nop, const In& in)
+{
+    using Sh = MiddleShape<LR, LT>;
+    if constexpr (R + 1 < Sh::NR) {
+        using At = Round<LR, R>;
+        constexpr int B = At::B, LB = At::LB, LST = At::LST, LG = LR - B;
+        static_assert(B == 3, "full rounds come first");
+        const int g = threadIdx.x;
+        const int t = g >> LG, gi = g & ((1 << LG) - 1);
+        const int j = gi & ((1 << LST) - 1);
+        const int base = ((gi >> LST) << LB) + j;
+        const int pb = (t << LR) + place(base);
+        GroupTw<B, LST> w;
+        w.load(tw, j);
+#pragma unroll 2
+        for (int a = 0; a < nop; a++) {
+            double x[8];
+            double* sa = s + a * Sh::TOT;
+#pragma unroll
+            for (int m = 0; m < 8; m++) {
+                if constexpr (R == 0) x[m] = in(a, t, base + (m << LST));
+                else x[m] = sa[pb ^ place(m << LST)];
+            }
+            fwd_group<B, LST>(x, w, L);
+#pragma unroll
+            for (int m = 0; m < 8; m++) sa[pb ^ place(m << LST)] = x[m];
+        }
+        __syncthreads();
+        forward_rounds<LR, LT, NOP, R + 1>(s, L, tw, nop, in);
+    }
+}
+
+// Inverse rounds R .. 0 of the results in rows act(i), i < nout; out(i, t, e, v)
+// writes result i's element e of the CTA's row t.
+template <int LR, int LT, int R, class Act, class Out>
+__device__ __forceinline__ void inverse_rounds(double* __restrict__ s, const Dbl::Ctx& L,
+                                               const double* __restrict__ tw, int nout, const Act& act, const Out& out)
+{
+    using Sh = MiddleShape<LR, LT>;
+    using At = Round<LR, R>;
+    constexpr int B = At::B, LB = At::LB, LST = At::LST, LG = LR - B;
+    const int g = threadIdx.x;
+    const int t = g >> LG, gi = g & ((1 << LG) - 1);
+    const int j = gi & ((1 << LST) - 1);
+    const int base = ((gi >> LST) << LB) + j;
+    const int pb = (t << LR) + place(base);
+    GroupTw<B, LST> w;
+    w.load(tw, j);
+    __syncthreads();
+#pragma unroll 2
+    for (int i = 0; i < nout; i++) {
+        double x[8];
+        double* sa = s + act(i) * Sh::TOT;
+#pragma unroll
+        for (int m = 0; m < 8; m++) x[m] = sa[pb ^ place(m << LST)];
+        inv_group<B, LST>(x, w, L);
+#pragma unroll
+        for (int m = 0; m < 8; m++) {
+            if constexpr (R == 0) out(i, t, base + (m << LST), x[m]);
+            else sa[pb ^ place(m << LST)] = x[m];
+        }
+    }
+    if constexpr (R > 0) inverse_rounds<LR, LT, R - 1>(s, L, tw, nout, act, out);
+}
+
+struct MergeMiddleDev {
+    uint64_t* arr[3];  // P, Q, R
+    SplitSrc src[3];
+    size_t stride;
+    uint32_t np;
+    uint32_t blocks;  // CTAs per prime
+    const uint8_t* sgn;
+    int need_r;
+    PrimeDev prime[3];
+};
+
+// Operand rows of a merge in shared memory: PL, PR, QL, QR, RL, RR.
+template <int LR, int LT, bool SRC>
+__global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::NT > 256 ? 1 : 2)
+    merge_middle_kernel(const __grid_constant__ MergeMiddleDev M, int lrow)
+{
+    using Sh = MiddleShape<LR, LT>;
+    constexpr int TOT = Sh::TOT;
+    extern __shared__ double ms[];
+    const uint32_t q = blockIdx.x / M.blocks, cb = blockIdx.x - q * M.blocks;
+    const PrimeDev& P = q == 0 ? M.prime[0] : (q == 1 ? M.prime[1] : M.prime[2]);
+    const Dbl::Ctx L = Dbl::ctx(P);
+    const double* __restrict__ tf = reinterpret_cast<const double*>(P.lvl_fwd);
+    const double* __restrict__ ti = reinterpret_cast<const double*>(P.lvl_inv);
+    const size_t row0 = (size_t)cb << LT;  // (parent, row) pairs, 2^lrow rows a parent
+    const size_t nrows = (size_t)M.np << lrow;
+    const size_t rmask = ((size_t)1 << lrow) - 1;
+    // element e of operand a's row t: child 2 i + (a & 1) of array a / 2
+    auto off = [&](int a, int t, int e) {
+        const size_t row = row0 + t;
+        const size_t item = (size_t)q * 2 * M.np + 2 * (row >> lrow) + (a & 1);
+        return item * M.stride + ((row & rmask) << LR) + e;
+    };
+    auto pick = [&](int a) { return a < 2 ? M.arr[0] : (a < 4 ? M.arr[1] : M.arr[2]); };
+    auto in = [&](int a, int t, int e) -> double {
+        if (LT > 0 && row0 + t >= nrows) return 0.0;
+        if constexpr (SRC) {  // lrow == 0: the row is child c of the source
+            const SplitSrc& S = a < 2 ? M.src[0] : (a < 4 ? M.src[1] : M.src[2]);
+            const size_t c = S.c0 + 2 * (row0 + t) + (a & 1);
+            const uint32_t n = __ldg(S.len + c);
+            return dpiece56(src_piece56_raw(S.words + c * (size_t)S.cap, n, S.first + e), L.p, L.pinv);
+        } else {
+            return dbits(pick(a)[off(a, t, e)]);
+        }
+    };
+    auto put = [&](int a, int t, int e, double v) {
+        if (LT == 0 || row0 + t < nrows) pick(a)[off(a, t, e)] = dstore(v);
+    };
+    const int nop = M.need_r ? 6 : 5;
+    forward_rounds<LR, LT, 6, 0>(ms, L, tf, nop, in);
+    // last forward round, pointwise products, first inverse round
+    {
+        using At = Round<LR, Sh::NR - 1>;
+        constexpr int B = At::B, LST = At::LST, LG = LR - B, E = 1 << B;
+        static_assert(LST == 0, "the last round has stride 1");
+        constexpr int G = 1 << (LT + LG);
+        GroupTw<B, 0> wf, wi;
+        wf.load(tf, 0);
+        wi.load(ti, 0);
+#pragma unroll 1
+        for (int g = threadIdx.x; g < G; g += Sh::NT) {
+            const int t = g >> LG;
+            const int pb = (t << LR) + place((g & ((1 << LG) - 1)) << B);
+            const int base = (g & ((1 << LG) - 1)) << B;
+            auto load = [&](int a, double(&x)[E]) {  // NR 1: the only round
+#pragma unroll
+                for (int m = 0; m < E; m++) x[m] = Sh::NR == 1 ? in(a, t, base + m) : ms[a * TOT + (pb ^ place(m))];
+                fwd_group<B, 0>(x, wf, L);
+            };
+            auto store = [&](int a, double(&x)[E]) {
+                inv_group<B, 0>(x, wi, L);
+#pragma unroll
+                for (int m = 0; m < E; m++) {
+                    if constexpr (Sh::NR == 1) put(a, t, base + m, x[m]);
+                    else ms[a * TOT + (pb ^ place(m))] = x[m];
+                }
+            };
+            double qr[E], rl[E], x[E], y[E];
+            load(3, qr);
+            load(4, rl);
+            load(0, x);
+            load(1, y);
+#pragma unroll
+            for (int m = 0; m < E; m++) {
+                x[m] = dmul_mod(x[m], qr[m], L.p, L.pinv);
+                y[m] = dmul_mod(y[m], rl[m], L.p, L.pinv);
+            }
+            if (M.sgn != nullptr) {
+                const size_t row = row0 + t;
+                const size_t i = LT > 0 && row >= nrows ? 0 : row >> lrow;
+                const bool same = (M.sgn[2 * i] != 0) == (M.sgn[2 * i + 1] != 0);
+#pragma unroll
+                for (int m = 0; m < E; m++) x[m] = __dadd_rn(x[m], same ? y[m] : -y[m]);
+            } else {
+                store(1, y);
+            }
+            store(0, x);
+            load(2, x);
+#pragma unroll
+            for (int m = 0; m < E; m++) x[m] = dmul_mod(x[m], qr[m], L.p, L.pinv);
+            store(2, x);
+            if (M.need_r) {
+                load(5, y);
+#pragma unroll
+                for (int m = 0; m < E; m++) y[m] = dmul_mod(y[m], rl[m], L.p, L.pinv);
+                store(4, y);
+            }
+        }
+    }
+    // results in rows 0 (T1 or V), 2 (Q), 4 (R), 1 (T2)
+    const int apart = M.sgn == nullptr;
+    const int nout = 2 + (M.need_r ? 1 : 0) + apart;
+    auto act = [&](int i) { return i == nout - 1 && apart ? 1 : 2 * i; };
+    auto out = [&](int i, int t, int e, double v) { put(act(i), t, e, v); };
+    if constexpr (Sh::NR > 1) inverse_rounds<LR, LT, Sh::NR - 2>(ms, L, ti, nout, act, out);
+}
+
+int merge_row_bits(int k) { return k <= 12 ? k : 11; }
+
+template <int LR, bool SRC>
+static void launch_merge_middle(const MergeMiddle& m, int k, cudaStream_t s)
+{
+    constexpr int LT = LR < 11 ? 11 - LR : 0;
+    using Sh = MiddleShape<LR, LT>;
+    MergeMiddleDev d;
+    d.arr[0] = m.P;
+    d.arr[1] = m.Q;
+    d.arr[2] = m.R;
+    d.src[0] = m.sP;
+    d.src[1] = m.sQ;
+    d.src[2] = m.sR;
+    d.stride = m.stride;
+    d.np = (uint32_t)m.np;
+    d.sgn = m.sgn;
+    d.need_r = m.need_r ? 1 : 0;
+    for (int q = 0; q < 3; q++) d.prime[q] = dbl_prime_tables(kDblPrimes[q]).dev;
+    const size_t rows = m.np << (k - LR);
+    const size_t blocks = (rows + ((size_t)1 << LT) - 1) >> LT;
+    PIC_REQUIRE(3 * blocks <= 0x7fffffffu, PIC_ERR_INVALID, "merge grid too large");
+    d.blocks = (uint32_t)blocks;
+    const size_t smem = sizeof(double) * 6 * Sh::TOT;
+    auto kern = merge_middle_kernel<LR, LT, SRC>;
+    PIC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<(unsigned)(3 * blocks), Sh::NT, smem, s>>>(d, k - LR);
+    PIC_CHECK_LAUNCH();
+    count_launch();
+}
+
+void ntt_merge_middle(const MergeMiddle& m, int k, cudaStream_t s)
+{
+    // 6 rows read and 3 (or 4) written per row of a parent
+    ProfScope ps(KC_NTT_MIDDLE, 3.0 * (double)m.np * (double)((size_t)1 << k) * 72.0, s);
+    const int lr = merge_row_bits(k);
+    if (lr < k) {
+        launch_merge_middle<11, false>(m, k, s);
+        return;
+    }
+    switch (lr) {
+    case 2: launch_merge_middle<2, true>(m, k, s); break;
+    case 3: launch_merge_middle<3, true>(m, k, s); break;
+    case 4: launch_merge_middle<4, true>(m, k, s); break;
+    case 5: launch_merge_middle<5, true>(m, k, s); break;
+    case 6: launch_merge_middle<6, true>(m, k, s); break;
+    case 7: launch_merge_middle<7, true>(m, k, s); break;
+    case 8: launch_merge_middle<8, true>(m, k, s); break;
+    case 9: launch_merge_middle<9, true>(m, k, s); break;
+    case 10: launch_merge_middle<10, true>(m, k, s); break;
+    case 11: launch_merge_middle<11, true>(m, k, s); break;
+    case 12: launch_merge_middle<12, true>(m, k, s); break;
+    default: throw Error(PIC_ERR_INVALID, "merge transform too short");
+    }
+}
+
+}  // namespace pic

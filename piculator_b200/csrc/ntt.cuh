@@ -101,10 +101,11 @@ enum NttForm { kFormInt = 0, kFormDbl = 1, kFormChosen = 2 };
 // item's prime.  Only the first pass reads it; every pass writes `data`.
 struct SplitSrc {
     const uint32_t* words = nullptr;  // null: the input is already in `data`
-    const uint32_t* len = nullptr;
+    const uint32_t* len = nullptr;  // null: every item has n words
     uint32_t cap = 0;
     size_t c0 = 0;
     size_t first = 0;
+    uint32_t n = 0;
 };
 
 struct NttBatch {
@@ -119,6 +120,37 @@ struct NttBatch {
 void ntt_forward_dif(const NttBatch& b, int k, cudaStream_t s);
 void ntt_inverse_dit(const NttBatch& b, int k, cudaStream_t s);
 void ntt_bitreverse(const NttBatch& b, int k, cudaStream_t s);
+
+// The column passes of a transform whose contiguous row pass has 2^row_bits
+// points: what precedes that row pass in the forward direction, what follows
+// it in the inverse one (nothing when k = row_bits).
+void ntt_forward_cols(const NttBatch& b, int k, int row_bits, cudaStream_t s);
+void ntt_inverse_cols(const NttBatch& b, int k, int row_bits, cudaStream_t s);
+
+// Fused middle passes of the FP64 form (middle.cu): the forward row pass of
+// every operand, the pointwise products and the inverse row pass of every
+// result in one kernel, so that a spectrum never leaves the chip.
+//
+// A merge: per prime q, parent i and row, the children's transforms at
+// P/Q/R + (q 2 np + c) stride (c = 2i, 2i + 1), row passes still to run, become
+// the products' transforms with the inverse row pass done:
+//   T1 = PL QR -> P[2i], T2 = PR RL -> P[2i + 1], Q = QL QR -> Q[2i],
+//   R = RL RR -> R[2i] (need_r),
+// or, with the children's P signs `sgn` (parent i at sgn[2i], sgn[2i + 1]),
+//   T1 +- T2 -> P[2i] (plus when the signs agree), nothing in P[2i + 1].
+// When k = middle_row_bits(k) the rows are whole transforms and the operands
+// are read from the source words.
+struct MergeMiddle {
+    uint64_t *P, *Q, *R;
+    SplitSrc sP, sQ, sR;  // k = row bits: the children's words (c0: the first child)
+    size_t stride;
+    size_t np;
+    const uint8_t* sgn;  // null: T1 and T2 apart
+    bool need_r;
+};
+void ntt_merge_middle(const MergeMiddle& m, int k, cudaStream_t s);
+// Row bits the fused merge uses at length 2^k.
+int merge_row_bits(int k);
 
 // out[i] = a[i] * b[i] * 2^-64 mod p over every transform of the batch
 // (b may equal a for squaring); b's transforms are b_stride apart (0: a's

@@ -371,7 +371,7 @@ const char* kernel_class_name(int c)
 {
     static const char* names[KC_COUNT] = {"ntt_cols", "ntt_rows", "ntt_pointwise", "split", "crt_carry",
                                           "carry_scan", "linear", "schoolbook", "fft_cols", "fft_rows",
-                                          "bsr_level", "other"};
+                                          "bsr_level", "other", "ntt_middle"};
     return (c >= 0 && c < KC_COUNT) ? names[c] : "?";
 }
 

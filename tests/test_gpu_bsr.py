@@ -69,3 +69,25 @@ def test_bsr_karatsuba_vs_oracle(pic, oracle, a, b, p, kara):
     assert _same(Q, wQ), "Q"
     assert _same(R, wR), "R"
     assert _same(P, wP), "P"
+
+
+# The FP64 form's fused merge kernel against the integer form's separate passes
+# at transform lengths 2^2 .. 2^19: rows of every length, ragged last CTAs,
+# column passes of 1 .. 8 bits before and after it.
+@pytest.mark.parametrize("a,b,p", [(3, 1027, 4096), (0, 70_001, 1 << 20), (11, 150_000, 200_000),
+                                   (0, 33_333, 30_000)])
+@pytest.mark.parametrize("wrap", [0, 1])
+def test_bsr_fp64_and_integer_forms_agree(pic, a, b, p, wrap):
+    knobs = {pic.TUNE_BSR_SCHOOL_MAX: 8, pic.TUNE_BSR_WRAP: wrap, pic.TUNE_NTT_FORM: 0}
+    saved = {k: pic.get_tuning(k) for k in knobs}
+    try:
+        for k, v in knobs.items():
+            pic.set_tuning(k, v)
+        want = [x.to_bf() for x in pic.bsr(a, b, p, pic.PI_CHOSEN)]
+        pic.set_tuning(pic.TUNE_NTT_FORM, 1)
+        got = pic.bsr(a, b, p, pic.PI_CHOSEN)
+    finally:
+        for k, v in saved.items():
+            pic.set_tuning(k, v)
+    for name, g, w in zip("PQR", got, want):
+        assert _same(g, w), name
