@@ -286,14 +286,17 @@ def arith_roof(P, torch, L, stream):
     0.8 * 2^23-word operands in the active form (a plain transform of length
     2^23 in both forms; 3 row passes per product, each over 3 x 2^23 points
     and row_bits levels) against the register-only butterfly ceiling of that
-    form's arithmetic."""
+    form's arithmetic.  The FP64 form runs its three 11-bit row passes and the
+    pointwise product in one kernel (`ntt_middle`)."""
     import ctypes as C
 
     form = P.get_tuning(P.TUNE_NTT_FORM)
     mode = "ntt3d" if form == P.FORM_DBL else "ntt3"
     k = 23
     n = int(0.8 * (1 << k))
-    row_bits = P.get_ntt_geometry(k, form)[0]
+    fused = form == P.FORM_DBL
+    kernel = "ntt_middle" if fused else "ntt_rows"
+    row_bits = 11 if fused else P.get_ntt_geometry(k, form)[0]
     a = torch.randint(-2**31, 2**31 - 1, (n,), dtype=torch.int32, device="cuda")
     b = torch.randint(-2**31, 2**31 - 1, (n,), dtype=torch.int32, device="cuda")
     z = torch.empty(2 * n, dtype=torch.int32, device="cuda")
@@ -307,15 +310,15 @@ def arith_roof(P, torch, L, stream):
     stats = (P.KernelStat * 32)()
     cnt = C.c_int()
     P.check(L.pic_profile_end(stats, 32, C.byref(cnt)))
-    rows = [s for s in stats[: cnt.value] if s.name.decode() == "ntt_rows"]
+    rows = [s for s in stats[: cnt.value] if s.name.decode() == kernel]
     if not rows or rows[0].seconds <= 0:
         return None
-    bfly = rows[0].launches * 3 * (1 << (k - 1)) * row_bits
+    bfly = rows[0].launches * (3 if fused else 1) * 3 * (1 << (k - 1)) * row_bits
     achieved = bfly / rows[0].seconds / 1e9
     ceiling = P.butterfly_rate(form)
-    basis = ("FP64 modular DIF butterflies (about nine FP64 instructions each)" if form == P.FORM_DBL
+    basis = ("FP64 modular DIF butterflies (about eight and a half FP64 instructions each)" if form == P.FORM_DBL
              else "lazy Shoup DIF butterflies") + " with operands in registers, no memory traffic"
-    return {"kernel": "ntt_rows", "form": "fp64" if form == P.FORM_DBL else "integer",
+    return {"kernel": kernel, "form": "fp64" if form == P.FORM_DBL else "integer",
             "workload": f"three-prime product of two {n}-word operands (transform length 2^{k})",
             "row_bits": row_bits, "achieved": achieved, "ceiling": ceiling, "unit": "G butterflies/s",
             "frac": achieved / ceiling, "ceiling_basis": basis}
@@ -541,12 +544,12 @@ def ours(args):
     # DRAM bytes per algorithmic byte (16 B per point and pass) of the NTT
     # passes: dram__bytes_read.sum + dram__bytes_write.sum of every launch of
     # the kernel in one 1e9-digit computation (ncu, one pass per launch), over
-    # the kernel's algorithmic bytes in the same computation.  FP64 form: rows
-    # 1591.5 GB / 1739.5 GB, columns 1786.5 GB / 1763.6 GB (their per-point
-    # twiddle tables mostly hit L2).  Integer form, from the 2^23-word product:
+    # the kernel's algorithmic bytes in the same computation.  FP64 form:
+    # columns 1786.5 GB / 1763.6 GB (their per-point twiddle tables mostly hit
+    # L2).  Integer form, from the 2^23-word product:
     # rows 14.9 B and columns 30.8 B per point.
     if P.get_tuning(P.TUNE_NTT_FORM) == P.FORM_DBL:
-        dram_per_alg = {"ntt_rows": 1591.5 / 1739.5, "ntt_cols": 1786.5 / 1763.6}
+        dram_per_alg = {"ntt_cols": 1786.5 / 1763.6}
         traffic_basis = ("ncu DRAM bytes of every launch of the kernel in one 1e9-digit computation over its "
                          "algorithmic bytes, times the kernel's average launch")
     else:

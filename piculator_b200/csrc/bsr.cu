@@ -1436,7 +1436,7 @@ static void ntt_products(const Level& ch, size_t p0, size_t np, const MergeShape
         // six forward transforms, the products and the inverse transforms at
         // length 2^kk over the arrays `arr3` (item stride `stride`)
         auto transform = [&](NttBatch b, uint64_t* const* arr3, int kk, size_t stride, size_t first) {
-            const int rows = merge_row_bits(kk);
+            const int rows = middle_row_bits(kk);
             for (int a = 0; a < 3; a++) {
                 b.data = arr3[a];
                 b.src = source(a, first);

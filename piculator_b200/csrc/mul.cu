@@ -583,19 +583,32 @@ uint64_t held_transform_reuses() { return g_held_reuses.load(); }
 
 static bool is_held(const uint32_t* x, size_t n) { return t_held && t_held->src == x && t_held->n == n; }
 
-void ntt3d_forward_operand(uint64_t* out, int k, const uint32_t* a, size_t na, cudaStream_t s);
-
-// The held operand's forward transform at length 2^k (stride 2^k) in the
-// given product form, computed on first use at that length and form.
-static const uint64_t* held_transform(int k, int form, cudaStream_t s)
+// The integer form: the held operand's forward transform at length 2^k (stride
+// 2^k), computed on first use at that length.
+static const uint64_t* held_transform(int k, cudaStream_t s)
 {
     HeldOperand* h = t_held;
-    if (h->k != k || h->form != form) {
+    if (h->k != k || h->form != kFormInt) {
         h->T = DevBuf<uint64_t>(3 * ((size_t)1 << k), s);
-        if (form == kFormDbl) ntt3d_forward_operand(h->T.get(), k, h->src, h->n, s);
-        else ntt3_forward_operand(h->T.get(), k, h->src, h->n, s);
+        ntt3_forward_operand(h->T.get(), k, h->src, h->n, s);
         h->k = k;
-        h->form = form;
+        h->form = kFormInt;
+    } else {
+        g_held_reuses.fetch_add(1);
+    }
+    return h->T.get();
+}
+
+// The FP64 form: the held operand's spectrum at length 2^k (stride 2^k); *ready
+// tells whether an earlier product has filled it, else this one must.
+static uint64_t* held_spectrum(int k, bool* ready, cudaStream_t s)
+{
+    HeldOperand* h = t_held;
+    *ready = h->k == k && h->form == kFormDbl;
+    if (!*ready) {
+        h->T = DevBuf<uint64_t>(3 * ((size_t)1 << k), s);
+        h->k = k;
+        h->form = kFormDbl;
     } else {
         g_held_reuses.fetch_add(1);
     }
@@ -622,7 +635,7 @@ static void mul_ntt3_wrapped(uint32_t* z, const uint32_t* a, size_t na, const ui
     const bool square = (a == b && na == nb);
     const uint64_t P0 = kProductPrimes[0], P1 = kProductPrimes[1], P2 = kProductPrimes[2];
     // a held b (or a held square) brings its main transform with it
-    const uint64_t* held = is_held(b, nb) ? held_transform(km, kFormInt, s) : nullptr;
+    const uint64_t* held = is_held(b, nb) ? held_transform(km, s) : nullptr;
     DevBuf<uint64_t> A(3 * ST, s), B(square || held ? 0 : 3 * ST, s), tA(3 * T, s), tB(square ? 0 : 3 * T, s);
     {
         ProfScope ps(KC_SPLIT, 4.0 * (double)(na + nb) + 24.0 * (double)(2 * (Nm + T)), s);
@@ -696,7 +709,7 @@ void mul_ntt3(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size
         }
     }
     const bool square = (a == b && na == nb);
-    const uint64_t* held = is_held(b, nb) ? held_transform(k, kFormInt, s) : nullptr;
+    const uint64_t* held = is_held(b, nb) ? held_transform(k, s) : nullptr;
     DevBuf<uint64_t> A(3 * N, s);
     DevBuf<uint64_t> B(square || held ? 0 : 3 * N, s);
     if (held && square) copy_transforms(A.get(), N, held, N, k, s);
@@ -738,36 +751,6 @@ static NttBatch ntt3d_batch_stride(uint64_t* data, size_t stride)
     bat.per_prime = 1;
     for (int q = 0; q < 3; q++) bat.prime[q] = dbl_prime_tables(kDblPrimes[q]).dev;
     return bat;
-}
-
-// out[q stride + j] = piece first + j of a mod p_q, j < N.
-__global__ void split3d_off_kernel(uint64_t* __restrict__ out, size_t stride, const uint32_t* __restrict__ a,
-                                   uint32_t na, size_t first, size_t N, DblPrimes3 P)
-{
-    for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < N; j += (size_t)gridDim.x * blockDim.x) {
-        const uint64_t v = src_piece56_raw(a, na, first + j);
-#pragma unroll
-        for (int q = 0; q < 3; q++) out[q * stride + j] = dstore(dpiece56(v, P.p[q], P.pinv[q]));
-    }
-}
-
-static void split3d(uint64_t* out, size_t stride, const uint32_t* a, size_t na, size_t first, size_t N,
-                    cudaStream_t s)
-{
-    PIC_REQUIRE(na < ((size_t)1 << 32), PIC_ERR_LENGTH, "operand too long for the FP64 form");
-    split3d_off_kernel<<<grid_for(N, 256), 256, 0, s>>>(out, stride, a, (uint32_t)na, first, N, dbl_primes3());
-    PIC_CHECK_LAUNCH();
-    count_launch();
-}
-
-void ntt3d_forward_operand(uint64_t* out, int k, const uint32_t* a, size_t na, cudaStream_t s)
-{
-    const size_t N = (size_t)1 << k;
-    {
-        ProfScope ps(KC_SPLIT, 4.0 * (double)na + 24.0 * (double)N, s);
-        split3d(out, N, a, na, 0, N, s);
-    }
-    ntt_forward_dif(ntt3d_batch_stride(out, N), k, s);
 }
 
 struct CrtDConsts {
@@ -1023,6 +1006,59 @@ void launch_wrap_fix_d(uint64_t* y, size_t ystride, const uint64_t* tail, size_t
 // coefficients below 2^28 (2^56 - 1)^2 < p0 p1 p2.
 constexpr size_t kDblMaxPieces = (size_t)1 << 28;
 
+// The operands' column passes (straight from the words), the fused middle pass
+// and the inverse column passes of one product at length 2^k: pieces from
+// index fa of a times pieces from index fb of b, residues at out + q stride.
+// spec: the held operand's spectrum at this length (see ProductMiddle).
+constexpr int kDblMinBits = 4;  // shortest transform of ntt_product_middle
+
+static void ntt3d_product(uint64_t* out, size_t stride, int k, const uint32_t* a, size_t na, size_t fa,
+                          const uint32_t* b, size_t nb, size_t fb, bool square, uint64_t* spec, bool spec_ready,
+                          cudaStream_t s)
+{
+    PIC_REQUIRE(na < ((size_t)1 << 32) && nb < ((size_t)1 << 32), PIC_ERR_LENGTH, "operand too long for the FP64 form");
+    auto source = [](const uint32_t* x, size_t n, size_t first) {
+        SplitSrc src;
+        src.words = x;
+        src.n = (uint32_t)n;
+        src.first = first;
+        return src;
+    };
+    const int rows = middle_row_bits(k);
+    const size_t N = (size_t)1 << k;
+    const bool cols = rows < k;
+    const bool need_a = !(square && spec_ready), need_b = !square && !spec_ready;
+    ProductMiddle m{};
+    m.out = out;
+    m.out_stride = stride;
+    m.square = square;
+    m.sa = source(a, na, fa);
+    m.sb = source(b, nb, fb);
+    m.spec = spec;
+    m.spec_ready = spec_ready;
+    DevBuf<uint64_t> B;
+    if (cols && need_a) {
+        NttBatch bt = ntt3d_batch_stride(out, stride);
+        bt.src = m.sa;
+        ntt_forward_cols(bt, k, rows, s);
+        m.a = out;
+        m.a_stride = stride;
+    }
+    if (cols && need_b) {
+        // a held b's column passes run in the buffer its spectrum will fill
+        if (!spec) B = DevBuf<uint64_t>(3 * N, s);
+        NttBatch bt = ntt3d_batch_stride(spec ? spec : B.get(), N);
+        bt.src = m.sb;
+        ntt_forward_cols(bt, k, rows, s);
+        m.b = bt.data;
+        m.b_stride = N;
+    }
+    ntt_product_middle(m, k, s);
+    if (cols) ntt_inverse_cols(ntt3d_batch_stride(out, stride), k, rows, s);
+}
+
+// The wrapped form (see wrap_fix_kernel): main transforms of length 2^km, tails
+// of length 2^kt over the top W pieces.
 static void mul_ntt3d_wrapped(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, int km,
                               int kt, cudaStream_t s)
 {
@@ -1032,31 +1068,11 @@ static void mul_ntt3d_wrapped(uint32_t* z, const uint32_t* a, size_t na, const u
     const size_t Nm = (size_t)1 << km, T = (size_t)1 << kt, W = L - Nm;
     const size_t ST = Nm + ((W + 15) & ~(size_t)15);
     const bool square = (a == b && na == nb);
-    const uint64_t* held = is_held(b, nb) ? held_transform(km, kFormDbl, s) : nullptr;
-    DevBuf<uint64_t> A(3 * ST, s), B(square || held ? 0 : 3 * ST, s), tA(3 * T, s), tB(square ? 0 : 3 * T, s);
-    {
-        ProfScope ps(KC_SPLIT, 4.0 * (double)(na + nb) + 24.0 * (double)(2 * (Nm + T)), s);
-        if (!(held && square)) split3d(A.get(), ST, a, na, 0, Nm, s);
-        split3d(tA.get(), T, a, na, Nm - pb + 1, T, s);
-        if (!square) {
-            if (!held) split3d(B.get(), ST, b, nb, 0, Nm, s);
-            split3d(tB.get(), T, b, nb, Nm - pa + 1, T, s);
-        }
-    }
-    const NttBatch mA = ntt3d_batch_stride(A.get(), ST), mB = ntt3d_batch_stride(B.get(), ST);
-    const NttBatch xA = ntt3d_batch_stride(tA.get(), T), xB = ntt3d_batch_stride(tB.get(), T);
-    if (held && square) copy_transforms(A.get(), ST, held, Nm, km, s);
-    else ntt_forward_dif(mA, km, s);
-    ntt_forward_dif(xA, kt, s);
-    if (!square) {
-        if (!held) ntt_forward_dif(mB, km, s);
-        ntt_forward_dif(xB, kt, s);
-    }
-    if (held) ntt_pointwise_mont(mA, held, km, s, Nm);
-    else ntt_pointwise_mont(mA, square ? A.get() : B.get(), km, s);
-    ntt_pointwise_mont(xA, square ? tA.get() : tB.get(), kt, s);
-    ntt_inverse_dit(mA, km, s);
-    ntt_inverse_dit(xA, kt, s);
+    bool ready = false;
+    uint64_t* spec = is_held(b, nb) ? held_spectrum(km, &ready, s) : nullptr;
+    DevBuf<uint64_t> A(3 * ST, s), tA(3 * T, s);
+    ntt3d_product(A.get(), ST, km, a, na, 0, b, nb, 0, square, spec, ready, s);
+    ntt3d_product(tA.get(), T, kt, a, na, Nm - pb + 1, b, nb, Nm - pa + 1, square, nullptr, false, s);
     {
         ProfScope ps(KC_NTT_POINTWISE, 3.0 * (double)W * 24.0, s);
         launch_wrap_fix_d(A.get(), ST, tA.get(), T, 1, 1, 1, Nm, W, s);
@@ -1081,15 +1097,15 @@ void mul_ntt3d(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, siz
     }
     const size_t ncoef = pa + pb - 1;
     int k = ceil_log2(ncoef);
-    if (k < 1) k = 1;
+    if (k < kDblMinBits) k = kDblMinBits;
     PIC_REQUIRE(k <= 30, PIC_ERR_LENGTH, "product too long for the FP64 three-prime NTT (2^30 points)");
     const size_t N = (size_t)1 << k;
-    if (g_mul_wrap && k >= 4) {
+    if (g_mul_wrap && k > kDblMinBits + 1) {
         const size_t Nm = N / 2;
         if (std::max(pa, pb) <= Nm && ncoef > Nm) {
             const size_t W = ncoef - Nm;
             int kt = ceil_log2(2 * W - 1);
-            if (kt < 2) kt = 2;
+            if (kt < kDblMinBits) kt = kDblMinBits;
             if (((size_t)1 << kt) <= Nm / 2) {
                 mul_ntt3d_wrapped(z, a, na, b, nb, k - 1, kt, s);
                 return;
@@ -1097,14 +1113,10 @@ void mul_ntt3d(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, siz
         }
     }
     const bool square = (a == b && na == nb);
-    const uint64_t* held = is_held(b, nb) ? held_transform(k, kFormDbl, s) : nullptr;
+    bool ready = false;
+    uint64_t* spec = is_held(b, nb) ? held_spectrum(k, &ready, s) : nullptr;
     DevBuf<uint64_t> A(3 * N, s);
-    DevBuf<uint64_t> B(square || held ? 0 : 3 * N, s);
-    if (held && square) copy_transforms(A.get(), N, held, N, k, s);
-    else ntt3d_forward_operand(A.get(), k, a, na, s);
-    if (!square && !held) ntt3d_forward_operand(B.get(), k, b, nb, s);
-    ntt_pointwise_mont(ntt3d_batch_stride(A.get(), N), held ? held : (square ? A.get() : B.get()), k, s);
-    ntt_inverse_dit(ntt3d_batch_stride(A.get(), N), k, s);
+    ntt3d_product(A.get(), N, k, a, na, 0, b, nb, 0, square, spec, ready, s);
     crt3d_to_words(A.get(), N, k, ncoef, z, zw, s);
 }
 

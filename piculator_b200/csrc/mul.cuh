@@ -15,10 +15,8 @@ void mul_ntt3(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size
 void mul_ntt3d(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s);
 // 56-bit pieces of an operand of n words.
 size_t pieces56(size_t nwords);
-// FP64-form building blocks: split + forward into out[3 * 2^k]; batched
-// inverse output like ntt3_batch_to_words (offset 2^140 per coefficient);
-// wrapped-product fix-up like launch_wrap_fix.
-void ntt3d_forward_operand(uint64_t* out, int k, const uint32_t* a, size_t na, cudaStream_t s);
+// FP64-form building blocks: batched inverse output like ntt3_batch_to_words
+// (offset 2^140 per coefficient); wrapped-product fix-up like launch_wrap_fix.
 void ntt3d_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, size_t count, int k, uint32_t* z,
                           uint32_t zcap, const uint32_t* zlen, cudaStream_t s, size_t ncoef, bool offset);
 void launch_wrap_fix_d(uint64_t* y, size_t ystride, const uint64_t* tail, size_t T, size_t nitems,

@@ -149,8 +149,28 @@ struct MergeMiddle {
     bool need_r;
 };
 void ntt_merge_middle(const MergeMiddle& m, int k, cudaStream_t s);
-// Row bits the fused merge uses at length 2^k.
-int merge_row_bits(int k);
+// Row bits the fused merge and product use at length 2^k.
+int middle_row_bits(int k);
+//
+// A product: out = a b per prime q (transforms at out + q out_stride, a and b
+// likewise), the operands' column passes done (k = row bits: read from the
+// source words).  out may be a.  b null: a square.  A held operand's spectrum
+// (stride 2^k) can take b's place, or a's in a square: `spec` receives that
+// operand's spectrum when spec_ready is false, and is read instead of
+// transforming it when it is true.
+struct ProductMiddle {
+    uint64_t* out;
+    size_t out_stride;
+    const uint64_t* a;  // null when the square's operand is `spec` ready
+    size_t a_stride;
+    const uint64_t* b;
+    size_t b_stride;
+    bool square;
+    SplitSrc sa, sb;
+    uint64_t* spec;
+    bool spec_ready;
+};
+void ntt_product_middle(const ProductMiddle& m, int k, cudaStream_t s);
 
 // out[i] = a[i] * b[i] * 2^-64 mod p over every transform of the batch
 // (b may equal a for squaring); b's transforms are b_stride apart (0: a's

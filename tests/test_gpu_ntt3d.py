@@ -183,3 +183,21 @@ def test_auto_products_in_chosen_form(pic, n):
     finally:
         pic.set_tuning(pic.TUNE_NTT_FORM, saved)
     assert _int(z) == _int(a) * _int(b)
+
+
+@pytest.mark.parametrize("na,nb", [(14_340, 14_340), (14_400, 14_500), (30_000, 28_000), (57_344, 57_344),
+                                   (57_400, 300), (229_300, 230_000), (3_670_000, 3_700_001)])
+def test_fused_product_lengths_match_integer_form(pic, torch_cuda, na, nb):
+    """The fused FP64 product against the integer form's separate passes, around
+    the lengths where a product takes another column pass or a wrapped tail of
+    another length, and the square of each."""
+    torch = torch_cuda
+    a, b = random_words(na, na), random_words(nb + 1, nb)
+    ta, tb = (torch.from_numpy(x.view(np.int32)).cuda() for x in (a, b))
+    for x, y in ((ta, tb), (ta, ta)):
+        z = [torch.empty(x.numel() + y.numel(), dtype=torch.int32, device="cuda") for _ in range(2)]
+        torch.cuda.synchronize()
+        for out, mode in zip(z, ("ntt3d", "ntt3")):
+            pic.mul_dev(out.data_ptr(), x.data_ptr(), x.numel(), y.data_ptr(), y.numel(), mode)
+        pic.synchronize()
+        assert torch.equal(z[0], z[1])
