@@ -43,8 +43,7 @@ BigFloat::BigFloat(uint32_t x, bool sign_) : sign(true), exp(0), L(1)
     }
     sign = sign_;
     store = alloc_words(1);
-    PIC_CUDA(cudaMemcpyAsync(store->base, &x, sizeof(uint32_t), cudaMemcpyHostToDevice, S()));
-    PIC_CUDA(cudaStreamSynchronize(S()));
+    lin_set(store->base, x, 0, 1, S());
     T = store->base;
 }
 
@@ -91,8 +90,12 @@ BigFloat BigFloat::from_host(bool sign, int64_t exp, const uint32_t* words, size
     z.L = L;
     if (L) {
         z.store = alloc_words(L);
-        PIC_CUDA(cudaMemcpyAsync(z.store->base, words, L * sizeof(uint32_t), cudaMemcpyHostToDevice, S()));
-        PIC_CUDA(cudaStreamSynchronize(S()));
+        if (L <= 2) {
+            lin_set(z.store->base, words[0], L > 1 ? words[1] : 0u, (int)L, S());
+        } else {
+            PIC_CUDA(cudaMemcpyAsync(z.store->base, words, L * sizeof(uint32_t), cudaMemcpyHostToDevice, S()));
+            PIC_CUDA(cudaStreamSynchronize(S()));
+        }
         z.T = z.store->base;
     }
     return z;
@@ -147,9 +150,7 @@ BigFloat BigFloat::mul(uint32_t x) const
 {
     if (L == 0 || x == 0) return BigFloat();
     auto st = alloc_words(L + 1);
-    lin_mul_u32(st->base, T, L, x, S());
-    uint32_t top;
-    read_words(&top, st->base + L, 1, S());
+    const uint32_t top = lin_mul_u32(st->base, T, L, x);
     return from_device(sign, exp, st, st->base, top != 0 ? L + 1 : L);
 }
 
@@ -169,14 +170,15 @@ BigFloat BigFloat::uadd(const BigFloat& x, size_t p) const
     TL = (int64_t)(uint32_t)TL;  // the reference stores z.L = (uint32_t)TL
     auto st = alloc_words((size_t)TL + 1);
     WordView a{T, exp, (int64_t)L}, b{x.T, x.exp, (int64_t)x.L};
-    lin_addsub(st->base, (size_t)TL, a, b, bot, false, st->base + TL, S());
-    uint32_t carry;
-    read_words(&carry, st->base + TL, 1, S());
+    const uint32_t carry = lin_add(st->base, (size_t)TL, a, b, bot);
     return from_device(sign, bot, st, st->base, (size_t)TL + (carry ? 1 : 0));
 }
 
-// usub -- BigFloat.cpp:233-287 (|this| >= |x|)
-BigFloat BigFloat::usub(const BigFloat& x, size_t p) const
+// ucmp and usub -- BigFloat.cpp:123-147, 233-287: |this| - |x| with the sign of
+// *this when |this| > |x| (*greater), else |x| - |this| with the sign of x.  The
+// window is the same for both orders; the comparison, where it needs words, and
+// the subtraction follow each other on the device.
+BigFloat BigFloat::udiff(const BigFloat& x, size_t p, bool* greater) const
 {
     const int64_t magA = exp + (int64_t)L, magB = x.exp + (int64_t)x.L;
     const int64_t top = magA > magB ? magA : magB;
@@ -191,27 +193,28 @@ BigFloat BigFloat::usub(const BigFloat& x, size_t p) const
     TL = (int64_t)(uint32_t)TL;
     auto st = alloc_words((size_t)TL + 1);
     WordView a{T, exp, (int64_t)L}, b{x.T, x.exp, (int64_t)x.L};
-    lin_addsub(st->base, (size_t)TL, a, b, bot, true, st->base + TL, S());
-    const size_t nz = lin_top_nonzero(st->base, (size_t)TL, S());
+    int order = lin_mag_order(a, b);
+    const size_t nz = lin_diff(st->base, (size_t)TL, a, b, bot, &order);
+    *greater = order > 0;
     if (nz == 0) return BigFloat();  // zero: exp 0, sign positive (BigFloat.cpp:280-284)
-    return from_device(sign, bot, st, st->base, nz);
+    return from_device(order > 0 ? sign : x.sign, bot, st, st->base, nz);
 }
 
 // add -- BigFloat.cpp:288-305
 BigFloat BigFloat::add(const BigFloat& x, size_t p) const
 {
     if (sign == x.sign) return uadd(x, p);
-    if (ucmp(x) > 0) return usub(x, p);
-    return x.usub(*this, p);
+    bool greater;
+    return udiff(x, p, &greater);
 }
 
 // sub -- BigFloat.cpp:306-325
 BigFloat BigFloat::sub(const BigFloat& x, size_t p) const
 {
     if (sign != x.sign) return uadd(x, p);
-    if (ucmp(x) > 0) return usub(x, p);
-    BigFloat z = x.usub(*this, p);
-    z.negate();
+    bool greater;
+    BigFloat z = udiff(x, p, &greater);
+    if (!greater) z.negate();
     return z;
 }
 
@@ -239,9 +242,11 @@ BigFloat BigFloat::mul(const BigFloat& x, size_t p, int) const
     }
     const size_t zl = AL + BL;
     auto st = alloc_words(zl);
-    mul_dispatch(st->base, AT, AL, BT, BL, t_mul_mode, S());
+    Mail mail(S());
+    mul_dispatch(st->base, AT, AL, BT, BL, t_mul_mode, S(), &mail);
     uint32_t top;
-    read_words(&top, st->base + zl - 1, 1, S());
+    if (mail.armed()) top = (uint32_t)mail.wait();
+    else read_words(&top, st->base + zl - 1, 1, S());
     return from_device(sign == x.sign, Aexp + Bexp, st, st->base, top == 0 ? zl - 1 : zl);
 }
 

@@ -75,7 +75,7 @@ private:
     std::shared_ptr<WordStore> store;
 
     BigFloat uadd(const BigFloat& x, size_t p) const;
-    BigFloat usub(const BigFloat& x, size_t p) const;
+    BigFloat udiff(const BigFloat& x, size_t p, bool* greater) const;
 
     friend BigFloat invsqrt(uint32_t x, size_t p, int threads);
 };

@@ -1066,12 +1066,11 @@ __global__ void __launch_bounds__(256) signed_add_kernel(const uint32_t* __restr
 
 // ---- the same signed sum spread over many CTAs per parent -------------------
 // For levels with few, long parents: one CTA per (parent, chunk of kWideWPC
-// words), the chunks' carries (or borrows) joined by a segmented scan.
+// words), the chunks' carries (or borrows) joined in a second launch.
 //   wide_cmp:    highest differing word of |T1|, |T2| per parent (atomicMax)
 //   wide_k1:     chunk digits with in-chunk carries, chunk (G, P) aggregate
-//   (carry_scan_segments: carry-in per chunk)
-//   wide_ripple: +1 / -1 rippled into chunks with a carry-in
-//   wide_final:  length (highest nonzero word, atomicMax), carry word, sign
+//   wide_fix:    +1 / -1 rippled into chunks with a carry-in, then the length
+//                (highest nonzero word, atomicMax), carry word and sign
 constexpr int kWideIPT = 8;
 constexpr uint32_t kWideWPC = 256 * kWideIPT;
 
@@ -1083,8 +1082,7 @@ struct WideAdd {
     uint32_t *Pw, *Pl, cP;
     uint8_t* Ps;
     uint32_t* hd;    // per parent: highest differing word + 1
-    uint32_t* agg;   // per (parent, chunk): (G, P), then carry-in
-    uint32_t* aggc;  // per (parent, chunk): (G, P) kept for the final carry
+    uint32_t* agg;   // per (parent, chunk): (G, P)
     uint32_t cpp;    // chunks per parent
 };
 
@@ -1184,46 +1182,29 @@ __global__ void __launch_bounds__(256) wide_k1_kernel(WideAdd w)
             cin = (uint32_t)(xs[u] < ys[u]) | ((uint32_t)(d == 0u) & cin);
         }
     }
-    if (threadIdx.x == 0) {
-        w.agg[blockIdx.x] = total;
-        w.aggc[blockIdx.x] = total;
-    }
+    if (threadIdx.x == 0) w.agg[blockIdx.x] = total;
 }
 
 // Chunks with a carry-in: +1 (add) or -1 (subtract) rippled from the chunk's
-// first word to the first word that absorbs it.
-__global__ void __launch_bounds__(256) wide_ripple_kernel(WideAdd w)
-{
-    if (w.agg[blockIdx.x] == 0) return;
-    const size_t i = blockIdx.x / w.cpp, c = blockIdx.x % w.cpp;
-    const uint32_t n = max(w.l1[i], w.l2[i]);
-    const WideOp o = wide_op(w, i);
-    if (o.zero) return;
-    uint32_t* z = w.Pw + (w.c0 + i) * (size_t)w.cP;
-    const uint32_t b0 = (uint32_t)c * kWideWPC, e = min(min(b0 + kWideWPC, n), w.cP);
-    if (b0 >= e) return;
-    const uint32_t stop = o.sub ? 0u : 0xffffffffu;  // words that pass the carry on
-    unsigned long long mine = ~0ull;
-    for (uint32_t k = b0 + threadIdx.x; k < e; k += blockDim.x)
-        if (z[k] != stop && k < mine) mine = k;
-    const uint32_t f = (uint32_t)min((unsigned long long)e, block_min_u64(mine));
-    for (uint32_t k = b0 + threadIdx.x; k < f; k += blockDim.x) z[k] = ~stop;
-    if (threadIdx.x == 0 && f < e) z[f] += o.sub ? 0xffffffffu : 1u;
-}
-
-// Length, carry word and sign.  Parent lengths start at zero.
-__global__ void __launch_bounds__(256) wide_final_kernel(WideAdd w)
+// first word.  Then length, carry word and sign; parent lengths start at zero.
+__global__ void __launch_bounds__(256) wide_fix_kernel(WideAdd w)
 {
     const size_t i = blockIdx.x / w.cpp, c = blockIdx.x % w.cpp;
     const uint32_t n = max(w.l1[i], w.l2[i]);
     const WideOp o = wide_op(w, i);
     const bool sa = w.cS[2 * i] != 0, sb = w.cS[2 * i + 1] != 0;
     uint32_t* z = w.Pw + (w.c0 + i) * (size_t)w.cP;
+    if (o.sub && c == 0 && threadIdx.x == 0) w.Ps[w.c0 + i] = o.zero ? 1 : ((o.swap ? sb : sa) ? 1 : 0);
+    if (o.zero) return;
+    const uint32_t* agg = w.agg + i * (size_t)w.cpp;
+    const uint32_t last = n ? (n - 1) / kWideWPC : 0;
+    if (c > last) return;
+    const uint32_t cin = chunk_carry_in(agg, c);
+    const uint32_t b0 = (uint32_t)c * kWideWPC, e = min(min(b0 + kWideWPC, n), w.cP);
+    if (cin) chunk_ripple(z, b0, e, o.sub);
     if (!o.sub) {
-        // the carry out of the last chunk: its (G, P) joined with its carry-in
-        const uint32_t last = n ? (n - 1) / kWideWPC : 0;
         if (c == last && threadIdx.x == 0) {
-            const uint32_t gp = w.aggc[blockIdx.x], cin = w.agg[blockIdx.x];
+            const uint32_t gp = agg[c];
             const uint32_t carry = n ? ((gp & 1u) | ((gp >> 1) & cin)) : 0u;
             if (carry && n < w.cP) z[n] = 1;
             w.Pl[w.c0 + i] = n + carry;
@@ -1231,9 +1212,7 @@ __global__ void __launch_bounds__(256) wide_final_kernel(WideAdd w)
         }
         return;
     }
-    if (c == 0 && threadIdx.x == 0) w.Ps[w.c0 + i] = o.zero ? 1 : ((o.swap ? sb : sa) ? 1 : 0);
-    if (o.zero) return;
-    const uint32_t b0 = (uint32_t)c * kWideWPC, e = min(min(b0 + kWideWPC, n), w.cP);
+    __syncthreads();
     unsigned long long mine = 0;
     for (uint32_t k = b0 + threadIdx.x; k < e; k += blockDim.x)
         if (z[k] != 0) mine = k + 1;
@@ -1550,20 +1529,18 @@ static void signed_sum(const uint32_t* A, const uint32_t* lA, uint32_t cA, const
     ProfScope ps(KC_LINEAR, 12.0 * (double)np * (double)nmax, s);
     const uint32_t cpp = (uint32_t)((nmax + kWideWPC - 1) / kWideWPC);
     if (g_wide_add && np < 2 * 148 && cpp > 1) {
-        DevBuf<uint32_t> hd(np, s), agg(np * cpp, s), aggc(np * cpp, s);
+        DevBuf<uint32_t> hd(np, s), agg(np * cpp, s);
         PIC_CUDA(cudaMemsetAsync(hd.get(), 0, 4 * np, s));
         PIC_CUDA(cudaMemsetAsync(par.P.len.get() + p0, 0, 4 * np, s));
         WideAdd w{A, lA, B, lB, cA, cB, cS, p0, par.P.w.get(), par.P.len.get(), par.P.cap, par.sign.get(), hd.get(),
-                  agg.get(), aggc.get(), cpp};
+                  agg.get(), cpp};
         const unsigned grid = (unsigned)(np * cpp);
         wide_cmp_kernel<<<grid, 256, 0, s>>>(w);
         wide_k1_kernel<<<grid, 256, 0, s>>>(w);
         PIC_CHECK_LAUNCH();
-        carry_scan_segments(agg.get(), np, cpp, s);
-        wide_ripple_kernel<<<grid, 256, 0, s>>>(w);
-        wide_final_kernel<<<grid, 256, 0, s>>>(w);
+        wide_fix_kernel<<<grid, 256, 0, s>>>(w);
         PIC_CHECK_LAUNCH();
-        count_launch(4);
+        count_launch(3);
     } else {
         signed_add_kernel<<<(unsigned)np, 256, 0, s>>>(A, lA, cA, B, lB, cB, cS, p0, par.P.w.get(), par.P.len.get(),
                                                       par.sign.get(), par.P.cap);
@@ -1583,9 +1560,9 @@ static bool g_combine = true;  // P formed in the transform domain (one inverse,
 // per word the peak outgrew it and runs stalled on pool growth.
 static size_t merge_budget(size_t p)
 {
-    size_t b = device_available_bytes() / 4;
-    b = std::min(b, p * 128);
-    return std::max(b, (size_t)1 << 30);
+    const size_t least = (size_t)1 << 30;
+    if (p * 128 <= least) return least;  // whatever is left: no need to ask (0.1 ms, at times 4)
+    return std::max(std::min(device_available_bytes() / 4, p * 128), least);
 }
 
 static void merge_ntt(Level& ch, Level& par, cudaStream_t s, size_t mem_budget)

@@ -6,102 +6,45 @@
 
 namespace pic {
 
-// ---- K2: scan of per-CTA (G, P) pairs, one CTA -----------------------------
-__global__ void __launch_bounds__(1024) carry_scan_kernel(uint32_t* agg, size_t n, uint32_t* final_carry)
-{
-    const size_t per = (n + blockDim.x - 1) / blockDim.x;
-    const size_t b = threadIdx.x * per, e = b + per < n ? b + per : n;
-    uint32_t acc = kGPIdentity;
-    for (size_t i = b; i < e; i++) acc = gp_combine(acc, agg[i]);
-    uint32_t total;
-    const uint32_t pre = block_gp_scan(acc, &total);
-    uint32_t cin = pre & 1u;  // carry into this segment (array carry-in 0)
-    for (size_t i = b; i < e; i++) {
-        const uint32_t gp = agg[i];
-        agg[i] = cin;
-        cin = (gp & 1u) | ((gp >> 1) & cin);
-    }
-    if (threadIdx.x == 0 && final_carry) *final_carry = total & 1u;
-}
-
-void carry_scan_aggregates(uint32_t* agg, size_t nctas, uint32_t* final_carry, cudaStream_t s)
-{
-    ProfScope ps(KC_CARRY, 8.0 * (double)nctas, s);
-    carry_scan_kernel<<<1, 1024, 0, s>>>(agg, nctas, final_carry);
-    PIC_CHECK_LAUNCH();
-    count_launch();
-}
-
-__global__ void __launch_bounds__(256) carry_scan_seg_kernel(uint32_t* agg, size_t cpp)
-{
-    uint32_t* a = agg + blockIdx.x * cpp;
-    const size_t per = (cpp + blockDim.x - 1) / blockDim.x;
-    const size_t b = threadIdx.x * per, e = b + per < cpp ? b + per : cpp;
-    uint32_t acc = kGPIdentity;
-    for (size_t i = b; i < e; i++) acc = gp_combine(acc, a[i]);
-    uint32_t total;
-    const uint32_t pre = block_gp_scan(acc, &total);
-    uint32_t cin = pre & 1u;
-    for (size_t i = b; i < e; i++) {
-        const uint32_t gp = a[i];
-        a[i] = cin;
-        cin = (gp & 1u) | ((gp >> 1) & cin);
-    }
-}
-
-void carry_scan_segments(uint32_t* agg, size_t count, size_t cpp, cudaStream_t s)
-{
-    ProfScope ps(KC_CARRY, 8.0 * (double)(count * cpp), s);
-    carry_scan_seg_kernel<<<(unsigned)count, 256, 0, s>>>(agg, cpp);
-    PIC_CHECK_LAUNCH();
-    count_launch();
-}
-
-__global__ void carry_ripple_batch_kernel(uint32_t* z, uint32_t zcap, const uint32_t* zlen, size_t wpc,
-                                          const uint32_t* cin, size_t cpp)
-{
-    if (cin[blockIdx.x] == 0) return;
-    const size_t prod = blockIdx.x / cpp, lc = blockIdx.x % cpp;
-    uint32_t* zz = z + prod * (size_t)zcap;
-    const size_t n = zlen[prod];
-    const size_t b = lc * wpc, e = b + wpc < n ? b + wpc : n;
-    unsigned long long mine = ~0ull;
-    for (size_t i = b + threadIdx.x; i < e; i += blockDim.x)
-        if (zz[i] != 0xffffffffu && i < mine) mine = i;
-    const size_t f = (size_t)block_min_u64(mine);
-    for (size_t i = b + threadIdx.x; i < e && i < f; i += blockDim.x) zz[i] = 0;
-    if (threadIdx.x == 0 && f < e) zz[f] += 1u;
-}
-
-void carry_ripple_batch(uint32_t* z, uint32_t zcap, const uint32_t* zlen, size_t words_per_cta,
-                        const uint32_t* agg_cin, size_t count, size_t cpp, cudaStream_t s)
-{
-    ProfScope ps(KC_CARRY, 4.0 * (double)(count * cpp), s);
-    carry_ripple_batch_kernel<<<(unsigned)(count * cpp), 256, 0, s>>>(z, zcap, zlen, words_per_cta, agg_cin, cpp);
-    PIC_CHECK_LAUNCH();
-    count_launch();
-}
-
-// ---- K3: ripple a carry-in of 1 through one CTA's words --------------------
-__global__ void carry_ripple_kernel(uint32_t* z, size_t n, size_t wpc, const uint32_t* cin, int mode)
+// ---- K2 ---------------------------------------------------------------------
+__global__ void __launch_bounds__(256) carry_fix_kernel(uint32_t* z, size_t n, size_t wpc,
+                                                        const uint32_t* __restrict__ agg, size_t nctas, MailRef mail)
 {
     const size_t c = blockIdx.x;
-    if (cin[c] == 0) return;
     const size_t b = c * wpc, e = b + wpc < n ? b + wpc : n;
-    const uint32_t stop_unless = mode == kCarryAdd ? 0xffffffffu : 0u;
-    unsigned long long mine = ~0ull;
-    for (size_t i = b + threadIdx.x; i < e; i += blockDim.x)
-        if (z[i] != stop_unless && i < mine) mine = i;
-    const size_t f = (size_t)block_min_u64(mine);
-    for (size_t i = b + threadIdx.x; i < e && i < f; i += blockDim.x) z[i] = ~stop_unless;
-    if (threadIdx.x == 0 && f < e) z[f] = mode == kCarryAdd ? z[f] + 1u : z[f] - 1u;
+    if (chunk_carry_in(agg, c)) chunk_ripple(z, b, e, false);
+    if (mail.slot != nullptr && c == nctas - 1) {
+        __syncthreads();
+        if (threadIdx.x == 0) mail_post(mail, z[n - 1]);
+    }
 }
 
-void carry_ripple(uint32_t* z, size_t nwords, size_t words_per_cta, const uint32_t* agg_cin,
-                  size_t nctas, CarryMode mode, cudaStream_t s)
+void carry_fix(uint32_t* z, size_t nwords, size_t words_per_cta, const uint32_t* agg, size_t nctas, cudaStream_t s,
+               MailRef mail)
 {
     ProfScope ps(KC_CARRY, 4.0 * (double)nctas, s);
-    carry_ripple_kernel<<<(unsigned)nctas, 256, 0, s>>>(z, nwords, words_per_cta, agg_cin, (int)mode);
+    carry_fix_kernel<<<(unsigned)nctas, 256, 0, s>>>(z, nwords, words_per_cta, agg, nctas, mail);
+    PIC_CHECK_LAUNCH();
+    count_launch();
+}
+
+__global__ void __launch_bounds__(256) carry_fix_batch_kernel(uint32_t* z, uint32_t zcap,
+                                                              const uint32_t* __restrict__ zlen, size_t wpc,
+                                                              const uint32_t* __restrict__ agg, size_t cpp, bool sub)
+{
+    const size_t prod = blockIdx.x / cpp, c = blockIdx.x - prod * cpp;
+    const size_t n = zlen[prod];
+    const size_t b = c * wpc, e = b + wpc < n ? b + wpc : n;
+    if (b >= e || !chunk_carry_in(agg + prod * cpp, c)) return;
+    chunk_ripple(z + prod * (size_t)zcap, b, e, sub);
+}
+
+void carry_fix_batch(uint32_t* z, uint32_t zcap, const uint32_t* zlen, size_t words_per_cta, const uint32_t* agg,
+                     size_t count, size_t cpp, cudaStream_t s, bool sub)
+{
+    if (cpp <= 1) return;  // one CTA per product: no carries between CTAs
+    ProfScope ps(KC_CARRY, 4.0 * (double)(count * cpp), s);
+    carry_fix_batch_kernel<<<(unsigned)(count * cpp), 256, 0, s>>>(z, zcap, zlen, words_per_cta, agg, cpp, sub);
     PIC_CHECK_LAUNCH();
     count_launch();
 }
@@ -119,10 +62,70 @@ __device__ __forceinline__ uint32_t word_at(const uint32_t* T, int64_t exp, int6
     return (i >= 0 && i < L) ? T[i] : 0u;
 }
 
-// Windowed add / subtract of two magnitudes: z[c] = a(bot+c) +/- b(bot+c).
-__global__ void __launch_bounds__(kLinThreads) addsub_k1(uint32_t* z, size_t TL, WordView a, WordView b,
-                                                         int64_t bot, int mode, uint32_t* agg)
+// How a linear operation on z[0, n) ends: the word above it and the result.
+enum LinKind { kLinAdd = 0, kLinSub = 1, kLinMul = 2 };
+
+struct LinEnd {
+    int kind;
+    uint32_t* carry_out;  // the carry's (kLinMul: the top word's) place, may be null
+    uint32_t top_hi;      // kLinMul: the top word's part of the last product, set by the kernels
+    const int* order;     // kLinSub: posted beside the length
+    unsigned long long* diff;  // kLinSub over several CTAs: zero before and after
+    uint32_t* ticket;
+    MailRef mail;
+};
+
+// The end of the CTA that holds words [b, e) of z, its carry-in resolved
+// (`carry` out of it).  Every thread calls.
+__device__ __forceinline__ void lin_end(const LinEnd& E, const uint32_t* z, size_t b, size_t e, uint32_t carry,
+                                        uint32_t nctas)
 {
+    if (E.kind == kLinSub) {
+        if (E.mail.slot == nullptr) return;
+        __syncthreads();
+        unsigned long long mine = 0;
+        for (size_t i = b + threadIdx.x; i < e; i += blockDim.x)
+            if (z[i] != 0u) mine = i + 1;
+        mine = block_max_u64(mine);
+        if (nctas > 1) {
+            if (threadIdx.x == 0 && mine) atomicMax(E.diff, mine);
+            if (!last_cta(E.ticket, nctas)) return;
+            if (threadIdx.x == 0) {
+                mine = __ldcg(E.diff);
+                *E.diff = 0;
+            }
+        }
+        if (threadIdx.x == 0) mail_post(E.mail, mine, E.order == nullptr || *E.order > 0 ? 1u : 0u);
+        return;
+    }
+    if (blockIdx.x == nctas - 1 && threadIdx.x == 0) {
+        const uint32_t v = carry + (E.kind == kLinMul ? E.top_hi : 0u);
+        if (E.carry_out != nullptr) *E.carry_out = v;
+        mail_post(E.mail, v);
+    }
+}
+
+// K2 of the linear operations (several CTAs).
+__global__ void __launch_bounds__(kLinThreads) lin_fix_kernel(uint32_t* z, size_t n, const uint32_t* __restrict__ agg,
+                                                              uint32_t nctas, LinEnd E, const uint32_t* a, uint32_t x)
+{
+    const size_t c = blockIdx.x;
+    const size_t b = c * kLinWPC, e = b + kLinWPC < n ? b + kLinWPC : n;
+    const uint32_t cin = chunk_carry_in(agg, c);
+    const uint32_t gp = agg[c];
+    if (cin) chunk_ripple(z, b, e, E.kind == kLinSub);
+    if (E.kind == kLinMul) E.top_hi = (uint32_t)(((uint64_t)a[n - 1] * x) >> 32);
+    lin_end(E, z, b, e, (gp & 1u) | ((gp >> 1) & cin), nctas);
+}
+
+// Windowed add / subtract of two magnitudes: z[c] = a(bot+c) +/- b(bot+c).
+// order (subtract): b - a when *order is not positive.  A single CTA ends the
+// operation itself.
+__global__ void __launch_bounds__(kLinThreads) addsub_k1(uint32_t* z, size_t TL, WordView va, WordView vb,
+                                                         int64_t bot, uint32_t* agg, LinEnd E)
+{
+    const bool ord = E.order == nullptr || *E.order > 0, add = E.kind == kLinAdd;
+    const WordView a = ord ? va : vb, b = ord ? vb : va;
     const size_t i0 = (size_t)blockIdx.x * kLinWPC + (size_t)threadIdx.x * kLinIPT;
     uint32_t d[kLinIPT], gg[kLinIPT];
     uint32_t gp = kGPIdentity;
@@ -133,7 +136,7 @@ __global__ void __launch_bounds__(kLinThreads) addsub_k1(uint32_t* z, size_t TL,
         if (i < TL) {
             const int64_t mag = bot + (int64_t)i;
             const uint32_t x = word_at(a.T, a.exp, a.L, mag), y = word_at(b.T, b.exp, b.L, mag);
-            if (mode == kCarryAdd) {
+            if (add) {
                 const uint64_t s = (uint64_t)x + y;
                 dig = (uint32_t)s;
                 g = (uint32_t)(s >> 32);
@@ -142,7 +145,7 @@ __global__ void __launch_bounds__(kLinThreads) addsub_k1(uint32_t* z, size_t TL,
                 g = x < y;
             }
         }
-        const uint32_t p = mode == kCarryAdd ? (dig == 0xffffffffu) : (dig == 0u);
+        const uint32_t p = add ? (dig == 0xffffffffu) : (dig == 0u);
         d[u] = dig;
         gg[u] = g;
         if (i < TL) gp = gp_combine(gp, g | (p << 1));  // padding is the scan identity
@@ -155,7 +158,7 @@ __global__ void __launch_bounds__(kLinThreads) addsub_k1(uint32_t* z, size_t TL,
         if (i >= TL) break;
         const uint32_t dig = d[u];
         uint32_t p;
-        if (mode == kCarryAdd) {
+        if (add) {
             z[i] = dig + cin;
             p = dig == 0xffffffffu;
         } else {
@@ -164,12 +167,16 @@ __global__ void __launch_bounds__(kLinThreads) addsub_k1(uint32_t* z, size_t TL,
         }
         cin = gg[u] | (p & cin);
     }
-    if (threadIdx.x == 0) agg[blockIdx.x] = total;
+    if (gridDim.x > 1) {
+        if (threadIdx.x == 0) agg[blockIdx.x] = total;
+    } else {
+        lin_end(E, z, 0, TL, total & 1u, 1);
+    }
 }
 
 // z[c] = low(a_c x) + high(a_(c-1) x), carries resolved; z[L] = final word.
 __global__ void __launch_bounds__(kLinThreads) mulu32_k1(uint32_t* z, const uint32_t* a, size_t L, uint32_t x,
-                                                         uint32_t* agg)
+                                                         uint32_t* agg, LinEnd E)
 {
     const size_t i0 = (size_t)blockIdx.x * kLinWPC + (size_t)threadIdx.x * kLinIPT;
     uint32_t d[kLinIPT], gg[kLinIPT];
@@ -200,51 +207,99 @@ __global__ void __launch_bounds__(kLinThreads) mulu32_k1(uint32_t* z, const uint
         z[i] = d[u] + cin;
         cin = gg[u] | ((uint32_t)(d[u] == 0xffffffffu) & cin);
     }
-    if (threadIdx.x == 0) agg[blockIdx.x] = total;
+    if (gridDim.x > 1) {
+        if (threadIdx.x == 0) agg[blockIdx.x] = total;
+    } else {
+        E.top_hi = (uint32_t)(((uint64_t)a[L - 1] * x) >> 32);
+        lin_end(E, z, 0, L, total & 1u, 1);
+    }
 }
 
-__global__ void mulu32_final_kernel(uint32_t* z, const uint32_t* a, size_t L, uint32_t x, const uint32_t* fc)
+__global__ void set_words_kernel(uint32_t* p, uint32_t lo, uint32_t hi, int n)
 {
-    // word L = high half of the top product + the carry out of word L-1
-    z[L] = (uint32_t)(((uint64_t)a[L - 1] * x) >> 32) + *fc;
+    p[0] = lo;
+    if (n > 1) p[1] = hi;
 }
 
-static size_t run_scan_phases(uint32_t* z, size_t n, uint32_t* agg, size_t nctas, uint32_t* final_carry,
-                              CarryMode mode, cudaStream_t s)
+void lin_set(uint32_t* p, uint32_t lo, uint32_t hi, int n, cudaStream_t s)
 {
-    carry_scan_aggregates(agg, nctas, final_carry, s);
-    carry_ripple(z, n, kLinWPC, agg, nctas, mode, s);
-    return nctas;
+    set_words_kernel<<<1, 1, 0, s>>>(p, lo, hi, n);
+    PIC_CHECK_LAUNCH();
+    count_launch();
+}
+
+static size_t lin_ctas(size_t n) { return (n + kLinWPC - 1) / kLinWPC; }
+
+static void lin_fix(uint32_t* z, size_t n, const uint32_t* agg, size_t nctas, const LinEnd& E, const uint32_t* a,
+                    uint32_t x, cudaStream_t s)
+{
+    if (nctas <= 1) return;
+    ProfScope ps(KC_CARRY, 4.0 * (double)nctas, s);
+    lin_fix_kernel<<<(unsigned)nctas, kLinThreads, 0, s>>>(z, n, agg, (uint32_t)nctas, E, a, x);
+    PIC_CHECK_LAUNCH();
+    count_launch();
+}
+
+static void addsub(uint32_t* z, size_t TL, const WordView& a, const WordView& b, int64_t bot, const LinEnd& E,
+                   cudaStream_t s)
+{
+    const size_t nctas = lin_ctas(TL);
+    DevBuf<uint32_t> agg(nctas, s);
+    ProfScope ps(KC_LINEAR, 12.0 * (double)TL, s);
+    addsub_k1<<<(unsigned)nctas, kLinThreads, 0, s>>>(z, TL, a, b, bot, agg.get(), E);
+    PIC_CHECK_LAUNCH();
+    count_launch();
+    lin_fix(z, TL, agg.get(), nctas, E, nullptr, 0, s);
 }
 
 void lin_addsub(uint32_t* z, size_t TL, const WordView& a, const WordView& b, int64_t bot, bool sub,
-                uint32_t* d_final, cudaStream_t s)
+                cudaStream_t s)
 {
-    if (TL == 0) {
-        PIC_CUDA(cudaMemsetAsync(d_final, 0, sizeof(uint32_t), s));
-        return;
-    }
-    const size_t nctas = (TL + kLinWPC - 1) / kLinWPC;
-    DevBuf<uint32_t> agg(nctas, s);
-    ProfScope ps(KC_LINEAR, 12.0 * (double)TL, s);
-    addsub_k1<<<(unsigned)nctas, kLinThreads, 0, s>>>(z, TL, a, b, bot, sub ? kCarrySub : kCarryAdd, agg.get());
-    PIC_CHECK_LAUNCH();
-    count_launch();
-    run_scan_phases(z, TL, agg.get(), nctas, d_final, sub ? kCarrySub : kCarryAdd, s);
+    if (TL == 0) return;
+    LinEnd E{};
+    E.kind = sub ? kLinSub : kLinAdd;
+    addsub(z, TL, a, b, bot, E, s);
 }
 
-void lin_mul_u32(uint32_t* z, const uint32_t* a, size_t L, uint32_t x, cudaStream_t s)
+// The words of ctx().scratch: kernels of the library's stream run one after
+// another, so one set serves them all.
+static uint32_t* scratch_ticket() { return ctx().scratch; }
+static int* scratch_order() { return reinterpret_cast<int*>(ctx().scratch + 1); }
+static unsigned long long* scratch_diff() { return reinterpret_cast<unsigned long long*>(ctx().scratch + 2); }
+
+uint32_t lin_add(uint32_t* z, size_t TL, const WordView& a, const WordView& b, int64_t bot)
 {
-    const size_t nctas = (L + kLinWPC - 1) / kLinWPC;
-    DevBuf<uint32_t> agg(nctas, s), fc(1, s);
-    ProfScope ps(KC_LINEAR, 8.0 * (double)L, s);
-    mulu32_k1<<<(unsigned)nctas, kLinThreads, 0, s>>>(z, a, L, x, agg.get());
-    PIC_CHECK_LAUNCH();
-    count_launch();
-    run_scan_phases(z, L, agg.get(), nctas, fc.get(), kCarryAdd, s);
-    mulu32_final_kernel<<<1, 1, 0, s>>>(z, a, L, x, fc.get());
-    PIC_CHECK_LAUNCH();
-    count_launch();
+    if (TL == 0) {
+        PIC_CUDA(cudaMemsetAsync(z, 0, sizeof(uint32_t), ctx().stream));
+        return 0;
+    }
+    Mail mail(ctx().stream);
+    LinEnd E{};
+    E.kind = kLinAdd;
+    E.carry_out = z + TL;
+    E.mail = mail.ref();
+    addsub(z, TL, a, b, bot, E, ctx().stream);
+    return (uint32_t)mail.wait();
+}
+
+uint32_t lin_mul_u32(uint32_t* z, const uint32_t* a, size_t L, uint32_t x)
+{
+    const cudaStream_t s = ctx().stream;
+    const size_t nctas = lin_ctas(L);
+    Mail mail(s);
+    DevBuf<uint32_t> agg(nctas, s);
+    LinEnd E{};
+    E.kind = kLinMul;
+    E.carry_out = z + L;
+    E.mail = mail.ref();
+    {
+        ProfScope ps(KC_LINEAR, 8.0 * (double)L, s);
+        mulu32_k1<<<(unsigned)nctas, kLinThreads, 0, s>>>(z, a, L, x, agg.get(), E);
+        PIC_CHECK_LAUNCH();
+        count_launch();
+        lin_fix(z, L, agg.get(), nctas, E, a, x, s);
+    }
+    return (uint32_t)mail.wait();
 }
 
 // ---- leading zeros / compare -------------------------------------------------
@@ -271,9 +326,12 @@ size_t lin_top_nonzero(const uint32_t* z, size_t n, cudaStream_t s)
     return (size_t)h[0] | ((size_t)h[1] << 32);
 }
 
-// Highest magnitude position where the two windows differ: atomicMax over
-// (mag - lo + 1); 0 when equal over [lo, hi).
-__global__ void ucmp_kernel(WordView a, WordView b, int64_t lo, int64_t hi, unsigned long long* out)
+// Highest magnitude position where the two windows differ (atomicMax over
+// mag - lo + 1, zero before and after); the last CTA compares the words there:
+// *order = 1, 0 or -1 as |a| >, =, < |b|, posted too.
+__global__ void __launch_bounds__(256) ucmp_kernel(WordView a, WordView b, int64_t lo, int64_t hi,
+                                                   unsigned long long* diff, uint32_t* ticket, int* order,
+                                                   MailRef mail)
 {
     const int64_t n = hi - lo;
     unsigned long long mine = 0;
@@ -282,32 +340,70 @@ __global__ void ucmp_kernel(WordView a, WordView b, int64_t lo, int64_t hi, unsi
         if (word_at(a.T, a.exp, a.L, mag) != word_at(b.T, b.exp, b.L, mag)) mine = (unsigned long long)(i + 1);
     }
     mine = warp_max_u64(mine);
-    if ((threadIdx.x & 31) == 0 && mine) atomicMax(out, mine);
+    if ((threadIdx.x & 31) == 0 && mine) atomicMax(diff, mine);
+    if (!last_cta(ticket, gridDim.x)) return;
+    if (threadIdx.x == 0) {
+        const unsigned long long r = __ldcg(diff);
+        int c = 0;
+        if (r) {
+            const int64_t mag = lo + (int64_t)r - 1;
+            c = word_at(a.T, a.exp, a.L, mag) < word_at(b.T, b.exp, b.L, mag) ? -1 : 1;
+        }
+        *diff = 0;
+        *order = c;
+        mail_post(mail, 0, (uint32_t)(c + 1));
+    }
 }
 
-int lin_ucmp(const WordView& a, const WordView& b, cudaStream_t s)
+// The comparison's launch on the library's stream (magnitudes equal).
+static void ucmp_launch(const WordView& a, const WordView& b, MailRef mail)
 {
-    // BigFloat::ucmp, BigFloat.cpp:123-147
-    const int64_t magA = a.exp + a.L, magB = b.exp + b.L;
-    if (magA > magB) return 1;
-    if (magA < magB) return -1;
-    const int64_t lo = a.exp < b.exp ? a.exp : b.exp;
-    const int64_t hi = magA;
-    if (hi <= lo) return 0;
-    DevBuf<unsigned long long> d(1, s);
-    PIC_CUDA(cudaMemsetAsync(d.get(), 0, sizeof(unsigned long long), s));
-    ucmp_kernel<<<grid_for((size_t)(hi - lo), 256), 256, 0, s>>>(a, b, lo, hi, d.get());
+    const int64_t lo = a.exp < b.exp ? a.exp : b.exp, hi = a.exp + a.L;
+    ucmp_kernel<<<grid_for((size_t)(hi - lo), 256), 256, 0, ctx().stream>>>(a, b, lo, hi, scratch_diff(),
+                                                                           scratch_ticket(), scratch_order(), mail);
     PIC_CHECK_LAUNCH();
     count_launch();
-    uint32_t h[2];
-    read_words(h, (const uint32_t*)d.get(), 2, s);
-    const unsigned long long r = (unsigned long long)h[0] | ((unsigned long long)h[1] << 32);
-    if (r == 0) return 0;
-    const int64_t mag = lo + (int64_t)r - 1;
-    uint32_t wa = 0, wb = 0;
-    if (mag >= a.exp && mag < a.exp + a.L) read_words(&wa, a.T + (mag - a.exp), 1, s);
-    if (mag >= b.exp && mag < b.exp + b.L) read_words(&wb, b.T + (mag - b.exp), 1, s);
-    return wa < wb ? -1 : 1;
+}
+
+int lin_ucmp(const WordView& a, const WordView& b, cudaStream_t)
+{
+    // BigFloat::ucmp, BigFloat.cpp:123-147
+    if (const int c = lin_mag_order(a, b)) return c;
+    if (a.exp + a.L <= (a.exp < b.exp ? a.exp : b.exp)) return 0;
+    Mail mail(ctx().stream);
+    {
+        std::lock_guard<std::recursive_mutex> pair(ctx().lock);
+        ucmp_launch(a, b, mail.ref());
+    }
+    uint32_t c;
+    mail.wait(&c);
+    return (int)c - 1;
+}
+
+size_t lin_diff(uint32_t* z, size_t TL, const WordView& a, const WordView& b, int64_t bot, int* order)
+{
+    const bool ask = *order == 0;
+    if (TL == 0) {
+        if (ask) *order = -1;
+        return 0;
+    }
+    Mail mail(ctx().stream);
+    LinEnd E{};
+    E.kind = kLinSub;
+    E.order = ask ? scratch_order() : nullptr;
+    E.diff = scratch_diff();
+    E.ticket = scratch_ticket();
+    E.mail = mail.ref();
+    {
+        // another thread's comparison may not come between this one and its use
+        std::lock_guard<std::recursive_mutex> pair(ctx().lock);
+        if (ask) ucmp_launch(a, b, MailRef{});
+        addsub(z, TL, *order >= 0 ? a : b, *order >= 0 ? b : a, bot, E, ctx().stream);
+    }
+    uint32_t greater;
+    const uint64_t nz = mail.wait(&greater);
+    if (ask) *order = greater ? 1 : -1;
+    return (size_t)nz;
 }
 
 }  // namespace pic

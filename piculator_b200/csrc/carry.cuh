@@ -9,13 +9,25 @@
 //     c_(i+1) = g_i | (p_i & c_i),   p_i = (d_i == all-ones)   [add]
 //     b_(i+1) = g_i | (p_i & b_i),   p_i = (d_i == 0)          [subtract]
 // which is associative, so it runs as a block scan inside each CTA plus a
-// reduce-then-scan across CTAs (no inter-CTA waiting, no spin loops):
+// second launch for the carries between CTAs (no inter-CTA waiting, no spin
+// loops):
 //   K1  raw digits -> in-block resolved words + one (G, P) per CTA
-//   K2  one CTA scans the per-CTA pairs -> carry-in per CTA + final carry
-//   K3  CTAs with carry-in 1 ripple it through their own words.
+//   K2  each CTA takes its carry-in from the aggregates below it and, if it is
+//       1, ripples it through its own words.
+// A chunk passes a carry on only when all its words are all-ones (zero), so
+// the aggregate just below decides almost always; where it does not, the CTA
+// scans all those below it.
+// Against a scan launch and a ripple launch (three in all): division and inverse
+// square root at 300,007 words 9.65 -> 4.17 ms together with the results posted
+// to the host (common.cuh) and the comparison of a difference left on the
+// device.  Doing K2 in the CTA of K1 that finishes last was slower (6.1 ms): its
+// fences, and the runs of all-ones words that a Newton step's x r ~ 1 leaves to
+// that one CTA.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include "common.cuh"
 
 namespace pic {
 
@@ -119,18 +131,68 @@ __device__ __forceinline__ unsigned long long block_min_u64(unsigned long long v
     return r;
 }
 
-enum CarryMode { kCarryAdd = 0, kCarrySub = 1 };
+// The last CTA of a launch: true in exactly one of `nctas` CTAs, after every
+// other one has arrived; what those wrote before is visible to it through
+// loads that bypass L1 (__ldcg).  *ticket is zero before the launch and after it.
+__device__ __forceinline__ bool last_cta(uint32_t* ticket, uint32_t nctas)
+{
+    __shared__ bool s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == nctas - 1;
+        if (s_last) {
+            *ticket = 0;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    return s_last;
+}
 
-// Cross-CTA phases (carry.cu).  agg[c] = (G, P) of CTA c; words_per_cta words
-// per CTA; K3 also needs the array length.
-void carry_scan_aggregates(uint32_t* agg, size_t nctas, uint32_t* final_carry, cudaStream_t s);
-void carry_ripple(uint32_t* z, size_t nwords, size_t words_per_cta, const uint32_t* agg_cin,
-                  size_t nctas, CarryMode mode, cudaStream_t s);
+// The carry into chunk c from the (G, P) of chunks 0 .. c - 1 (every thread
+// calls, the same result in each).
+__device__ __forceinline__ uint32_t chunk_carry_in(const uint32_t* __restrict__ agg, size_t c)
+{
+    if (c == 0) return 0;
+    const uint32_t below = agg[c - 1];
+    if (!(below & 2u)) return below & 1u;
+    const size_t per = (c + blockDim.x - 1) / blockDim.x;
+    const size_t b = threadIdx.x * per < c ? threadIdx.x * per : c, e = b + per < c ? b + per : c;
+    uint32_t acc = kGPIdentity;
+    for (size_t i = b; i < e; i++) acc = gp_combine(acc, agg[i]);
+    uint32_t total;
+    block_gp_scan(acc, &total);
+    return total & 1u;
+}
 
-// Segmented forms for batches of products: `count` segments of `cpp` CTAs;
-// product i writes zlen[i] words at z + i * zcap.
-void carry_scan_segments(uint32_t* agg, size_t count, size_t cpp, cudaStream_t s);
-void carry_ripple_batch(uint32_t* z, uint32_t zcap, const uint32_t* zlen, size_t words_per_cta,
-                        const uint32_t* agg_cin, size_t count, size_t cpp, cudaStream_t s);
+// A carry (borrow) of one into words z[b, e): passed on over words equal to
+// `stop` (which become ~stop) to the first that takes it.
+__device__ __forceinline__ void chunk_ripple(uint32_t* z, size_t b, size_t e, bool sub)
+{
+    const uint32_t stop = sub ? 0u : 0xffffffffu;
+    if (b >= e) return;
+    const uint32_t w = z[b];
+    if (w != stop) {  // the same for every thread: they have all read it
+        __syncthreads();
+        if (threadIdx.x == 0) z[b] = sub ? w - 1u : w + 1u;
+        return;
+    }
+    unsigned long long mine = ~0ull;
+    for (size_t i = b + threadIdx.x; i < e; i += blockDim.x)
+        if (z[i] != stop && i < mine) mine = i;
+    const size_t f = (size_t)block_min_u64(mine);
+    for (size_t i = b + threadIdx.x; i < e && i < f; i += blockDim.x) z[i] = ~stop;
+    if (threadIdx.x == 0 && f < e) z[f] += sub ? 0xffffffffu : 1u;
+}
+
+// K2 (carry.cu).  agg[c] = (G, P) of CTA c, which owns words_per_cta words.
+// mail: receives the top word z[nwords - 1].
+void carry_fix(uint32_t* z, size_t nwords, size_t words_per_cta, const uint32_t* agg, size_t nctas, cudaStream_t s,
+               MailRef mail = MailRef{});
+// For batches of products: `count` segments of `cpp` CTAs; product i writes
+// zlen[i] words at z + i * zcap.
+void carry_fix_batch(uint32_t* z, uint32_t zcap, const uint32_t* zlen, size_t words_per_cta, const uint32_t* agg,
+                     size_t count, size_t cpp, cudaStream_t s, bool sub = false);
 
 }  // namespace pic

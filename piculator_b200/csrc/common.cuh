@@ -49,6 +49,9 @@ struct Context {
     std::atomic<uint64_t> fft_recomputes{0};  // FFT products redone with the NTT
     uint32_t* pinned_words = nullptr;    // small pinned staging for metadata reads
     size_t pinned_words_cap = 0;
+    // Words on the device that kernels of the library's stream use one after the
+    // other (see carry.cuh): zero between kernels.
+    uint32_t* scratch = nullptr;
 };
 
 Context& ctx();
@@ -125,6 +128,41 @@ struct DevBuf {
 
 // Reads `count` words from device memory (stream-ordered, then synchronises).
 void read_words(uint32_t* host, const uint32_t* dev, size_t count, cudaStream_t s);
+
+// A result that a kernel hands to the host: one 8-byte store into pinned host
+// memory, a sequence number of 14 bits, two bits and a value of 48 bits, which
+// the host polls.  A BigFloat operation's length or carry arrives this way
+// without a copy and a stream synchronisation (about 9 us of an operation on
+// short numbers).
+struct MailRef {  // kernel argument; slot null: nothing to deliver
+    unsigned long long* slot = nullptr;
+    uint32_t seq = 0;
+};
+
+__device__ __forceinline__ void mail_post(const MailRef& m, uint64_t value, uint32_t bits = 0)
+{
+    if (m.slot != nullptr)
+        *reinterpret_cast<volatile unsigned long long*>(m.slot) =
+            ((uint64_t)m.seq << 50) | ((uint64_t)(bits & 3u) << 48) | (value & 0xffffffffffffull);
+}
+
+class Mail {
+public:
+    explicit Mail(cudaStream_t s);
+    ~Mail();  // a posted but unread mail is waited for before its slot is reused
+    Mail(const Mail&) = delete;
+    Mail& operator=(const Mail&) = delete;
+    MailRef ref();  // pass to the one kernel that posts
+    bool armed() const { return armed_; }
+    uint64_t wait(uint32_t* bits = nullptr);  // the value, once the kernel has posted it
+
+private:
+    cudaStream_t s_;
+    unsigned long long* slot_;
+    uint32_t seq_;
+    bool armed_ = false;
+    unsigned long long v_ = 0;
+};
 
 // ---- live kernel timing -------------------------------------------------------
 // When enabled (pic_profile_begin), each instrumented launch is bracketed by a

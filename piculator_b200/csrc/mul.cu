@@ -324,8 +324,7 @@ __global__ void __launch_bounds__(kCvtThreads) coefbits_k1(Loader ld, size_t nco
 // per CTA; the CRT conversions own kCrtLPC and ripple with kCrtWPC).
 static void finish_scan(uint32_t* z, size_t zw, uint32_t* agg, size_t nctas, cudaStream_t s)
 {
-    carry_scan_aggregates(agg, nctas, nullptr, s);
-    carry_ripple(z, zw, kCvtWPC, agg, nctas, kCarryAdd, s);
+    carry_fix(z, zw, kCvtWPC, agg, nctas, s);
 }
 
 void coef16_to_words(const uint64_t* c, size_t ncoef, uint64_t scale_mont, uint64_t p, uint64_t pinv_neg,
@@ -434,8 +433,7 @@ void ntt3_inverse_to_words(uint64_t* y, int k, size_t ncoef, int depth, uint32_t
     crt3_k1<<<(unsigned)nctas, kCvtThreads, 0, s>>>(y, (size_t)1 << k, ncoef, C, z, zw, agg.get());
     PIC_CHECK_LAUNCH();
     count_launch();
-    carry_scan_aggregates(agg.get(), nctas, nullptr, s);
-    carry_ripple(z, zw, kCrtWPC, agg.get(), nctas, kCarryAdd, s);
+    carry_fix(z, zw, kCrtWPC, agg.get(), nctas, s);
 }
 
 void ntt3_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, size_t count, int k, uint32_t* z,
@@ -456,8 +454,7 @@ void ntt3_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, size
         PIC_CHECK_LAUNCH();
         count_launch();
     }
-    carry_scan_segments(agg.get(), count, cpp, s);
-    carry_ripple_batch(z, zcap, zlen, kCrtWPC, agg.get(), count, cpp, s);
+    carry_fix_batch(z, zcap, zlen, kCrtWPC, agg.get(), count, cpp, s);
 }
 
 // Pieces used by the allocation-free product (noalloc.cu): the same split and
@@ -480,8 +477,7 @@ void crt3_to_words_scratch(const uint64_t* y, int k, size_t ncoef, uint32_t* z, 
     crt3_k1<<<(unsigned)nctas, kCvtThreads, 0, s>>>(y, (size_t)1 << k, ncoef, C, z, zw, agg);
     PIC_CHECK_LAUNCH();
     count_launch();
-    carry_scan_aggregates(agg, nctas, nullptr, s);
-    carry_ripple(z, zw, kCrtWPC, agg, nctas, kCarryAdd, s);
+    carry_fix(z, zw, kCrtWPC, agg, nctas, s);
 }
 
 // Wrapped products.  A product of operands of sa and sb pieces has
@@ -678,8 +674,7 @@ static void mul_ntt3_wrapped(uint32_t* z, const uint32_t* a, size_t na, const ui
     crt3_k1<<<(unsigned)nctas, kCvtThreads, 0, s>>>(A.get(), ST, L, C, z, zw, agg.get());
     PIC_CHECK_LAUNCH();
     count_launch();
-    carry_scan_aggregates(agg.get(), nctas, nullptr, s);
-    carry_ripple(z, zw, kCrtWPC, agg.get(), nctas, kCarryAdd, s);
+    carry_fix(z, zw, kCrtWPC, agg.get(), nctas, s);
 }
 
 void mul_ntt3(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s)
@@ -915,11 +910,15 @@ __device__ __forceinline__ void crt3d_block(const uint64_t* __restrict__ Y, size
     limbs_to_words<7>(dig, gen, 7 * (size_t)u, z, zw < zend ? zw : zend, agg_slot);
 }
 
+// A single CTA posts the top word; several leave their carries to carry_fix.
 __global__ void __launch_bounds__(kCrtDThreads) crt3d_k1(const uint64_t* __restrict__ Y, size_t pstride,
-                                                         size_t ncoef, CrtDConsts C, uint32_t* __restrict__ z,
-                                                         size_t zw, uint32_t* agg)
+                                                         size_t ncoef, CrtDConsts C, uint32_t* z, size_t zw,
+                                                         uint32_t* agg, MailRef mail)
 {
     crt3d_block(Y, pstride, ncoef, C, z, zw, (int64_t)blockIdx.x, agg + blockIdx.x);
+    if (mail.slot == nullptr) return;
+    __syncthreads();
+    if (threadIdx.x == 0) mail_post(mail, z[zw - 1]);
 }
 
 __global__ void __launch_bounds__(kCrtDThreads) crt3d_batch_k1(const uint64_t* __restrict__ Y, size_t istride,
@@ -936,19 +935,20 @@ __global__ void __launch_bounds__(kCrtDThreads) crt3d_batch_k1(const uint64_t* _
 static size_t crt3d_ctas(size_t zw) { return ((zw + 1) / 2 + kCrtDLPC - 1) / kCrtDLPC; }
 
 // Inverse-transformed residues (product length 2^k, prime q at y + q pstride)
-// -> zw words.
+// -> zw words; mail receives the top one.
 static void crt3d_to_words(const uint64_t* y, size_t pstride, int k, size_t ncoef, uint32_t* z, size_t zw,
-                           cudaStream_t s)
+                           Mail* mail, cudaStream_t s)
 {
     const CrtDConsts C = make_crtd(k, false);
     const size_t nctas = crt3d_ctas(zw);
     DevBuf<uint32_t> agg(nctas, s);
+    const MailRef m = mail ? mail->ref() : MailRef{};
     ProfScope ps(KC_CRT, 24.0 * (double)ncoef + 4.0 * (double)zw, s);
-    crt3d_k1<<<(unsigned)nctas, kCrtDThreads, 0, s>>>(y, pstride, ncoef, C, z, zw, agg.get());
+    crt3d_k1<<<(unsigned)nctas, kCrtDThreads, 0, s>>>(y, pstride, ncoef, C, z, zw, agg.get(),
+                                                     nctas == 1 ? m : MailRef{});
     PIC_CHECK_LAUNCH();
     count_launch();
-    carry_scan_aggregates(agg.get(), nctas, nullptr, s);
-    carry_ripple(z, zw, kCrtDWPC, agg.get(), nctas, kCarryAdd, s);
+    if (nctas > 1) carry_fix(z, zw, kCrtDWPC, agg.get(), nctas, s, m);
 }
 
 void ntt3d_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, size_t count, int k, uint32_t* z,
@@ -967,8 +967,7 @@ void ntt3d_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, siz
         PIC_CHECK_LAUNCH();
         count_launch();
     }
-    carry_scan_segments(agg.get(), count, cpp, s);
-    carry_ripple_batch(z, zcap, zlen, kCrtDWPC, agg.get(), count, cpp, s);
+    carry_fix_batch(z, zcap, zlen, kCrtDWPC, agg.get(), count, cpp, s);
 }
 
 // The wrapped form's fix-up (see wrap_fix_kernel) on FP64 residues:
@@ -1060,7 +1059,7 @@ static void ntt3d_product(uint64_t* out, size_t stride, int k, const uint32_t* a
 // The wrapped form (see wrap_fix_kernel): main transforms of length 2^km, tails
 // of length 2^kt over the top W pieces.
 static void mul_ntt3d_wrapped(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, int km,
-                              int kt, cudaStream_t s)
+                              int kt, Mail* mail, cudaStream_t s)
 {
     const size_t zw = na + nb;
     const size_t pa = pieces56(na), pb = pieces56(nb);
@@ -1078,12 +1077,12 @@ static void mul_ntt3d_wrapped(uint32_t* z, const uint32_t* a, size_t na, const u
         launch_wrap_fix_d(A.get(), ST, tA.get(), T, 1, 1, 1, Nm, W, s);
         count_launch();
     }
-    crt3d_to_words(A.get(), ST, km, L, z, zw, s);
+    crt3d_to_words(A.get(), ST, km, L, z, zw, mail, s);
 }
 
 // The FP64 form of mul_ntt3 (PIC_MUL_NTT3D): products whose shorter operand
 // has more than 2^28 pieces go to the integer form.
-void mul_ntt3d(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s)
+void mul_ntt3d(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s, Mail* mail)
 {
     if (is_held(a, na) && !(a == b && na == nb)) {  // the held operand goes second
         std::swap(a, b);
@@ -1107,7 +1106,7 @@ void mul_ntt3d(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, siz
             int kt = ceil_log2(2 * W - 1);
             if (kt < kDblMinBits) kt = kDblMinBits;
             if (((size_t)1 << kt) <= Nm / 2) {
-                mul_ntt3d_wrapped(z, a, na, b, nb, k - 1, kt, s);
+                mul_ntt3d_wrapped(z, a, na, b, nb, k - 1, kt, mail, s);
                 return;
             }
         }
@@ -1117,7 +1116,7 @@ void mul_ntt3d(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, siz
     uint64_t* spec = is_held(b, nb) ? held_spectrum(k, &ready, s) : nullptr;
     DevBuf<uint64_t> A(3 * N, s);
     ntt3d_product(A.get(), N, k, a, na, 0, b, nb, 0, square, spec, ready, s);
-    crt3d_to_words(A.get(), N, k, ncoef, z, zw, s);
+    crt3d_to_words(A.get(), N, k, ncoef, z, zw, mail, s);
 }
 
 void mul_ntt_ref(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s)
@@ -1162,7 +1161,8 @@ constexpr int kSchThreads = 256;
 constexpr int kSchWPT = (int)(kSchoolMaxWords / kSchThreads);
 
 __global__ void __launch_bounds__(kSchThreads) school_kernel(uint32_t* __restrict__ z, const uint32_t* __restrict__ a,
-                                                             uint32_t na, const uint32_t* __restrict__ b, uint32_t nb)
+                                                             uint32_t na, const uint32_t* __restrict__ b, uint32_t nb,
+                                                             MailRef mail)
 {
     extern __shared__ uint32_t sm[];
     uint32_t* sa = sm;
@@ -1215,18 +1215,19 @@ __global__ void __launch_bounds__(kSchThreads) school_kernel(uint32_t* __restric
     for (int u = 0; u < kSchWPT; u++) {
         const uint32_t w = w0 + u;
         if (w < zw) z[w] = d[u] + cin;
+        if (w + 1 == zw) mail_post(mail, d[u] + cin);  // the top word
         cin = gg[u] | ((uint32_t)(d[u] == 0xffffffffu) & cin);
     }
 }
 
-void mul_school(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s)
+void mul_school(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s, Mail* mail)
 {
     PIC_REQUIRE(na + nb <= kSchoolMaxWords, PIC_ERR_INVALID, "schoolbook product too long");
     const size_t smem = (na + nb) * 4 + (na + nb) * 12;
     if (smem > 48 * 1024)
         PIC_CUDA(cudaFuncSetAttribute(school_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     ProfScope ps(KC_SCHOOL, 4.0 * (double)(2 * (na + nb)), s);
-    school_kernel<<<1, kSchThreads, smem, s>>>(z, a, (uint32_t)na, b, (uint32_t)nb);
+    school_kernel<<<1, kSchThreads, smem, s>>>(z, a, (uint32_t)na, b, (uint32_t)nb, mail ? mail->ref() : MailRef{});
     PIC_CHECK_LAUNCH();
     count_launch();
 }
@@ -1335,7 +1336,7 @@ void mul_set_fft_accept(double max_dist) { g_fft_accept = max_dist; }
 double mul_fft_accept() { return g_fft_accept; }
 
 void mul_dispatch(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, int mode,
-                  cudaStream_t s)
+                  cudaStream_t s, Mail* mail)
 {
     PIC_REQUIRE(na > 0 && nb > 0, PIC_ERR_INVALID, "empty operand");
     if (mode == PIC_MUL_AUTO) mode = mul_auto_mode(na, nb);
@@ -1343,14 +1344,14 @@ void mul_dispatch(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, 
     switch (mode) {
     case PIC_MUL_SCHOOL:
         if (na + nb <= kSchoolMaxWords) {
-            mul_school(z, a, na, b, nb, s);
+            mul_school(z, a, na, b, nb, s, mail);
             return;
         }
         mul_ntt3(z, a, na, b, nb, s);
         return;
     case PIC_MUL_NTT_REF: mul_ntt_ref(z, a, na, b, nb, s); return;
     case PIC_MUL_NTT3: mul_ntt3(z, a, na, b, nb, s); return;
-    case PIC_MUL_NTT3D: mul_ntt3d(z, a, na, b, nb, s); return;
+    case PIC_MUL_NTT3D: mul_ntt3d(z, a, na, b, nb, s, mail); return;
     case PIC_MUL_FFT: {
         double e = 0;
         if (!mul_fft(z, a, na, b, nb, s, &e) || e > g_fft_accept) {

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common.cuh"
 #include "ntt.cuh"
 #include "piculator_b200.h"
 
@@ -12,7 +13,8 @@ namespace pic {
 // Three-prime NTT: 64-bit pieces, primes kProductPrimes, Garner CRT.
 void mul_ntt3(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s);
 // The same in FP64 arithmetic: 56-bit pieces, primes kDblPrimes (fp64mod.cuh).
-void mul_ntt3d(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s);
+void mul_ntt3d(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s,
+               Mail* mail = nullptr);
 // 56-bit pieces of an operand of n words.
 size_t pieces56(size_t nwords);
 // FP64-form building blocks: batched inverse output like ntt3_batch_to_words
@@ -51,7 +53,8 @@ uint64_t held_transform_reuses();
 void mul_ntt_ref(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s);
 // One CTA per product, column sums in shared memory (na + nb <= kSchoolMax).
 constexpr size_t kSchoolMaxWords = 4096;
-void mul_school(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s);
+void mul_school(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s,
+                Mail* mail = nullptr);
 // FP64 FFT product; returns false (and leaves z undefined) when the largest
 // rounding distance exceeded 0.25, so the caller can recompute exactly.
 bool mul_fft(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s,
@@ -102,9 +105,11 @@ size_t crt3_scratch_ctas(size_t zw);
 void crt3_to_words_scratch(const uint64_t* y, int k, size_t ncoef, uint32_t* z, size_t zw, uint32_t* agg,
                            cudaStream_t s);
 
-// Dispatch on mode (PIC_MUL_*).
+// Dispatch on mode (PIC_MUL_*).  mail: the schoolbook and FP64 forms post the
+// product's top word to it where one kernel resolves the carries (mail->armed()
+// afterwards tells).
 void mul_dispatch(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, int mode,
-                  cudaStream_t s);
+                  cudaStream_t s, Mail* mail = nullptr);
 int mul_auto_mode(size_t na, size_t nb);
 void mul_set_thresholds(int64_t school_max, int64_t fft_max);
 int64_t mul_school_max();

@@ -3,6 +3,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <map>
 #include <tuple>
 #include <vector>
@@ -1333,11 +1334,13 @@ static bool launch_cols_fast(const NttBatch& b, int k, int lpre, int lc, int lw,
 // g_cols_bulk: 0 off, else log2 of the largest tile (points) the kernel
 // takes; tiles are narrowed to it so that more CTAs share an SM.
 static int g_cols_bulk = 0;
+static std::atomic<bool> g_bulk_ran{false};  // since the last ntt_take_bulk_error
 void ntt_set_cols_bulk(int bits) { g_cols_bulk = bits; }
 int ntt_cols_bulk() { return g_cols_bulk; }
 
 bool ntt_take_bulk_error()
 {
+    if (!g_bulk_ran.exchange(false)) return false;
     int e = 0, zero = 0;
     PIC_CUDA(cudaMemcpyFromSymbol(&e, g_ntt_bulk_error, sizeof e));
     if (e) PIC_CUDA(cudaMemcpyToSymbol(g_ntt_bulk_error, &zero, sizeof zero));
@@ -1354,6 +1357,7 @@ static bool launch_cols_bulk_tab(const NttBatch& b, int k, int lpre, const PassT
     PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
     if (per_sm < 1) return false;
     const size_t grid = std::min(ntiles, (size_t)ctx().num_sms * (size_t)per_sm);
+    g_bulk_ran.store(true);
     kern<<<(unsigned)grid, 256, smem, s>>>(b, k, lpre, pt, ntiles);
     return true;
 }

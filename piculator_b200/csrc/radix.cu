@@ -115,19 +115,13 @@ __global__ void __launch_bounds__(kDecThreads) dec_sub_k1(uint32_t* __restrict__
     if (threadIdx.x == 0) agg[blockIdx.x] = total;
 }
 
-// K3: CTAs with a borrow in subtract it from their own words.
-__global__ void dec_sub_ripple(uint32_t* r, size_t r_stride, size_t n, size_t cpi, const uint32_t* bin)
+// K2: CTAs with a borrow in subtract it from their own words.
+__global__ void __launch_bounds__(256) dec_sub_fix(uint32_t* r, size_t r_stride, size_t n, size_t cpi,
+                                                   const uint32_t* __restrict__ agg)
 {
-    if (bin[blockIdx.x] == 0) return;
     const size_t it = blockIdx.x / cpi, c = blockIdx.x - it * cpi;
-    uint32_t* z = r + it * r_stride;
     const size_t b = c * kDecWPC, e = b + kDecWPC < n ? b + kDecWPC : n;
-    unsigned long long mine = ~0ull;
-    for (size_t i = b + threadIdx.x; i < e; i += blockDim.x)
-        if (z[i] != 0u && i < mine) mine = i;
-    const size_t f = (size_t)block_min_u64(mine);
-    for (size_t i = b + threadIdx.x; i < e && i < f; i += blockDim.x) z[i] = 0xffffffffu;
-    if (threadIdx.x == 0 && f < e) z[f] -= 1u;
+    if (chunk_carry_in(agg + it * cpi, c)) chunk_ripple(r + it * r_stride, b, e, true);
 }
 
 static void dec_sub(uint32_t* r, size_t r_stride, const uint32_t* a, size_t a_stride, const uint32_t* b,
@@ -139,10 +133,11 @@ static void dec_sub(uint32_t* r, size_t r_stride, const uint32_t* a, size_t a_st
     dec_sub_k1<<<(unsigned)(count * cpi), kDecThreads, 0, s>>>(r, r_stride, a, a_stride, b, b_stride, b_words, n,
                                                               cpi, agg.get());
     PIC_CHECK_LAUNCH();
-    carry_scan_segments(agg.get(), count, cpi, s);
-    dec_sub_ripple<<<(unsigned)(count * cpi), 256, 0, s>>>(r, r_stride, n, cpi, agg.get());
+    count_launch();
+    if (cpi == 1) return;
+    dec_sub_fix<<<(unsigned)(count * cpi), 256, 0, s>>>(r, r_stride, n, cpi, agg.get());
     PIC_CHECK_LAUNCH();
-    count_launch(2);
+    count_launch();
 }
 
 // hi[i] = 1 + the highest word index where item i of x differs from t (0:
@@ -288,9 +283,7 @@ Divisor make_divisor(Nat T, cudaStream_t s)
     d.V.L = vw;
     d.V.st = alloc_words(vw);
     const BigFloat two(2u);
-    DevBuf<uint32_t> fin(1, s);
-    lin_addsub(d.V.st->base, vw, WordView{v.st->base, 0, (int64_t)vw}, WordView{two.device_words(), 0, 1}, 0, true,
-               fin.get(), s);
+    lin_addsub(d.V.st->base, vw, WordView{v.st->base, 0, (int64_t)vw}, WordView{two.device_words(), 0, 1}, 0, true, s);
     return d;
 }
 
@@ -379,9 +372,8 @@ void dec_digits(const BigFloat& x, size_t groups, char* d_out)
             DevBuf<unsigned long long> hi(count, s);
             DevBuf<uint8_t> ge(count, s);
             DevBuf<unsigned int> nge(1, s);
-            DevBuf<uint32_t> fin(1, s), d1(1, s);
-            const uint32_t one = 1;
-            PIC_CUDA(cudaMemcpyAsync(d1.get(), &one, 4, cudaMemcpyHostToDevice, s));
+            DevBuf<uint32_t> d1(1, s);
+            lin_set(d1.get(), 1, 0, 1, s);
             for (int round = 0;; round++) {
                 PIC_CUDA(cudaMemsetAsync(hi.get(), 0, 8 * count, s));
                 PIC_CUDA(cudaMemsetAsync(nge.get(), 0, 4, s));
@@ -403,9 +395,8 @@ void dec_digits(const BigFloat& x, size_t groups, char* d_out)
                     uint32_t* q = nxt.get() + 2 * i * ccap;
                     uint32_t* r = q + ccap;
                     lin_addsub(r, ccap, WordView{r, 0, (int64_t)ccap}, WordView{dv.T.w(), 0, (int64_t)tw}, 0, true,
-                               fin.get(), s);
-                    lin_addsub(q, ccap, WordView{q, 0, (int64_t)ccap}, WordView{d1.get(), 0, 1}, 0, false, fin.get(),
                                s);
+                    lin_addsub(q, ccap, WordView{q, 0, (int64_t)ccap}, WordView{d1.get(), 0, 1}, 0, false, s);
                 }
             }
         }

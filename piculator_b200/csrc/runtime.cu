@@ -5,6 +5,7 @@
 #include <stdlib.h>
 
 #include <chrono>
+#include <condition_variable>
 #include <mutex>
 #include <vector>
 
@@ -37,6 +38,80 @@ void require_init()
 
 cudaStream_t resolve(pic_stream s) { return s ? (cudaStream_t)s : g_ctx.stream; }
 
+namespace {
+constexpr size_t kScratchWords = 16;
+// Mail slots, handed out one per Mail; a thread that finds none free waits for
+// another thread's operation to end.
+constexpr int kMailSlots = 64;
+unsigned long long* g_mail = nullptr;
+std::vector<unsigned long long*> g_mail_free;
+std::mutex g_mail_lock;
+std::condition_variable g_mail_cv;
+
+void mail_init()
+{
+    std::lock_guard<std::mutex> g(g_mail_lock);
+    PIC_CUDA(cudaMallocHost((void**)&g_mail, kMailSlots * sizeof(unsigned long long)));
+    memset(g_mail, 0, kMailSlots * sizeof(unsigned long long));
+    g_mail_free.clear();
+    for (int i = 0; i < kMailSlots; i++) g_mail_free.push_back(g_mail + i);
+}
+
+void mail_shutdown()
+{
+    std::lock_guard<std::mutex> g(g_mail_lock);
+    if (g_mail) cudaFreeHost(g_mail);
+    g_mail = nullptr;
+    g_mail_free.clear();
+}
+}  // namespace
+
+Mail::Mail(cudaStream_t s) : s_(s)
+{
+    std::unique_lock<std::mutex> g(g_mail_lock);
+    g_mail_cv.wait(g, [] { return !g_mail_free.empty(); });
+    slot_ = g_mail_free.back();
+    g_mail_free.pop_back();
+    seq_ = (uint32_t)((*slot_ >> 50) + 1) & 0x3fffu;
+}
+
+Mail::~Mail()
+{
+    if (armed_) cudaStreamSynchronize(s_);
+    {
+        std::lock_guard<std::mutex> g(g_mail_lock);
+        g_mail_free.push_back(slot_);
+    }
+    g_mail_cv.notify_one();
+}
+
+MailRef Mail::ref()
+{
+    armed_ = true;
+    MailRef r;
+    r.slot = slot_;
+    r.seq = seq_;
+    return r;
+}
+
+uint64_t Mail::wait(uint32_t* bits)
+{
+    if (armed_) {
+        const volatile unsigned long long* p = slot_;
+        for (uint32_t n = 1; (v_ = *p) >> 50 != seq_; n++) {
+            if (n % 4096) continue;
+            const cudaError_t e = cudaStreamQuery(s_);
+            if (e == cudaErrorNotReady) continue;
+            PIC_CUDA(e);
+            if (*p >> 50 != seq_) throw Error(PIC_ERR_CUDA, "a kernel ended without its result");
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);
+        armed_ = false;
+    }
+    if (bits) *bits = (uint32_t)(v_ >> 48) & 3u;
+    return v_ & 0xffffffffffffull;
+}
+
 void init_context(int device)
 {
     std::lock_guard<std::recursive_mutex> g(g_ctx.lock);
@@ -68,6 +143,9 @@ void init_context(int device)
     PIC_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowOpportunistic, &no));
     g_ctx.pinned_words_cap = 1 << 16;
     PIC_CUDA(cudaMallocHost((void**)&g_ctx.pinned_words, g_ctx.pinned_words_cap * sizeof(uint32_t)));
+    PIC_CUDA(cudaMalloc((void**)&g_ctx.scratch, kScratchWords * sizeof(uint32_t)));
+    PIC_CUDA(cudaMemset(g_ctx.scratch, 0, kScratchWords * sizeof(uint32_t)));
+    mail_init();
     g_init.store(true);
 }
 
@@ -83,6 +161,9 @@ void shutdown_context()
     if (cudaDeviceGetDefaultMemPool(&pool, g_ctx.device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
     if (g_ctx.pinned_words) cudaFreeHost(g_ctx.pinned_words);
     g_ctx.pinned_words = nullptr;
+    if (g_ctx.scratch) cudaFree(g_ctx.scratch);
+    g_ctx.scratch = nullptr;
+    mail_shutdown();
     cudaStreamDestroy(g_ctx.stream);
     g_ctx.stream = nullptr;
     g_init.store(false);

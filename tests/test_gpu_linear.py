@@ -1,0 +1,82 @@
+"""BigFloat's linear operations at the edges of their kernels: a CTA owns 2048
+words and takes its carry-in from the aggregates below it, so numbers of one
+CTA, of a word more, and of many CTAs, with carries and borrows that run
+through all of them, against Python integers; and the comparison that orders a
+subtraction, from several threads at once."""
+from __future__ import annotations
+
+import threading
+
+import numpy as np
+import pytest
+
+from oracle.ffi import random_words
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1, 2, 2047, 2048, 2049, 4096, 6149, 300_001, 2_200_003]
+
+
+def _num(pic, words, sign=True):
+    return pic.DeviceBigFloat.from_words(sign, 0, np.ascontiguousarray(words, dtype=np.uint32))
+
+
+def _int(x):
+    bf = x.to_bf()
+    assert bf.words.size == 0 or bf.words[-1] != 0
+    v = int.from_bytes(bf.words.astype("<u4").tobytes(), "little") << (32 * bf.exp)
+    return v if bf.sign else -v
+
+
+def _val(words):
+    return int.from_bytes(np.ascontiguousarray(words, dtype="<u4").tobytes(), "little")
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_long_carries_and_borrows(pic, n):
+    ones = np.full(n, 0xFFFFFFFF, dtype=np.uint32)
+    power = np.zeros(n + 1, dtype=np.uint32)
+    power[n] = 1
+    one = pic.DeviceBigFloat.from_u32(1)
+    assert _int(_num(pic, ones).add(one)) == _val(ones) + 1          # a carry through every word
+    assert _int(_num(pic, power).sub(one)) == _val(power) - 1        # a borrow through every word
+    assert _int(one.sub(_num(pic, power))) == 1 - _val(power)
+    assert _int(_num(pic, ones).mul_u32(0xFFFFFFFF)) == _val(ones) * 0xFFFFFFFF
+    mid = np.zeros(n + 1, dtype=np.uint32)                           # the borrow clears the only word
+    mid[n] = 1
+    low = np.zeros(n + 1, dtype=np.uint32)
+    low[n], low[0] = 1, 1
+    assert _int(_num(pic, low).sub(_num(pic, mid))) == 1
+    assert _int(_num(pic, mid).sub(_num(pic, low))) == -1
+    assert _num(pic, low).sub(_num(pic, low)).info()[2] == 0
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_random_sums_and_differences(pic, n):
+    a, b = random_words(n, n), random_words(n + 7, n)
+    a[-1] |= 1
+    b[-1] = a[-1]  # equal top words: the comparison needs words further down
+    x, y = _num(pic, a), _num(pic, b)
+    assert _int(x.add(y)) == _val(a) + _val(b)
+    assert _int(x.sub(y)) == _val(a) - _val(b)
+    assert _int(y.sub(x)) == _val(b) - _val(a)
+    assert _int(x.add(_num(pic, b, sign=False))) == _val(a) - _val(b)
+    assert x.ucmp(y) == (_val(a) > _val(b)) - (_val(a) < _val(b))
+
+
+def test_ordered_differences_from_several_threads(pic):
+    def work(seed, bad):
+        a, b = random_words(seed, 5000), random_words(seed + 1, 5000)
+        a[-1] = b[-1] = 9
+        x, y = _num(pic, a), _num(pic, b)
+        for _ in range(40):
+            if _int(x.sub(y)) != _val(a) - _val(b) or _int(y.sub(x)) != _val(b) - _val(a):
+                bad.append(seed)
+
+    bad: list[int] = []
+    threads = [threading.Thread(target=work, args=(100 + 2 * i, bad)) for i in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
