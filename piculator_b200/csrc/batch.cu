@@ -6,6 +6,8 @@
 //   * products of at most kSchoolMaxWords words go to one persistent
 //     schoolbook launch: a grid of at most 148 x 8 CTAs pulls product indices
 //     from an atomic counter (longest first) until the list is exhausted;
+//   * products of the FP64 form with at most 2^13 coefficients go to one launch
+//     per transform length (small.cu), a cluster of three CTAs per product;
 //   * the rest are binned by transform length 2^k (three-prime NTT, 64-bit
 //     pieces); each bin is one batched split, forward, pointwise, inverse and
 //     CRT sequence for all its products, then a scatter to their outputs.
@@ -26,13 +28,6 @@
 #include "ntt.cuh"
 
 namespace pic {
-
-struct DevDesc {
-    uint32_t* z;
-    const uint32_t* a;
-    const uint32_t* b;
-    uint32_t na, nb;
-};
 
 // ---- persistent schoolbook ------------------------------------------------------
 constexpr int kPSchThreads = 256;
@@ -156,6 +151,7 @@ __global__ void bin_scatter_kernel(const uint32_t* __restrict__ zt, uint32_t zca
 namespace {
 struct Bin {
     int k;
+    bool small = false;  // FP64 form, one launch
     uint32_t zcap;
     std::vector<uint32_t> idx;  // descriptor indices
     DevBuf<uint32_t> didx;
@@ -187,12 +183,21 @@ bool g_use_graphs = true;
 
 void mul_batch_set_graphs(bool on) { g_use_graphs = on; }
 
+constexpr int kSmallClass = 64;
+
 static int batch_class(const pic_mul_desc& d, int mode)
 {
-    // -1: persistent schoolbook; k >= 1: three-prime NTT bin of length 2^k
+    // -1: persistent schoolbook; k >= 1: three-prime NTT bin of length 2^k, or
+    // kSmallClass + k: short products of the FP64 form
     const size_t zw = d.na + d.nb;
     int m = mode == PIC_MUL_AUTO ? mul_auto_mode(d.na, d.nb) : mode;
     if (m == PIC_MUL_SCHOOL && zw <= kSchoolMaxWords) return -1;
+    if (m == PIC_MUL_NTT3D) {
+        const size_t nc = pieces56(d.na) + pieces56(d.nb) - 1;
+        int ks = kSmallMinBits;
+        while (((size_t)1 << ks) < nc) ks++;
+        if (ks <= kSmallMaxBits) return kSmallClass + ks;
+    }
     const size_t ncoef = (d.na + 1) / 2 + (d.nb + 1) / 2 - 1;
     int k = 1;
     while (((size_t)1 << k) < ncoef) k++;
@@ -215,6 +220,10 @@ static void enqueue_plan(Plan& P, cudaStream_t s)
     }
     for (Bin& B : P.bins) {
         const size_t m = B.idx.size();
+        if (B.small) {
+            mul_small_batch(P.desc.get(), B.didx.get(), m, B.k, s);
+            continue;
+        }
         const size_t N = (size_t)1 << B.k;
         DevBuf<uint64_t> A(3 * m * N, s), Bb(3 * m * N, s);
         DevBuf<uint32_t> zt(m * (size_t)B.zcap, s), zl(m, s);
@@ -266,7 +275,8 @@ static std::unique_ptr<Plan> build_plan(const pic_mul_desc* d, size_t count, int
             P->school_max_zw = std::max<uint32_t>(P->school_max_zw, (uint32_t)(d[i].na + d[i].nb));
         } else {
             Bin& B = bins[c];
-            B.k = c;
+            B.small = c >= kSmallClass;
+            B.k = B.small ? c - kSmallClass : c;
             B.zcap = std::max<uint32_t>(B.zcap, (uint32_t)(d[i].na + d[i].nb));
             B.idx.push_back((uint32_t)i);
         }
@@ -284,7 +294,10 @@ static std::unique_ptr<Plan> build_plan(const pic_mul_desc* d, size_t count, int
         PIC_CUDA(cudaMemcpyAsync(B.didx.get(), B.idx.data(), 4 * B.idx.size(), cudaMemcpyHostToDevice, s));
         P->bins.push_back(std::move(B));
     }
-    for (int q = 0; q < 3; q++) prime_tables(kProductPrimes[q]);  // tables exist before any capture
+    for (int q = 0; q < 3; q++) {  // tables exist before any capture
+        prime_tables(kProductPrimes[q]);
+        dbl_prime_tables(kDblPrimes[q]);
+    }
     PIC_CUDA(cudaStreamSynchronize(s));
     return P;
 }

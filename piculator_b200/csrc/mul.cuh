@@ -17,6 +17,18 @@ void mul_ntt3d(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, siz
                Mail* mail = nullptr);
 // 56-bit pieces of an operand of n words.
 size_t pieces56(size_t nwords);
+// Short products of the FP64 form, one launch each or one for a batch of them
+// (small.cu): at most 2^kSmallMaxBits coefficients.
+constexpr int kSmallMinBits = 8, kSmallMaxBits = 13;
+struct DevDesc {
+    uint32_t* z;
+    const uint32_t* a;
+    const uint32_t* b;
+    uint32_t na, nb;
+};
+void mul_small(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s, Mail* mail);
+// Products d[idx[i]], i < count, of at most 2^k coefficients.
+void mul_small_batch(const DevDesc* d, const uint32_t* idx, size_t count, int k, cudaStream_t s);
 // FP64-form building blocks: batched inverse output like ntt3_batch_to_words
 // (offset 2^140 per coefficient); wrapped-product fix-up like launch_wrap_fix.
 void ntt3d_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, size_t count, int k, uint32_t* z,

@@ -201,3 +201,16 @@ def test_fused_product_lengths_match_integer_form(pic, torch_cuda, na, nb):
             pic.mul_dev(out.data_ptr(), x.data_ptr(), x.numel(), y.data_ptr(), y.numel(), mode)
         pic.synchronize()
         assert torch.equal(z[0], z[1])
+
+
+@pytest.mark.parametrize("na,nb", [(1, 1), (223, 224), (224, 225), (448, 449), (447, 449), (896, 896), (897, 898),
+                                   (3584, 3584), (3585, 3585), (7168, 7168), (7169, 7168), (14000, 336),
+                                   (14320, 16)])
+def test_one_launch_products(pic, oracle, na, nb):
+    """Products of up to 2^13 coefficients in one launch, at the lengths where
+    the transform doubles and the three CTAs' thirds are uneven, with random
+    and all-ones operands (carries through the CTAs' borders)."""
+    a, b = random_words(na, na), random_words(nb + 3, nb)
+    assert _int(pic.mul_host(a, b, "ntt3d")) == _int(a) * _int(b)
+    a[:], b[:] = 0xFFFFFFFF, 0xFFFFFFFF
+    assert _int(pic.mul_host(a, b, "ntt3d")) == _int(a) * _int(b)
