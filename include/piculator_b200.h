@@ -311,8 +311,8 @@ enum {
                                      0 integer (PIC_MUL_NTT3), 1 FP64 (PIC_MUL_NTT3D), 2 chosen per
                                      product (or merge level) by the transform work of the two forms */
     PIC_TUNE_DBL_PASS_TABLES = 11, /* FP64 column passes over blocks of at most 2^value points (0..24,
-                                     default 20) stream per-point twiddle tables; longer blocks form the
-                                     twiddles from the two-level tables */
+                                     default 20) read their twiddles from tables; longer blocks form them
+                                     from the two-level tables */
     PIC_TUNE_COLS_BULK = 12       /* 8..12: FP64 column passes of 2^5 .. 2^9 rows run the persistent
                                      kernel whose tiles (at most 2^value points) arrive by TMA bulk
                                      copies (bounded waits: a wait past ~1 s of SM clocks ends the pass

@@ -68,15 +68,19 @@ __device__ __forceinline__ double dreduce(double s, double p, double pinv)
 // The representative in [0, p) of a residue with |x| < p.
 __device__ __forceinline__ double dcanon(double x, double p) { return x < 0.0 ? __dadd_rn(x, p) : x; }
 
-// A 56-bit piece v (< 2^56) as a residue, |result| <= p / 2 + 2^28:
-// v = H 2^28 + L; H 2^28 and L are built exactly from their bits
-// (2^80 + H 2^28 and 2^52 + L are doubles whose mantissas hold H and L).
-__device__ __forceinline__ double dpiece56(uint64_t v, double p, double pinv)
+// A 56-bit piece H 2^28 + L as a residue, |result| <= p / 2 + 2^28: H 2^28 and
+// L are built exactly from their bits (2^80 + H 2^28 and 2^52 + L are doubles
+// whose mantissas hold H and L).
+__device__ __forceinline__ double dpiece28(uint32_t H, uint32_t L, double p, double pinv)
 {
-    const uint32_t H = (uint32_t)(v >> 28), L = (uint32_t)v & 0x0fffffffu;
     const double h = __dadd_rn(__hiloint2double(0x44f00000, (int)H), -1208925819614629174706176.0);  // - 2^80
     const double l = __dadd_rn(__hiloint2double(0x43300000, (int)L), -4503599627370496.0);          // - 2^52
     return __dadd_rn(dreduce(h, p, pinv), l);
+}
+
+__device__ __forceinline__ double dpiece56(uint64_t v, double p, double pinv)
+{
+    return dpiece28((uint32_t)(v >> 28), (uint32_t)v & 0x0fffffffu, p, pinv);
 }
 
 // Piece J of a word array x[0 .. n) in 56-bit pieces: bits 56 J .. 56 J + 55

@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
             const int base = (g & ((1 << LG) - 1)) << B;
             auto load = [&](int a, double(&x)[E]) {  // NR 1: the only round
 #pragma unroll
-                for (int m = 0; m < E; m++) x[m] = Sh::NR == 1 ? in(a, t, base + m) : ms[a * TOT + (pb ^ place(m))];
+                for (int m = 0; m < E; m++) x[m] = Sh::NR == 1 ? in(a, t, base + m) : ms[a * TOT + place_at(pb, m)];
                 fwd_group<B, 0>(x, wf, L);
             };
             auto store = [&](int a, double(&x)[E]) {
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
 #pragma unroll
                 for (int m = 0; m < E; m++) {
                     if constexpr (Sh::NR == 1) put(a, t, base + m, x[m]);
-                    else ms[a * TOT + (pb ^ place(m))] = x[m];
+                    else ms[a * TOT + place_at(pb, m)] = x[m];
                 }
             };
             double qr[E], rl[E], x[E], y[E];
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
             double x[E], y[E];
             auto load = [&](int i, double(&v)[E]) {
 #pragma unroll
-                for (int m = 0; m < E; m++) v[m] = ms[i * TOT + (pb ^ place(m))];
+                for (int m = 0; m < E; m++) v[m] = ms[i * TOT + place_at(pb, m)];
                 fwd_group<B, 0>(v, wf, L);
             };
             if (need_a) load(0, x);
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
             for (int m = 0; m < E; m++) x[m] = dmul_mod(x[m], M.square ? x[m] : y[m], L.p, L.pinv);
             inv_group<B, 0>(x, wi, L);
 #pragma unroll
-            for (int m = 0; m < E; m++) ms[pb ^ place(m)] = x[m];
+            for (int m = 0; m < E; m++) ms[place_at(pb, m)] = x[m];
         }
     }
     auto act = [](int) { return 0; };

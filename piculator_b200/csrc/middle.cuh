@@ -71,6 +71,11 @@ __host__ __device__ constexpr int place(int e)
     return e ^ ((e >> 4) & 1) ^ (((e >> 5) & 1) * 6) ^ (((e >> 6) & 1) << 3);
 }
 
+// The place of element base + m (disjoint bits) from pb = place(base): only the
+// low four bits of place(m) need the XOR, the others are zero in pb and become
+// the access's constant offset.
+__host__ __device__ constexpr int place_at(int pb, int m) { return (pb ^ (place(m) & 15)) + (place(m) & ~15); }
+
 // Rounds of a 2^LR row: radix 8, the remainder last (smallest stride).
 template <int LR, int R>
 using Round = typename RoundPlan<LR, 3>::template At<R>;
@@ -109,11 +114,11 @@ __device__ __forceinline__ void forward_rounds(double* __restrict__ s, const Dbl
 #pragma unroll
             for (int m = 0; m < 8; m++) {
                 if constexpr (R == 0) x[m] = in(a, t, base + (m << LST));
-                else x[m] = sa[pb ^ place(m << LST)];
+                else x[m] = sa[place_at(pb, m << LST)];
             }
             fwd_group<B, LST>(x, w, L);
 #pragma unroll
-            for (int m = 0; m < 8; m++) sa[pb ^ place(m << LST)] = x[m];
+            for (int m = 0; m < 8; m++) sa[place_at(pb, m << LST)] = x[m];
         }
         __syncthreads();
         forward_rounds<LR, LT, NOP, R + 1>(s, L, tw, nop, in);
@@ -142,12 +147,12 @@ __device__ __forceinline__ void inverse_rounds(double* __restrict__ s, const Dbl
         double x[8];
         double* sa = s + act(i) * Sh::TOT;
 #pragma unroll
-        for (int m = 0; m < 8; m++) x[m] = sa[pb ^ place(m << LST)];
+        for (int m = 0; m < 8; m++) x[m] = sa[place_at(pb, m << LST)];
         inv_group<B, LST>(x, w, L);
 #pragma unroll
         for (int m = 0; m < 8; m++) {
             if constexpr (R == 0) out(i, t, base + (m << LST), x[m]);
-            else sa[pb ^ place(m << LST)] = x[m];
+            else sa[place_at(pb, m << LST)] = x[m];
         }
     }
     if constexpr (R > 0) inverse_rounds<LR, LT, R - 1>(s, L, tw, nout, act, out);

@@ -1293,8 +1293,6 @@ static bool launch_cols_fast_lc(const NttBatch& b, int k, int lpre, int lw, size
     case 4: if constexpr (LC + 4 <= 13) { launch_cols_fast_t<INV, LC, 4, RB, A>(b, k, lpre, grid, s); return true; } break;
     case 5: if constexpr (LC + 5 <= 13) { launch_cols_fast_t<INV, LC, 5, RB, A>(b, k, lpre, grid, s); return true; } break;
     case 6: if constexpr (LC + 6 <= 13) { launch_cols_fast_t<INV, LC, 6, RB, A>(b, k, lpre, grid, s); return true; } break;
-    case 7: if constexpr (LC <= 4) { launch_cols_fast_t<INV, LC, 7, RB, A>(b, k, lpre, grid, s); return true; } break;
-    case 8: if constexpr (LC <= 3) { launch_cols_fast_t<INV, LC, 8, RB, A>(b, k, lpre, grid, s); return true; } break;
     default: break;
     }
     return false;
@@ -1413,30 +1411,17 @@ static bool launch_cols_bulk(const NttBatch& b, int k, int lpre, int lc, int lw,
     }
 }
 
-template <bool INV>
-static bool launch_rows_fast_any(const NttBatch& b, int k, int lr, cudaStream_t s)
-{
-    return b.prime[0].fp64 ? launch_rows_fast<INV, ArithDbl>(b, k, lr, s) : launch_rows_fast<INV, ArithInt>(b, k, lr, s);
-}
-
-template <bool INV>
-static bool launch_cols_fast_any(const NttBatch& b, int k, int lpre, int lc, int lw, size_t grid, cudaStream_t s)
-{
-    return b.prime[0].fp64 ? launch_cols_fast<INV, ArithDbl>(b, k, lpre, lc, lw, grid, s)
-                           : launch_cols_fast<INV, ArithInt>(b, k, lpre, lc, lw, grid, s);
-}
-
 static void launch_rows(bool inv, const NttBatch& b, int k, int lr, cudaStream_t s)
 {
+    PIC_REQUIRE(!b.prime[0].fp64, PIC_ERR_INVALID, "the FP64 form's row passes are the fused middle passes");
     if (fast_ok(b, k)) {
         ProfScope ps(KC_NTT_ROWS, 16.0 * (double)b.count * (double)((size_t)1 << k), s);
-        if (inv ? launch_rows_fast_any<true>(b, k, lr, s) : launch_rows_fast_any<false>(b, k, lr, s)) {
+        if (inv ? launch_rows_fast<true, ArithInt>(b, k, lr, s) : launch_rows_fast<false, ArithInt>(b, k, lr, s)) {
             PIC_CHECK_LAUNCH();
             count_launch();
             return;
         }
     }
-    PIC_REQUIRE(!b.prime[0].fp64, PIC_ERR_INVALID, "FP64 NTT row pass outside the fast kernels' shapes");
     if (!inv && b.src.words != nullptr) materialize_src(b, k, s);  // the general kernels read `data`
     int lrpc = 0;
     if (lr == k) {
@@ -1482,11 +1467,7 @@ static void launch_cols(bool inv, const NttBatch& b, int k, int lpre, int lc, cu
     const int lM = k - lpre - lc;
     if (lc + lw > kInnerBits) lw = kInnerBits - lc;  // tile <= 2^13 points (64 KB)
     if (lw < 2) lw = 2;
-    // short columns: wide enough that each of the CTA's 256 threads has a group
-    // of the first round (64 columns of 2^2 or 2^3 rows gave 64 threads work:
-    // the merge level of 2^13 points took 169 ms of the 1e9 run, now 46)
     const bool fast = fast_ok(b, k) && b.prime[0].slo_fwd != nullptr;
-    if (fast && lc <= 4) lw = std::max(lw, lc == 4 ? 7 : 8);
     if (lw > lM) lw = lM;
     const size_t grid = (size_t)b.count << (lM - lw + lpre);
     const size_t smem = sizeof(uint64_t) << (lc + lw);
@@ -1497,14 +1478,17 @@ static void launch_cols(bool inv, const NttBatch& b, int k, int lpre, int lc, cu
         count_launch();
         return;
     }
+    if (b.prime[0].fp64) {
+        ntt_cols56(inv, b, k, lpre, lc, gm.col_lw ? gm.col_lw : col_width_log2(lc), s);
+        return;
+    }
     if (fast &&
-        (inv ? launch_cols_fast_any<true>(b, k, lpre, lc, lw, grid, s)
-             : launch_cols_fast_any<false>(b, k, lpre, lc, lw, grid, s))) {
+        (inv ? launch_cols_fast<true, ArithInt>(b, k, lpre, lc, lw, grid, s)
+             : launch_cols_fast<false, ArithInt>(b, k, lpre, lc, lw, grid, s))) {
         PIC_CHECK_LAUNCH();
         count_launch();
         return;
     }
-    PIC_REQUIRE(!b.prime[0].fp64, PIC_ERR_INVALID, "FP64 NTT column pass outside the fast kernels' shapes");
     if (!inv && b.src.words != nullptr) materialize_src(b, k, s);  // the general kernels read `data`
     const bool lazy = b.prime[0].lazy != 0;
 #define PIC_COLS(I, Z, R)                                                                          \

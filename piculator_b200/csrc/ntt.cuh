@@ -127,6 +127,10 @@ void ntt_bitreverse(const NttBatch& b, int k, cudaStream_t s);
 void ntt_forward_cols(const NttBatch& b, int k, int row_bits, cudaStream_t s);
 void ntt_inverse_cols(const NttBatch& b, int k, int row_bits, cudaStream_t s);
 
+// One column pass of the FP64 form (cols.cu): 2^lc rows, tiles about 2^lw
+// columns wide.
+void ntt_cols56(bool inv, const NttBatch& b, int k, int lpre, int lc, int lw, cudaStream_t s);
+
 // Fused middle passes of the FP64 form (middle.cu): the forward row pass of
 // every operand, the pointwise products and the inverse row pass of every
 // result in one kernel, so that a spectrum never leaves the chip.

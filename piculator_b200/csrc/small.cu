@@ -78,7 +78,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(MiddleShape<LR, 0>::
             double x[E], y[E];
             auto load = [&](int i, double(&v)[E]) {
 #pragma unroll
-                for (int m = 0; m < E; m++) v[m] = ms[i * TOT + (pb ^ place(m))];
+                for (int m = 0; m < E; m++) v[m] = ms[i * TOT + place_at(pb, m)];
                 fwd_group<B, 0>(v, wf, L);
             };
             load(0, x);
@@ -87,7 +87,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(MiddleShape<LR, 0>::
             for (int m = 0; m < E; m++) x[m] = dmul_mod(x[m], square ? x[m] : y[m], L.p, L.pinv);
             inv_group<B, 0>(x, wi, L);
 #pragma unroll
-            for (int m = 0; m < E; m++) ms[pb ^ place(m)] = x[m];
+            for (int m = 0; m < E; m++) ms[place_at(pb, m)] = x[m];
         }
     }
     auto act = [](int) { return 0; };

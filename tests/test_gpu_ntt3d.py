@@ -214,3 +214,27 @@ def test_one_launch_products(pic, oracle, na, nb):
     assert _int(pic.mul_host(a, b, "ntt3d")) == _int(a) * _int(b)
     a[:], b[:] = 0xFFFFFFFF, 0xFFFFFFFF
     assert _int(pic.mul_host(a, b, "ntt3d")) == _int(a) * _int(b)
+
+
+@pytest.mark.parametrize("lg", range(14, 25))
+def test_column_passes_of_every_height(pic, torch_cuda, lg):
+    """Products whose transforms take column passes of 1 .. 11 bits (and two of
+    them), with the tables of group twiddles and with the two-level tables,
+    against the integer form: operands that end inside a column tile, and one
+    much shorter than the other."""
+    torch = torch_cuda
+    n = (1 << lg) * 56 // 32 // 2
+    na, nb = n - 37, n - n // 3
+    a, b = (torch.randint(-2**31, 2**31 - 1, (m,), dtype=torch.int32, device="cuda") for m in (na, nb))
+    z = [torch.empty(na + nb, dtype=torch.int32, device="cuda") for _ in range(3)]
+    torch.cuda.synchronize()
+    pic.mul_dev(z[0].data_ptr(), a.data_ptr(), na, b.data_ptr(), nb, "ntt3")
+    saved = pic.get_tuning(pic.TUNE_DBL_PASS_TABLES)
+    try:
+        for out, bits in ((z[1], 24), (z[2], 0)):
+            pic.set_tuning(pic.TUNE_DBL_PASS_TABLES, bits)
+            pic.mul_dev(out.data_ptr(), a.data_ptr(), na, b.data_ptr(), nb, "ntt3d")
+    finally:
+        pic.set_tuning(pic.TUNE_DBL_PASS_TABLES, saved)
+    pic.synchronize()
+    assert torch.equal(z[0], z[1]) and torch.equal(z[0], z[2])
