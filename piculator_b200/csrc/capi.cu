@@ -188,6 +188,7 @@ pic_status pic_ntt_forward(uint64_t* T, int k, pic_stream s)
         require_init();
         PIC_REQ_PTR(T);
         const PrimeDev P = ref_prime_dev(k);
+        if (ntt_natural(T, k, P, false, resolve(s))) return;
         NttBatch b = single(T, k, P);
         ntt_forward_dif(b, k, resolve(s));
         ntt_bitreverse(b, k, resolve(s));
@@ -200,6 +201,7 @@ pic_status pic_ntt_inverse(uint64_t* T, int k, pic_stream s)
         require_init();
         PIC_REQ_PTR(T);
         const PrimeDev P = ref_prime_dev(k);
+        if (ntt_natural(T, k, P, true, resolve(s))) return;
         NttBatch b = single(T, k, P);
         ntt_bitreverse(b, k, resolve(s));
         ntt_inverse_dit(b, k, resolve(s));

@@ -40,35 +40,6 @@ namespace pic {
 
 constexpr int kColThreads = 256;
 
-// Radix-8 rounds with the remainder first (the largest stride).
-template <int LC>
-struct ColPlan {
-    static constexpr int REM = LC % 3, NR = LC / 3 + (REM ? 1 : 0);
-    template <int R>
-    struct At {
-        static constexpr int B = (R == 0 && REM) ? REM : 3;
-        static constexpr int LB = R == 0 ? LC : LC - (REM ? REM : 3) - 3 * (R - 1);  // log2 sub-block
-        static constexpr int LST = LB - B;                                           // log2 stride
-    };
-};
-
-// Shared-memory place of element (row << LW) + column: half a warp that holds
-// several rows eight apart falls in different banks.  Linear, like place().
-template <int LW>
-__host__ __device__ constexpr int col_place(int e)
-{
-    return LW == 2 ? e ^ (((e >> 5) & 3) << 2) : (LW == 3 ? e ^ (((e >> 6) & 1) << 3) : e);
-}
-
-// Place of element base + m (disjoint bits) from pb = col_place(base).
-template <int LW>
-__host__ __device__ constexpr int col_at(int pb, int m)
-{
-    return (pb ^ (col_place<LW>(m) & 15)) + (col_place<LW>(m) & ~15);
-}
-
-constexpr int brev3(int i, int bits) { return bits == 3 ? ((i & 1) << 2 | (i & 2) | i >> 2) : (bits == 2 ? ((i & 1) << 1 | i >> 1) : i); }
-
 // Butterflies of the smallest-stride round: t.at(l, u) = root_(2^(B - l))^u, so
 // u = 0 needs no product and the unit level none.  Forward: |x| <= 2 p gives
 // |x| <= 16 p, unreduced.

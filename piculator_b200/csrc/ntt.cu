@@ -158,6 +158,21 @@ const PrimeTables& prime_tables(uint64_t p)
     d.ohi_fwd = upload(hif);
     d.olo_inv = upload(loi);
     d.ohi_inv = upload(hii);
+    if (IB == kInnerBits) {
+        // per-level inner tables from the order-2^IB tables: the root of
+        // order 2^m is inner root^(2^(IB - m))
+        std::vector<uint64_t> lf((size_t)2 << IB), li((size_t)2 << IB);
+        for (int lm = 1; lm <= IB; lm++)
+            for (size_t e = 0; e < ((size_t)1 << (lm - 1)); e++) {
+                const size_t dst = ((size_t)1 << (lm - 1)) - 1 + e, src = e << (IB - lm);
+                lf[2 * dst] = inf[2 * src];
+                lf[2 * dst + 1] = inf[2 * src + 1];
+                li[2 * dst] = ini[2 * src];
+                li[2 * dst + 1] = ini[2 * src + 1];
+            }
+        d.lvl_fwd = upload(lf);
+        d.lvl_inv = upload(li);
+    }
     if (d.lazy) {
         // the same outer roots as Shoup pairs (plain value, companion)
         auto pairs = [&](const std::vector<uint64_t>& mont) {
@@ -174,21 +189,6 @@ const PrimeTables& prime_tables(uint64_t p)
         d.shi_fwd = pairs(hif);
         d.slo_inv = pairs(loi);
         d.shi_inv = pairs(hii);
-        if (IB == kInnerBits) {
-            // per-level inner tables from the order-2^IB tables: the root of
-            // order 2^m is inner root^(2^(IB - m))
-            std::vector<uint64_t> lf((size_t)2 << IB), li((size_t)2 << IB);
-            for (int lm = 1; lm <= IB; lm++)
-                for (size_t e = 0; e < ((size_t)1 << (lm - 1)); e++) {
-                    const size_t dst = ((size_t)1 << (lm - 1)) - 1 + e, src = e << (IB - lm);
-                    lf[2 * dst] = inf[2 * src];
-                    lf[2 * dst + 1] = inf[2 * src + 1];
-                    li[2 * dst] = ini[2 * src];
-                    li[2 * dst + 1] = ini[2 * src + 1];
-                }
-            d.lvl_fwd = upload(lf);
-            d.lvl_inv = upload(li);
-        }
     }
     g_tabs[p] = t;
     return *t;
@@ -588,17 +588,6 @@ __device__ void cta_ntt(uint64_t* s, int logn, int lnt, int les, int lts, bool t
         }
         __syncthreads();
     }
-}
-
-// Root of unity w_(2^lM)^e in Montgomery form from the two-level tables.
-template <bool INV>
-__device__ __forceinline__ uint64_t outer_root(const PrimeDev& P, uint64_t e, int lM)
-{
-    const uint64_t E = e << (P.K - lM);
-    const uint64_t lo = E & ((1ull << P.S) - 1), hi = E >> P.S;
-    const uint64_t* tl = INV ? P.olo_inv : P.olo_fwd;
-    const uint64_t* th = INV ? P.ohi_inv : P.ohi_fwd;
-    return mont_mul(__ldg(th + hi), __ldg(tl + lo), P.p, P.pinv_neg);
 }
 
 // Contiguous row pass: rows of 2^lr elements; 2^lrpc rows per CTA.

@@ -51,7 +51,7 @@ struct PrimeDev {
     const uint64_t* shi_fwd;
     const uint64_t* slo_inv;
     const uint64_t* shi_inv;
-    // Lazy primes only (else null): inner roots by level, Shoup pairs.  The
+    // Inner tables of order 2^13 (else null): inner roots by level, Shoup pairs.  The
     // roots of order 2^m (m = 1 .. 13), root^e for e < 2^(m-1), sit at pair
     // index 2^(m-1) - 1 + e, so consecutive e are consecutive pairs.
     const uint64_t* lvl_fwd;
@@ -120,6 +120,13 @@ struct NttBatch {
 void ntt_forward_dif(const NttBatch& b, int k, cudaStream_t s);
 void ntt_inverse_dit(const NttBatch& b, int k, cudaStream_t s);
 void ntt_bitreverse(const NttBatch& b, int k, cudaStream_t s);
+
+// Natural-order transforms modulo a reference prime (natural.cu): forward = DIF
+// and bit reversal, inverse = bit reversal, DIT and the factor 2^-k, the
+// reversal done by the row pass through a second buffer.  False (nothing done)
+// for lengths or primes outside these kernels, or without room for the buffer:
+// the general passes then serve them.
+bool ntt_natural(uint64_t* T, int k, const PrimeDev& P, bool inverse, cudaStream_t s);
 
 // The column passes of a transform whose contiguous row pass has 2^row_bits
 // points: what precedes that row pass in the forward direction, what follows

@@ -1,7 +1,6 @@
-// Device code shared by the NTT pass kernels (ntt.cu) and the fused middle
-// passes (middle.cu): the prime of a batch item, the shared-memory swizzle,
-// reading pieces from source words, the butterflies of both product forms and
-// the register rounds of one group.
+// Device code shared by the pass kernels: the prime of a batch item, the
+// shared-memory swizzles, reading pieces from source words, the butterflies of
+// both product forms, the register rounds of one group and their plans.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -267,5 +266,45 @@ struct RoundPlan {
         static constexpr int LST = LB - B;         // log2 stride inside a group
     };
 };
+
+// Radix-8 rounds with the remainder first (the largest stride).
+template <int LC>
+struct ColPlan {
+    static constexpr int REM = LC % 3, NR = LC / 3 + (REM ? 1 : 0);
+    template <int R>
+    struct At {
+        static constexpr int B = (R == 0 && REM) ? REM : 3;
+        static constexpr int LB = R == 0 ? LC : LC - (REM ? REM : 3) - 3 * (R - 1);  // log2 sub-block
+        static constexpr int LST = LB - B;                                           // log2 stride
+    };
+};
+
+// Shared-memory place of element (row << LW) + column: half a warp that holds
+// several rows eight apart falls in different banks.  Linear, like place().
+template <int LW>
+__host__ __device__ constexpr int col_place(int e)
+{
+    return LW == 2 ? e ^ (((e >> 5) & 3) << 2) : (LW == 3 ? e ^ (((e >> 6) & 1) << 3) : e);
+}
+
+// Place of element base + m (disjoint bits) from pb = col_place(base).
+template <int LW>
+__host__ __device__ constexpr int col_at(int pb, int m)
+{
+    return (pb ^ (col_place<LW>(m) & 15)) + (col_place<LW>(m) & ~15);
+}
+
+constexpr int brev3(int i, int bits) { return bits == 3 ? ((i & 1) << 2 | (i & 2) | i >> 2) : (bits == 2 ? ((i & 1) << 1 | i >> 1) : i); }
+
+// Root of unity w_(2^lM)^e in Montgomery form from the two-level tables.
+template <bool INV>
+__device__ __forceinline__ uint64_t outer_root(const PrimeDev& P, uint64_t e, int lM)
+{
+    const uint64_t E = e << (P.K - lM);
+    const uint64_t lo = E & ((1ull << P.S) - 1), hi = E >> P.S;
+    const uint64_t* tl = INV ? P.olo_inv : P.olo_fwd;
+    const uint64_t* th = INV ? P.ohi_inv : P.ohi_fwd;
+    return mont_mul(__ldg(th + hi), __ldg(tl + lo), P.p, P.pinv_neg);
+}
 
 }  // namespace pic

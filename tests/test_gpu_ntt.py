@@ -156,3 +156,30 @@ def test_fft_matches_reference_fft(pic, torch_cuda, reference, k):
         torch.cuda.synchronize()
         want = reference.fft(k, x, inverse=inv)
         assert np.allclose(t.cpu().numpy(), want, rtol=1e-9, atol=1e-8 * (1 << (k // 2)))
+
+
+@pytest.mark.parametrize("k", [13, 14, 15, 17, 19, 20, 21, 23])
+def test_ntt_flow_product_of_every_pass_split(pic, torch_cuda, k):
+    """The NTT.h flow (convert, forward, pointwise, inverse, convert) at lengths
+    whose transforms take column passes of 2 .. 11 bits and two of them, filled
+    to the last word: the product's words."""
+    torch = torch_cuda
+    L, s = pic.lib(), None
+    na = (1 << (k - 1)) // 2 - 1
+    nb = (1 << (k - 1)) - na
+    a, b = random_words(k, na), random_words(k + 1, nb)
+    ta, tb = (torch.empty(1 << k, dtype=torch.int64, device="cuda") for _ in range(2))
+    da, db = (torch.from_numpy(x.view(np.int32)).cuda() for x in (a, b))
+    z = torch.empty(na + nb, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for t, x in ((ta, da), (tb, db)):
+        pic.check(L.pic_int_to_ntt(t.data_ptr(), k, x.data_ptr(), x.numel(), s))
+        pic.check(L.pic_ntt_forward(t.data_ptr(), k, s))
+    pic.check(L.pic_ntt_pointwise(ta.data_ptr(), tb.data_ptr(), k, s))
+    pic.check(L.pic_ntt_inverse(ta.data_ptr(), k, s))
+    pic.check(L.pic_ntt_to_int(ta.data_ptr(), k, z.data_ptr(), z.numel(), s))
+    pic.synchronize()
+    want = torch.empty_like(z)
+    pic.mul_dev(want.data_ptr(), da.data_ptr(), na, db.data_ptr(), nb, "ntt3")
+    pic.synchronize()
+    assert torch.equal(z, want)
