@@ -9,6 +9,7 @@
 #include "fft.cuh"
 #include "mul.cuh"
 #include "ntt.cuh"
+#include "passes.cuh"
 
 namespace pic {
 
@@ -18,6 +19,7 @@ static constexpr int kFftS = 15;          // outer split e = hi * 2^15 + lo
 
 struct FftTables {
     double2* inner = nullptr;  // exp(+2 pi i j / 2^13), j < 2^12
+    double2* lvl = nullptr;    // the same by level: exp(+2 pi i e / 2^m), e < 2^(m-1), at 2^(m-1) - 1 + e
     double2* olo = nullptr;    // exp(+2 pi i j / 2^30), j < 2^15
     double2* ohi = nullptr;    // exp(+2 pi i j 2^15 / 2^30), j < 2^15
 };
@@ -53,7 +55,12 @@ static const FftTables& fft_tables()
             const double a = two_pi * (double)j / (double)(1u << (kFftK - kFftS));
             hi[j] = make_double2(cos(a), sin(a));
         }
+        std::vector<double2> lv((size_t)1 << kFftInnerBits);
+        for (int m = 1; m <= kFftInnerBits; m++)
+            for (size_t e = 0; e < ((size_t)1 << (m - 1)); e++)
+                lv[((size_t)1 << (m - 1)) - 1 + e] = in[e << (kFftInnerBits - m)];
         g_fft.inner = upload2(in);
+        g_fft.lvl = upload2(lv);
         g_fft.olo = upload2(lo);
         g_fft.ohi = upload2(hi);
     });
@@ -177,43 +184,160 @@ __global__ void __launch_bounds__(512) fft_rows_kernel(FftBatch B, int k, int lr
     }
 }
 
-template <bool INV>
-__global__ void __launch_bounds__(256) fft_cols_kernel(FftBatch B, int k, int lpre, int lc, int W,
-                                                       const double2* tw, const double2* olo, const double2* ohi)
+// ---- passes with compile-time rounds (transforms longer than one CTA's) --------
+// The butterflies, twiddle values and their order are those of the general
+// kernels above, which serve the single-pass lengths; here the strides fold away,
+// consecutive lanes read consecutive twiddles, the first round reads and the
+// last writes global memory, and the shared-memory places keep eight lanes' 16
+// bytes in different banks.  Bound by latency (three CTAs
+// per SM, 64 - 84 registers) while the data stays in L2: forward passes of 2^20
+// points 28.9 us (rows) and 27.8 (columns) before, 12.2 and 15.4 here; the FFT.h
+// flow at 2^20 245 -> 148 us.
+
+// Bits 3, 4, 5 of a row's element XORed into bits 0, 1, 2 (rounds at strides
+// 2^8, 2^5, 2^2, 1 of 11-bit rows).
+__host__ __device__ constexpr int fft_place(int e) { return e ^ ((e >> 3) & 7); }
+// A column tile's (row << LW) + column, 2^LW >= 4: rows eight apart.
+template <int LW>
+__host__ __device__ constexpr int fft_col_place(int e)
 {
+    return LW == 2 ? e ^ (((e >> 5) & 1) << 2) : e;
+}
+
+template <int B, bool INV, int LST>
+__device__ __forceinline__ void fft_levels(double2 (&x)[1 << B], int j, const double2* __restrict__ lvl)
+{
+#pragma unroll
+    for (int q = 0; q < B; q++) {
+        const int l = INV ? B - 1 - q : q;
+        const int hm = 1 << (B - 1 - l);
+#pragma unroll
+        for (int m = 0; m < (1 << B); m++) {
+            if (m & hm) continue;
+            const double2 w = __ldg(lvl + ((1 << (B - l + LST - 1)) - 1) + j + ((m & (hm - 1)) << LST));
+            if (!INV) {
+                const double2 a = x[m], b = x[m + hm];
+                x[m] = cadd(a, b);
+                x[m + hm] = cmul(csub(a, b), w);
+            } else {
+                const double2 a = x[m], b = cmulc(x[m + hm], w);
+                x[m] = cadd(a, b);
+                x[m + hm] = csub(a, b);
+            }
+        }
+    }
+}
+
+constexpr int kFftThreads = 256;
+constexpr int kFftRowBits = 11;
+
+template <bool INV>
+__global__ void __launch_bounds__(kFftThreads, 3) fft_rows_fast_kernel(FftBatch B, int k,
+                                                                       const double2* __restrict__ lvl)
+{
+    constexpr int LR = kFftRowBits, NR = RoundPlan<LR, 3>::NR;
     extern __shared__ double2 fsm[];
-    const int lM = k - lpre - lc;
-    const size_t M = (size_t)1 << lM;
-    const size_t tiles_per_block = M / W;
-    const size_t ctas_per_tr = tiles_per_block << lpre;
+    const int lrow = k - LR;
+    double2* row = B.data + (blockIdx.x >> lrow) * B.stride + ((blockIdx.x & (((size_t)1 << lrow) - 1)) << LR);
+    auto round = [&](auto rc) {
+        constexpr int RR = INV ? NR - 1 - decltype(rc)::value : decltype(rc)::value;
+        using At = typename RoundPlan<LR, 3>::template At<RR>;
+        constexpr int Bb = At::B, LB = At::LB, LST = At::LST, E = 1 << Bb, G = 1 << (LR - Bb);
+        constexpr bool FIRST = decltype(rc)::value == 0, LAST = decltype(rc)::value == NR - 1;
+#pragma unroll 1
+        for (int g = threadIdx.x; g < G; g += kFftThreads) {
+            const int j = g & ((1 << LST) - 1), base = ((g >> LST) << LB) + j;
+            double2 x[E];
+#pragma unroll
+            for (int m = 0; m < E; m++) {
+                const int e = base + (m << LST);
+                x[m] = FIRST ? row[e] : fsm[fft_place(e)];
+            }
+            fft_levels<Bb, INV, LST>(x, j, lvl);
+#pragma unroll
+            for (int m = 0; m < E; m++) {
+                const int e = base + (m << LST);
+                if (LAST) row[e] = x[m];
+                else fsm[fft_place(e)] = x[m];
+            }
+        }
+        if constexpr (!LAST) __syncthreads();
+    };
+    static_assert(NR == 4, "11-bit rows");
+    round(std::integral_constant<int, 0>{});
+    round(std::integral_constant<int, 1>{});
+    round(std::integral_constant<int, 2>{});
+    round(std::integral_constant<int, 3>{});
+}
+
+template <bool INV, int LC, int LW>
+__global__ void __launch_bounds__(kFftThreads, 3)
+    fft_cols_fast_kernel(FftBatch B, int k, int lpre, const double2* __restrict__ lvl, const double2* __restrict__ olo,
+                         const double2* __restrict__ ohi)
+{
+    using Plan = RoundPlan<LC, 3>;
+    constexpr int NR = Plan::NR, WMASK = (1 << LW) - 1;
+    extern __shared__ double2 fsm[];
+    const int lblock = k - lpre, lM = lblock - LC, ltiles = lM - LW;
     const size_t cta = blockIdx.x;
-    const size_t tr = cta / ctas_per_tr;
-    const size_t rem = cta % ctas_per_tr;
-    const size_t ob = rem / tiles_per_block;
-    const size_t c0 = (rem % tiles_per_block) * W;
-    double2* base = B.data + tr * B.stride + (ob << (k - lpre)) + c0;
-    const int N1 = 1 << lc;
-    const int lblock = k - lpre;
-    for (int idx = threadIdx.x; idx < N1 * W; idx += blockDim.x) {
-        const int m = idx / W, w = idx % W;
-        double2 v = base[((size_t)m << lM) + w];
-        if (INV) {
-            const uint64_t k1 = __brev((unsigned)m) >> (32 - lc);
-            v = cmulc(v, fft_outer_root(olo, ohi, (c0 + w) * k1, lblock));
+    const size_t tr = cta >> (ltiles + lpre), rem = cta & (((size_t)1 << (ltiles + lpre)) - 1);
+    const size_t ob = rem >> ltiles;
+    const int w = threadIdx.x & WMASK;
+    const uint64_t c = ((rem & (((size_t)1 << ltiles) - 1)) << LW) + w;
+    double2* col = B.data + tr * B.stride + (ob << lblock) + c;
+    auto root = [&](int r) { return fft_outer_root(olo, ohi, c * (__brev((unsigned)r) >> (32 - LC)), lblock); };
+    auto round = [&](auto rc) {
+        constexpr int RR = INV ? NR - 1 - decltype(rc)::value : decltype(rc)::value;
+        using At = typename Plan::template At<RR>;
+        constexpr int Bb = At::B, LB = At::LB, LST = At::LST, E = 1 << Bb, G = 1 << (LC - Bb + LW);
+        constexpr bool FIRST = decltype(rc)::value == 0, LAST = decltype(rc)::value == NR - 1;
+#pragma unroll 1
+        for (int g = threadIdx.x; g < G; g += kFftThreads) {
+            const int gi = g >> LW, j = gi & ((1 << LST) - 1), r0 = ((gi >> LST) << LB) + j;
+            double2 x[E];
+#pragma unroll
+            for (int m = 0; m < E; m++) {
+                const int r = r0 + (m << LST);
+                if (FIRST) {
+                    x[m] = col[(size_t)r << lM];
+                    if (INV) x[m] = cmulc(x[m], root(r));
+                } else {
+                    x[m] = fsm[fft_col_place<LW>((r << LW) + w)];
+                }
+            }
+            fft_levels<Bb, INV, LST>(x, j, lvl);
+#pragma unroll
+            for (int m = 0; m < E; m++) {
+                const int r = r0 + (m << LST);
+                if (LAST) col[(size_t)r << lM] = INV ? x[m] : cmul(x[m], root(r));
+                else fsm[fft_col_place<LW>((r << LW) + w)] = x[m];
+            }
         }
-        fsm[idx] = v;
-    }
-    __syncthreads();
-    cta_fft<INV>(fsm, lc, W, W, 1, true, tw);
-    for (int idx = threadIdx.x; idx < N1 * W; idx += blockDim.x) {
-        const int m = idx / W, w = idx % W;
-        double2 v = fsm[idx];
-        if (!INV) {
-            const uint64_t k1 = __brev((unsigned)m) >> (32 - lc);
-            v = cmul(v, fft_outer_root(olo, ohi, (c0 + w) * k1, lblock));
-        }
-        base[((size_t)m << lM) + w] = v;
-    }
+        if constexpr (!LAST) __syncthreads();
+    };
+    round(std::integral_constant<int, 0>{});
+    if constexpr (NR > 1) round(std::integral_constant<int, 1>{});
+    if constexpr (NR > 2) round(std::integral_constant<int, 2>{});
+}
+
+static void fft_rows_fast(bool inv, const FftBatch& b, int k, cudaStream_t s)
+{
+    const size_t grid = (size_t)b.count << (k - kFftRowBits);
+    const size_t smem = sizeof(double2) << kFftRowBits;
+    if (inv) fft_rows_fast_kernel<true><<<(unsigned)grid, kFftThreads, smem, s>>>(b, k, fft_tables().lvl);
+    else fft_rows_fast_kernel<false><<<(unsigned)grid, kFftThreads, smem, s>>>(b, k, fft_tables().lvl);
+}
+
+// 2^11-point tiles: a group of every round per thread.
+template <int LC>
+static void fft_cols_fast(bool inv, const FftBatch& b, int k, int lpre, cudaStream_t s)
+{
+    constexpr int LW = 11 - LC > 8 ? 8 : 11 - LC;
+    const FftTables& T = fft_tables();
+    const size_t grid = (size_t)b.count << (k - LC - LW);
+    const size_t smem = RoundPlan<LC, 3>::NR > 1 ? sizeof(double2) << (LC + LW) : 0;
+    if (inv) fft_cols_fast_kernel<true, LC, LW><<<(unsigned)grid, kFftThreads, smem, s>>>(b, k, lpre, T.lvl, T.olo, T.ohi);
+    else fft_cols_fast_kernel<false, LC, LW><<<(unsigned)grid, kFftThreads, smem, s>>>(b, k, lpre, T.lvl, T.olo, T.ohi);
 }
 
 static std::vector<int> fft_pass_bits(int k)
@@ -223,7 +347,7 @@ static std::vector<int> fft_pass_bits(int k)
         bits.push_back(k);
         return bits;
     }
-    const int row = 11, colmax = 9;  // 16-byte points: half the NTT's tile
+    const int row = kFftRowBits, colmax = 9;  // 16-byte points: half the NTT's tile
     int rest = k - row;
     const int ncol = (rest + colmax - 1) / colmax;
     for (int i = 0; i < ncol; i++) {
@@ -247,6 +371,12 @@ static void fft_launch_rows(bool inv, const FftBatch& b, int k, int lr, cudaStre
     }
     const size_t grid = ((size_t)b.count << (k - lr)) / rpc;
     ProfScope ps(KC_FFT_ROWS, 32.0 * (double)b.count * (double)((size_t)1 << k), s);
+    if (lr < k) {
+        fft_rows_fast(inv, b, k, s);
+        PIC_CHECK_LAUNCH();
+        count_launch();
+        return;
+    }
     const size_t smem = (size_t)rpc * n * sizeof(double2);
     int threads = (rpc * n) / 8;
     if (threads < 32) threads = 32;
@@ -266,20 +396,16 @@ static void fft_launch_rows(bool inv, const FftBatch& b, int k, int lr, cudaStre
 
 static void fft_launch_cols(bool inv, const FftBatch& b, int k, int lpre, int lc, cudaStream_t s)
 {
-    const FftTables& T = fft_tables();
-    const int W = 4;
-    const size_t M = (size_t)1 << (k - lpre - lc);
-    const size_t grid = ((size_t)b.count * (M / W)) << lpre;
-    const size_t smem = ((size_t)W << lc) * sizeof(double2);
     ProfScope ps(KC_FFT_COLS, 32.0 * (double)b.count * (double)((size_t)1 << k), s);
-    if (inv) {
-        if (smem > 48 * 1024)
-            PIC_CUDA(cudaFuncSetAttribute(fft_cols_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        fft_cols_kernel<true><<<(unsigned)grid, 256, smem, s>>>(b, k, lpre, lc, W, T.inner, T.olo, T.ohi);
-    } else {
-        if (smem > 48 * 1024)
-            PIC_CUDA(cudaFuncSetAttribute(fft_cols_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        fft_cols_kernel<false><<<(unsigned)grid, 256, smem, s>>>(b, k, lpre, lc, W, T.inner, T.olo, T.ohi);
+    switch (lc) {
+    case 3: fft_cols_fast<3>(inv, b, k, lpre, s); break;
+    case 4: fft_cols_fast<4>(inv, b, k, lpre, s); break;
+    case 5: fft_cols_fast<5>(inv, b, k, lpre, s); break;
+    case 6: fft_cols_fast<6>(inv, b, k, lpre, s); break;
+    case 7: fft_cols_fast<7>(inv, b, k, lpre, s); break;
+    case 8: fft_cols_fast<8>(inv, b, k, lpre, s); break;
+    case 9: fft_cols_fast<9>(inv, b, k, lpre, s); break;
+    default: throw Error(PIC_ERR_INVALID, "FFT column pass outside its kernels' shapes");
     }
     PIC_CHECK_LAUNCH();
     count_launch();

@@ -183,3 +183,27 @@ def test_ntt_flow_product_of_every_pass_split(pic, torch_cuda, k):
     pic.mul_dev(want.data_ptr(), da.data_ptr(), na, db.data_ptr(), nb, "ntt3")
     pic.synchronize()
     assert torch.equal(z, want)
+
+
+@pytest.mark.parametrize("k", [14, 15, 16, 17, 18, 19, 20, 21, 22])
+def test_fft_passes_of_every_height(pic, torch_cuda, k):
+    """Forward (bit-reversed output) against torch's transform, and back: column
+    passes of 3 .. 9 bits and two of them.  A radix-2 level adds at most about
+    three roundings, so the relative error stays below 4 k 2^-52."""
+    torch = torch_cuda
+    n = 1 << k
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.view_as_complex(torch.randn((n, 2), generator=g, device="cuda", dtype=torch.float64))
+    t = x.clone()
+    torch.cuda.synchronize()
+    pic.check(pic.lib().pic_fft_forward(t.data_ptr(), k, None))
+    pic.synchronize()
+    i, r = torch.arange(n, device="cuda"), torch.zeros(n, dtype=torch.int64, device="cuda")
+    for b in range(k):
+        r |= ((i >> b) & 1) << (k - 1 - b)
+    want = torch.fft.ifft(x, norm="forward")
+    bound = 4 * k * 2.0 ** -52
+    assert float(torch.linalg.norm(t[r] - want) / torch.linalg.norm(want)) < bound
+    pic.check(pic.lib().pic_fft_inverse(t.data_ptr(), k, None))
+    pic.synchronize()
+    assert float(torch.linalg.norm(t / n - x) / torch.linalg.norm(x)) < 2 * bound
