@@ -98,10 +98,4 @@ __device__ __forceinline__ uint64_t src_piece56_raw(const uint32_t* __restrict__
     return v & ((1ull << 56) - 1);
 }
 
-// A residue x with 0 <= x < 2^52 as an integer (the bits of x + 2^52).
-__device__ __forceinline__ uint64_t dto_u64(double x)
-{
-    return (uint64_t)__double_as_longlong(__dadd_rn(x, 4503599627370496.0)) & ((1ull << 52) - 1);
-}
-
 }  // namespace pic

@@ -139,6 +139,40 @@ __device__ __forceinline__ void crt3(const Crt3Consts& C, uint64_t y0, uint64_t 
     l2 = b2 + c1;
 }
 
+// Shared tail of the limb conversions: limb digits (T = D_i + C_(i-1)) -> words
+// with in-block carry resolution; writes the CTA's (G, P).
+template <int NL>
+__device__ __forceinline__ void limbs_to_words(const uint64_t (&dig)[NL], const uint32_t (&gen)[NL],
+                                               size_t first_limb, uint32_t* z, size_t zw, uint32_t* agg_slot)
+{
+    uint32_t gp = kGPIdentity;
+#pragma unroll
+    for (int u = 0; u < NL; u++) {
+        const size_t w = 2 * (first_limb + u);
+        const uint32_t lo = (uint32_t)dig[u], hi = (uint32_t)(dig[u] >> 32);
+        if (w < zw) gp = gp_combine(gp, (uint32_t)(lo == 0xffffffffu) << 1);
+        if (w + 1 < zw) gp = gp_combine(gp, gen[u] | ((uint32_t)(hi == 0xffffffffu) << 1));
+    }
+    uint32_t total;
+    uint32_t cin = block_gp_scan(gp, &total) & 1u;
+#pragma unroll
+    for (int u = 0; u < NL; u++) {
+        const size_t w = 2 * (first_limb + u);
+        const uint32_t lo = (uint32_t)dig[u], hi = (uint32_t)(dig[u] >> 32);
+        if (w < zw) z[w] = lo + cin;
+        cin = (uint32_t)(lo == 0xffffffffu) & cin;
+        if (w + 1 < zw) z[w + 1] = hi + cin;
+        cin = gen[u] | ((uint32_t)(hi == 0xffffffffu) & cin);
+    }
+    if (threadIdx.x == 0) *agg_slot = total;
+}
+
+__device__ __forceinline__ void add128(uint64_t& lo, uint64_t& hi, uint64_t v)
+{
+    lo += v;
+    hi += (lo < v);
+}
+
 // Three-prime residues y[q * pstride + j] -> words.  Limb i (64 bits)
 // collects x_i.l0 + x_(i-1).l1 + x_(i-2).l2 (< 3 * 2^64).  One CTA handles
 // limbs [i0, i0 + kCrtLPC) of one product; slot t of xs holds coefficient
@@ -785,52 +819,61 @@ CrtDConsts make_crtd(int k, bool offset)
     dbl_pair(host_powmod(P0 % P1, P1 - 2, P1), P1, C.i01, C.i01p);
     dbl_pair(host_powmod(host_mulmod(P0 % P2, P1 % P2, P2), P2 - 2, P2), P2, C.i012, C.i012p);
     dbl_pair(host_powmod(P1 % P2, P2 - 2, P2), P2, C.q012, C.q012p);
-    const unsigned __int128 p01 = (unsigned __int128)P0 * P1;
-    C.p0 = P0;
-    C.p01_lo = (uint64_t)p01;
-    C.p01_hi = (uint64_t)(p01 >> 64);
+    C.off[0] -= 2 * C.p[0];
+    const uint64_t c0 = P0 >> 32, c1 = P1 >> 32;
+    C.c0 = (uint32_t)c0;
+    C.c01 = (uint32_t)(c0 + c1);
+    C.cc = (uint32_t)(c0 * c1);
     return C;
 }
 
 // 128 threads convert 127 groups of 8 coefficients and the three before them
-// (1019 coefficients, eight per thread).  The 64 registers and 28 KB of shared
-// memory let eight CTAs share an SM.  Binary splitting at 1e8 digits: 10.3 ms
-// of CRT with each thread's eight coefficients in registers (uncoalesced
-// residue reads, 33 limb registers), 9.7 ms so.
+// (1019 coefficients, eight per thread), eight CTAs per SM.  Bound by instruction
+// issue (about 150 a coefficient, 57 of them FP64).  2^24-word operands: 255 us
+// with three-limb coefficients of one thread each, 234 with the coefficients
+// spread over the threads, 207 with base-2^56 digits and the short products of
+// c 2^32 + 1, 152 with the next residues loaded ahead and the words written
+// through shared memory.
 constexpr int kCrtDThreads = 128;
 constexpr int kCrtDGroups = 127;
-constexpr size_t kCrtDLPC = 7 * (size_t)kCrtDGroups;  // limbs per CTA
-constexpr size_t kCrtDWPC = 2 * kCrtDLPC;
+constexpr size_t kCrtDWPC = 14 * (size_t)kCrtDGroups;  // words per CTA
 constexpr int kCrtDCoefs = 8 * kCrtDGroups + 3;
 constexpr int kCrtDSlots = crt_slot(kCrtDCoefs);
+
+// Coefficients with words below zw.
+__device__ __forceinline__ int64_t crt_limit(size_t ncoef, size_t zw)
+{
+    const int64_t climit = (int64_t)((32 * zw + 55) / 56);
+    return climit < (int64_t)ncoef ? climit : (int64_t)ncoef;
+}
 
 __device__ __forceinline__ void crt3d_block(const uint64_t* __restrict__ Y, size_t pstride, size_t ncoef,
                                             const CrtDConsts& C, uint32_t* __restrict__ z, size_t zw, int64_t cta,
                                             uint32_t* agg_slot)
 {
-    __shared__ uint64_t X[3 * kCrtDSlots];
-    const int64_t climit = (int64_t)((32 * zw + 55) / 56);  // coefficients below the last word
-    const int64_t jlim = climit < (int64_t)ncoef ? climit : (int64_t)ncoef;
-    crt_coefs<kCrtDSlots>(X, 8 * cta * kCrtDGroups - 3, kCrtDCoefs, jlim, C,
-                          [&](int64_t j, double& y0, double& y1, double& y2) {
-                              y0 = dbits(Y[j]);
-                              y1 = dbits(Y[pstride + j]);
-                              y2 = dbits(Y[2 * pstride + j]);
-                          });
+    __shared__ CrtDigits<kCrtDSlots> X;
+    const int64_t j0 = 8 * cta * kCrtDGroups - 3, jlim = crt_limit(ncoef, zw);
+    crt_coefs(X, kCrtDCoefs, C, [&](int i) { return j0 + i < jlim ? j0 + i : (int64_t)-1; },
+              [&](int64_t j, double& y0, double& y1, double& y2) {
+                  y0 = dbits(Y[j]);
+                  y1 = dbits(Y[pstride + j]);
+                  y2 = dbits(Y[2 * pstride + j]);
+              });
     __syncthreads();
-    uint64_t dig[7] = {0, 0, 0, 0, 0, 0, 0};
-    uint32_t gen[7] = {0, 0, 0, 0, 0, 0, 0};
+    uint64_t t[8];
     const bool mine = threadIdx.x < kCrtDGroups;
-    if (mine) crt_digits<kCrtDSlots>(X, threadIdx.x, dig, gen);
-    const size_t zend = 2 * ((size_t)cta * kCrtDLPC + kCrtDLPC);
-    limbs_to_words<7>(dig, gen, mine ? 7 * ((size_t)cta * kCrtDGroups + threadIdx.x) : zw, z, zw < zend ? zw : zend,
-                      agg_slot);
+    if (mine) crt_group(X, 8 * (int)threadIdx.x + 3, t);
+    uint32_t* W = reinterpret_cast<uint32_t*>(&X);
+    digits_to_words(t, mine, false, W, agg_slot);
+    const size_t w0 = (size_t)cta * kCrtDWPC;
+    const int n = w0 >= zw ? 0 : (int)(zw - w0 < kCrtDWPC ? zw - w0 : kCrtDWPC);
+    for (int i = threadIdx.x; i < n; i += kCrtDThreads) z[w0 + i] = W[i];
 }
 
 // A single CTA posts the top word; several leave their carries to carry_fix.
 __global__ void __launch_bounds__(kCrtDThreads, 8) crt3d_k1(const uint64_t* __restrict__ Y, size_t pstride,
-                                                         size_t ncoef, CrtDConsts C, uint32_t* z, size_t zw,
-                                                         uint32_t* agg, MailRef mail)
+                                                            size_t ncoef, CrtDConsts C, uint32_t* z, size_t zw,
+                                                            uint32_t* agg, MailRef mail)
 {
     crt3d_block(Y, pstride, ncoef, C, z, zw, (int64_t)blockIdx.x, agg + blockIdx.x);
     if (mail.slot == nullptr) return;
@@ -839,17 +882,55 @@ __global__ void __launch_bounds__(kCrtDThreads, 8) crt3d_k1(const uint64_t* __re
 }
 
 __global__ void __launch_bounds__(kCrtDThreads, 8) crt3d_batch_k1(const uint64_t* __restrict__ Y, size_t istride,
-                                                               size_t pstride, size_t ncoef, CrtDConsts C,
-                                                               uint32_t* __restrict__ z, uint32_t zcap,
-                                                               const uint32_t* __restrict__ zlen, size_t cpp,
-                                                               uint32_t* agg)
+                                                                  size_t pstride, size_t ncoef, CrtDConsts C,
+                                                                  uint32_t* __restrict__ z, uint32_t zcap,
+                                                                  const uint32_t* __restrict__ zlen, size_t cpp,
+                                                                  uint32_t* agg)
 {
     const size_t prod = blockIdx.x / cpp, lc = blockIdx.x % cpp;
     crt3d_block(Y + prod * istride, pstride, ncoef, C, z + prod * (size_t)zcap, zlen[prod], (int64_t)lc,
                 agg + blockIdx.x);
 }
 
-static size_t crt3d_ctas(size_t zw) { return ((zw + 1) / 2 + kCrtDLPC - 1) / kCrtDLPC; }
+// Short products: `per` groups each, `pack` products per CTA (at most 128 groups
+// and kCrtDCoefs coefficients), where one product would leave most of a CTA idle.
+__global__ void __launch_bounds__(kCrtDThreads, 8) crt3d_pack_k1(const uint64_t* __restrict__ Y, size_t istride,
+                                                                 size_t pstride, size_t ncoef, CrtDConsts C,
+                                                                 uint32_t* __restrict__ z, uint32_t zcap,
+                                                                 const uint32_t* __restrict__ zlen, size_t count,
+                                                                 int per, int pack)
+{
+    __shared__ CrtDigits<kCrtDSlots> X;
+    __shared__ uint32_t s_agg;
+    const int stride = 8 * per + 3;  // a product's coefficients, three zeros first
+    const size_t p0 = (size_t)blockIdx.x * pack;
+    const int n = (int)(count - p0 < (size_t)pack ? count - p0 : (size_t)pack);
+    const uint64_t* Yp = Y + p0 * istride;
+    crt_coefs(X, n * stride, C,
+              [&](int i) {
+                  const int q = i / stride, j = i - q * stride - 3;
+                  return j >= 0 && j < crt_limit(ncoef, zlen[p0 + q]) ? (int64_t)q * (int64_t)istride + j : (int64_t)-1;
+              },
+              [&](int64_t at, double& y0, double& y1, double& y2) {
+                  y0 = dbits(Yp[at]);
+                  y1 = dbits(Yp[pstride + at]);
+                  y2 = dbits(Yp[2 * pstride + at]);
+              });
+    __syncthreads();
+    uint64_t t[8];
+    const int q = (int)threadIdx.x / per, g = (int)threadIdx.x - q * per;
+    const bool mine = q < n;
+    if (mine) crt_group(X, q * stride + 8 * g + 3, t);
+    uint32_t* W = reinterpret_cast<uint32_t*>(&X);
+    digits_to_words(t, mine, g == per - 1, W, &s_agg);
+    const int words = 14 * per;
+    for (int i = threadIdx.x; i < n * words; i += kCrtDThreads) {
+        const int r = i / words, w = i - r * words;
+        if ((uint32_t)w < zlen[p0 + r]) z[(p0 + r) * (size_t)zcap + w] = W[i];
+    }
+}
+
+static size_t crt3d_ctas(size_t zw) { return (zw + kCrtDWPC - 1) / kCrtDWPC; }
 
 // Inverse-transformed residues (product length 2^k, prime q at y + q pstride)
 // -> zw words; mail receives the top one.
@@ -874,6 +955,17 @@ void ntt3d_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, siz
     if (count == 0) return;
     if (ncoef == 0) ncoef = (size_t)1 << k;
     const CrtDConsts C = make_crtd(k, offset);
+    // products of at most half a CTA's groups share CTAs
+    const int per = (int)((zcap + 13) / 14);
+    const int pack = std::min(kCrtDThreads / std::max(per, 1), kCrtDCoefs / (8 * per + 3));
+    if (per >= 1 && pack >= 2) {
+        ProfScope ps(KC_CRT, (24.0 * (double)ncoef + 4.0 * zcap) * (double)count, s);
+        crt3d_pack_k1<<<(unsigned)((count + pack - 1) / pack), kCrtDThreads, 0, s>>>(y, istride, pstride, ncoef, C, z,
+                                                                                  zcap, zlen, count, per, pack);
+        PIC_CHECK_LAUNCH();
+        count_launch();
+        return;
+    }
     const size_t cpp = crt3d_ctas(zcap);
     const size_t nctas = count * cpp;
     DevBuf<uint32_t> agg(nctas, s);

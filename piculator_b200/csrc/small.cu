@@ -4,7 +4,7 @@
 // A cluster of three CTAs multiplies two operands, one CTA per prime: it reads
 // the operands' pieces, transforms both in shared memory, multiplies and
 // transforms back (middle.cuh), all without leaving the SM; then each CTA
-// takes a third of the product's limbs, reads the other two primes' residues
+// takes a third of the product's words, reads the other two primes' residues
 // through distributed shared memory for the CRT and passes its carry on the
 // same way.  A product of this length is bound by latency: as separate
 // launches (forward, product and inverse of a main and a tail transform,
@@ -38,8 +38,8 @@ template <int LR>
 struct SmallShape {
     static constexpr int TOT = 1 << LR;
     static constexpr int PER = (TOT / 8 + 3) / 3;                // groups per CTA, at most
-    static constexpr int XS = crt_slot(8 * PER + 3);             // slots per limb
-    static constexpr size_t SMEM = 8 * (size_t)(TOT + (3 * XS > TOT ? 3 * XS : TOT));
+    static constexpr int XS = (crt_slot(8 * PER + 3) + 1) & ~1;  // digit slots
+    static constexpr size_t SMEM = 8 * (size_t)TOT + std::max(8 * (size_t)TOT, sizeof(CrtDigits<XS>));
 };
 
 // Operand rows a, b; afterwards row 0 holds the residues and b's place the
@@ -94,30 +94,33 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(MiddleShape<LR, 0>::
     auto out = [&](int, int, int e, double v) { ms[place(e)] = v; };
     inverse_rounds<LR, 0, Sh::NR - 2>(ms, L, ti, 1, act, out);
     cluster.sync();
-    // limbs: 7 per group of 8 coefficients, a third of the groups per CTA
+    // words: 14 per group of 8 coefficients, a third of the groups per CTA
     const double* Y[3];
 #pragma unroll
     for (int r = 0; r < 3; r++) Y[r] = cluster.map_shared_rank(ms, r);
     const uint32_t zw = D.na + D.nb;
     const int ncoef = (int)((32 * (size_t)D.na + 55) / 56 + (32 * (size_t)D.nb + 55) / 56 - 1);
     const int jlim = min(ncoef, (int)((32 * (size_t)zw + 55) / 56));
-    const int groups = (int)(((zw + 1) / 2 + 6) / 7), per = (groups + 2) / 3;
+    const int groups = (int)((zw + 13) / 14), per = (groups + 2) / 3;
     const int u = (int)q * per + (int)threadIdx.x;
     const bool mine = (int)threadIdx.x < per && u < groups;
-    uint64_t* X = reinterpret_cast<uint64_t*>(ms + TOT);  // b's place and some more
-    constexpr int XS = SmallShape<LR>::XS;
-    crt_coefs<XS>(X, 8 * (int)q * per - 3, 8 * per + 3, jlim, M.C, [&](int64_t j, double& y0, double& y1, double& y2) {
-        const int at = place((int)j);
-        y0 = Y[0][at];
-        y1 = Y[1][at];
-        y2 = Y[2][at];
-    });
+    using Digits = CrtDigits<SmallShape<LR>::XS>;
+    Digits& X = *reinterpret_cast<Digits*>(ms + TOT);  // b's place and some more
+    const int j0 = 8 * (int)q * per - 3;
+    crt_coefs(X, 8 * per + 3, M.C, [&](int i) { return j0 + i < jlim ? (int64_t)(j0 + i) : (int64_t)-1; },
+              [&](int64_t j, double& y0, double& y1, double& y2) {
+                  const int at = place((int)j);
+                  y0 = Y[0][at];
+                  y1 = Y[1][at];
+                  y2 = Y[2][at];
+              });
     __syncthreads();
-    uint64_t dig[7] = {0, 0, 0, 0, 0, 0, 0};
-    uint32_t gen[7] = {0, 0, 0, 0, 0, 0, 0};
-    if (mine) crt_digits<XS>(X, threadIdx.x, dig, gen);
+    uint64_t t[8];
+    if (mine) crt_group(X, 8 * (int)threadIdx.x + 3, t);
     const size_t wb = 14 * (size_t)q * per, we = min((size_t)zw, wb + 14 * (size_t)per);
-    limbs_to_words<7>(dig, gen, mine ? 7 * (size_t)u : (size_t)zw, D.z, we, &s_total);
+    uint32_t* W = reinterpret_cast<uint32_t*>(ms + TOT);
+    digits_to_words(t, mine, false, W, &s_total);
+    for (size_t i = wb + threadIdx.x; i < we; i += NT) D.z[i] = W[i - wb];
     cluster.sync();
     uint32_t cin = 0;
     for (uint32_t r = 0; r < q; r++) {

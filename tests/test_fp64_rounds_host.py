@@ -1,6 +1,8 @@
 """The FP64 form's forward register rounds (tests/host/fp64_round_check.c):
 with only the named outputs reduced, values stay in the FP64 quotient's range
-and every output within what the next round accepts, exactly congruent."""
+and every output within what the next round accepts, exactly congruent.  And
+its CRT (tests/host/crt56_check.c): the coefficient's base-2^56 digits from any
+representatives the inverse transforms leave."""
 from __future__ import annotations
 
 import os
@@ -19,4 +21,13 @@ def test_forward_round_ranges(tmp_path, bits):
     subprocess.run(["gcc", "-O2", "-ffp-contract=off", "-o", str(exe),
                     os.path.join(HERE, "host", "fp64_round_check.c"), "-lm"], check=True)
     out = subprocess.run([str(exe), str(bits), "200000"], capture_output=True, text=True)
+    assert out.returncode == 0 and out.stdout.startswith("bad=0"), out.stdout + out.stderr
+
+
+@pytest.mark.skipif(shutil.which("gcc") is None, reason="gcc not available")
+def test_crt_digits_exact(tmp_path):
+    exe = tmp_path / "crt56_check"
+    subprocess.run(["gcc", "-O2", "-ffp-contract=off", "-o", str(exe), os.path.join(HERE, "host", "crt56_check.c"),
+                    "-lm"], check=True)
+    out = subprocess.run([str(exe), "300000"], capture_output=True, text=True)
     assert out.returncode == 0 and out.stdout.startswith("bad=0"), out.stdout + out.stderr

@@ -91,3 +91,22 @@ def test_bsr_fp64_and_integer_forms_agree(pic, a, b, p, wrap):
             pic.set_tuning(k, v)
     for name, g, w in zip("PQR", got, want):
         assert _same(g, w), name
+
+
+# Short merged products share the conversion's CTAs: many parents of 2 .. 128
+# groups each, a ragged last CTA, against the integer form.
+@pytest.mark.parametrize("terms,p", [(1001, 40), (1500, 100), (2999, 300), (777, 700)])
+def test_bsr_packed_conversions(pic, terms, p):
+    knobs = {pic.TUNE_BSR_SCHOOL_MAX: 8, pic.TUNE_NTT_FORM: 0}
+    saved = {k: pic.get_tuning(k) for k in knobs}
+    try:
+        for k, v in knobs.items():
+            pic.set_tuning(k, v)
+        want = [x.to_bf() for x in pic.bsr(5, 5 + terms, p, pic.PI_CHOSEN)]
+        pic.set_tuning(pic.TUNE_NTT_FORM, 1)
+        got = pic.bsr(5, 5 + terms, p, pic.PI_CHOSEN)
+    finally:
+        for k, v in saved.items():
+            pic.set_tuning(k, v)
+    for name, g, w in zip("PQR", got, want):
+        assert _same(g, w), name
