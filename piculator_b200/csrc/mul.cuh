@@ -27,6 +27,10 @@ struct DevDesc {
     uint32_t na, nb;
 };
 void mul_small(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s, Mail* mail);
+// z + i zs = (a + i as) b for i < count, operands of na and nb words, where AUTO
+// would take this form for each; false (nothing done) where it would not.
+bool mul_small_uniform(uint32_t* z, size_t zs, const uint32_t* a, size_t as, size_t na, const uint32_t* b, size_t nb,
+                       size_t count, cudaStream_t s);
 // Products d[idx[i]], i < count, of at most 2^k coefficients.
 void mul_small_batch(const DevDesc* d, const uint32_t* idx, size_t count, int k, cudaStream_t s);
 // FP64-form building blocks: batched inverse output like ntt3_batch_to_words

@@ -26,9 +26,10 @@ namespace cg = cooperative_groups;
 namespace pic {
 
 struct SmallArgs {
-    const DevDesc* d;     // null: the one product below
+    const DevDesc* d;     // null: the product(s) below
     const uint32_t* idx;  // product i is d[idx[i]]
     DevDesc one;
+    size_t zs, as;  // without d: product i is one.z + i zs = (one.a + i as) one.b
     MailRef mail;  // the product's top word
     CrtDConsts C;
     PrimeDev prime[3];
@@ -60,7 +61,13 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(MiddleShape<LR, 0>::
     const Dbl::Ctx L = Dbl::ctx(P);
     const double* __restrict__ tf = reinterpret_cast<const double*>(P.lvl_fwd);
     const double* __restrict__ ti = reinterpret_cast<const double*>(P.lvl_inv);
-    const DevDesc D = M.d != nullptr ? M.d[M.idx[item]] : M.one;
+    DevDesc D = M.one;
+    if (M.d != nullptr) {
+        D = M.d[M.idx[item]];
+    } else {
+        D.z += item * M.zs;
+        D.a += item * M.as;
+    }
     const bool square = D.a == D.b && D.na == D.nb;
     auto in = [&](int i, int, int e) -> double {
         return dpiece56(src_piece56_raw(i == 0 ? D.a : D.b, i == 0 ? D.na : D.nb, e), L.p, L.pinv);
@@ -175,6 +182,23 @@ void mul_small(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, siz
     m.one = DevDesc{z, a, b, (uint32_t)na, (uint32_t)nb};
     if (mail) m.mail = mail->ref();
     small_products(m, 1, k, s);
+}
+
+bool mul_small_uniform(uint32_t* z, size_t zs, const uint32_t* a, size_t as, size_t na, const uint32_t* b, size_t nb,
+                       size_t count, cudaStream_t s)
+{
+    if (count == 0) return true;
+    const size_t ncoef = pieces56(na) + pieces56(nb) - 1;
+    if (mul_auto_mode(na, nb) != PIC_MUL_NTT3D || ncoef > ((size_t)1 << kSmallMaxBits)) return false;
+    int k = kSmallMinBits;
+    while (((size_t)1 << k) < ncoef) k++;
+    SmallArgs m{};
+    m.one = DevDesc{z, a, b, (uint32_t)na, (uint32_t)nb};
+    m.zs = zs;
+    m.as = as;
+    count_products(count);
+    small_products(m, count, k, s);
+    return true;
 }
 
 void mul_small_batch(const DevDesc* d, const uint32_t* idx, size_t count, int k, cudaStream_t s)
