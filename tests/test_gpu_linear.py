@@ -64,6 +64,24 @@ def test_random_sums_and_differences(pic, n):
     assert x.ucmp(y) == (_val(a) > _val(b)) - (_val(a) < _val(b))
 
 
+@pytest.mark.parametrize("n", [8191, 8192, 8193, 16385, 65535, 65536, 65537])
+def test_one_launch_edges(pic, n):
+    """Up to 65,536 words a cluster of CTAs of 8192 words does all of an operation;
+    a difference cut to a window compares the words under it as well."""
+    a, b = random_words(3 * n, n), random_words(3 * n + 1, n)
+    a[n // 2:] = b[n // 2:]
+    x, y = _num(pic, a), _num(pic, b)
+    assert _int(x.add(y)) == _val(a) + _val(b)
+    assert _int(x.sub(y)) == _val(a) - _val(b)
+    assert _int(x.mul_u32(0xFFFFFFFB)) == _val(a) * 0xFFFFFFFB
+    ones = np.full(n, 0xFFFFFFFF, dtype=np.uint32)
+    assert _int(_num(pic, ones).add(pic.DeviceBigFloat.from_u32(1))) == _val(ones) + 1
+    for lo in (0, 5, n // 2 - 1):  # the window drops the words that differ: zero
+        c = a.copy()
+        c[lo] ^= 1
+        assert _num(pic, c).sub(x, n // 2 - 4).info()[2] == 0
+
+
 def test_ordered_differences_from_several_threads(pic):
     def work(seed, bad):
         a, b = random_words(seed, 5000), random_words(seed + 1, 5000)
