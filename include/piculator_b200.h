@@ -299,7 +299,7 @@ enum {
     PIC_TUNE_MUL_FFT_MAX = 2,    /* products up to this many words: FP64 FFT in AUTO (0: never) */
     PIC_TUNE_BATCH_GRAPHS = 3,   /* 1: pic_mul_batch replays captured CUDA graphs (default) */
     PIC_TUNE_BSR_WRAP = 4,       /* 1: binary-splitting NTT merges use wrapped products (default) */
-    PIC_TUNE_BSR_SMALL_MERGE = 5, /* short schoolbook levels: 0 CTA, 1 + warp, 2 + thread per parent (default) */
+    PIC_TUNE_BSR_SMALL_MERGE = 5, /* 2: the shortest nodes' merges a thread per parent (default); 0, 1: not */
     PIC_TUNE_MUL_WRAP = 6,        /* 1: three-prime products use the wrapped form when it is shorter (default) */
     PIC_TUNE_BSR_COMBINE = 7,     /* 1: binary-splitting NTT merges form P in the transform domain (default) */
     PIC_TUNE_FFT_ACCEPT_PPM = 8,  /* FFT products whose max rounding distance exceeds value * 1e-6 are

@@ -1,0 +1,119 @@
+// Schoolbook products in 8 x 8-word register blocks.
+//
+// An operand of n words is ceil(n / 8) blocks.  Thread d of a product of na by
+// nb blocks (na <= nb) takes the blocks (i, (d - i) mod nb) for i = 0 .. na-1:
+// first the diagonal d, then, past the wrap, the diagonal d + nb, so every
+// thread does the same work (a thread per diagonal or per column would do
+// between none and all of it) and block i of the first operand is one address
+// for all threads.  A diagonal's sum (17 words) goes to shared memory, where
+// three neighbouring diagonals make a result word.
+#pragma once
+#include <stdint.h>
+
+namespace pic {
+
+constexpr int kDiagWords = 17;  // 16 words and the overflow of up to 2^32 blocks; odd: no bank conflicts
+
+// e[0..8] += a * (b0, b2, b4, b6) at even distances (e[8]: the carry out)
+__device__ __forceinline__ void mad_row(uint32_t* e, uint32_t a, uint32_t b0, uint32_t b2, uint32_t b4, uint32_t b6)
+{
+    asm("mad.lo.cc.u32 %0,%9,%10,%0; madc.hi.cc.u32 %1,%9,%10,%1;"
+        "madc.lo.cc.u32 %2,%9,%11,%2; madc.hi.cc.u32 %3,%9,%11,%3;"
+        "madc.lo.cc.u32 %4,%9,%12,%4; madc.hi.cc.u32 %5,%9,%12,%5;"
+        "madc.lo.cc.u32 %6,%9,%13,%6; madc.hi.cc.u32 %7,%9,%13,%7; addc.u32 %8,%8,0;"
+        : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]), "+r"(e[8])
+        : "r"(a), "r"(b0), "r"(b2), "r"(b4), "r"(b6));
+}
+
+// x[0..17) += y[0..16)
+__device__ __forceinline__ void add16(uint32_t* x, const uint32_t* y)
+{
+    asm("add.cc.u32 %0,%0,%17; "
+        "addc.cc.u32 %1,%1,%18; addc.cc.u32 %2,%2,%19; addc.cc.u32 %3,%3,%20; addc.cc.u32 %4,%4,%21; "
+        "addc.cc.u32 %5,%5,%22; addc.cc.u32 %6,%6,%23; addc.cc.u32 %7,%7,%24; addc.cc.u32 %8,%8,%25; "
+        "addc.cc.u32 %9,%9,%26; addc.cc.u32 %10,%10,%27; addc.cc.u32 %11,%11,%28; addc.cc.u32 %12,%12,%29; "
+        "addc.cc.u32 %13,%13,%30; addc.cc.u32 %14,%14,%31; addc.cc.u32 %15,%15,%32; addc.u32 %16,%16,0;"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]), "+r"(x[8]),
+          "+r"(x[9]), "+r"(x[10]), "+r"(x[11]), "+r"(x[12]), "+r"(x[13]), "+r"(x[14]), "+r"(x[15]), "+r"(x[16])
+        : "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]), "r"(y[4]), "r"(y[5]), "r"(y[6]), "r"(y[7]),
+          "r"(y[8]), "r"(y[9]), "r"(y[10]), "r"(y[11]), "r"(y[12]), "r"(y[13]), "r"(y[14]), "r"(y[15]));
+}
+
+// acc[0..17) += a[0..8) * b[0..8).  The products at even and at odd word
+// distances are summed apart, each a chain of 64-bit multiply-adds whose carry
+// ends in a word that was zero; the two sums are then added to acc.
+__device__ __forceinline__ void mac_block(uint32_t (&acc)[kDiagWords], const uint32_t (&a)[8], const uint32_t (&b)[8])
+{
+    uint32_t e[18], o[18];  // o[k]: word k as well; o[0] stays 0
+#pragma unroll
+    for (int x = 0; x < 18; x++) e[x] = o[x] = 0;
+#pragma unroll
+    for (int x = 0; x < 8; x++) {
+        mad_row((x & 1 ? o : e) + x, a[x], b[0], b[2], b[4], b[6]);
+        mad_row((x & 1 ? e : o) + x + 1, a[x], b[1], b[3], b[5], b[7]);
+    }
+    add16(acc, e);
+    add16(acc, o);
+}
+
+__device__ __forceinline__ void load_block(uint32_t (&x)[8], const uint32_t* p)
+{
+    const uint4 lo = *reinterpret_cast<const uint4*>(p), hi = *reinterpret_cast<const uint4*>(p + 4);
+    x[0] = lo.x, x[1] = lo.y, x[2] = lo.z, x[3] = lo.w;
+    x[4] = hi.x, x[5] = hi.y, x[6] = hi.z, x[7] = hi.w;
+}
+
+// Thread d's share of a product of na x nb blocks (na <= nb, d < nb): diagonals
+// d and d + nb (where there are) to diag[kDiagWords * diagonal].
+__device__ __forceinline__ void block_diagonals(const uint32_t* a, int na, const uint32_t* b, int nb, int d,
+                                                uint32_t* diag)
+{
+    uint32_t acc[kDiagWords];
+#pragma unroll
+    for (int w = 0; w < kDiagWords; w++) acc[w] = 0;
+    int j = d;
+    uint32_t* out = diag + kDiagWords * d;
+#pragma unroll 1
+    for (int i = 0; i < na; i++) {
+        if (j < 0) {  // past the wrap
+            j += nb;
+#pragma unroll
+            for (int w = 0; w < kDiagWords; w++) {
+                out[w] = acc[w];
+                acc[w] = 0;
+            }
+            out += kDiagWords * nb;
+        }
+        uint32_t x[8], y[8];
+        load_block(x, a + 8 * i);
+        load_block(y, b + 8 * j);
+        mac_block(acc, x, y);
+        j--;
+    }
+#pragma unroll
+    for (int w = 0; w < kDiagWords; w++) out[w] = acc[w];
+}
+
+// Result words of block c (words 8 c .. 8 c + 7) of a product whose nd
+// diagonals are at diag: f(r, t, g) for r = 0 .. 7 in order, the digit t before
+// carries and its generate bit g (a digit with g is at most 1, so it cannot
+// propagate as well).
+template <class F>
+__device__ __forceinline__ void block_digits(const uint32_t* diag, int nd, int c, const F& f)
+{
+    const uint32_t* lo = diag + kDiagWords * c;
+    const uint32_t* hi = lo - kDiagWords + 8;
+    const bool hl = c < nd, hh = c >= 1;
+    uint64_t prev = 0;  // the sum one word below
+    if (hh) prev = (uint64_t)lo[7 - kDiagWords] + (c >= 2 ? hi[7 - kDiagWords] : 0u);
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        uint64_t s = (uint64_t)(hl ? lo[r] : 0u) + (hh ? hi[r] : 0u);
+        if (r == 0 && c >= 2) s += lo[16 - 2 * kDiagWords];
+        const uint64_t t = (s & 0xffffffffu) + (prev >> 32);
+        f(r, (uint32_t)t, (uint32_t)(t >> 32));
+        prev = s;
+    }
+}
+
+}  // namespace pic

@@ -9,8 +9,8 @@
 // in a few launches, with every value resident in HBM in fixed-capacity slots:
 //   * bottom depth (node lengths 1 or 2): one thread per node, leaf formulas
 //     (PI.h:67-88) and the two-leaf merge in registers;
-//   * short children: one CTA per parent, schoolbook column sums and
-//     carry-lookahead scans in shared memory;
+//   * short children: schoolbook products in registers, one thread per parent
+//     of the shortest nodes, else one CTA whose threads take 8 x 8-word blocks;
 //   * long children: batched three-prime NTT, each child transformed once and
 //     reused by the two products that need it (the transform-domain reuse that
 //     Transform.h was written for), CRT + carry per product, then a batched
@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "bigfloat.hpp"
+#include "blockmul.cuh"
 #include "bsr.cuh"
 #include "carry.cuh"
 #include "common.cuh"
@@ -588,6 +589,157 @@ __global__ void __launch_bounds__(256) merge_school_kernel(MergeArgs m)
 }
 
 // ---------------------------------------------------------------------------
+// The same merge with the four products side by side, each in register blocks
+// (blockmul.cuh): one CTA per parent, a thread per block row of a product, one
+// carry scan over the words of all four.  The column sums below spend most of
+// their issue slots on carries, shared-memory reads and columns of uneven
+// length; here a block of 64 multiply-adds costs 8 shared-memory words' reads
+// (two 16-byte loads an operand) and about 250 slots for 200 at the multiplier's
+// full rate.  Levels of a 1e9-digit computation with children of up to 75, 150
+// and 300 words: 23, 38 and 75 -> 17, 17 and 25 ms; of up to 38 words, which had
+// a warp per parent, 23 -> 13 ms.
+struct BlockMergeShape {
+    uint32_t bP, bQ, bR;  // blocks of a child slot
+    __host__ __device__ uint32_t operands() const { return 2 * (bP + bQ + bR); }
+    __host__ __device__ uint32_t diagonals() const { return 2 * bP + 3 * bQ + 3 * bR; }  // of the four products
+    __host__ __device__ uint32_t words() const { return 8 * operands() + kDiagWords * diagonals(); }
+    uint32_t rows() const { return std::max(bP, bQ) + std::max(bP, bR) + bQ + bR; }
+};
+constexpr int kBlockMergeThreads = 512;
+
+__global__ void __launch_bounds__(kBlockMergeThreads, 2) merge_block_kernel(MergeArgs m, BlockMergeShape S)
+{
+    extern __shared__ __align__(16) uint32_t sm[];
+    __shared__ uint32_t s_top[4];  // a product's highest word
+    const size_t i = blockIdx.x;
+    const size_t L = 2 * i, R = 2 * i + 1;
+    const uint32_t T = blockDim.x;
+    const uint32_t nPL = m.cPl[L], nQL = m.cQl[L], nRL = m.cRl[L];
+    const uint32_t nPR = m.cPl[R], nQR = m.cQl[R], nRR = m.cRl[R];
+    const bool sL = m.cS[L] != 0, sR = m.cS[R] != 0;
+    uint32_t* PL = sm;
+    uint32_t* PR = PL + 8 * S.bP;
+    uint32_t* QL = PR + 8 * S.bP;
+    uint32_t* QR = QL + 8 * S.bQ;
+    uint32_t* RL = QR + 8 * S.bQ;
+    uint32_t* RR = RL + 8 * S.bR;
+    uint32_t* diag = RR + 8 * S.bR;
+    // operands, whole blocks, zero above their length
+    const uint32_t bmax = 8 * max(S.bP, max(S.bQ, S.bR));
+    for (uint32_t k = threadIdx.x; k < bmax; k += T) {
+        const uint32_t pl = k < nPL ? m.cPw[L * m.ccP + k] : 0u, pr = k < nPR ? m.cPw[R * m.ccP + k] : 0u;
+        const uint32_t ql = k < nQL ? m.cQw[L * m.ccQ + k] : 0u, qr = k < nQR ? m.cQw[R * m.ccQ + k] : 0u;
+        const uint32_t rl = k < nRL ? m.cRw[L * m.ccR + k] : 0u, rr = k < nRR ? m.cRw[R * m.ccR + k] : 0u;
+        if (k < 8 * S.bP) PL[k] = pl, PR[k] = pr;
+        if (k < 8 * S.bQ) QL[k] = ql, QR[k] = qr;
+        if (k < 8 * S.bR) RL[k] = rl, RR[k] = rr;
+    }
+    __syncthreads();
+    // product p: PL QR, PR RL, QL QR, RL RR, the operand of fewer blocks first
+    auto op = [&](int p, const uint32_t*& a, uint32_t& na, const uint32_t*& b, uint32_t& nb) {
+        a = p == 0 ? PL : (p == 1 ? PR : (p == 2 ? QL : RL));
+        na = p == 0 ? nPL : (p == 1 ? nPR : (p == 2 ? nQL : nRL));
+        b = p == 0 || p == 2 ? QR : (p == 1 ? RL : RR);
+        nb = p == 0 || p == 2 ? nQR : (p == 1 ? nRL : nRR);
+        if (na > nb) {
+            const uint32_t* x = a;
+            a = b;
+            b = x;
+            const uint32_t n = na;
+            na = nb;
+            nb = n;
+        }
+    };
+    auto blocks = [](uint32_t n) { return (n + 7) / 8; };
+    uint32_t first_row[5], first_blk[5];  // of each product, in the lists of rows and of result blocks
+    first_row[0] = first_blk[0] = 0;
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+        const uint32_t *a, *b;
+        uint32_t na, nb;
+        op(p, a, na, b, nb);
+        first_row[p + 1] = first_row[p] + (na ? blocks(nb) : 0u);
+        first_blk[p + 1] = first_blk[p] + (na ? blocks(na) + blocks(nb) : 0u);
+    }
+    for (uint32_t t = threadIdx.x; t < first_row[4]; t += T) {
+        const int p = t < first_row[1] ? 0 : (t < first_row[2] ? 1 : (t < first_row[3] ? 2 : 3));
+        const uint32_t r0 = p == 0 ? 0u : (p == 1 ? first_row[1] : (p == 2 ? first_row[2] : first_row[3]));
+        const uint32_t b0 = p == 0 ? 0u : (p == 1 ? first_blk[1] : (p == 2 ? first_blk[2] : first_blk[3]));
+        const uint32_t *a, *b;
+        uint32_t na, nb;
+        op(p, a, na, b, nb);
+        block_diagonals(a, (int)blocks(na), b, (int)blocks(nb), (int)(t - r0), diag + kDiagWords * b0);
+    }
+    if (threadIdx.x < 4) s_top[threadIdx.x] = 0;
+    __syncthreads();
+    // words: a thread takes consecutive result blocks.  No carry leaves a product
+    // (its blocks reach past its highest word), so one scan serves all four.
+    const uint32_t nblk = first_blk[4], per = (nblk + T - 1) / T;
+    const uint32_t q0 = min(threadIdx.x * per, nblk), q1 = min(q0 + per, nblk);
+    auto at = [&](uint32_t q, int& p, uint32_t& b0, uint32_t& nd) {
+        p = q < first_blk[1] ? 0 : (q < first_blk[2] ? 1 : (q < first_blk[3] ? 2 : 3));
+        b0 = p == 0 ? 0u : (p == 1 ? first_blk[1] : (p == 2 ? first_blk[2] : first_blk[3]));
+        nd = (p == 0 ? first_blk[1] : (p == 1 ? first_blk[2] : (p == 2 ? first_blk[3] : first_blk[4]))) - b0 - 1;
+    };
+    uint32_t gp = kGPIdentity;
+    for (uint32_t q = q0; q < q1; q++) {
+        int p;
+        uint32_t b0, nd;
+        at(q, p, b0, nd);
+        block_digits(diag + kDiagWords * b0, (int)nd, (int)(q - b0), [&](int, uint32_t t, uint32_t g) {
+            gp = gp_combine(gp, g | ((uint32_t)(t == 0xffffffffu) << 1));
+        });
+    }
+    uint32_t total;
+    uint32_t cin = block_gp_scan(gp, &total) & 1u;
+    // T1 and T2 over the operands (read above), Q and R to the parent's slots
+    uint32_t* t1 = sm;
+    uint32_t* t2 = t1 + 8 * first_blk[1];
+    for (uint32_t q = q0; q < q1; q++) {
+        int p;
+        uint32_t b0, nd;
+        at(q, p, b0, nd);
+        const uint32_t zw = p == 0 ? nPL + nQR : (p == 1 ? nPR + nRL : (p == 2 ? nQL + nQR : nRL + nRR));
+        uint32_t* z = p == 0 ? t1 : (p == 1 ? t2 : (p == 2 ? m.pQw + i * m.pcQ : m.pRw + i * m.pcR));
+        const uint32_t w0 = 8 * (q - b0);
+        block_digits(diag + kDiagWords * b0, (int)nd, (int)(q - b0), [&](int r, uint32_t t, uint32_t g) {
+            const uint32_t w = w0 + r, v = t + cin;
+            cin = g | ((uint32_t)(t == 0xffffffffu) & cin);
+            if (w + 1 < zw || (w + 1 == zw && v != 0)) z[w] = v;
+            if (w + 1 == zw) s_top[p] = v;
+        });
+    }
+    __syncthreads();
+    auto len = [&](int p, uint32_t na, uint32_t nb) {
+        return na == 0 || nb == 0 ? 0u : na + nb - (s_top[p] == 0 ? 1u : 0u);
+    };
+    const uint32_t n1 = len(0, nPL, nQR), n2 = len(1, nPR, nRL), nQ = len(2, nQL, nQR), nR = len(3, nRL, nRR);
+    // P = PL QR + PR RL (PI.h:110)
+    bool sP;
+    const uint32_t nP = cta_signed_add(sL, t1, n1, sR, t2, n2, diag, &sP);
+    for (uint32_t k = threadIdx.x; k < nP; k += T) m.pPw[i * m.pcP + k] = diag[k];
+    if (threadIdx.x == 0) {
+        m.pPl[i] = nP;
+        m.pQl[i] = nQ;
+        m.pRl[i] = nR;
+        m.pS[i] = sP ? 1 : 0;
+    }
+}
+
+// Whether the children fit the register-block merge's shared memory.
+static bool launch_merge_block(const MergeArgs& m, cudaStream_t s)
+{
+    BlockMergeShape S{(m.ccP + 7) / 8, (m.ccQ + 7) / 8, (m.ccR + 7) / 8};
+    const size_t smem = sizeof(uint32_t) * (size_t)S.words();
+    if (smem > 200 * 1024) return false;
+    if (smem > 48 * 1024)
+        PIC_CUDA(cudaFuncSetAttribute(merge_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const uint32_t threads = std::min<uint32_t>(kBlockMergeThreads, (S.rows() + 31) / 32 * 32);
+    merge_block_kernel<<<(unsigned)m.count, threads, smem, s>>>(m, S);
+    return true;
+}
+
+// ---------------------------------------------------------------------------
 // Thread-per-parent merge for the shortest nodes: every operand and product
 // in registers (fixed capacities CP, CQ, CR >= the child slots), fully
 // unrolled word loops, the same results as merge_school_kernel.
@@ -667,210 +819,6 @@ static bool launch_merge_thread(const MergeArgs& m, cudaStream_t s)
     if (m.ccP > (uint32_t)CP || m.ccQ > (uint32_t)CQ || m.ccR > (uint32_t)CR) return false;
     merge_thread_kernel<CP, CQ, CR><<<(unsigned)((m.count + 127) / 128), 128, 0, s>>>(m);
     return true;
-}
-
-// ---------------------------------------------------------------------------
-// Warp-per-parent schoolbook merge for short nodes (every child slot <= 64
-// words): the same arithmetic as merge_school_kernel with warp-wide scans and
-// __syncwarp instead of block barriers, several parents per CTA, and the six
-// child operands fetched with independent loads.
-
-constexpr int kWarpMergeMax = 64;  // largest child slot (words)
-constexpr int kWarpMergeWarps = 8;
-
-// Exclusive warp scan of one (g, p) per lane, lanes in position order.
-__device__ __forceinline__ uint32_t warp_gp_scan(uint32_t gp, uint32_t* total)
-{
-    const int lane = threadIdx.x & 31;
-    uint32_t v = gp;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t o = __shfl_up_sync(0xffffffffu, v, off);
-        if (lane >= off) v = gp_combine(o, v);
-    }
-    uint32_t excl = __shfl_up_sync(0xffffffffu, v, 1);
-    if (lane == 0) excl = kGPIdentity;
-    *total = __shfl_sync(0xffffffffu, v, 31);
-    return excl;
-}
-
-// z[0..na+nb) = a * b in the warp's shared region; col holds 3 (na + nb)
-// words.  Returns the length without the leading zero word (0 if empty).
-__device__ uint32_t warp_mul(const uint32_t* a, uint32_t na, const uint32_t* b, uint32_t nb, uint32_t* z,
-                             uint32_t* col)
-{
-    const int lane = threadIdx.x & 31;
-    if (na == 0 || nb == 0) return 0;
-    const uint32_t zw = na + nb;
-    for (uint32_t g = lane; 4 * g < zw; g += 32) colsum4(a, (int)na, b, (int)nb, (int)(4 * g), zw, col);
-    __syncwarp();
-    const uint32_t per = (zw + 31) / 32;
-    const uint32_t w0 = lane * per, w1 = min(w0 + per, zw);
-    auto digit = [&](uint32_t w, uint32_t& g) -> uint32_t {
-        uint64_t sw = col[3 * w], sp = 0;
-        if (w >= 1) {
-            sw += col[3 * (w - 1) + 1];
-            sp += col[3 * (w - 1)];
-        }
-        if (w >= 2) {
-            sw += col[3 * (w - 2) + 2];
-            sp += col[3 * (w - 2) + 1];
-        }
-        if (w >= 3) sp += col[3 * (w - 3) + 2];
-        const uint64_t t = (sw & 0xffffffffu) + (sp >> 32);
-        g = (uint32_t)(t >> 32);
-        return (uint32_t)t;
-    };
-    uint32_t gp = kGPIdentity;
-    for (uint32_t w = w0; w < w1; w++) {
-        uint32_t g;
-        const uint32_t d = digit(w, g);
-        gp = gp_combine(gp, g | ((uint32_t)(d == 0xffffffffu) << 1));
-    }
-    uint32_t total;
-    uint32_t cin = warp_gp_scan(gp, &total) & 1u;
-    for (uint32_t w = w0; w < w1; w++) {
-        uint32_t g;
-        const uint32_t d = digit(w, g);
-        z[w] = d + cin;
-        cin = g | ((uint32_t)(d == 0xffffffffu) & cin);
-    }
-    __syncwarp();
-    return z[zw - 1] == 0 ? zw - 1 : zw;
-}
-
-// Signed sum of magnitudes into z (capacity max(na, nb) + 1); the reference's
-// sign dispatch (BigFloat.cpp:288-305) on exact operands.
-__device__ uint32_t warp_signed_add(bool sa, const uint32_t* a, uint32_t na, bool sb, const uint32_t* b, uint32_t nb,
-                                    uint32_t* z, bool* sz)
-{
-    const int lane = threadIdx.x & 31;
-    const uint32_t n = max(na, nb);
-    auto A = [&](uint32_t i) -> uint32_t { return i < na ? a[i] : 0u; };
-    auto B = [&](uint32_t i) -> uint32_t { return i < nb ? b[i] : 0u; };
-    const bool sub = sa != sb;
-    bool swap = false;
-    if (sub) {
-        unsigned long long mine = 0;
-        for (uint32_t i = lane; i < n; i += 32)
-            if (A(i) != B(i)) mine = i + 1;
-        const uint32_t h = (uint32_t)warp_max_u64(mine);
-        if (h == 0) {
-            *sz = true;
-            return 0;
-        }
-        swap = A(h - 1) < B(h - 1);
-    }
-    const uint32_t per = (n + 31) / 32;
-    const uint32_t w0 = lane * per, w1 = min(w0 + per, n);
-    uint32_t gp = kGPIdentity;
-    for (uint32_t i = w0; i < w1; i++) {
-        const uint32_t x = swap ? B(i) : A(i), y = swap ? A(i) : B(i);
-        uint32_t d, g, p;
-        if (!sub) {
-            const uint64_t s = (uint64_t)x + y;
-            d = (uint32_t)s;
-            g = (uint32_t)(s >> 32);
-            p = d == 0xffffffffu;
-        } else {
-            d = x - y;
-            g = x < y;
-            p = d == 0u;
-        }
-        gp = gp_combine(gp, g | (p << 1));
-    }
-    uint32_t total;
-    uint32_t cin = warp_gp_scan(gp, &total) & 1u;
-    for (uint32_t i = w0; i < w1; i++) {
-        const uint32_t x = swap ? B(i) : A(i), y = swap ? A(i) : B(i);
-        if (!sub) {
-            const uint64_t s = (uint64_t)x + y;
-            const uint32_t d = (uint32_t)s;
-            z[i] = d + cin;
-            cin = (uint32_t)(s >> 32) | ((uint32_t)(d == 0xffffffffu) & cin);
-        } else {
-            const uint32_t d = x - y;
-            z[i] = d - cin;
-            cin = (uint32_t)(x < y) | ((uint32_t)(d == 0u) & cin);
-        }
-    }
-    __syncwarp();
-    if (!sub) {
-        const uint32_t c = total & 1u;
-        if (lane == 0) z[n] = c;
-        __syncwarp();
-        *sz = sa;
-        return n + c;
-    }
-    unsigned long long mine = 0;
-    for (uint32_t i = lane; i < n; i += 32)
-        if (z[i] != 0) mine = i + 1;
-    const uint32_t len = (uint32_t)warp_max_u64(mine);
-    *sz = len == 0 ? true : (swap ? sb : sa);
-    return len;
-}
-
-// Shared words per warp for child slots (cP, cQ, cR).
-__host__ __device__ inline uint32_t warp_merge_words(uint32_t cP, uint32_t cQ, uint32_t cR)
-{
-    return 2 * (cP + cQ + cR) + (cP + cQ) + (cP + cR) + 3 * (cP + cQ);
-}
-
-__global__ void __launch_bounds__(32 * kWarpMergeWarps) merge_warp_kernel(MergeArgs m)
-{
-    extern __shared__ uint32_t sm[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const size_t i = (size_t)blockIdx.x * kWarpMergeWarps + wid;
-    if (i >= m.count) return;  // whole warps leave together
-    uint32_t* base = sm + (size_t)wid * warp_merge_words(m.ccP, m.ccQ, m.ccR);
-    uint32_t* PL = base;
-    uint32_t* QL = PL + m.ccP;
-    uint32_t* RL = QL + m.ccQ;
-    uint32_t* PR = RL + m.ccR;
-    uint32_t* QR = PR + m.ccP;
-    uint32_t* RR = QR + m.ccQ;
-    uint32_t* t1 = RR + m.ccR;
-    uint32_t* t2 = t1 + m.ccP + m.ccQ;
-    uint32_t* col = t2 + m.ccP + m.ccR;
-    const size_t L = 2 * i, R = 2 * i + 1;
-    const uint32_t nPL = m.cPl[L], nQL = m.cQl[L], nRL = m.cRl[L];
-    const uint32_t nPR = m.cPl[R], nQR = m.cQl[R], nRR = m.cRl[R];
-    const bool sL = m.cS[L] != 0, sR = m.cS[R] != 0;
-    // all six operands' loads issued before any is stored
-    for (uint32_t k = lane; k < (uint32_t)kWarpMergeMax; k += 32) {
-        const uint32_t pl = k < nPL ? m.cPw[L * m.ccP + k] : 0u;
-        const uint32_t ql = k < nQL ? m.cQw[L * m.ccQ + k] : 0u;
-        const uint32_t rl = k < nRL ? m.cRw[L * m.ccR + k] : 0u;
-        const uint32_t pr = k < nPR ? m.cPw[R * m.ccP + k] : 0u;
-        const uint32_t qr = k < nQR ? m.cQw[R * m.ccQ + k] : 0u;
-        const uint32_t rr = k < nRR ? m.cRw[R * m.ccR + k] : 0u;
-        if (k < nPL) PL[k] = pl;
-        if (k < nQL) QL[k] = ql;
-        if (k < nRL) RL[k] = rl;
-        if (k < nPR) PR[k] = pr;
-        if (k < nQR) QR[k] = qr;
-        if (k < nRR) RR[k] = rr;
-    }
-    __syncwarp();
-    const uint32_t nQ = warp_mul(QL, nQL, QR, nQR, t1, col);
-    for (uint32_t k = lane; k < nQ; k += 32) m.pQw[i * m.pcQ + k] = t1[k];
-    __syncwarp();
-    const uint32_t nR = warp_mul(RL, nRL, RR, nRR, t1, col);
-    for (uint32_t k = lane; k < nR; k += 32) m.pRw[i * m.pcR + k] = t1[k];
-    __syncwarp();
-    // P = PL QR + PR RL (PI.h:110)
-    const uint32_t n1 = warp_mul(PL, nPL, QR, nQR, t1, col);
-    const uint32_t n2 = warp_mul(PR, nPR, RL, nRL, t2, col);
-    bool sP;
-    uint32_t* pz = col;  // max(n1, n2) + 1 <= 3 (ccP + ccQ)
-    const uint32_t nP = warp_signed_add(sL, t1, n1, sR, t2, n2, pz, &sP);
-    for (uint32_t k = lane; k < nP; k += 32) m.pPw[i * m.pcP + k] = pz[k];
-    if (lane == 0) {
-        m.pPl[i] = nP;
-        m.pQl[i] = nQ;
-        m.pRl[i] = nR;
-        m.pS[i] = sP ? 1 : 0;
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1232,7 +1180,7 @@ static Mod64 prime_mod(int q) { return make_mod(kProductPrimes[q]); }
 
 static bool g_wrap = true;
 static uint32_t g_kara_min = 0;  // CTA schoolbook merges: Karatsuba level from this many words (0: off)
-static int g_small_merge = 2;  // 0: CTA schoolbook, 1: + warp per parent, 2: + thread per parent
+static int g_small_merge = 2;  // 2: the shortest nodes' merges in registers, a thread per parent; else none
 static bool g_top_batched = true;
 static bool g_wide_add = true;
 
@@ -1647,12 +1595,6 @@ static void merge_school(Level& ch, Level& par, cudaStream_t s)
     m.pcR = par.R.cap;
     m.count = par.count;
     m.kara_min = g_kara_min;
-    const size_t words = 2 * ((size_t)m.ccP + m.ccQ + m.ccR) + (m.ccP + m.ccQ) + (m.ccP + m.ccR) +
-                         3 * ((size_t)m.ccP + m.ccQ) + (g_kara_min ? 3 * ((size_t)m.ccP + m.ccQ) + 8 : 0);
-    const size_t smem = words * sizeof(uint32_t);
-    PIC_REQUIRE(smem <= 200 * 1024, PIC_ERR_INVALID, "schoolbook merge tile too large");
-    if (smem > 48 * 1024)
-        PIC_CUDA(cudaFuncSetAttribute(merge_school_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint32_t cmax = std::max(m.ccP, std::max(m.ccQ, m.ccR));
     count_products(4 * par.count);  // P0 Q1, P1 R0, Q0 Q1, R0 R1 per parent (PI.h:110-112)
     ProfScope ps(KC_BSR, 4.0 * (double)par.count * 2.0 * (m.ccP + m.ccQ + m.ccR), s);
@@ -1662,16 +1604,17 @@ static void merge_school(Level& ch, Level& par, cudaStream_t s)
         count_launch();
         return;
     }
-    if (cmax <= (uint32_t)kWarpMergeMax && g_small_merge >= 1) {
-        const size_t wsmem = sizeof(uint32_t) * warp_merge_words(m.ccP, m.ccQ, m.ccR) * kWarpMergeWarps;
-        if (wsmem > 48 * 1024)
-            PIC_CUDA(cudaFuncSetAttribute(merge_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsmem));
-        const size_t grid = (par.count + kWarpMergeWarps - 1) / kWarpMergeWarps;
-        merge_warp_kernel<<<(unsigned)grid, 32 * kWarpMergeWarps, wsmem, s>>>(m);
+    if (m.kara_min == 0 && launch_merge_block(m, s)) {
         PIC_CHECK_LAUNCH();
         count_launch();
         return;
     }
+    const size_t words = 2 * ((size_t)m.ccP + m.ccQ + m.ccR) + (m.ccP + m.ccQ) + (m.ccP + m.ccR) +
+                         3 * ((size_t)m.ccP + m.ccQ) + (g_kara_min ? 3 * ((size_t)m.ccP + m.ccQ) + 8 : 0);
+    const size_t smem = words * sizeof(uint32_t);
+    PIC_REQUIRE(smem <= 200 * 1024, PIC_ERR_INVALID, "schoolbook merge tile too large");
+    if (smem > 48 * 1024)
+        PIC_CUDA(cudaFuncSetAttribute(merge_school_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int threads = cmax <= 16 ? 32 : (cmax <= 64 ? 64 : (cmax <= 256 ? 128 : 256));
     merge_school_kernel<<<(unsigned)par.count, threads, smem, s>>>(m);
     PIC_CHECK_LAUNCH();

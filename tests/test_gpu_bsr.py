@@ -71,6 +71,28 @@ def test_bsr_karatsuba_vs_oracle(pic, oracle, a, b, p, kara):
     assert _same(P, wP), "P"
 
 
+# The register-block merges (blocks of 8 words, threads past a CTA's loop, numbers
+# of one block, nodes of different lengths side by side) against the column-sum
+# kernel, which a Karatsuba threshold above every length selects; short nodes
+# with the thread-per-parent kernel off as well.
+@pytest.mark.parametrize("small", [0, 2])
+@pytest.mark.parametrize("terms", [4, 5, 7, 16, 33, 100, 333, 700, 1001, 1500])
+def test_bsr_block_merges_agree(pic, terms, small):
+    knobs = {pic.TUNE_BSR_SCHOOL_MAX: 2000, pic.TUNE_BSR_SMALL_MERGE: small, pic.TUNE_BSR_KARATSUBA: 0}
+    saved = {k: pic.get_tuning(k) for k in knobs}
+    res = []
+    try:
+        for kara in (0, 4096):
+            for k, v in {**knobs, pic.TUNE_BSR_KARATSUBA: kara}.items():
+                pic.set_tuning(k, v)
+            res.append(pic.bsr(5, 5 + terms, 1 << 16, pic.PI_CHOSEN))
+    finally:
+        for k, v in saved.items():
+            pic.set_tuning(k, v)
+    for x, y in zip(*res):
+        assert _same(x, y.to_bf())
+
+
 # The FP64 form's fused merge kernel against the integer form's separate passes
 # at transform lengths 2^2 .. 2^19: rows of every length, ragged last CTAs,
 # column passes of 1 .. 8 bits before and after it.
