@@ -14,6 +14,8 @@ namespace pic {
 
 constexpr int kDiagWords = 17;  // 16 words and the overflow of up to 2^32 blocks; odd: no bank conflicts
 
+constexpr int kDiagZeros = kDiagWords + 1;  // zero words in front of a CTA's first diagonal
+
 // e[0..8] += a * (b0, b2, b4, b6) at even distances (e[8]: the carry out)
 __device__ __forceinline__ void mad_row(uint32_t* e, uint32_t a, uint32_t b0, uint32_t b2, uint32_t b4, uint32_t b6)
 {
@@ -94,26 +96,54 @@ __device__ __forceinline__ void block_diagonals(const uint32_t* a, int na, const
     for (int w = 0; w < kDiagWords; w++) out[w] = acc[w];
 }
 
-// Result words of block c (words 8 c .. 8 c + 7) of a product whose nd
-// diagonals are at diag: f(r, t, g) for r = 0 .. 7 in order, the digit t before
-// carries and its generate bit g (a digit with g is at most 1, so it cannot
-// propagate as well).
-template <class F>
-__device__ __forceinline__ void block_digits(const uint32_t* diag, int nd, int c, const F& f)
+// The words of one result block before carries.  `lo` is its diagonal.  A product
+// is followed by a zero diagonal, which is also the one before the next product's
+// first; before a CTA's first are kDiagZeros words of zero (and any word before
+// them: alone it makes no carry).  Word r takes the low half of its own diagonal, the high
+// half of the one before and, as the lowest word, the overflow of the one before
+// that; its digit adds the carry of the sum one word below.  *gen and *prop: a bit
+// for each word that makes a carry, and that passes one on (never both: a digit
+// that makes a carry is at most 1).
+__device__ __forceinline__ void block_digits(const uint32_t* lo, uint32_t (&t)[8], uint32_t* gen, uint32_t* prop)
 {
-    const uint32_t* lo = diag + kDiagWords * c;
     const uint32_t* hi = lo - kDiagWords + 8;
-    const bool hl = c < nd, hh = c >= 1;
-    uint64_t prev = 0;  // the sum one word below
-    if (hh) prev = (uint64_t)lo[7 - kDiagWords] + (c >= 2 ? hi[7 - kDiagWords] : 0u);
+    uint32_t g = 0, p = 0;
+    uint32_t up = (uint32_t)(((uint64_t)lo[7 - kDiagWords] + hi[7 - kDiagWords]) >> 32);
 #pragma unroll
     for (int r = 0; r < 8; r++) {
-        uint64_t s = (uint64_t)(hl ? lo[r] : 0u) + (hh ? hi[r] : 0u);
-        if (r == 0 && c >= 2) s += lo[16 - 2 * kDiagWords];
-        const uint64_t t = (s & 0xffffffffu) + (prev >> 32);
-        f(r, (uint32_t)t, (uint32_t)(t >> 32));
-        prev = s;
+        uint64_t s = (uint64_t)lo[r] + hi[r];
+        if (r == 0) s += lo[16 - 2 * kDiagWords];
+        t[r] = (uint32_t)s + up;
+        g |= (uint32_t)(t[r] < up) << r;
+        p |= (uint32_t)(t[r] == 0xffffffffu) << r;
+        up = (uint32_t)(s >> 32);
     }
+    *gen = g;
+    *prop = p;
+}
+
+// Bit i: the carry into word i, from generate and propagate bits and a carry in.
+__device__ __forceinline__ uint32_t carry_bits(uint32_t gen, uint32_t prop, uint32_t cin)
+{
+    return (((gen << 1) | cin) + prop) ^ prop;
+}
+
+// The carry into the calling thread's words, threads in order, each with a
+// generate and a propagate bit (never both); `cin` into the first, *cout out of
+// the last (whole warps, at most 32; s_w: 32 words for each call before the next
+// barrier after it).  Ballots and additions in place of a scan by shuffles.
+__device__ __forceinline__ uint32_t block_carry(uint32_t gen, uint32_t prop, uint32_t cin, uint32_t* s_w, uint32_t* cout)
+{
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const uint32_t g = __ballot_sync(0xffffffffu, gen), p = __ballot_sync(0xffffffffu, prop);
+    const uint64_t sum = ((uint64_t)g << 1) + p;
+    if (lane == 0) s_w[wid] = (uint32_t)(sum >> 32) | ((uint32_t)(p == 0xffffffffu) << 1);
+    __syncthreads();
+    const uint32_t w = lane < nw ? s_w[lane] : 0u;
+    const uint32_t gw = __ballot_sync(0xffffffffu, w & 1u), pw = __ballot_sync(0xffffffffu, w >> 1);
+    const uint64_t cw = ((((uint64_t)gw << 1) | cin) + pw) ^ pw;  // bit i: into warp i
+    *cout = (uint32_t)(cw >> nw) & 1u;
+    return (uint32_t)((((((uint64_t)g << 1) | ((cw >> wid) & 1u)) + p) ^ p) >> lane) & 1u;
 }
 
 }  // namespace pic

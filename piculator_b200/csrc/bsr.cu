@@ -590,152 +590,271 @@ __global__ void __launch_bounds__(256) merge_school_kernel(MergeArgs m)
 
 // ---------------------------------------------------------------------------
 // The same merge with the four products side by side, each in register blocks
-// (blockmul.cuh): one CTA per parent, a thread per block row of a product, one
-// carry scan over the words of all four.  The column sums below spend most of
-// their issue slots on carries, shared-memory reads and columns of uneven
+// (blockmul.cuh): a thread per block row of a product, one carry scan over the
+// words of all products.  A CTA takes as many parents as give it 256 rows, so the
+// rows of short nodes fill its warps (a parent of two-block children has eight)
+// and a scan serves several parents: a product's carries end inside its words and
+// so do a sum's, which has a zero word on top.  The column sums below spend most
+// of their issue slots on carries, shared-memory reads and columns of uneven
 // length; here a block of 64 multiply-adds costs 8 shared-memory words' reads
-// (two 16-byte loads an operand) and about 250 slots for 200 at the multiplier's
-// full rate.  Levels of a 1e9-digit computation with children of up to 75, 150
-// and 300 words: 23, 38 and 75 -> 17, 17 and 25 ms; of up to 38 words, which had
-// a warp per parent, 23 -> 13 ms.
+// (two 16-byte loads an operand), and the multiplier, 7.7 T multiply-adds a second
+// in this form without the rest, is what bounds the longer levels.  Levels of a
+// 1e9-digit computation with children of up to 41, 74, 144 and 284 words: 23 (a
+// warp per parent), 23, 38 and 75 -> 10.8, 10.6, 15.5 and 24.2 ms (the last one's
+// multiply-adds alone: 16.5); one parent a CTA and digits made twice, before and
+// after a scan by shuffles, took 12.5, 17.3, 17.5 and 25.4.
+constexpr int kBlockMergeThreads = 512;
+constexpr int kBlockMergeParents = 8;  // 4 products each: one warp scans their lengths
+
 struct BlockMergeShape {
     uint32_t bP, bQ, bR;  // blocks of a child slot
+    uint32_t G;           // parents of a CTA
     __host__ __device__ uint32_t operands() const { return 2 * (bP + bQ + bR); }
     __host__ __device__ uint32_t diagonals() const { return 2 * bP + 3 * bQ + 3 * bR; }  // of the four products
-    __host__ __device__ uint32_t words() const { return 8 * operands() + kDiagWords * diagonals(); }
+    // the operands, zeros, the diagonals
+    uint32_t words() const { return G * (8 * operands() + kDiagWords * diagonals()) + kDiagZeros; }
     uint32_t rows() const { return std::max(bP, bQ) + std::max(bP, bR) + bQ + bR; }
 };
-constexpr int kBlockMergeThreads = 512;
+
+// Eight words to z + w (w a multiple of 8), those below `cap`.
+__device__ __forceinline__ void store_block(uint32_t* z, uint32_t w, uint32_t cap, const uint32_t (&v)[8])
+{
+    if (w + 8 <= cap && (cap & 3) == 0) {  // slots start at multiples of cap words
+        reinterpret_cast<uint4*>(z + w)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        reinterpret_cast<uint4*>(z + w)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+        return;
+    }
+#pragma unroll
+    for (int r = 0; r < 8; r++)
+        if (w + r < cap) z[w + r] = v[r];
+}
 
 __global__ void __launch_bounds__(kBlockMergeThreads, 2) merge_block_kernel(MergeArgs m, BlockMergeShape S)
 {
     extern __shared__ __align__(16) uint32_t sm[];
-    __shared__ uint32_t s_top[4];  // a product's highest word
-    const size_t i = blockIdx.x;
-    const size_t L = 2 * i, R = 2 * i + 1;
-    const uint32_t T = blockDim.x;
-    const uint32_t nPL = m.cPl[L], nQL = m.cQl[L], nRL = m.cRl[L];
-    const uint32_t nPR = m.cPl[R], nQR = m.cQl[R], nRR = m.cRl[R];
-    const bool sL = m.cS[L] != 0, sR = m.cS[R] != 0;
-    uint32_t* PL = sm;
-    uint32_t* PR = PL + 8 * S.bP;
-    uint32_t* QL = PR + 8 * S.bP;
-    uint32_t* QR = QL + 8 * S.bQ;
-    uint32_t* RL = QR + 8 * S.bQ;
-    uint32_t* RR = RL + 8 * S.bR;
-    uint32_t* diag = RR + 8 * S.bR;
-    // operands, whole blocks, zero above their length
-    const uint32_t bmax = 8 * max(S.bP, max(S.bQ, S.bR));
-    for (uint32_t k = threadIdx.x; k < bmax; k += T) {
-        const uint32_t pl = k < nPL ? m.cPw[L * m.ccP + k] : 0u, pr = k < nPR ? m.cPw[R * m.ccP + k] : 0u;
-        const uint32_t ql = k < nQL ? m.cQw[L * m.ccQ + k] : 0u, qr = k < nQR ? m.cQw[R * m.ccQ + k] : 0u;
-        const uint32_t rl = k < nRL ? m.cRw[L * m.ccR + k] : 0u, rr = k < nRR ? m.cRw[R * m.ccR + k] : 0u;
-        if (k < 8 * S.bP) PL[k] = pl, PR[k] = pr;
-        if (k < 8 * S.bQ) QL[k] = ql, QR[k] = qr;
-        if (k < 8 * S.bR) RL[k] = rl, RR[k] = rr;
+    constexpr int NP = 4 * kBlockMergeParents;
+    __shared__ uint32_t s_len[kBlockMergeParents][6];  // PL PR QL QR RL RR
+    __shared__ uint32_t s_row[NP + 1], s_blk[NP + 1], s_sum[kBlockMergeParents + 1];  // first row, result block, sum block
+    __shared__ uint32_t s_top[NP];                     // a product's highest word
+    __shared__ uint32_t s_w[2][32];
+    __shared__ uint32_t s_hi[kBlockMergeParents], s_nP[kBlockMergeParents];
+    __shared__ uint8_t s_sgn[kBlockMergeParents][2];
+    const uint32_t T = blockDim.x, tid = threadIdx.x;
+    const size_t i0 = (size_t)blockIdx.x * S.G;
+    const uint32_t G = m.count - i0 < S.G ? (uint32_t)(m.count - i0) : S.G;
+    const uint32_t ow = 8 * S.operands();  // operand words of a parent
+    uint32_t* diag = sm + S.G * ow + kDiagZeros;
+    auto blocks = [](uint32_t n) { return (n + 7) / 8; };
+    if (tid < 6 * G) {
+        const uint32_t g = tid / 6, a = tid - 6 * g;
+        const size_t c = 2 * (i0 + g) + (a & 1);
+        s_len[g][a] = a < 2 ? m.cPl[c] : (a < 4 ? m.cQl[c] : m.cRl[c]);
+        if (a < 2) s_sgn[g][a] = m.cS[c] != 0;
     }
     __syncthreads();
-    // product p: PL QR, PR RL, QL QR, RL RR, the operand of fewer blocks first
-    auto op = [&](int p, const uint32_t*& a, uint32_t& na, const uint32_t*& b, uint32_t& nb) {
-        a = p == 0 ? PL : (p == 1 ? PR : (p == 2 ? QL : RL));
-        na = p == 0 ? nPL : (p == 1 ? nPR : (p == 2 ? nQL : nRL));
-        b = p == 0 || p == 2 ? QR : (p == 1 ? RL : RR);
-        nb = p == 0 || p == 2 ? nQR : (p == 1 ? nRL : nRR);
+    // operand a of a parent starts at word opw(a)
+    auto opw = [&](uint32_t a) {
+        return 8 * (a < 2 ? a * S.bP : (a < 4 ? 2 * S.bP + (a - 2) * S.bQ : 2 * (S.bP + S.bQ) + (a - 4) * S.bR));
+    };
+    // product p = 0..3: PL QR, PR RL, QL QR, RL RR
+    auto first = [](uint32_t p) { return p < 2 ? p : 2 * p - 2; };
+    auto second = [](uint32_t p) { return p == 1 ? 4u : (p == 3 ? 5u : 3u); };
+    if (tid < 32) {
+        uint32_t rows = 0, blk = 0;
+        if (tid < 4 * G) {
+            const uint32_t na = s_len[tid >> 2][first(tid & 3)], nb = s_len[tid >> 2][second(tid & 3)];
+            if (na && nb) {
+                rows = blocks(max(na, nb));
+                blk = blocks(na) + blocks(nb);
+            }
+        }
+        uint32_t ir = rows, ib = blk;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t r = __shfl_up_sync(0xffffffffu, ir, off), b = __shfl_up_sync(0xffffffffu, ib, off);
+            if (tid >= (uint32_t)off) ir += r, ib += b;
+        }
+        s_row[tid + 1] = ir;
+        s_blk[tid + 1] = ib;
+        s_top[tid] = 0;
+        if (tid == 0) s_row[0] = s_blk[0] = s_sum[0] = 0;
+        if (tid < (uint32_t)kBlockMergeParents) s_hi[tid] = s_nP[tid] = 0;
+    }
+    // operands, whole blocks, zero above their length: 16 threads each
+    for (uint32_t x = tid >> 4; x < 6 * G; x += T >> 4) {
+        const uint32_t g = x / 6, a = x - 6 * g, n = s_len[g][a];
+        const size_t c = 2 * (i0 + g) + (a & 1);
+        const uint32_t* src = a < 2 ? m.cPw + c * m.ccP : (a < 4 ? m.cQw + c * m.ccQ : m.cRw + c * m.ccR);
+        uint32_t* dst = sm + g * ow + opw(a);
+        const uint32_t pad = 8 * (a < 2 ? S.bP : (a < 4 ? S.bQ : S.bR));
+        for (uint32_t k = tid & 15; k < pad; k += 16) dst[k] = k < n ? src[k] : 0u;
+    }
+    if (tid < kDiagZeros) diag[(int)tid - kDiagZeros] = 0;
+    __syncthreads();
+    // the product (or sum) whose run holds t: the last that starts at or before it
+    auto find = [](const uint32_t* run, uint32_t n, uint32_t t) {
+        uint32_t x = 0;
+#pragma unroll
+        for (uint32_t step = NP / 2; step >= 1; step >>= 1)
+            if (x + step < n && run[x + step] <= t) x += step;
+        return x;
+    };
+    const uint32_t nprod = 4 * G;
+    for (uint32_t t = tid; t < s_row[nprod]; t += T) {
+        const uint32_t x = find(s_row, nprod, t), g = x >> 2, p = x & 3;
+        uint32_t a = first(p), b = second(p);
+        uint32_t na = s_len[g][a], nb = s_len[g][b];
         if (na > nb) {
-            const uint32_t* x = a;
-            a = b;
-            b = x;
-            const uint32_t n = na;
-            na = nb;
-            nb = n;
+            const uint32_t c = a, n = na;
+            a = b, b = c;
+            na = nb, nb = n;
+        }
+        const uint32_t* o = sm + g * ow;
+        const int d = (int)(t - s_row[x]);
+        block_diagonals(o + opw(a), (int)blocks(na), o + opw(b), (int)blocks(nb), d, diag + kDiagWords * s_blk[x]);
+        if (d == 0)
+            for (int w = 0; w < kDiagWords; w++) diag[kDiagWords * (s_blk[x + 1] - 1) + w] = 0;
+    }
+    __syncthreads();
+    // words: two consecutive result blocks a thread (there are at most two a row)
+    const uint32_t nblk = s_blk[nprod];
+    // T1 and T2 over the parent's operands (read above), Q and R to its slots
+    auto t1_of = [&](uint32_t g) { return sm + g * ow; };
+    auto t2_of = [&](uint32_t g) { return sm + g * ow + 8 * (s_blk[4 * g + 1] - s_blk[4 * g]); };
+    uint32_t cin = 0;
+    for (uint32_t base = 0; base < nblk; base += 2 * T) {
+        uint32_t v[2][8], gen[2] = {0, 0}, prop[2] = {0, 0};
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const uint32_t q = base + 2 * tid + u;
+            if (q < nblk) block_digits(diag + kDiagWords * q, v[u], &gen[u], &prop[u]);
+        }
+        const uint32_t g2 = gen[0] | (gen[1] << 8), p2 = prop[0] | (prop[1] << 8);
+        uint32_t cout;
+        const uint32_t c = block_carry(((g2 << 1) + p2) >> 16, p2 == 0xffffu, cin, s_w[0], &cout);
+        const uint32_t carries = carry_bits(g2, p2, c);
+        cin = cout;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const uint32_t q = base + 2 * tid + u;
+            if (q >= nblk) continue;
+#pragma unroll
+            for (int r = 0; r < 8; r++) v[u][r] += (carries >> (8 * u + r)) & 1u;
+            const uint32_t x = find(s_blk, nprod, q), g = x >> 2, p = x & 3;
+            const uint32_t w0 = 8 * (q - s_blk[x]);
+            if (p < 2) store_block((p == 0 ? t1_of(g) : t2_of(g)), w0, w0 + 8, v[u]);
+            else if (p == 2) store_block(m.pQw + (i0 + g) * m.pcQ, w0, m.pcQ, v[u]);
+            else store_block(m.pRw + (i0 + g) * m.pcR, w0, m.pcR, v[u]);
+            const uint32_t top = s_len[g][first(p)] + s_len[g][second(p)] - 1 - w0;
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+                if (top == (uint32_t)r) s_top[x] = v[u][r];
+        }
+        if (base + 2 * T < nblk) __syncthreads();  // s_w again
+    }
+    __syncthreads();
+    // P = PL QR + PR RL (PI.h:110), signed: the same blocks of both, enough for a carry word
+    auto len = [&](uint32_t x) {
+        const uint32_t na = s_len[x >> 2][first(x & 3)], nb = s_len[x >> 2][second(x & 3)];
+        return na == 0 || nb == 0 ? 0u : na + nb - (s_top[x] == 0 ? 1u : 0u);
+    };
+    if (tid < G) s_sum[tid + 1] = blocks(max(len(4 * tid), len(4 * tid + 1)) + 1);
+    __syncthreads();
+    if (tid == 0)
+        for (uint32_t g = 0; g < G; g++) s_sum[g + 1] += s_sum[g];
+    __syncthreads();
+    auto load = [&](uint32_t g, int which, uint32_t c, uint32_t(&v)[8]) {
+        const uint32_t x = 4 * g + which;
+        if (c < s_blk[x + 1] - s_blk[x]) {
+            load_block(v, (which ? t2_of(g) : t1_of(g)) + 8 * c);
+        } else {
+#pragma unroll
+            for (int r = 0; r < 8; r++) v[r] = 0;
         }
     };
-    auto blocks = [](uint32_t n) { return (n + 7) / 8; };
-    uint32_t first_row[5], first_blk[5];  // of each product, in the lists of rows and of result blocks
-    first_row[0] = first_blk[0] = 0;
+    const uint32_t nsum = s_sum[G];
+    for (uint32_t q = tid; q < nsum; q += T) {  // differences: the highest word that differs
+        const uint32_t g = find(s_sum, G, q);
+        if (s_sgn[g][0] == s_sgn[g][1]) continue;
+        uint32_t a[8], b[8], h = 0;
+        load(g, 0, q - s_sum[g], a);
+        load(g, 1, q - s_sum[g], b);
 #pragma unroll
-    for (int p = 0; p < 4; p++) {
-        const uint32_t *a, *b;
-        uint32_t na, nb;
-        op(p, a, na, b, nb);
-        first_row[p + 1] = first_row[p] + (na ? blocks(nb) : 0u);
-        first_blk[p + 1] = first_blk[p] + (na ? blocks(na) + blocks(nb) : 0u);
-    }
-    for (uint32_t t = threadIdx.x; t < first_row[4]; t += T) {
-        const int p = t < first_row[1] ? 0 : (t < first_row[2] ? 1 : (t < first_row[3] ? 2 : 3));
-        const uint32_t r0 = p == 0 ? 0u : (p == 1 ? first_row[1] : (p == 2 ? first_row[2] : first_row[3]));
-        const uint32_t b0 = p == 0 ? 0u : (p == 1 ? first_blk[1] : (p == 2 ? first_blk[2] : first_blk[3]));
-        const uint32_t *a, *b;
-        uint32_t na, nb;
-        op(p, a, na, b, nb);
-        block_diagonals(a, (int)blocks(na), b, (int)blocks(nb), (int)(t - r0), diag + kDiagWords * b0);
-    }
-    if (threadIdx.x < 4) s_top[threadIdx.x] = 0;
-    __syncthreads();
-    // words: a thread takes consecutive result blocks.  No carry leaves a product
-    // (its blocks reach past its highest word), so one scan serves all four.
-    const uint32_t nblk = first_blk[4], per = (nblk + T - 1) / T;
-    const uint32_t q0 = min(threadIdx.x * per, nblk), q1 = min(q0 + per, nblk);
-    auto at = [&](uint32_t q, int& p, uint32_t& b0, uint32_t& nd) {
-        p = q < first_blk[1] ? 0 : (q < first_blk[2] ? 1 : (q < first_blk[3] ? 2 : 3));
-        b0 = p == 0 ? 0u : (p == 1 ? first_blk[1] : (p == 2 ? first_blk[2] : first_blk[3]));
-        nd = (p == 0 ? first_blk[1] : (p == 1 ? first_blk[2] : (p == 2 ? first_blk[3] : first_blk[4]))) - b0 - 1;
-    };
-    uint32_t gp = kGPIdentity;
-    for (uint32_t q = q0; q < q1; q++) {
-        int p;
-        uint32_t b0, nd;
-        at(q, p, b0, nd);
-        block_digits(diag + kDiagWords * b0, (int)nd, (int)(q - b0), [&](int, uint32_t t, uint32_t g) {
-            gp = gp_combine(gp, g | ((uint32_t)(t == 0xffffffffu) << 1));
-        });
-    }
-    uint32_t total;
-    uint32_t cin = block_gp_scan(gp, &total) & 1u;
-    // T1 and T2 over the operands (read above), Q and R to the parent's slots
-    uint32_t* t1 = sm;
-    uint32_t* t2 = t1 + 8 * first_blk[1];
-    for (uint32_t q = q0; q < q1; q++) {
-        int p;
-        uint32_t b0, nd;
-        at(q, p, b0, nd);
-        const uint32_t zw = p == 0 ? nPL + nQR : (p == 1 ? nPR + nRL : (p == 2 ? nQL + nQR : nRL + nRR));
-        uint32_t* z = p == 0 ? t1 : (p == 1 ? t2 : (p == 2 ? m.pQw + i * m.pcQ : m.pRw + i * m.pcR));
-        const uint32_t w0 = 8 * (q - b0);
-        block_digits(diag + kDiagWords * b0, (int)nd, (int)(q - b0), [&](int r, uint32_t t, uint32_t g) {
-            const uint32_t w = w0 + r, v = t + cin;
-            cin = g | ((uint32_t)(t == 0xffffffffu) & cin);
-            if (w + 1 < zw || (w + 1 == zw && v != 0)) z[w] = v;
-            if (w + 1 == zw) s_top[p] = v;
-        });
+        for (int r = 0; r < 8; r++)
+            if (a[r] != b[r]) h = 8 * (q - s_sum[g]) + r + 1;
+        if (h) atomicMax(&s_hi[g], h);
     }
     __syncthreads();
-    auto len = [&](int p, uint32_t na, uint32_t nb) {
-        return na == 0 || nb == 0 ? 0u : na + nb - (s_top[p] == 0 ? 1u : 0u);
+    auto swapped = [&](uint32_t g) {  // a difference whose second number is the larger
+        const uint32_t h = s_hi[g];
+        if (h == 0) return false;
+        uint32_t a[2];
+        for (int which = 0; which < 2; which++) {
+            const uint32_t x = 4 * g + which;
+            a[which] = h - 1 < 8 * (s_blk[x + 1] - s_blk[x]) ? (which ? t2_of(g) : t1_of(g))[h - 1] : 0u;
+        }
+        return a[0] < a[1];
     };
-    const uint32_t n1 = len(0, nPL, nQR), n2 = len(1, nPR, nRL), nQ = len(2, nQL, nQR), nR = len(3, nRL, nRR);
-    // P = PL QR + PR RL (PI.h:110)
-    bool sP;
-    const uint32_t nP = cta_signed_add(sL, t1, n1, sR, t2, n2, diag, &sP);
-    for (uint32_t k = threadIdx.x; k < nP; k += T) m.pPw[i * m.pcP + k] = diag[k];
-    if (threadIdx.x == 0) {
-        m.pPl[i] = nP;
-        m.pQl[i] = nQ;
-        m.pRl[i] = nR;
-        m.pS[i] = sP ? 1 : 0;
+    cin = 0;
+    for (uint32_t base = 0; base < nsum; base += T) {
+        const uint32_t q = base + tid, g = find(s_sum, G, q);
+        const bool sub = s_sgn[g][0] != s_sgn[g][1], sw = sub && swapped(g);
+        uint32_t v[8], gen = 0, prop = 0;
+        if (q < nsum) {
+            uint32_t b[8];
+            load(g, sw ? 1 : 0, q - s_sum[g], v);
+            load(g, sw ? 0 : 1, q - s_sum[g], b);
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                const uint32_t a = v[r];
+                v[r] = sub ? a - b[r] : a + b[r];
+                gen |= (uint32_t)(sub ? a < b[r] : v[r] < a) << r;
+                prop |= (uint32_t)(v[r] == (sub ? 0u : 0xffffffffu)) << r;
+            }
+        }
+        prop &= ~gen;
+        uint32_t cout;
+        const uint32_t c = block_carry(((gen << 1) + prop) >> 8, prop == 0xffu, cin, s_w[1], &cout);
+        const uint32_t carries = carry_bits(gen, prop, c);
+        cin = cout;
+        if (q < nsum) {
+            uint32_t h = 0;
+            const uint32_t w0 = 8 * (q - s_sum[g]);
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                const uint32_t cr = (carries >> r) & 1u;
+                v[r] = sub ? v[r] - cr : v[r] + cr;
+                if (v[r]) h = w0 + r + 1;
+            }
+            store_block(m.pPw + (i0 + g) * m.pcP, w0, m.pcP, v);
+            if (h) atomicMax(&s_nP[g], h);
+        }
+        if (base + T < nsum) __syncthreads();  // s_w again
+    }
+    __syncthreads();
+    if (tid < G) {
+        const bool sL = s_sgn[tid][0] != 0, sR = s_sgn[tid][1] != 0;
+        const uint32_t nP = s_nP[tid];
+        m.pPl[i0 + tid] = nP;
+        m.pQl[i0 + tid] = len(4 * tid + 2);
+        m.pRl[i0 + tid] = len(4 * tid + 3);
+        m.pS[i0 + tid] = (sL == sR ? sL : (nP == 0 || (swapped(tid) ? sR : sL))) ? 1 : 0;
     }
 }
 
 // Whether the children fit the register-block merge's shared memory.
 static bool launch_merge_block(const MergeArgs& m, cudaStream_t s)
 {
-    BlockMergeShape S{(m.ccP + 7) / 8, (m.ccQ + 7) / 8, (m.ccR + 7) / 8};
+    BlockMergeShape S{(m.ccP + 7) / 8, (m.ccQ + 7) / 8, (m.ccR + 7) / 8, 1};
+    // several parents a CTA only where there are CTAs enough for every SM
+    S.G = std::max<uint32_t>(1, std::min<uint32_t>(kBlockMergeParents, 256 / S.rows()));
+    S.G = (uint32_t)std::max<size_t>(1, std::min<size_t>(S.G, m.count / (4 * (size_t)ctx().num_sms)));
     const size_t smem = sizeof(uint32_t) * (size_t)S.words();
     if (smem > 200 * 1024) return false;
     if (smem > 48 * 1024)
         PIC_CUDA(cudaFuncSetAttribute(merge_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const uint32_t threads = std::min<uint32_t>(kBlockMergeThreads, (S.rows() + 31) / 32 * 32);
-    merge_block_kernel<<<(unsigned)m.count, threads, smem, s>>>(m, S);
+    const uint32_t threads = std::min<uint32_t>(kBlockMergeThreads, (S.G * S.rows() + 31) / 32 * 32);
+    merge_block_kernel<<<(unsigned)((m.count + S.G - 1) / S.G), std::max<uint32_t>(threads, 64), smem, s>>>(m, S);
     return true;
 }
 
@@ -1598,8 +1717,13 @@ static void merge_school(Level& ch, Level& par, cudaStream_t s)
     const uint32_t cmax = std::max(m.ccP, std::max(m.ccQ, m.ccR));
     count_products(4 * par.count);  // P0 Q1, P1 R0, Q0 Q1, R0 R1 per parent (PI.h:110-112)
     ProfScope ps(KC_BSR, 4.0 * (double)par.count * 2.0 * (m.ccP + m.ccQ + m.ccR), s);
-    if (g_small_merge >= 2 && (launch_merge_thread<16, 16, 12>(m, s) || launch_merge_thread<20, 20, 14>(m, s) ||
-                               launch_merge_thread<28, 28, 20>(m, s))) {
+    // A thread per parent has no idle lanes, but one parent's time is the whole of a
+    // merge on one thread: 16.8M parents of 9-word children 13.5 ms (blocks 31), 8.4M
+    // of 17 words 16.1 (20.6), but 8192 parents 27 us (16), a few 25 (8); 4.2M of 26
+    // words 15.5 ms (12.9).  So up to 20 words, where every SM has 100 of them.
+    const bool many = m.count >= 100 * (size_t)ctx().num_sms || m.kara_min != 0;
+    if (g_small_merge >= 2 && many &&
+        (launch_merge_thread<16, 16, 12>(m, s) || launch_merge_thread<20, 20, 14>(m, s))) {
         PIC_CHECK_LAUNCH();
         count_launch();
         return;
