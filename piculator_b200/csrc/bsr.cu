@@ -1509,11 +1509,11 @@ static void ntt_products(const Level& ch, size_t p0, size_t np, const MergeShape
         transform(fb, mains, k, ST, 0);
         if (sh.wrap) {
             transform(tb, tails, sh.kt, T, sh.t0);
+        }
+        if (sh.wrap && !dbl) {  // the FP64 form's CRT reads the tails itself
             ProfScope ps(KC_NTT_POINTWISE, 3.0 * 4 * np * (double)sh.W * 24.0, s);
-            const size_t W = sh.W;
             auto fix = [&](uint64_t* y, const uint64_t* tail, size_t nitems, size_t item_mul) {
-                if (dbl) launch_wrap_fix_d(y, ST, tail, T, nitems, item_mul, nc, N, W, s);
-                else launch_wrap_fix(y, ST, tail, T, nitems, item_mul, nc, N, W, cT, s);
+                launch_wrap_fix(y, ST, tail, T, nitems, item_mul, nc, N, sh.W, cT, s);
             };
             if (comb) fix(PB, PT, np, 2);
             else fix(PB, PT, nc, 1);
@@ -1535,18 +1535,20 @@ static void ntt_products(const Level& ch, size_t p0, size_t np, const MergeShape
         count_launch(needR ? 4 : 3);
         // T1: residues at bP items 2i (stride 2 ST), T2 at items 2i+1
         const size_t pstride = nc * ST;  // [prime][child][ST]
-        auto to_words = [&](const uint64_t* y, uint32_t* z, uint32_t zcap, const uint32_t* zlen, bool offset) {
-            if (dbl) ntt3d_batch_to_words(y, 2 * ST, pstride, np, k, z, zcap, zlen, s, ncoef, offset);
+        auto to_words = [&](const uint64_t* y, const uint64_t* tail, uint32_t* z, uint32_t zcap, const uint32_t* zlen,
+                            bool offset) {
+            const CrtWrap wrap = sh.wrap ? crt_wrap(tail, 2 * T, nc * T, T, N, sh.W) : CrtWrap{};
+            if (dbl) ntt3d_batch_to_words(y, 2 * ST, pstride, np, k, z, zcap, zlen, s, ncoef, offset, wrap);
             else ntt3_batch_to_words(y, 2 * ST, pstride, np, k, z, zcap, zlen, s, ncoef, offset);
         };
         if (comb) {
-            to_words(PB, o.T1, o.c1, o.l1, true);
+            to_words(PB, PT, o.T1, o.c1, o.l1, true);
         } else {
-            to_words(PB, o.T1, o.c1, o.l1, false);
-            to_words(PB + ST, o.T2, o.c2, o.l2, false);
+            to_words(PB, PT, o.T1, o.c1, o.l1, false);
+            to_words(PB + ST, PT + T, o.T2, o.c2, o.l2, false);
         }
-        to_words(QB, o.Q, o.cQ, o.lQ, false);
-        if (needR) to_words(RB, o.R, o.cR, o.lR, false);
+        to_words(QB, QT, o.Q, o.cQ, o.lQ, false);
+        if (needR) to_words(RB, RT, o.R, o.cR, o.lR, false);
         if (!comb) {
             fix_top_kernel<<<grid_for(np, 256), 256, 0, s>>>(o.T1, o.c1, o.l1, np);
             fix_top_kernel<<<grid_for(np, 256), 256, 0, s>>>(o.T2, o.c2, o.l2, np);

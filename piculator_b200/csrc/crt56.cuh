@@ -76,23 +76,27 @@ struct CrtDigits {
 };
 
 // Coefficients at[i], i < n: index(i) names the i-th (negative or past the last
-// one: zero), res(j, y0, y1, y2) gives its residues.
-template <int XS, class Index, class Res>
+// one: zero), res(j, y0, y1, y2) gives its residues, ahead of their use;
+// fix(j, y0, y1, y2) may change them when they have arrived.
+template <int XS, class Index, class Res, class Fix>
 __device__ __forceinline__ void crt_coefs(CrtDigits<XS>& X, int n, const CrtDConsts& C, const Index& index,
-                                          const Res& res)
+                                          const Res& res, const Fix& fix)
 {
     // the next coefficient's residues are on the way while one is converted
     double n0 = 0, n1 = 0, n2 = 0;
     int64_t nj = (int)threadIdx.x < n ? index((int)threadIdx.x) : -1;
     if (nj >= 0) res(nj, n0, n1, n2);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double y0 = n0, y1 = n1, y2 = n2;
-        const bool live = nj >= 0;
+        double y0 = n0, y1 = n1, y2 = n2;
+        const int64_t j = nj;
         nj = i + (int)blockDim.x < n ? index(i + (int)blockDim.x) : -1;
         if (nj >= 0) res(nj, n0, n1, n2);
         uint64_t d0 = 0, d1 = 0;
         uint32_t d2 = 0;
-        if (live) crt3d(C, y0, y1, y2, d0, d1, d2);
+        if (j >= 0) {
+            fix(j, y0, y1, y2);
+            crt3d(C, y0, y1, y2, d0, d1, d2);
+        }
         const int at = crt_slot(i);
         X.d0[at] = d0;
         X.d1[at] = d1;

@@ -774,20 +774,6 @@ void mul_ntt3(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size
 
 size_t pieces56(size_t nwords) { return (32 * nwords + 55) / 56; }
 
-struct DblPrimes3 {
-    double p[3], pinv[3];
-};
-
-static DblPrimes3 dbl_primes3()
-{
-    DblPrimes3 d;
-    for (int q = 0; q < 3; q++) {
-        d.p[q] = (double)kDblPrimes[q];
-        d.pinv[q] = 1.0 / d.p[q];
-    }
-    return d;
-}
-
 static NttBatch ntt3d_batch_stride(uint64_t* data, size_t stride)
 {
     NttBatch bat;
@@ -847,18 +833,59 @@ __device__ __forceinline__ int64_t crt_limit(size_t ncoef, size_t zw)
     return climit < (int64_t)ncoef ? climit : (int64_t)ncoef;
 }
 
-__device__ __forceinline__ void crt3d_block(const uint64_t* __restrict__ Y, size_t pstride, size_t ncoef,
+CrtWrap crt_wrap(const uint64_t* tail, size_t istride, size_t pstride, size_t T, size_t N, size_t W)
+{
+    CrtWrap w{tail, istride, pstride, (int64_t)N, (int64_t)W, (double)(N / T), {}};  // N / T: below every prime
+    for (int q = 0; q < 3; q++) w.cwp[q] = w.cw / (double)kDblPrimes[q];
+    return w;
+}
+
+// Residues of coefficient j of one product.  Wrapped: from N on they are the
+// tail's h(j - N) = d_(W - 1 + j - N) N / T, and the first W have h(j) taken out.
+// Three kernels of their own that rewrote those residues took 34 ms of a
+// computation of 1e9 digits, at the bandwidth of the memory; here it is one more
+// read of the tail (1.217 -> 1.195 s for the whole).
+template <bool WRAP>
+struct CrtSource {
+    const uint64_t *Y, *D;  // the product's residues, its tail's from W - 1 on
+    size_t pstride;
+
+    __device__ __forceinline__ void load(const CrtWrap& w, int64_t j, double& y0, double& y1, double& y2) const
+    {
+        const bool tail = WRAP && j >= w.N;
+        const uint64_t* p = tail ? D + (j - w.N) : Y + j;
+        const size_t st = tail ? w.pstride : pstride;
+        y0 = dbits(p[0]);
+        y1 = dbits(p[st]);
+        y2 = dbits(p[2 * st]);
+    }
+    __device__ __forceinline__ void fix(const CrtWrap& w, const CrtDConsts& C, int64_t j, double& y0, double& y1,
+                                        double& y2) const
+    {
+        if constexpr (WRAP) {
+            if (j >= w.N) {
+                y0 = dmul_tw(y0, w.cw, w.cwp[0], C.p[0]);
+                y1 = dmul_tw(y1, w.cw, w.cwp[1], C.p[1]);
+                y2 = dmul_tw(y2, w.cw, w.cwp[2], C.p[2]);
+            } else if (j < w.W) {
+                y0 = __dadd_rn(y0, -dmul_tw(dbits(D[j]), w.cw, w.cwp[0], C.p[0]));
+                y1 = __dadd_rn(y1, -dmul_tw(dbits(D[w.pstride + j]), w.cw, w.cwp[1], C.p[1]));
+                y2 = __dadd_rn(y2, -dmul_tw(dbits(D[2 * w.pstride + j]), w.cw, w.cwp[2], C.p[2]));
+            }
+        }
+    }
+};
+
+template <bool WRAP>
+__device__ __forceinline__ void crt3d_block(const CrtSource<WRAP>& S, const CrtWrap& wrap, size_t ncoef,
                                             const CrtDConsts& C, uint32_t* __restrict__ z, size_t zw, int64_t cta,
                                             uint32_t* agg_slot)
 {
     __shared__ CrtDigits<kCrtDSlots> X;
     const int64_t j0 = 8 * cta * kCrtDGroups - 3, jlim = crt_limit(ncoef, zw);
     crt_coefs(X, kCrtDCoefs, C, [&](int i) { return j0 + i < jlim ? j0 + i : (int64_t)-1; },
-              [&](int64_t j, double& y0, double& y1, double& y2) {
-                  y0 = dbits(Y[j]);
-                  y1 = dbits(Y[pstride + j]);
-                  y2 = dbits(Y[2 * pstride + j]);
-              });
+              [&](int64_t j, double& y0, double& y1, double& y2) { S.load(wrap, j, y0, y1, y2); },
+              [&](int64_t j, double& y0, double& y1, double& y2) { S.fix(wrap, C, j, y0, y1, y2); });
     __syncthreads();
     uint64_t t[8];
     const bool mine = threadIdx.x < kCrtDGroups;
@@ -871,31 +898,41 @@ __device__ __forceinline__ void crt3d_block(const uint64_t* __restrict__ Y, size
 }
 
 // A single CTA posts the top word; several leave their carries to carry_fix.
+template <bool WRAP>
 __global__ void __launch_bounds__(kCrtDThreads, 8) crt3d_k1(const uint64_t* __restrict__ Y, size_t pstride,
-                                                            size_t ncoef, CrtDConsts C, uint32_t* z, size_t zw,
-                                                            uint32_t* agg, MailRef mail)
+                                                            size_t ncoef, const __grid_constant__ CrtDConsts C,
+                                                            const __grid_constant__ CrtWrap wrap, uint32_t* z,
+                                                            size_t zw, uint32_t* agg, MailRef mail)
 {
-    crt3d_block(Y, pstride, ncoef, C, z, zw, (int64_t)blockIdx.x, agg + blockIdx.x);
+    const CrtSource<WRAP> S{Y, WRAP ? wrap.tail + wrap.W - 1 : nullptr, pstride};
+    crt3d_block(S, wrap, ncoef, C, z, zw, (int64_t)blockIdx.x, agg + blockIdx.x);
     if (mail.slot == nullptr) return;
     __syncthreads();
     if (threadIdx.x == 0) mail_post(mail, z[zw - 1]);
 }
 
+template <bool WRAP>
 __global__ void __launch_bounds__(kCrtDThreads, 8) crt3d_batch_k1(const uint64_t* __restrict__ Y, size_t istride,
-                                                                  size_t pstride, size_t ncoef, CrtDConsts C,
+                                                                  size_t pstride, size_t ncoef,
+                                                                  const __grid_constant__ CrtDConsts C,
+                                                                  const __grid_constant__ CrtWrap wrap,
                                                                   uint32_t* __restrict__ z, uint32_t zcap,
                                                                   const uint32_t* __restrict__ zlen, size_t cpp,
                                                                   uint32_t* agg)
 {
     const size_t prod = blockIdx.x / cpp, lc = blockIdx.x % cpp;
-    crt3d_block(Y + prod * istride, pstride, ncoef, C, z + prod * (size_t)zcap, zlen[prod], (int64_t)lc,
+    const CrtSource<WRAP> S{Y + prod * istride, WRAP ? wrap.tail + prod * wrap.istride + wrap.W - 1 : nullptr, pstride};
+    crt3d_block(S, wrap, ncoef, C, z + prod * (size_t)zcap, zlen[prod], (int64_t)lc,
                 agg + blockIdx.x);
 }
 
 // Short products: `per` groups each, `pack` products per CTA (at most 128 groups
 // and kCrtDCoefs coefficients), where one product would leave most of a CTA idle.
+template <bool WRAP>
 __global__ void __launch_bounds__(kCrtDThreads, 8) crt3d_pack_k1(const uint64_t* __restrict__ Y, size_t istride,
-                                                                 size_t pstride, size_t ncoef, CrtDConsts C,
+                                                                 size_t pstride, size_t ncoef,
+                                                                 const __grid_constant__ CrtDConsts C,
+                                                                 const __grid_constant__ CrtWrap wrap,
                                                                  uint32_t* __restrict__ z, uint32_t zcap,
                                                                  const uint32_t* __restrict__ zlen, size_t count,
                                                                  int per, int pack)
@@ -905,16 +942,20 @@ __global__ void __launch_bounds__(kCrtDThreads, 8) crt3d_pack_k1(const uint64_t*
     const int stride = 8 * per + 3;  // a product's coefficients, three zeros first
     const size_t p0 = (size_t)blockIdx.x * pack;
     const int n = (int)(count - p0 < (size_t)pack ? count - p0 : (size_t)pack);
-    const uint64_t* Yp = Y + p0 * istride;
+    auto source = [&](int64_t at) {
+        const size_t prod = p0 + (size_t)(at >> 32);
+        return CrtSource<WRAP>{Y + prod * istride, WRAP ? wrap.tail + prod * wrap.istride + wrap.W - 1 : nullptr, pstride};
+    };
     crt_coefs(X, n * stride, C,
               [&](int i) {
                   const int q = i / stride, j = i - q * stride - 3;
-                  return j >= 0 && j < crt_limit(ncoef, zlen[p0 + q]) ? (int64_t)q * (int64_t)istride + j : (int64_t)-1;
+                  return j >= 0 && j < crt_limit(ncoef, zlen[p0 + q]) ? ((int64_t)q << 32) + j : (int64_t)-1;
               },
               [&](int64_t at, double& y0, double& y1, double& y2) {
-                  y0 = dbits(Yp[at]);
-                  y1 = dbits(Yp[pstride + at]);
-                  y2 = dbits(Yp[2 * pstride + at]);
+                  source(at).load(wrap, (int64_t)(uint32_t)at, y0, y1, y2);
+              },
+              [&](int64_t at, double& y0, double& y1, double& y2) {
+                  if constexpr (WRAP) source(at).fix(wrap, C, (int64_t)(uint32_t)at, y0, y1, y2);
               });
     __syncthreads();
     uint64_t t[8];
@@ -934,23 +975,25 @@ static size_t crt3d_ctas(size_t zw) { return (zw + kCrtDWPC - 1) / kCrtDWPC; }
 
 // Inverse-transformed residues (product length 2^k, prime q at y + q pstride)
 // -> zw words; mail receives the top one.
-static void crt3d_to_words(const uint64_t* y, size_t pstride, int k, size_t ncoef, uint32_t* z, size_t zw,
-                           Mail* mail, cudaStream_t s)
+static void crt3d_to_words(const uint64_t* y, size_t pstride, int k, size_t ncoef, const CrtWrap& wrap, uint32_t* z,
+                           size_t zw, Mail* mail, cudaStream_t s)
 {
     const CrtDConsts C = make_crtd(k, false);
     const size_t nctas = crt3d_ctas(zw);
     DevBuf<uint32_t> agg(nctas, s);
     const MailRef m = mail ? mail->ref() : MailRef{};
     ProfScope ps(KC_CRT, 24.0 * (double)ncoef + 4.0 * (double)zw, s);
-    crt3d_k1<<<(unsigned)nctas, kCrtDThreads, 0, s>>>(y, pstride, ncoef, C, z, zw, agg.get(),
-                                                     nctas == 1 ? m : MailRef{});
+    auto kern = wrap.tail ? crt3d_k1<true> : crt3d_k1<false>;
+    kern<<<(unsigned)nctas, kCrtDThreads, 0, s>>>(y, pstride, ncoef, C, wrap, z, zw, agg.get(),
+                                                 nctas == 1 ? m : MailRef{});
     PIC_CHECK_LAUNCH();
     count_launch();
     if (nctas > 1) carry_fix(z, zw, kCrtDWPC, agg.get(), nctas, s, m);
 }
 
 void ntt3d_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, size_t count, int k, uint32_t* z,
-                          uint32_t zcap, const uint32_t* zlen, cudaStream_t s, size_t ncoef, bool offset)
+                          uint32_t zcap, const uint32_t* zlen, cudaStream_t s, size_t ncoef, bool offset,
+                          const CrtWrap& wrap)
 {
     if (count == 0) return;
     if (ncoef == 0) ncoef = (size_t)1 << k;
@@ -960,8 +1003,9 @@ void ntt3d_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, siz
     const int pack = std::min(kCrtDThreads / std::max(per, 1), kCrtDCoefs / (8 * per + 3));
     if (per >= 1 && pack >= 2) {
         ProfScope ps(KC_CRT, (24.0 * (double)ncoef + 4.0 * zcap) * (double)count, s);
-        crt3d_pack_k1<<<(unsigned)((count + pack - 1) / pack), kCrtDThreads, 0, s>>>(y, istride, pstride, ncoef, C, z,
-                                                                                  zcap, zlen, count, per, pack);
+        auto kern = wrap.tail ? crt3d_pack_k1<true> : crt3d_pack_k1<false>;
+        kern<<<(unsigned)((count + pack - 1) / pack), kCrtDThreads, 0, s>>>(y, istride, pstride, ncoef, C, wrap, z, zcap,
+                                                                            zlen, count, per, pack);
         PIC_CHECK_LAUNCH();
         count_launch();
         return;
@@ -971,43 +1015,12 @@ void ntt3d_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, siz
     DevBuf<uint32_t> agg(nctas, s);
     {
         ProfScope ps(KC_CRT, (24.0 * (double)ncoef + 4.0 * zcap) * (double)count, s);
-        crt3d_batch_k1<<<(unsigned)nctas, kCrtDThreads, 0, s>>>(y, istride, pstride, ncoef, C, z, zcap, zlen, cpp,
-                                                               agg.get());
+        auto kern = wrap.tail ? crt3d_batch_k1<true> : crt3d_batch_k1<false>;
+        kern<<<(unsigned)nctas, kCrtDThreads, 0, s>>>(y, istride, pstride, ncoef, C, wrap, z, zcap, zlen, cpp, agg.get());
         PIC_CHECK_LAUNCH();
         count_launch();
     }
     carry_fix_batch(z, zcap, zlen, kCrtDWPC, agg.get(), count, cpp, s);
-}
-
-// The wrapped form's fix-up (see wrap_fix_kernel) on FP64 residues:
-// y[j] -= h, y[Nm + j] = h with h = d_(W-1+j) Nm / T mod p.
-__global__ void wrap_fix_d_kernel(uint64_t* __restrict__ y, size_t ystride, const uint64_t* __restrict__ tail,
-                                  size_t T, size_t nitems, size_t item_mul, size_t nchild, size_t Nm, size_t W,
-                                  DblPrimes3 P, double cw, double cwp0, double cwp1, double cwp2)
-{
-    const size_t total = 3 * nitems * W;
-    for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < total; g += (size_t)gridDim.x * blockDim.x) {
-        const size_t q = g / (nitems * W);
-        const size_t r = g - q * nitems * W;
-        const size_t it = r / W, j = r - it * W;
-        const double p = q == 0 ? P.p[0] : (q == 1 ? P.p[1] : P.p[2]);
-        const double wp = q == 0 ? cwp0 : (q == 1 ? cwp1 : cwp2);
-        const size_t child = q * nchild + it * item_mul;
-        const double h = dmul_tw(dbits(tail[child * T + W - 1 + j]), cw, wp, p);
-        uint64_t* yi = y + child * ystride;
-        yi[j] = dstore(__dadd_rn(dbits(yi[j]), -h));
-        yi[Nm + j] = dstore(h);
-    }
-}
-
-void launch_wrap_fix_d(uint64_t* y, size_t ystride, const uint64_t* tail, size_t T, size_t nitems,
-                       size_t item_mul, size_t nchild, size_t Nm, size_t W, cudaStream_t s)
-{
-    const double cw = (double)(Nm / T);  // below every prime
-    wrap_fix_d_kernel<<<grid_for(3 * nitems * W, 256), 256, 0, s>>>(
-        y, ystride, tail, T, nitems, item_mul, nchild, Nm, W, dbl_primes3(), cw, cw / (double)kDblPrimes[0],
-        cw / (double)kDblPrimes[1], cw / (double)kDblPrimes[2]);
-    PIC_CHECK_LAUNCH();
 }
 
 // Largest shorter operand (in pieces) the FP64 form multiplies exactly:
@@ -1074,19 +1087,13 @@ static void mul_ntt3d_wrapped(uint32_t* z, const uint32_t* a, size_t na, const u
     const size_t pa = pieces56(na), pb = pieces56(nb);
     const size_t L = pa + pb - 1;
     const size_t Nm = (size_t)1 << km, T = (size_t)1 << kt, W = L - Nm;
-    const size_t ST = Nm + ((W + 15) & ~(size_t)15);
     const bool square = (a == b && na == nb);
     bool ready = false;
     uint64_t* spec = is_held(b, nb) ? held_spectrum(km, &ready, s) : nullptr;
-    DevBuf<uint64_t> A(3 * ST, s), tA(3 * T, s);
-    ntt3d_product(A.get(), ST, km, a, na, 0, b, nb, 0, square, spec, ready, s);
+    DevBuf<uint64_t> A(3 * Nm, s), tA(3 * T, s);
+    ntt3d_product(A.get(), Nm, km, a, na, 0, b, nb, 0, square, spec, ready, s);
     ntt3d_product(tA.get(), T, kt, a, na, Nm - pb + 1, b, nb, Nm - pa + 1, square, nullptr, false, s);
-    {
-        ProfScope ps(KC_NTT_POINTWISE, 3.0 * (double)W * 24.0, s);
-        launch_wrap_fix_d(A.get(), ST, tA.get(), T, 1, 1, 1, Nm, W, s);
-        count_launch();
-    }
-    crt3d_to_words(A.get(), ST, km, L, z, zw, mail, s);
+    crt3d_to_words(A.get(), Nm, km, L, crt_wrap(tA.get(), 0, T, T, Nm, W), z, zw, mail, s);
 }
 
 // The FP64 form of mul_ntt3 (PIC_MUL_NTT3D): products whose shorter operand
@@ -1129,7 +1136,7 @@ void mul_ntt3d(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, siz
     uint64_t* spec = is_held(b, nb) ? held_spectrum(k, &ready, s) : nullptr;
     DevBuf<uint64_t> A(3 * N, s);
     ntt3d_product(A.get(), N, k, a, na, 0, b, nb, 0, square, spec, ready, s);
-    crt3d_to_words(A.get(), N, k, ncoef, z, zw, mail, s);
+    crt3d_to_words(A.get(), N, k, ncoef, CrtWrap{}, z, zw, mail, s);
 }
 
 void mul_ntt_ref(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s)

@@ -33,12 +33,21 @@ bool mul_small_uniform(uint32_t* z, size_t zs, const uint32_t* a, size_t as, siz
                        size_t count, cudaStream_t s);
 // Products d[idx[i]], i < count, of at most 2^k coefficients.
 void mul_small_batch(const DevDesc* d, const uint32_t* idx, size_t count, int k, cudaStream_t s);
-// FP64-form building blocks: batched inverse output like ntt3_batch_to_words
-// (offset 2^140 per coefficient); wrapped-product fix-up like launch_wrap_fix.
+// A wrapped product's tail in the FP64 form (see wrap_fix_kernel): the middle
+// product of length T whose outputs W - 1 .. 2 W - 2 are the coefficients of
+// the product from N on, which wrapped onto the first W of the main transform.
+struct CrtWrap {
+    const uint64_t* tail = nullptr;  // null: not wrapped
+    size_t istride = 0, pstride = 0;  // of the products, of the primes
+    int64_t N = 0, W = 0;
+    double cw = 0, cwp[3] = {};  // N / T, the tails' other scale
+};
+CrtWrap crt_wrap(const uint64_t* tail, size_t istride, size_t pstride, size_t T, size_t N, size_t W);
+// FP64-form building block: batched inverse output like ntt3_batch_to_words
+// (offset 2^140 per coefficient), a wrapped form's tails folded in.
 void ntt3d_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, size_t count, int k, uint32_t* z,
-                          uint32_t zcap, const uint32_t* zlen, cudaStream_t s, size_t ncoef, bool offset);
-void launch_wrap_fix_d(uint64_t* y, size_t ystride, const uint64_t* tail, size_t T, size_t nitems,
-                       size_t item_mul, size_t nchild, size_t Nm, size_t W, cudaStream_t s);
+                          uint32_t zcap, const uint32_t* zlen, cudaStream_t s, size_t ncoef, bool offset,
+                          const CrtWrap& wrap);
 // The three-prime form of AUTO products and binary-splitting merges
 // (kFormInt, kFormDbl, or kFormChosen: per product by transform work).
 void mul_set_ntt_form(int form);

@@ -120,7 +120,8 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(MiddleShape<LR, 0>::
                   y0 = Y[0][at];
                   y1 = Y[1][at];
                   y2 = Y[2][at];
-              });
+              },
+              [](int64_t, double&, double&, double&) {});
     __syncthreads();
     uint64_t t[8];
     if (mine) crt_group(X, 8 * (int)threadIdx.x + 3, t);

@@ -55,6 +55,18 @@ def test_wrapped_and_plain_forms(pic, na, nb):
         pic.set_tuning(pic.TUNE_MUL_WRAP, saved)
 
 
+@pytest.mark.parametrize("W", [1, 2, 1018, 1020, 2048, 4096])
+def test_wrapped_tails(pic, W):
+    """pa + pb - 1 = 2^14 + W pieces of 56 bits: W coefficients wrap, from one to
+    all that the tail's half length allows; the CRT takes them from the tail, in
+    CTAs of 1019 coefficients."""
+    pa, pb = 8193, 8192 + W
+    a, b = (random_words(W + i, 56 * p // 32) for i, p in enumerate((pa, pb)))  # 56 p / 32 words: p pieces
+    a[-1], b[-1] = 0xFFFFFFFF, 0xFFFFFFFF
+    assert [(32 * x.size + 55) // 56 for x in (a, b)] == [pa, pb]
+    assert _int(pic.mul_host(a, b, "ntt3d")) == _int(a) * _int(b)
+
+
 def test_squaring_same_pointer(pic, torch_cuda, oracle):
     torch = torch_cuda
     for n in (3000, 2200):
