@@ -40,42 +40,6 @@ namespace pic {
 
 constexpr int kColThreads = 256;
 
-// Butterflies of the smallest-stride round: t.at(l, u) = root_(2^(B - l))^u, so
-// u = 0 needs no product and the unit level none.  Forward: |x| <= 2 p gives
-// |x| <= 16 p, unreduced.
-template <int B>
-__device__ __forceinline__ void fwd_tail(double (&x)[1 << B], const GroupTw<B, 0>& t, const Dbl::Ctx& L)
-{
-#pragma unroll
-    for (int l = 0; l < B; l++) {
-        const int hm = 1 << (B - 1 - l);
-#pragma unroll
-        for (int m = 0; m < (1 << B); m++) {
-            if (m & hm) continue;
-            if ((m & (hm - 1)) == 0) Dbl::dif_unit<false>(x[m], x[m + hm], L);
-            else Dbl::dif<false>(x[m], x[m + hm], t.at(l, m & (hm - 1)), L);
-        }
-    }
-}
-
-// Inverse: |x| <= p gives |x| <= 8 p, or 5 p with the products of the last
-// level's u = 0 kept (KEEP: tall columns, which add up to 8 p more after it and
-// must end below 15 p).
-template <int B, bool KEEP>
-__device__ __forceinline__ void inv_head(double (&x)[1 << B], const GroupTw<B, 0>& t, const Dbl::Ctx& L)
-{
-#pragma unroll
-    for (int l = B - 1; l >= 0; l--) {
-        const int hm = 1 << (B - 1 - l);
-#pragma unroll
-        for (int m = 0; m < (1 << B); m++) {
-            if (m & hm) continue;
-            if ((m & (hm - 1)) == 0 && !(KEEP && l == 0)) Dbl::dit_unit(x[m], x[m + hm], L);
-            else Dbl::dit(x[m], x[m + hm], t.at(l, m & (hm - 1)), L);
-        }
-    }
-}
-
 struct ColTables {
     const double* w[3];  // per prime: W(g, c) at g M + c, or null
 };

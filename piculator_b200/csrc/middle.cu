@@ -15,13 +15,16 @@
 // Merges of a pi computation at 1e9 digits (binary splitting, one B200): a
 // level of 2^17-point transforms 64.4 -> 54.5 ms, of 2^12 points 55.8 -> 38.6,
 // the whole computation 1.73 -> 1.49 s, against the same passes launched
-// apart.  What is left in the kernel is FP64 work (about 430 instructions per
-// parent point and prime: 6 forward and 3 inverse rows of 11 levels) with two
+// apart.  What is left in the kernel is FP64 work (about 415 instructions per
+// parent point and prime: 6 forward and 3 inverse rows of 11 levels; 16 more with
+// the products by one and a reduction of every last sum: the whole computation
+// then 0.8 % slower, a product of 4096 words 32.3 us for 30.7) with two
 // CTAs of 256 threads per SM, the rows' 96 KB of shared memory being the limit.
 // One product (two operands, 24 B a point instead of 72): 2^24-word operands
 // 4.00 -> 3.32 ms, 1,048,573 x 400,009 words 186 -> 146 us, 4096 words 82 -> 45
 // us (the operands' pieces are read by the first pass, 16 launches -> 8).
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "middle.cuh"
@@ -92,13 +95,15 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
             const int t = g >> LG;
             const int pb = (t << LR) + place((g & ((1 << LG) - 1)) << B);
             const int base = (g & ((1 << LG) - 1)) << B;
-            auto load = [&](int a, double(&x)[E]) {  // NR 1: the only round
+            auto load = [&](int a, double(&x)[E], auto red) {  // NR 1: the only round
 #pragma unroll
                 for (int m = 0; m < E; m++) x[m] = Sh::NR == 1 ? in(a, t, base + m) : ms[a * TOT + place_at(pb, m)];
-                fwd_group<B, 0>(x, wf, L);
+                fwd_last<B, red.value>(x, wf, L);
             };
+            constexpr std::true_type kReduced{};
+            constexpr std::false_type kRaw{};
             auto store = [&](int a, double(&x)[E]) {
-                inv_group<B, 0>(x, wi, L);
+                inv_first<B, LR, 2>(x, wi, L);
 #pragma unroll
                 for (int m = 0; m < E; m++) {
                     if constexpr (Sh::NR == 1) put(a, t, base + m, x[m]);
@@ -106,10 +111,10 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
                 }
             };
             double qr[E], rl[E], x[E], y[E];
-            load(3, qr);
-            load(4, rl);
-            load(0, x);
-            load(1, y);
+            load(3, qr, kReduced);
+            load(4, rl, kReduced);
+            load(0, x, kRaw);
+            load(1, y, kRaw);
 #pragma unroll
             for (int m = 0; m < E; m++) {
                 x[m] = dmul_mod(x[m], qr[m], L.p, L.pinv);
@@ -125,12 +130,12 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
                 store(1, y);
             }
             store(0, x);
-            load(2, x);
+            load(2, x, kRaw);
 #pragma unroll
             for (int m = 0; m < E; m++) x[m] = dmul_mod(x[m], qr[m], L.p, L.pinv);
             store(2, x);
             if (M.need_r) {
-                load(5, y);
+                load(5, y, kRaw);
 #pragma unroll
                 for (int m = 0; m < E; m++) y[m] = dmul_mod(y[m], rl[m], L.p, L.pinv);
                 store(4, y);
@@ -261,7 +266,8 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
             auto load = [&](int i, double(&v)[E]) {
 #pragma unroll
                 for (int m = 0; m < E; m++) v[m] = ms[i * TOT + place_at(pb, m)];
-                fwd_group<B, 0>(v, wf, L);
+                if (i == 1 || M.square) fwd_last<B, true>(v, wf, L);
+                else fwd_last<B, false>(v, wf, L);
             };
             if (need_a) load(0, x);
             if (need_b) load(1, y);
@@ -275,7 +281,7 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
             }
 #pragma unroll
             for (int m = 0; m < E; m++) x[m] = dmul_mod(x[m], M.square ? x[m] : y[m], L.p, L.pinv);
-            inv_group<B, 0>(x, wi, L);
+            inv_first<B, LR, 1>(x, wi, L);
 #pragma unroll
             for (int m = 0; m < E; m++) ms[place_at(pb, m)] = x[m];
         }

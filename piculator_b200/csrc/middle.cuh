@@ -61,6 +61,65 @@ __device__ __forceinline__ void inv_group(double (&x)[1 << B], const GroupTw<B, 
     }
 }
 
+// The same for the smallest-stride round, where t.at(l, u) = root_(2^(B - l))^u,
+// so u = 0 needs no product and the unit level none.  Forward: |x| <= 2 p gives
+// |x| <= 16 p (8 p for B = 2), unreduced, for a product that follows at once.
+template <int B>
+__device__ __forceinline__ void fwd_tail(double (&x)[1 << B], const GroupTw<B, 0>& t, const Dbl::Ctx& L)
+{
+#pragma unroll
+    for (int l = 0; l < B; l++) {
+        const int hm = 1 << (B - 1 - l);
+#pragma unroll
+        for (int m = 0; m < (1 << B); m++) {
+            if (m & hm) continue;
+            if ((m & (hm - 1)) == 0) Dbl::dif_unit<false>(x[m], x[m + hm], L);
+            else Dbl::dif<false>(x[m], x[m + hm], t.at(l, m & (hm - 1)), L);
+        }
+    }
+}
+
+// Inverse: |x| <= X gives |x| <= 2^B X, or 2^(B - 1) X + p with the products of
+// the last level's u = 0 kept (KEEP: the levels after it add up to p each and
+// must end below 15.75 p).
+template <int B, bool KEEP>
+__device__ __forceinline__ void inv_head(double (&x)[1 << B], const GroupTw<B, 0>& t, const Dbl::Ctx& L)
+{
+#pragma unroll
+    for (int l = B - 1; l >= 0; l--) {
+        const int hm = 1 << (B - 1 - l);
+#pragma unroll
+        for (int m = 0; m < (1 << B); m++) {
+            if (m & hm) continue;
+            if ((m & (hm - 1)) == 0 && !(KEEP && l == 0)) Dbl::dit_unit(x[m], x[m + hm], L);
+            else Dbl::dit(x[m], x[m + hm], t.at(l, m & (hm - 1)), L);
+        }
+    }
+}
+
+// The last forward round of a row, for pointwise products: of two factors one is
+// reduced (|x| <= p / 2 + 1) and the other left at up to 16 p, a product of at
+// most 8 p^2 and below 0.75 p after its reduction.
+template <int B, bool RED>
+__device__ __forceinline__ void fwd_last(double (&x)[1 << B], const GroupTw<B, 0>& t, const Dbl::Ctx& L)
+{
+    fwd_tail<B>(x, t, L);
+    if constexpr (RED) {
+#pragma unroll
+        for (int m = 0; m < (1 << B); m++) x[m] = dreduce(x[m], L.p, L.pinv);
+    }
+}
+
+// The first inverse round of a 2^LR row whose points are below X = 0.75 TERMS p
+// (a sum of TERMS products): at most 4 X, the LR - 2 levels (or LR - 1, of 2 X)
+// after it p each, and the row ends below 15.75 p.
+template <int B, int LR, int TERMS>
+__device__ __forceinline__ void inv_first(double (&x)[1 << B], const GroupTw<B, 0>& t, const Dbl::Ctx& L)
+{
+    if constexpr (B == 1 || 4 * 0.75 * TERMS + (LR - 2) > 15.75) inv_group<B, 0>(x, t, L);
+    else inv_head<B, B == 3>(x, t, L);
+}
+
 // Shared-memory place of a row's element e: bits 4, 5, 6 of e are XORed into
 // bits 0, (1 and 2), 3.  The map is linear, so the place of base + (m << LST)
 // (disjoint bits) is place(base) ^ place(m << LST), the latter a constant.

@@ -86,13 +86,14 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(MiddleShape<LR, 0>::
             auto load = [&](int i, double(&v)[E]) {
 #pragma unroll
                 for (int m = 0; m < E; m++) v[m] = ms[i * TOT + place_at(pb, m)];
-                fwd_group<B, 0>(v, wf, L);
+                if (i == 1 || square) fwd_last<B, true>(v, wf, L);
+                else fwd_last<B, false>(v, wf, L);
             };
             load(0, x);
             if (!square) load(1, y);
 #pragma unroll
             for (int m = 0; m < E; m++) x[m] = dmul_mod(x[m], square ? x[m] : y[m], L.p, L.pinv);
-            inv_group<B, 0>(x, wi, L);
+            inv_first<B, LR, 1>(x, wi, L);
 #pragma unroll
             for (int m = 0; m < E; m++) ms[place_at(pb, m)] = x[m];
         }

@@ -25,6 +25,19 @@ def test_forward_round_ranges(tmp_path, bits):
 
 
 @pytest.mark.skipif(shutil.which("gcc") is None, reason="gcc not available")
+@pytest.mark.parametrize("terms", [1, 2])
+@pytest.mark.parametrize("row_bits", [4, 5, 9, 10, 11, 12, 13])
+def test_middle_round_ranges(tmp_path, row_bits, terms):
+    """The last forward and the first inverse round of a row without the products
+    by one (tests/host/fp64_middle_check.c)."""
+    exe = tmp_path / "fp64_middle_check"
+    subprocess.run(["gcc", "-O2", "-ffp-contract=off", "-o", str(exe),
+                    os.path.join(HERE, "host", "fp64_middle_check.c"), "-lm"], check=True)
+    out = subprocess.run([str(exe), str(row_bits), str(terms), "50000"], capture_output=True, text=True)
+    assert out.returncode == 0 and out.stdout.startswith("bad=0"), out.stdout + out.stderr
+
+
+@pytest.mark.skipif(shutil.which("gcc") is None, reason="gcc not available")
 def test_crt_digits_exact(tmp_path):
     exe = tmp_path / "crt56_check"
     subprocess.run(["gcc", "-O2", "-ffp-contract=off", "-o", str(exe), os.path.join(HERE, "host", "crt56_check.c"),
