@@ -17,14 +17,13 @@
 // the whole computation 1.73 -> 1.49 s, against the same passes launched
 // apart.  What is left in the kernel is FP64 work (about 415 instructions per
 // parent point and prime: 6 forward and 3 inverse rows of 11 levels; 16 more with
-// the products by one and a reduction of every last sum: the whole computation
-// then 0.8 % slower, a product of 4096 words 32.3 us for 30.7) with two
+// the products by one and a reduction of every last sum: the merges' middle
+// passes 409 ms for 401, a whole computation 1.2005 s for 1.1945) with two
 // CTAs of 256 threads per SM, the rows' 96 KB of shared memory being the limit.
 // One product (two operands, 24 B a point instead of 72): 2^24-word operands
 // 4.00 -> 3.32 ms, 1,048,573 x 400,009 words 186 -> 146 us, 4096 words 82 -> 45
 // us (the operands' pieces are read by the first pass, 16 launches -> 8).
 #include <algorithm>
-#include <type_traits>
 
 #include "common.cuh"
 #include "middle.cuh"
@@ -95,13 +94,12 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
             const int t = g >> LG;
             const int pb = (t << LR) + place((g & ((1 << LG) - 1)) << B);
             const int base = (g & ((1 << LG) - 1)) << B;
-            auto load = [&](int a, double(&x)[E], auto red) {  // NR 1: the only round
+            auto load = [&](int a, double(&x)[E]) {  // NR 1: the only round
 #pragma unroll
                 for (int m = 0; m < E; m++) x[m] = Sh::NR == 1 ? in(a, t, base + m) : ms[a * TOT + place_at(pb, m)];
-                fwd_last<B, red.value>(x, wf, L);
+                if (a == 3 || a == 4) fwd_last<B, true>(x, wf, L);  // QR and RL, in two products each
+                else fwd_last<B, false>(x, wf, L);
             };
-            constexpr std::true_type kReduced{};
-            constexpr std::false_type kRaw{};
             auto store = [&](int a, double(&x)[E]) {
                 inv_first<B, LR, 2>(x, wi, L);
 #pragma unroll
@@ -111,10 +109,10 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
                 }
             };
             double qr[E], rl[E], x[E], y[E];
-            load(3, qr, kReduced);
-            load(4, rl, kReduced);
-            load(0, x, kRaw);
-            load(1, y, kRaw);
+            load(3, qr);
+            load(4, rl);
+            load(0, x);
+            load(1, y);
 #pragma unroll
             for (int m = 0; m < E; m++) {
                 x[m] = dmul_mod(x[m], qr[m], L.p, L.pinv);
@@ -130,12 +128,12 @@ __global__ void __launch_bounds__(MiddleShape<LR, LT>::NT, MiddleShape<LR, LT>::
                 store(1, y);
             }
             store(0, x);
-            load(2, x, kRaw);
+            load(2, x);
 #pragma unroll
             for (int m = 0; m < E; m++) x[m] = dmul_mod(x[m], qr[m], L.p, L.pinv);
             store(2, x);
             if (M.need_r) {
-                load(5, y, kRaw);
+                load(5, y);
 #pragma unroll
                 for (int m = 0; m < E; m++) y[m] = dmul_mod(y[m], rl[m], L.p, L.pinv);
                 store(4, y);
