@@ -22,6 +22,7 @@
 #include <mutex>
 #include <vector>
 
+#include "blockmul.cuh"
 #include "carry.cuh"
 #include "common.cuh"
 #include "mul.cuh"
@@ -36,70 +37,15 @@ __global__ void __launch_bounds__(kPSchThreads) school_persistent_kernel(const D
                                                                          const uint32_t* __restrict__ order,
                                                                          uint32_t n, uint32_t* counter)
 {
-    extern __shared__ uint32_t sm[];
-    __shared__ uint32_t s_item;
+    extern __shared__ __align__(16) uint32_t sch[];
+    __shared__ uint32_t s_item, s_w[32];
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1u);
         __syncthreads();
         const uint32_t it = s_item;
-        __syncthreads();
         if (it >= n) return;
         const DevDesc D = d[order[it]];
-        const uint32_t na = D.na, nb = D.nb, zw = na + nb;
-        uint32_t* sa = sm;
-        uint32_t* sb = sa + na;
-        uint32_t* col = sb + nb;
-        for (uint32_t i = threadIdx.x; i < na; i += blockDim.x) sa[i] = D.a[i];
-        for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x) sb[i] = D.b[i];
-        __syncthreads();
-        for (uint32_t c = threadIdx.x; c < zw; c += blockDim.x) {
-            uint64_t lo = 0;
-            uint32_t hi = 0;
-            if (c + 1 < zw) {
-                const uint32_t i_lo = c + 1 > nb ? c + 1 - nb : 0;
-                const uint32_t i_hi = c < na - 1 ? c : na - 1;
-                for (uint32_t i = i_lo; i <= i_hi; i++) {
-                    const uint64_t pr = (uint64_t)sa[i] * sb[c - i];
-                    lo += pr;
-                    hi += (lo < pr);
-                }
-            }
-            col[3 * c] = (uint32_t)lo;
-            col[3 * c + 1] = (uint32_t)(lo >> 32);
-            col[3 * c + 2] = hi;
-        }
-        __syncthreads();
-        const uint32_t per = (zw + blockDim.x - 1) / blockDim.x;
-        const uint32_t w0 = threadIdx.x * per, w1 = min(w0 + per, zw);
-        auto digit = [&](uint32_t w, uint32_t& g) -> uint32_t {
-            uint64_t sw = col[3 * w], sp = 0;
-            if (w >= 1) {
-                sw += col[3 * (w - 1) + 1];
-                sp += col[3 * (w - 1)];
-            }
-            if (w >= 2) {
-                sw += col[3 * (w - 2) + 2];
-                sp += col[3 * (w - 2) + 1];
-            }
-            if (w >= 3) sp += col[3 * (w - 3) + 2];
-            const uint64_t t = (sw & 0xffffffffu) + (sp >> 32);
-            g = (uint32_t)(t >> 32);
-            return (uint32_t)t;
-        };
-        uint32_t gp = kGPIdentity;
-        for (uint32_t w = w0; w < w1; w++) {
-            uint32_t g;
-            const uint32_t dd = digit(w, g);
-            gp = gp_combine(gp, g | ((uint32_t)(dd == 0xffffffffu) << 1));
-        }
-        uint32_t total;
-        uint32_t cin = block_gp_scan(gp, &total) & 1u;
-        for (uint32_t w = w0; w < w1; w++) {
-            uint32_t g;
-            const uint32_t dd = digit(w, g);
-            D.z[w] = dd + cin;
-            cin = g | ((uint32_t)(dd == 0xffffffffu) & cin);
-        }
+        block_product(sch, s_w, D.a, D.na, D.b, D.nb, [&](uint32_t w, uint32_t v) { D.z[w] = v; });
         __syncthreads();
     }
 }
@@ -165,7 +111,7 @@ struct Plan {
     std::vector<uint32_t> school;  // descriptor indices, longest first
     DevBuf<uint32_t> dschool;
     DevBuf<uint32_t> counter;
-    uint32_t school_max_zw = 0;
+    uint32_t school_words = 0;  // shared memory of the schoolbook CTAs
     std::vector<Bin> bins;
     cudaGraphExec_t exec = nullptr;
     uint64_t kernels = 0;
@@ -208,7 +154,7 @@ static void enqueue_plan(Plan& P, cudaStream_t s)
 {
     if (!P.school.empty()) {
         PIC_CUDA(cudaMemsetAsync(P.counter.get(), 0, sizeof(uint32_t), s));
-        const size_t smem = (size_t)P.school_max_zw * 16;
+        const size_t smem = sizeof(uint32_t) * (size_t)P.school_words;
         if (smem > 48 * 1024)
             PIC_CUDA(cudaFuncSetAttribute(school_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
@@ -272,7 +218,7 @@ static std::unique_ptr<Plan> build_plan(const pic_mul_desc* d, size_t count, int
         const int c = batch_class(d[i], mode);
         if (c < 0) {
             P->school.push_back((uint32_t)i);
-            P->school_max_zw = std::max<uint32_t>(P->school_max_zw, (uint32_t)(d[i].na + d[i].nb));
+            P->school_words = std::max(P->school_words, BlockProduct((uint32_t)d[i].na, (uint32_t)d[i].nb, kPSchThreads).words());
         } else {
             Bin& B = bins[c];
             B.small = c >= kSmallClass;

@@ -146,4 +146,77 @@ __device__ __forceinline__ uint32_t block_carry(uint32_t gen, uint32_t prop, uin
     return (uint32_t)((((((uint64_t)g << 1) | ((cw >> wid) & 1u)) + p) ^ p) >> lane) & 1u;
 }
 
+// One product by a whole CTA of T threads (whole warps): rows of at most T
+// threads, and where they leave threads idle the first operand's blocks are split
+// into up to eight runs, each with diagonals of its own.
+struct BlockProduct {
+    uint32_t ma, mb, S;  // blocks of the shorter and of the longer operand; runs
+    __host__ __device__ BlockProduct(uint32_t na, uint32_t nb, uint32_t T)
+    {
+        const uint32_t x = (na + 7) / 8, y = (nb + 7) / 8;
+        ma = x < y ? x : y;
+        mb = x < y ? y : x;
+        S = mb ? T / mb : 1;
+        if (S > 8) S = 8;
+        if (S > ma) S = ma;
+        if (S < 1) S = 1;
+    }
+    __host__ __device__ uint32_t words() const { return (ma + mb) * (8 + S * kDiagWords); }
+};
+
+// put(w, v): word w of a * b, w < na + nb, from one thread each.  sm: 16-byte
+// aligned, words() words; s_w: 32 words.  Ends without a barrier.
+template <class Put>
+__device__ __forceinline__ void block_product(uint32_t* sm, uint32_t* s_w, const uint32_t* __restrict__ a, uint32_t na,
+                                              const uint32_t* __restrict__ b, uint32_t nb, const Put& put)
+{
+    const uint32_t T = blockDim.x, tid = threadIdx.x, lane = tid & 31, zw = na + nb;
+    if (na > nb) {
+        const uint32_t* p = a;
+        a = b, b = p;
+        const uint32_t n = na;
+        na = nb, nb = n;
+    }
+    const BlockProduct P(na, nb, T);
+    const uint32_t slots = P.ma + P.mb;
+    uint32_t* sa = sm;
+    uint32_t* sb = sa + 8 * P.ma;
+    uint32_t* diag = sb + 8 * P.mb;
+    for (uint32_t i = tid; i < 8 * P.ma; i += T) sa[i] = i < na ? a[i] : 0u;
+    for (uint32_t i = tid; i < 8 * P.mb; i += T) sb[i] = i < nb ? b[i] : 0u;
+    for (uint32_t i = tid; i < P.S * slots * kDiagWords; i += T) diag[i] = 0;  // slots a run does not reach
+    __syncthreads();
+    for (uint32_t t = tid; t < P.S * P.mb; t += T) {
+        const uint32_t run = t / P.mb, d = t - run * P.mb;
+        const uint32_t i0 = run * P.ma / P.S, i1 = (run + 1) * P.ma / P.S;
+        block_diagonals(sa + 8 * i0, (int)(i1 - i0), sb, (int)P.mb, (int)d, diag + kDiagWords * (run * slots + i0));
+    }
+    __syncthreads();
+    // a thread per word; sums of at most 2^32 (2 S + 1): digits as in block_digits
+    auto sum = [&](uint32_t w) {
+        const uint32_t c = w >> 3, r = w & 7;
+        uint64_t s = 0;
+        for (uint32_t run = 0; run < P.S; run++) {
+            const uint32_t* p = diag + kDiagWords * (run * slots + c) + r;
+            s += p[0];
+            if (c >= 1) s += p[8 - kDiagWords];
+            if (c >= 2 && r == 0) s += p[16 - 2 * kDiagWords];
+        }
+        return s;
+    };
+    uint32_t cin = 0;
+    for (uint32_t base = 0; base < zw; base += T) {
+        const uint32_t w = base + tid;
+        const uint64_t s = w < zw ? sum(w) : 0;
+        uint32_t up = __shfl_up_sync(0xffffffffu, (uint32_t)(s >> 32), 1);
+        if (lane == 0) up = w > 0 && w < zw ? (uint32_t)(sum(w - 1) >> 32) : 0u;
+        const uint32_t t = (uint32_t)s + up;
+        uint32_t cout;
+        const uint32_t c = block_carry(t < up, t == 0xffffffffu, cin, s_w, &cout);
+        cin = cout;
+        if (w < zw) put(w, t + c);
+        if (base + T < zw) __syncthreads();  // s_w again
+    }
+}
+
 }  // namespace pic

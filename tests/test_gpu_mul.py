@@ -32,6 +32,29 @@ def test_products_vs_oracle(pic, oracle, mode, na, nb):
     assert np.array_equal(z, oracle.mul_words(a, b))
 
 
+@pytest.mark.parametrize("na,nb", [(8, 8), (9, 8), (16, 17), (63, 65), (72, 80), (128, 128), (129, 127), (250, 260),
+                                   (48, 2040), (5, 4091), (256, 1023), (2048, 2048)])
+def test_school_blocks(pic, torch_cuda, na, nb):
+    """Schoolbook products in 8-word blocks, alone (CTAs of 256 threads: rows split
+    into one to eight runs, more rows than threads) and in a batch, with words
+    that make the longest carries."""
+    for fill in (False, True):
+        a, b = (np.full(n, 0xFFFFFFFF, dtype=np.uint32) if fill else random_words(na + 3 * i, n)
+                for i, n in enumerate((na, nb)))
+        want = _int(a) * _int(b)
+        assert _int(pic.mul_host(a, b, "school")) == want
+        assert _int(pic.mul_host(b, a, "school")) == want
+        x, y = (torch_cuda.from_numpy(w.view(np.int32)).cuda() for w in (a, b))
+        z = torch_cuda.zeros(3, na + nb, dtype=torch_cuda.int32, device="cuda")
+        ptr = [r.data_ptr() for r in z]
+        torch_cuda.cuda.synchronize()
+        pic.mul_batch_dev([(ptr[0], x.data_ptr(), na, y.data_ptr(), nb), (ptr[1], y.data_ptr(), nb, x.data_ptr(), na),
+                           (ptr[2], x.data_ptr(), na, y.data_ptr(), 1)], "school")
+        pic.synchronize()
+        got = [_int(r.cpu().numpy().view(np.uint32)) for r in z]
+        assert got == [want, want, _int(a) * int(b[0])]
+
+
 @pytest.mark.parametrize("mode", ["ntt_ref", "ntt3", "fft", "auto"])
 @pytest.mark.parametrize("n", [5000, 1 << 14, 40000, 1 << 17])
 def test_products_vs_python_int(pic, mode, n):
