@@ -543,14 +543,15 @@ def ours(args):
     total_k = sum(k["seconds"] for k in kstats) or 1.0
     # DRAM bytes per algorithmic byte (16 B per point and pass) of the NTT
     # passes: dram__bytes_read.sum + dram__bytes_write.sum of every launch of
-    # the kernel in one 1e9-digit computation (ncu, one pass per launch), over
-    # the kernel's algorithmic bytes in the same computation.  FP64 form:
-    # columns 1786.5 GB / 1763.6 GB (their per-point twiddle tables mostly hit
-    # L2).  Integer form, from the 2^23-word product:
-    # rows 14.9 B and columns 30.8 B per point.
+    # the kernel in one computation (ncu, one pass per launch), over the kernel's
+    # algorithmic bytes in the same computation.  FP64 form, 1e8 digits: columns
+    # 88.2 GB / 123.6 GB (their first pass reads 56-bit pieces from the words, and
+    # a batch's results stay partly in L2), fused middle passes 55.8 / 65.2.
+    # Integer form, from the 2^23-word product: rows 14.9 B and columns 30.8 B
+    # per point.
     if P.get_tuning(P.TUNE_NTT_FORM) == P.FORM_DBL:
-        dram_per_alg = {"ntt_cols": 1786.5 / 1763.6}
-        traffic_basis = ("ncu DRAM bytes of every launch of the kernel in one 1e9-digit computation over its "
+        dram_per_alg = {"ntt_cols": 88.2 / 123.6, "ntt_middle": 55.8 / 65.2}
+        traffic_basis = ("ncu DRAM bytes of every launch of the kernel in one 1e8-digit computation over its "
                          "algorithmic bytes, times the kernel's average launch")
     else:
         dram_per_alg = {"ntt_rows": 14.9 / 16.0, "ntt_cols": 30.8 / 16.0}

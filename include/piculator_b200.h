@@ -327,7 +327,8 @@ int64_t pic_get_tuning(int knob);
 pic_status pic_set_ntt_geometry(int k, int row_bits, int col_width_log2, int radix_log2);
 pic_status pic_get_ntt_geometry(int k, int* row_bits, int* col_width_log2, int* radix_log2);
 /* The same per product form (0 integer, 1 FP64; the FP64 form takes row bits
- * 11..13 and radix bits 3..4, its passes having no general fallback). */
+ * 11..13 and radix bits 3..4, but its rows are 11 bits in radix-8 rounds whatever
+ * these say: of the three only the column width changes its passes). */
 pic_status pic_set_ntt_geometry_form(int form, int k, int row_bits, int col_width_log2, int radix_log2);
 pic_status pic_get_ntt_geometry_form(int form, int k, int* row_bits, int* col_width_log2, int* radix_log2);
 

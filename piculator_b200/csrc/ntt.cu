@@ -889,18 +889,14 @@ __global__ void pass_table_kernel(void* __restrict__ out_v, PrimeDev P, int inv,
 // register round and written by the last, without staging.
 // RB 4: radix-16 rounds, 16 residues per thread, two CTAs per SM.
 // Resident CTAs per SM the column kernels are compiled for (the register
-// budget): radix-16 two; radix-8 integer four forward, three inverse; FP64
-// PIC_DBL_COLS_MINB.
-#ifndef PIC_DBL_COLS_MINB
-#define PIC_DBL_COLS_MINB 4
-#endif
-template <class A, int RB, bool INV>
+// budget): radix-16 two; radix-8 four forward, three inverse.
+template <int RB, bool INV>
 struct ColsMinBlocks {
-    static constexpr int value = RB == 4 ? 2 : (std::is_same<A, ArithDbl>::value ? PIC_DBL_COLS_MINB : (INV ? 3 : 4));
+    static constexpr int value = RB == 4 ? 2 : (INV ? 3 : 4);
 };
 
 template <bool INV, int LC, int LW, int RB, class A>
-__global__ void __launch_bounds__(256, ColsMinBlocks<A, RB, INV>::value)
+__global__ void __launch_bounds__(256, ColsMinBlocks<RB, INV>::value)
     ntt_cols_fast_kernel(NttBatch B, int k, int lpre, PassTw pt)
 {
     extern __shared__ uint64_t smem[];
@@ -1225,10 +1221,11 @@ constexpr int kPassTableMaxBits = 24;
 static std::mutex g_pass_lock;
 static std::map<std::tuple<int, uint64_t, int, int, int>, void*> g_pass_tables;
 
-// FP64 column passes stream the per-point table only for blocks of at most
-// 2^g_dbl_pass_bits points (tables that stay in L2); longer ones form each
-// twiddle from the two-level tables (two products on the FP64 pipe, which
-// has room), saving 16 bytes of DRAM traffic per point.
+// The bulk-copy FP64 column kernel streams the per-point table only for blocks of
+// at most 2^g_dbl_pass_bits points (tables that stay in L2); longer ones form each
+// twiddle from the two-level tables (two products on the FP64 pipe, which has
+// room), saving 8 bytes of DRAM traffic per point.  The kernel that runs by
+// default has its own tables (cols.cu).
 static int g_dbl_pass_bits = 20;
 void ntt_set_dbl_pass_bits(int bits) { g_dbl_pass_bits = bits; }
 int ntt_dbl_pass_bits() { return g_dbl_pass_bits; }

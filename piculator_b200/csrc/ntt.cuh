@@ -202,10 +202,11 @@ double butterfly_ceiling_dbl(cudaStream_t s);
 std::vector<int> ntt_pass_bits(int k, int form = kFormInt);
 // Tunable geometry per length and form (row-pass bits 8..13, column tile
 // log2 width 0..6 with 0 = automatic, bits per register round 2..4; the FP64
-// form runs only the fast passes: row bits 11..13, rounds of 3 or 4 bits).
+// form accepts row bits 11..13 and rounds of 3 or 4 bits, but its row passes are
+// the fused middle passes, 11 bits in rounds of 3: only the width changes them).
 void ntt_set_geometry(int k, int row_bits, int col_lw, int rbits, int form = kFormInt);
-// FP64 column passes use per-point twiddle tables for blocks of at most
-// 2^bits points (0: never), else the two-level tables.
+// The bulk-copy FP64 column kernel uses per-point twiddle tables for blocks of at
+// most 2^bits points (0: never), else the two-level tables.
 void ntt_set_dbl_pass_bits(int bits);
 int ntt_dbl_pass_bits();
 // FP64 column passes of 2^5 .. 2^9 rows through the persistent kernel fed by
