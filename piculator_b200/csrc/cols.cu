@@ -14,8 +14,9 @@
 //    (or the two-level outer tables), the powers of Q are made once per thread:
 //    one more FP64 product per point instead of a streamed 8-byte table entry.
 //    That round's smallest-stride butterflies have twiddles that are constants,
-//    one in four of them 1, and nothing after it needs a reduction (the twiddle
-//    product takes any |y| < 2^51).
+//    one in four of them 1, and nothing after it needs a reduction: the twiddle
+//    product takes any |y| < 2^51.  In a pass of at most three bits row 0 meets no
+//    twiddle; it alone is reduced, in both directions (cols.cuh).
 //  * The first forward pass reads its points from the operand's words.  The
 //    rows of one thread are a multiple of four pieces apart, hence a whole
 //    number of words: one shift and one word address serve all of them.
@@ -33,6 +34,7 @@
 #include <tuple>
 #include <type_traits>
 
+#include "cols.cuh"
 #include "common.cuh"
 #include "middle.cuh"
 
@@ -49,62 +51,6 @@ struct ColArgs {
     ColTables t;
     int lblock;  // log2 points of a block
     int lpre;    // log2 blocks of a transform
-};
-
-// Twiddles of one thread's column c: Q^1 .. Q^7 (or fewer rows), and W of a
-// group.
-template <bool INV, int LC>
-struct ColTwiddle {
-    static constexpr int BL = LC < 3 ? LC : 3;
-    double q[1 << BL];  // q[i] = Q^i, i >= 1
-    const double* w;
-    const double *lo, *hi;
-    int S, esh;
-    uint32_t c;
-    __device__ __forceinline__ double root(uint64_t e, const Dbl::Ctx& L) const  // root_(2^lblock)^e
-    {
-        const uint64_t E = e << esh;
-        return dmul_w(__ldg(hi + (E >> S)), __ldg(lo + (E & (((uint64_t)1 << S) - 1))), L.p, L.pinv);
-    }
-    __device__ __forceinline__ void init(const PrimeDev& P, const double* table, int lblock, uint32_t col,
-                                         const Dbl::Ctx& L)
-    {
-        lo = reinterpret_cast<const double*>(INV ? P.slo_inv : P.slo_fwd);
-        hi = reinterpret_cast<const double*>(INV ? P.shi_inv : P.shi_fwd);
-        S = P.S;
-        esh = P.K - lblock;
-        c = col;
-        w = table != nullptr ? table + col : nullptr;
-        q[1] = root((uint64_t)c << (LC - BL), L);
-    }
-    // made just before the round that uses them, so that they hold no registers
-    // in the others
-    __device__ __forceinline__ void powers(const Dbl::Ctx& L)
-    {
-        if constexpr (BL >= 2) {
-            q[2] = dmul_w(q[1], q[1], L.p, L.pinv);
-            q[3] = dmul_w(q[2], q[1], L.p, L.pinv);
-        }
-        if constexpr (BL >= 3) {
-            q[4] = dmul_w(q[2], q[2], L.p, L.pinv);
-            q[5] = dmul_w(q[3], q[2], L.p, L.pinv);
-            q[6] = dmul_w(q[3], q[3], L.p, L.pinv);
-            q[7] = dmul_w(q[4], q[3], L.p, L.pinv);
-        }
-    }
-    // W of group g (rows 8 g ..): loaded early by the caller
-    __device__ __forceinline__ double group(int g, int lM, const Dbl::Ctx& L) const
-    {
-        if constexpr (LC <= 3) return 1.0;
-        if (w != nullptr) return __ldg(w + ((size_t)g << lM));
-        return root((uint64_t)c * (__brev((unsigned)g) >> (32 - (LC > 3 ? LC - 3 : 1))), L);
-    }
-    __device__ __forceinline__ double apply(double v, int i, double wg, const Dbl::Ctx& L) const
-    {
-        const int r = brev3(i, BL);
-        if (LC > 3) v = dmul_w(v, wg, L.p, L.pinv);
-        return r ? dmul_w(v, q[r], L.p, L.pinv) : v;
-    }
 };
 
 // The pieces of rows r0 + m 2^LST (m < 2^B) of a column from the operand's
@@ -209,17 +155,13 @@ __global__ void __launch_bounds__(kColThreads, 4) cols56_kernel(const __grid_con
             if constexpr (LST > 0) t.load(tw, j);
             if constexpr (!INV) {
                 if constexpr (TAIL) {
-                    fwd_tail<B>(x, t, L);
-#pragma unroll
-                    for (int m = 0; m < E; m++) x[m] = T.apply(x[m], m, wg, L);
+                    T.forward_tail(x, t, wg, L);
                 } else {
                     fwd_group<B, LST>(x, t, L);
                 }
             } else {
                 if constexpr (TAIL) {
-#pragma unroll
-                    for (int m = 0; m < E; m++) x[m] = T.apply(x[m], m, wg, L);
-                    inv_head<B, (LC > 10)>(x, t, L);
+                    T.inverse_head(x, t, wg, L);
                 } else {
                     inv_group<B, LST>(x, t, L);
                 }

@@ -771,7 +771,8 @@ void mul_ntt3(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size
 // modulo kDblPrimes held as doubles (fp64mod.cuh), the same transform passes
 // with FP64 butterflies, pointwise products without a Montgomery factor, and a
 // CRT that places coefficient j (below p0 p1 p2 < 2^141) at bit 56 j.  Inverse
-// outputs arrive with |y| < 12 p (unscaled).
+// outputs arrive with |y| <= 15 p (unscaled), 15.75 p with a wrapped tail taken
+// out of them, below 2^51.
 
 size_t pieces56(size_t nwords) { return (32 * nwords + 55) / 56; }
 

@@ -44,3 +44,17 @@ def test_crt_digits_exact(tmp_path):
                     "-lm"], check=True)
     out = subprocess.run([str(exe), "300000"], capture_output=True, text=True)
     assert out.returncode == 0 and out.stdout.startswith("bad=0"), out.stdout + out.stderr
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="g++ not available")
+def test_short_column_passes_meet_the_rows_in_range(tmp_path):
+    """Column passes of one to three bits (and the round beside the twiddles of
+    longer ones) from the largest pieces into a row's first round, and from the
+    largest values a row leaves to what the CRT accepts: the device templates
+    themselves, built for the host (tests/host/fp64_columns_check.cpp)."""
+    exe = tmp_path / "fp64_columns_check"
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I", os.path.join(HERE, "host", "cuda_shim"),
+                    "-I", os.path.join(os.path.dirname(HERE), "piculator_b200", "csrc"), "-o", str(exe),
+                    os.path.join(HERE, "host", "fp64_columns_check.cpp")], check=True)
+    out = subprocess.run([str(exe), "20000"], capture_output=True, text=True)
+    assert out.returncode == 0 and out.stdout.startswith("bad=0"), out.stdout + out.stderr

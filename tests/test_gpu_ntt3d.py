@@ -250,3 +250,30 @@ def test_column_passes_of_every_height(pic, torch_cuda, lg):
         pic.set_tuning(pic.TUNE_DBL_PASS_TABLES, saved)
     pic.synchronize()
     assert torch.equal(z[0], z[1]) and torch.equal(z[0], z[2])
+
+
+def _words_of_pieces(v):
+    """The words of 56-bit pieces."""
+    b = np.ascontiguousarray(v, dtype="<u8").view(np.uint8).reshape(-1, 8)[:, :7].ravel()
+    return np.concatenate([b, np.zeros(-b.size % 4, np.uint8)]).view(np.uint32)
+
+
+@pytest.mark.parametrize("bits", [(8,), (9,), (10,), (8, 9), (8, 10), (9, 10), (8, 9, 10)])
+@pytest.mark.parametrize("pa,pb", [(16_184, 200), (12_288, 4_000), (16_184, 300)])
+def test_largest_residues_through_three_bit_columns(pic, pa, pb, bits):
+    """Transforms of 2^14 points (the third a wrapped product's main one) of a long
+    operand whose pieces are the largest residues of one of the primes, their signs
+    by bits of the column index: the sums of eight rows of a column, and their
+    differences in the row, reach their bounds."""
+    rng = np.random.default_rng(pa + pb + sum(bits))
+    j = np.arange(pa)
+    sign = np.zeros(pa, dtype=np.int64)
+    for b in bits:
+        sign ^= (j >> b) & 1
+    y = _words_of_pieces(rng.integers(0, 1 << 56, pb, dtype=np.int64))
+    for p in (140496970186753, 140458315481089, 140449725546497):
+        m = rng.integers(1, 511, pa, dtype=np.int64)
+        x = _words_of_pieces(m * p + (1 - 2 * sign) * ((p - 1) // 2 - (1 << 31)))
+        got = pic.mul_host(x, y, "ntt3d")
+        assert np.array_equal(got, pic.mul_host(x, y, "ntt3")), p
+        assert _int(got) == _int(x) * _int(y), p
