@@ -272,8 +272,9 @@ def test_largest_residues_through_three_bit_columns(pic, pa, pb, bits):
         sign ^= (j >> b) & 1
     y = _words_of_pieces(rng.integers(0, 1 << 56, pb, dtype=np.int64))
     for p in (140496970186753, 140458315481089, 140449725546497):
-        m = rng.integers(1, 511, pa, dtype=np.int64)
-        x = _words_of_pieces(m * p + (1 - 2 * sign) * ((p - 1) // 2 - (1 << 31)))
-        got = pic.mul_host(x, y, "ntt3d")
-        assert np.array_equal(got, pic.mul_host(x, y, "ntt3")), p
-        assert _int(got) == _int(x) * _int(y), p
+        for s in (1 - 2 * sign, 2 * sign - 1):  # a quotient may leave its range at either end
+            m = rng.integers(1, 511, pa, dtype=np.int64)
+            x = _words_of_pieces(m * p + s * ((p - 1) // 2 - (1 << 31)))
+            got = pic.mul_host(x, y, "ntt3d")
+            assert np.array_equal(got, pic.mul_host(x, y, "ntt3")), p
+            assert _int(got) == _int(x) * _int(y), p
