@@ -253,8 +253,9 @@ void mul_batch(const pic_mul_desc* d, size_t count, int mode, cudaStream_t s)
     count_products(count);
     if (count == 0) return;
     std::vector<uint32_t> sig;
-    sig.reserve(2 * count + 1);
+    sig.reserve(2 * count + 1 + 5);
     sig.push_back((uint32_t)mode);
+    if (mode == PIC_MUL_AUTO) mul_auto_settings(sig);  // batch_class asks them for each product
     for (size_t i = 0; i < count; i++) {
         PIC_REQUIRE(d[i].z && d[i].a && d[i].b && d[i].na && d[i].nb, PIC_ERR_INVALID, "bad product descriptor");
         PIC_REQUIRE(d[i].na < (1ull << 31) && d[i].nb < (1ull << 31), PIC_ERR_INVALID, "operand too long");

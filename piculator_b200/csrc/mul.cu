@@ -1274,6 +1274,16 @@ int mul_auto_mode(size_t na, size_t nb)
     return product_form(na, nb) == kFormDbl ? PIC_MUL_NTT3D : PIC_MUL_NTT3;
 }
 
+void mul_auto_settings(std::vector<uint32_t>& out)
+{
+    // zw, which the thresholds are compared with, is below 2^32 in every batch
+    auto word = [](int64_t v) { return (uint32_t)std::min<int64_t>(v, 0xffffffff); };
+    out.push_back(word(g_school_max_words));
+    out.push_back(word(g_fft_max_words));
+    out.push_back((uint32_t)g_ntt_form);
+    out.push_back(g_mul_wrap ? 1u : 0u);
+}
+
 static std::atomic<uint64_t> g_fft_err_bits{0};
 static std::atomic<uint64_t> g_fft_err_max_bits{0};  // largest since fft_reset_max_err
 double fft_last_max_err()

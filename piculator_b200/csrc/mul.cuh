@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "common.cuh"
 #include "ntt.cuh"
 #include "piculator_b200.h"
@@ -136,6 +138,9 @@ void crt3_to_words_scratch(const uint64_t* y, int k, size_t ncoef, uint32_t* z, 
 void mul_dispatch(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, int mode,
                   cudaStream_t s, Mail* mail = nullptr);
 int mul_auto_mode(size_t na, size_t nb);
+// Appends the settings that mul_auto_mode reads (plans made from its answers hold
+// for these only).
+void mul_auto_settings(std::vector<uint32_t>& out);
 void mul_set_thresholds(int64_t school_max, int64_t fft_max);
 int64_t mul_school_max();
 int64_t mul_fft_max();

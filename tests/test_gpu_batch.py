@@ -96,3 +96,32 @@ def test_batch_config3_workload_and_graph_replay(pic, torch_cuda, oracle):
         for i in range(0, 8192, 257):  # exact words for a sample
             a, b = ops[i]
             assert np.array_equal(got[i], oracle.mul_words(a, b)), (call, i)
+
+
+def test_batch_follows_the_product_form(pic, torch_cuda):
+    """A repeated batch after the product form has changed runs the new form's
+    kernels, not the plan made for the other one."""
+    import ctypes as C
+    sizes = [1000 + 7 * i for i in range(24)]
+    ops, descs, (ta, tb, tz) = _setup(torch_cuda, sizes, sizes[::-1], 900)
+    torch_cuda.cuda.synchronize()
+    lib = pic.lib()
+
+    def classes():
+        pic.check(lib.pic_profile_begin())
+        pic.mul_batch_dev(descs, "auto")
+        stats, n = (pic.KernelStat * 32)(), C.c_int()
+        pic.check(lib.pic_profile_end(stats, 32, C.byref(n)))
+        for (a, b), z in zip(ops, _outputs(tz, ops)):
+            assert _int(z) == _int(a) * _int(b)
+        return {s.name.decode() for s in stats[: n.value]}
+
+    saved = {k: pic.get_tuning(k) for k in (pic.TUNE_BATCH_GRAPHS, pic.TUNE_NTT_FORM)}
+    try:
+        pic.set_tuning(pic.TUNE_BATCH_GRAPHS, 0)  # launches of a graph are not profiled
+        for form, fused in ((pic.FORM_DBL, True), (pic.FORM_INT, False), (pic.FORM_DBL, True)):
+            pic.set_tuning(pic.TUNE_NTT_FORM, form)
+            assert ("ntt_middle" in classes()) == fused
+    finally:
+        for k, v in saved.items():
+            pic.set_tuning(k, v)
