@@ -292,7 +292,6 @@ struct OneArgs {
     int ask;             // kLinSub: compare first
     const uint32_t *a, *b;
     int64_t da, db, la, lb;  // the window's word i is a[i + da] (0 outside [0, la)), b likewise
-    int64_t below;       // words of either number under the window (they count in the comparison)
     uint32_t x;          // kLinMul
     MailRef mail;
 };
@@ -315,7 +314,7 @@ __device__ __forceinline__ unsigned long long cluster_max(cg::cluster_group& clu
 __global__ void __launch_bounds__(1024) lin_one_kernel(const __grid_constant__ OneArgs A)
 {
     cg::cluster_group cluster = cg::this_cluster();
-    __shared__ unsigned long long s_v[3];
+    __shared__ unsigned long long s_v[2];
     __shared__ uint32_t s_gp;
     const int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * kOneIPT;
     auto at = [](const uint32_t* p, int64_t i, int64_t l) -> uint32_t { return (uint64_t)i < (uint64_t)l ? p[i] : 0u; };
@@ -332,18 +331,11 @@ __global__ void __launch_bounds__(1024) lin_one_kernel(const __grid_constant__ O
         unsigned long long mine = 0;
 #pragma unroll
         for (int u = 0; u < kOneIPT; u++)
-            if (x[u] != y[u]) mine = (unsigned long long)(A.below + i0 + u + 1);
-        unsigned long long h = cluster_max(cluster, &s_v[0], mine);
-        if (h == 0 && A.below > 0) {  // equal in the window: the words under it decide
-            mine = 0;
-            for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.below;
-                 i += (int64_t)gridDim.x * blockDim.x)
-                if (at(A.a, i - A.below + A.da, A.la) != at(A.b, i - A.below + A.db, A.lb))
-                    mine = (unsigned long long)(i + 1);
-            h = cluster_max(cluster, &s_v[1], mine);
-        }
-        const int64_t i = (int64_t)h - 1 - A.below;
-        swap = h == 0 || at(A.a, i + A.da, A.la) < at(A.b, i + A.db, A.lb);
+            if (x[u] != y[u]) mine = (unsigned long long)(i0 + u + 1);
+        // equal in the window: zero in either order, whatever lies under it (a search
+        // there by one cluster took 31 ms for two numbers of 2^24 words)
+        const int64_t i = (int64_t)cluster_max(cluster, &s_v[0], mine) - 1;
+        swap = i < 0 || at(A.a, i + A.da, A.la) < at(A.b, i + A.db, A.lb);
     }
     uint32_t d[kOneIPT], gg[kOneIPT];
     uint32_t gp = kGPIdentity;
@@ -388,7 +380,7 @@ __global__ void __launch_bounds__(1024) lin_one_kernel(const __grid_constant__ O
         cin = gg[u] | (p & cin);
     }
     if (!add) {
-        top = cluster_max(cluster, &s_v[2], top);
+        top = cluster_max(cluster, &s_v[1], top);
         if (blockIdx.x == 0 && threadIdx.x == 0) mail_post(A.mail, top, swap ? 0u : 1u);
     } else if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
         uint32_t v = (total & 1u) | ((total >> 1) & cc);
@@ -571,7 +563,6 @@ size_t lin_diff(uint32_t* z, size_t TL, const WordView& a, const WordView& b, in
     if (TL <= kOneWords && bot + (int64_t)TL >= reach) {  // the comparison sees no word above the window
         OneArgs A = *order >= 0 ? one_args(z, TL, a, b, bot, kLinSub) : one_args(z, TL, b, a, bot, kLinSub);
         A.ask = ask ? 1 : 0;
-        A.below = ask ? bot - (a.exp < b.exp ? a.exp : b.exp) : 0;
         uint32_t greater;
         const uint64_t nz = lin_one(A, &greater);
         if (ask) *order = greater ? 1 : -1;

@@ -22,8 +22,9 @@ void lin_addsub(uint32_t* z, size_t TL, const WordView& a, const WordView& b, in
 // z[0..TL) = a + b over the window, z[TL] = the carry out, which is returned.
 uint32_t lin_add(uint32_t* z, size_t TL, const WordView& a, const WordView& b, int64_t bot);
 // z[0..TL) = |a| - |b| over the window when |a| > |b|, else |b| - |a| (order 1,
-// -1: known to the caller; 0: compared on the device).  *order tells which of
-// the two (1 or -1); returns 1 + the index of the highest nonzero word of z.
+// -1: known to the caller; 0: compared on the device).  Returns 1 + the index of
+// the highest nonzero word of z; *order tells which of the two (1 or -1) where
+// there is one.
 size_t lin_diff(uint32_t* z, size_t TL, const WordView& a, const WordView& b, int64_t bot, int* order);
 // z[0..L] = a[0..L) * x (z has L+1 words); returns z[L], which may be 0.
 uint32_t lin_mul_u32(uint32_t* z, const uint32_t* a, size_t L, uint32_t x);
