@@ -116,3 +116,29 @@ def test_equal_windows_of_long_numbers(pic):
         seconds.append(time.perf_counter() - t)
         assert d.info()[2] == 0
     assert sorted(seconds)[3] < 2e-3  # 2^24 words read by one CTA: 31 ms
+
+
+def test_long_ordered_differences_from_several_threads(pic):
+    """Above 65,536 words a comparison and the subtraction that reads its result are
+    launches of their own over shared scratch words: no other thread's comparison may
+    come between them."""
+    n = 70_000
+
+    def work(seed, bad):
+        a, b = random_words(seed, n), random_words(seed + 1, n)
+        a[-1] = b[-1] = 9
+        a[n // 2:] = b[n // 2:]
+        a[n // 2], b[n // 2] = (9, 8) if seed & 2 else (8, 9)  # the larger one differs from thread to thread
+        want = _val(a) - _val(b)
+        x, y = _num(pic, a), _num(pic, b)
+        for _ in range(40):
+            if _int(x.sub(y)) != want or _int(y.sub(x)) != -want:
+                bad.append(seed)
+
+    bad: list[int] = []
+    threads = [threading.Thread(target=work, args=(200 + 2 * i, bad)) for i in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
