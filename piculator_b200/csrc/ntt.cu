@@ -1318,13 +1318,15 @@ static bool launch_cols_fast(const NttBatch& b, int k, int lpre, int lc, int lw,
 // g_cols_bulk: 0 off, else log2 of the largest tile (points) the kernel
 // takes; tiles are narrowed to it so that more CTAs share an SM.
 static int g_cols_bulk = 0;
-static std::atomic<bool> g_bulk_ran{false};  // since the last ntt_take_bulk_error
+// Set by the first launch (or capture) and kept: a graph replays its passes without
+// coming here, and another thread's may still be running when one thread asks.
+static std::atomic<bool> g_bulk_ran{false};
 void ntt_set_cols_bulk(int bits) { g_cols_bulk = bits; }
 int ntt_cols_bulk() { return g_cols_bulk; }
 
 bool ntt_take_bulk_error()
 {
-    if (!g_bulk_ran.exchange(false)) return false;
+    if (!g_bulk_ran.load()) return false;
     int e = 0, zero = 0;
     PIC_CUDA(cudaMemcpyFromSymbol(&e, g_ntt_bulk_error, sizeof e));
     if (e) PIC_CUDA(cudaMemcpyToSymbol(g_ntt_bulk_error, &zero, sizeof zero));
