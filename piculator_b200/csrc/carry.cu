@@ -178,9 +178,10 @@ __global__ void __launch_bounds__(kLinThreads) addsub_k1(uint32_t* z, size_t TL,
     }
 }
 
-// z[c] = low(a_c x) + high(a_(c-1) x), carries resolved; z[L] = final word.
+// z[c] = low(a_c x) + high(a_(c-1) x), carries inside each CTA resolved (several
+// CTAs: lin_one serves shorter numbers); lin_fix passes on the others and writes z[L].
 __global__ void __launch_bounds__(kLinThreads) mulu32_k1(uint32_t* z, const uint32_t* a, size_t L, uint32_t x,
-                                                         uint32_t* agg, LinEnd E)
+                                                         uint32_t* agg)
 {
     const size_t i0 = (size_t)blockIdx.x * kLinWPC + (size_t)threadIdx.x * kLinIPT;
     uint32_t d[kLinIPT], gg[kLinIPT];
@@ -211,12 +212,7 @@ __global__ void __launch_bounds__(kLinThreads) mulu32_k1(uint32_t* z, const uint
         z[i] = d[u] + cin;
         cin = gg[u] | ((uint32_t)(d[u] == 0xffffffffu) & cin);
     }
-    if (gridDim.x > 1) {
-        if (threadIdx.x == 0) agg[blockIdx.x] = total;
-    } else {
-        E.top_hi = (uint32_t)(((uint64_t)a[L - 1] * x) >> 32);
-        lin_end(E, z, 0, L, total & 1u, 1);
-    }
+    if (threadIdx.x == 0) agg[blockIdx.x] = total;
 }
 
 __global__ void set_words_kernel(uint32_t* p, uint32_t lo, uint32_t hi, int n)
@@ -466,7 +462,7 @@ uint32_t lin_mul_u32(uint32_t* z, const uint32_t* a, size_t L, uint32_t x)
     E.mail = mail.ref();
     {
         ProfScope ps(KC_LINEAR, 8.0 * (double)L, s);
-        mulu32_k1<<<(unsigned)nctas, kLinThreads, 0, s>>>(z, a, L, x, agg.get(), E);
+        mulu32_k1<<<(unsigned)nctas, kLinThreads, 0, s>>>(z, a, L, x, agg.get());
         PIC_CHECK_LAUNCH();
         count_launch();
         lin_fix(z, L, agg.get(), nctas, E, a, x, s);

@@ -324,7 +324,7 @@ static std::vector<int> col_bits(int k, int row_bits)
     return bits;
 }
 
-std::vector<int> ntt_pass_bits(int k, int form)
+std::vector<int> ntt_pass_bits(int k)
 {
     // One in-CTA pass up to 2^13 points; then column passes of at most 11
     // bits (balanced) and the row pass.
@@ -333,7 +333,7 @@ std::vector<int> ntt_pass_bits(int k, int form)
         bits.push_back(k);
         return bits;
     }
-    const int row = g_geom_forms[form == kFormDbl ? 1 : 0][k].row_bits;
+    const int row = g_geom_forms[0][k].row_bits;
     bits = col_bits(k, row);
     bits.push_back(row);
     return bits;
@@ -737,10 +737,11 @@ struct RowsFastShape {
 // hold fewer than 2^LRPC transforms.  Forward passes stage their output
 // through shared memory (their last round has the smallest stride); inverse
 // passes write it directly.
-template <bool INV, int LR, int LRPC, int RB, class A>
+template <bool INV, int LR, int LRPC, int RB>
 __global__ void __launch_bounds__(RowsFastShape<LR, LRPC, RB>::NT, RowsFastShape<LR, LRPC, RB>::MINB)
     ntt_rows_fast_kernel(NttBatch B, int k)
 {
+    using A = ArithInt;
     extern __shared__ uint64_t smem[];
     constexpr int TOT = RowsFastShape<LR, LRPC, RB>::TOT, NT = RowsFastShape<LR, LRPC, RB>::NT;
     constexpr int EMASK = (1 << LR) - 1;
@@ -895,10 +896,11 @@ struct ColsMinBlocks {
     static constexpr int value = RB == 4 ? 2 : (INV ? 3 : 4);
 };
 
-template <bool INV, int LC, int LW, int RB, class A>
+template <bool INV, int LC, int LW, int RB>
 __global__ void __launch_bounds__(256, ColsMinBlocks<RB, INV>::value)
     ntt_cols_fast_kernel(NttBatch B, int k, int lpre, PassTw pt)
 {
+    using A = ArithInt;
     extern __shared__ uint64_t smem[];
     const int lM = k - lpre - LC;
     const int ltiles = lM - LW;
@@ -1125,10 +1127,6 @@ __global__ void src_split_kernel(NttBatch B, int k)
         const size_t j = g & (N - 1);
         const PrimeDev P = pick_prime(B, tr);
         const SrcRow r = src_row(B, tr);
-        if (P.fp64) {
-            B.data[(size_t)tr * B.stride + j] = dstore(dpiece56(src_piece56_raw(r.x, r.n, B.src.first + j), P.pd, P.pinv));
-            continue;
-        }
         const uint64_t v = src_piece_raw(B, r, j);
         B.data[(size_t)tr * B.stride + j] = P.lazy ? piece_to_strict(v, P.p) : v % P.p;
     }
@@ -1166,7 +1164,7 @@ static bool fast_ok(const NttBatch& b, int k)
 
 constexpr int fast_lrpc(int lr) { return lr < 11 ? 11 - lr : 0; }
 
-template <bool INV, int LR, int RB, class A>
+template <bool INV, int LR, int RB>
 static void launch_rows_fast_t(const NttBatch& b, int k, cudaStream_t s)
 {
     constexpr int LRPC = fast_lrpc(LR);
@@ -1174,36 +1172,36 @@ static void launch_rows_fast_t(const NttBatch& b, int k, cudaStream_t s)
     const size_t rows = (size_t)b.count << (k - LR);
     const size_t grid = (rows + ((size_t)1 << LRPC) - 1) >> LRPC;
     const size_t smem = sizeof(uint64_t) * Sh::TOT;
-    set_smem(ntt_rows_fast_kernel<INV, LR, LRPC, RB, A>, smem);
-    ntt_rows_fast_kernel<INV, LR, LRPC, RB, A><<<(unsigned)grid, Sh::NT, smem, s>>>(b, k);
+    set_smem(ntt_rows_fast_kernel<INV, LR, LRPC, RB>, smem);
+    ntt_rows_fast_kernel<INV, LR, LRPC, RB><<<(unsigned)grid, Sh::NT, smem, s>>>(b, k);
 }
 
-template <bool INV, class A>
+template <bool INV>
 static bool launch_rows_fast(const NttBatch& b, int k, int lr, cudaStream_t s)
 {
     if (!(lr == k || lr >= 11)) return false;
     if (geom_of(b, k).rbits == 4) {
         switch (lr) {
-        case 11: launch_rows_fast_t<INV, 11, 4, A>(b, k, s); return true;
-        case 12: launch_rows_fast_t<INV, 12, 4, A>(b, k, s); return true;
-        case 13: launch_rows_fast_t<INV, 13, 4, A>(b, k, s); return true;
+        case 11: launch_rows_fast_t<INV, 11, 4>(b, k, s); return true;
+        case 12: launch_rows_fast_t<INV, 12, 4>(b, k, s); return true;
+        case 13: launch_rows_fast_t<INV, 13, 4>(b, k, s); return true;
         default: break;  // shorter rows keep radix-8 rounds
         }
     }
     switch (lr) {
-    case 1: launch_rows_fast_t<INV, 1, 3, A>(b, k, s); break;
-    case 2: launch_rows_fast_t<INV, 2, 3, A>(b, k, s); break;
-    case 3: launch_rows_fast_t<INV, 3, 3, A>(b, k, s); break;
-    case 4: launch_rows_fast_t<INV, 4, 3, A>(b, k, s); break;
-    case 5: launch_rows_fast_t<INV, 5, 3, A>(b, k, s); break;
-    case 6: launch_rows_fast_t<INV, 6, 3, A>(b, k, s); break;
-    case 7: launch_rows_fast_t<INV, 7, 3, A>(b, k, s); break;
-    case 8: launch_rows_fast_t<INV, 8, 3, A>(b, k, s); break;
-    case 9: launch_rows_fast_t<INV, 9, 3, A>(b, k, s); break;
-    case 10: launch_rows_fast_t<INV, 10, 3, A>(b, k, s); break;
-    case 11: launch_rows_fast_t<INV, 11, 3, A>(b, k, s); break;
-    case 12: launch_rows_fast_t<INV, 12, 3, A>(b, k, s); break;
-    case 13: launch_rows_fast_t<INV, 13, 3, A>(b, k, s); break;
+    case 1: launch_rows_fast_t<INV, 1, 3>(b, k, s); break;
+    case 2: launch_rows_fast_t<INV, 2, 3>(b, k, s); break;
+    case 3: launch_rows_fast_t<INV, 3, 3>(b, k, s); break;
+    case 4: launch_rows_fast_t<INV, 4, 3>(b, k, s); break;
+    case 5: launch_rows_fast_t<INV, 5, 3>(b, k, s); break;
+    case 6: launch_rows_fast_t<INV, 6, 3>(b, k, s); break;
+    case 7: launch_rows_fast_t<INV, 7, 3>(b, k, s); break;
+    case 8: launch_rows_fast_t<INV, 8, 3>(b, k, s); break;
+    case 9: launch_rows_fast_t<INV, 9, 3>(b, k, s); break;
+    case 10: launch_rows_fast_t<INV, 10, 3>(b, k, s); break;
+    case 11: launch_rows_fast_t<INV, 11, 3>(b, k, s); break;
+    case 12: launch_rows_fast_t<INV, 12, 3>(b, k, s); break;
+    case 13: launch_rows_fast_t<INV, 13, 3>(b, k, s); break;
     default: return false;
     }
     return true;
@@ -1255,7 +1253,7 @@ static const void* pass_table(const PrimeDev& P, bool inv, int lblock, int lc, c
     return d;
 }
 
-template <bool INV, int LC, int LW, int RB, class A>
+template <bool INV, int LC, int LW, int RB>
 static void launch_cols_fast_t(const NttBatch& b, int k, int lpre, size_t grid, cudaStream_t s)
 {
     constexpr size_t smem = sizeof(uint64_t) << (LC + LW);
@@ -1266,48 +1264,48 @@ static void launch_cols_fast_t(const NttBatch& b, int k, int lpre, size_t grid, 
         all = all && pt.t[q] != nullptr;
     }
     if (!all) pt = PassTw{};  // one form for every prime of the launch
-    set_smem(ntt_cols_fast_kernel<INV, LC, LW, RB, A>, smem);
-    ntt_cols_fast_kernel<INV, LC, LW, RB, A><<<(unsigned)grid, 256, smem, s>>>(b, k, lpre, pt);
+    set_smem(ntt_cols_fast_kernel<INV, LC, LW, RB>, smem);
+    ntt_cols_fast_kernel<INV, LC, LW, RB><<<(unsigned)grid, 256, smem, s>>>(b, k, lpre, pt);
 }
 
-template <bool INV, int LC, int RB, class A>
+template <bool INV, int LC, int RB>
 static bool launch_cols_fast_lc(const NttBatch& b, int k, int lpre, int lw, size_t grid, cudaStream_t s)
 {
     switch (lw) {
-    case 2: if constexpr (LC + 2 <= 13) { launch_cols_fast_t<INV, LC, 2, RB, A>(b, k, lpre, grid, s); return true; } break;
-    case 3: if constexpr (LC + 3 <= 13) { launch_cols_fast_t<INV, LC, 3, RB, A>(b, k, lpre, grid, s); return true; } break;
-    case 4: if constexpr (LC + 4 <= 13) { launch_cols_fast_t<INV, LC, 4, RB, A>(b, k, lpre, grid, s); return true; } break;
-    case 5: if constexpr (LC + 5 <= 13) { launch_cols_fast_t<INV, LC, 5, RB, A>(b, k, lpre, grid, s); return true; } break;
-    case 6: if constexpr (LC + 6 <= 13) { launch_cols_fast_t<INV, LC, 6, RB, A>(b, k, lpre, grid, s); return true; } break;
+    case 2: if constexpr (LC + 2 <= 13) { launch_cols_fast_t<INV, LC, 2, RB>(b, k, lpre, grid, s); return true; } break;
+    case 3: if constexpr (LC + 3 <= 13) { launch_cols_fast_t<INV, LC, 3, RB>(b, k, lpre, grid, s); return true; } break;
+    case 4: if constexpr (LC + 4 <= 13) { launch_cols_fast_t<INV, LC, 4, RB>(b, k, lpre, grid, s); return true; } break;
+    case 5: if constexpr (LC + 5 <= 13) { launch_cols_fast_t<INV, LC, 5, RB>(b, k, lpre, grid, s); return true; } break;
+    case 6: if constexpr (LC + 6 <= 13) { launch_cols_fast_t<INV, LC, 6, RB>(b, k, lpre, grid, s); return true; } break;
     default: break;
     }
     return false;
 }
 
-template <bool INV, class A>
+template <bool INV>
 static bool launch_cols_fast(const NttBatch& b, int k, int lpre, int lc, int lw, size_t grid, cudaStream_t s)
 {
     if (geom_of(b, k).rbits == 4) {  // radix-16 rounds for the tall columns of long transforms
         switch (lc) {
-        case 8: return launch_cols_fast_lc<INV, 8, 4, A>(b, k, lpre, lw, grid, s);
-        case 9: return launch_cols_fast_lc<INV, 9, 4, A>(b, k, lpre, lw, grid, s);
-        case 10: return launch_cols_fast_lc<INV, 10, 4, A>(b, k, lpre, lw, grid, s);
-        case 11: return launch_cols_fast_lc<INV, 11, 4, A>(b, k, lpre, lw, grid, s);
+        case 8: return launch_cols_fast_lc<INV, 8, 4>(b, k, lpre, lw, grid, s);
+        case 9: return launch_cols_fast_lc<INV, 9, 4>(b, k, lpre, lw, grid, s);
+        case 10: return launch_cols_fast_lc<INV, 10, 4>(b, k, lpre, lw, grid, s);
+        case 11: return launch_cols_fast_lc<INV, 11, 4>(b, k, lpre, lw, grid, s);
         default: break;
         }
     }
     switch (lc) {
-    case 1: return launch_cols_fast_lc<INV, 1, 3, A>(b, k, lpre, lw, grid, s);
-    case 2: return launch_cols_fast_lc<INV, 2, 3, A>(b, k, lpre, lw, grid, s);
-    case 3: return launch_cols_fast_lc<INV, 3, 3, A>(b, k, lpre, lw, grid, s);
-    case 4: return launch_cols_fast_lc<INV, 4, 3, A>(b, k, lpre, lw, grid, s);
-    case 5: return launch_cols_fast_lc<INV, 5, 3, A>(b, k, lpre, lw, grid, s);
-    case 6: return launch_cols_fast_lc<INV, 6, 3, A>(b, k, lpre, lw, grid, s);
-    case 7: return launch_cols_fast_lc<INV, 7, 3, A>(b, k, lpre, lw, grid, s);
-    case 8: return launch_cols_fast_lc<INV, 8, 3, A>(b, k, lpre, lw, grid, s);
-    case 9: return launch_cols_fast_lc<INV, 9, 3, A>(b, k, lpre, lw, grid, s);
-    case 10: return launch_cols_fast_lc<INV, 10, 3, A>(b, k, lpre, lw, grid, s);
-    case 11: return launch_cols_fast_lc<INV, 11, 3, A>(b, k, lpre, lw, grid, s);
+    case 1: return launch_cols_fast_lc<INV, 1, 3>(b, k, lpre, lw, grid, s);
+    case 2: return launch_cols_fast_lc<INV, 2, 3>(b, k, lpre, lw, grid, s);
+    case 3: return launch_cols_fast_lc<INV, 3, 3>(b, k, lpre, lw, grid, s);
+    case 4: return launch_cols_fast_lc<INV, 4, 3>(b, k, lpre, lw, grid, s);
+    case 5: return launch_cols_fast_lc<INV, 5, 3>(b, k, lpre, lw, grid, s);
+    case 6: return launch_cols_fast_lc<INV, 6, 3>(b, k, lpre, lw, grid, s);
+    case 7: return launch_cols_fast_lc<INV, 7, 3>(b, k, lpre, lw, grid, s);
+    case 8: return launch_cols_fast_lc<INV, 8, 3>(b, k, lpre, lw, grid, s);
+    case 9: return launch_cols_fast_lc<INV, 9, 3>(b, k, lpre, lw, grid, s);
+    case 10: return launch_cols_fast_lc<INV, 10, 3>(b, k, lpre, lw, grid, s);
+    case 11: return launch_cols_fast_lc<INV, 11, 3>(b, k, lpre, lw, grid, s);
     default: return false;
     }
 }
@@ -1404,7 +1402,7 @@ static void launch_rows(bool inv, const NttBatch& b, int k, int lr, cudaStream_t
     PIC_REQUIRE(!b.prime[0].fp64, PIC_ERR_INVALID, "the FP64 form's row passes are the fused middle passes");
     if (fast_ok(b, k)) {
         ProfScope ps(KC_NTT_ROWS, 16.0 * (double)b.count * (double)((size_t)1 << k), s);
-        if (inv ? launch_rows_fast<true, ArithInt>(b, k, lr, s) : launch_rows_fast<false, ArithInt>(b, k, lr, s)) {
+        if (inv ? launch_rows_fast<true>(b, k, lr, s) : launch_rows_fast<false>(b, k, lr, s)) {
             PIC_CHECK_LAUNCH();
             count_launch();
             return;
@@ -1471,8 +1469,8 @@ static void launch_cols(bool inv, const NttBatch& b, int k, int lpre, int lc, cu
         return;
     }
     if (fast &&
-        (inv ? launch_cols_fast<true, ArithInt>(b, k, lpre, lc, lw, grid, s)
-             : launch_cols_fast<false, ArithInt>(b, k, lpre, lc, lw, grid, s))) {
+        (inv ? launch_cols_fast<true>(b, k, lpre, lc, lw, grid, s)
+             : launch_cols_fast<false>(b, k, lpre, lc, lw, grid, s))) {
         PIC_CHECK_LAUNCH();
         count_launch();
         return;
@@ -1515,7 +1513,7 @@ static void check_batch(const NttBatch& b, int k)
 void ntt_forward_dif(const NttBatch& b, int k, cudaStream_t s)
 {
     check_batch(b, k);
-    std::vector<int> bits = ntt_pass_bits(k, b.prime[0].fp64 ? kFormDbl : kFormInt);
+    std::vector<int> bits = ntt_pass_bits(k);
     NttBatch rest = b;
     rest.src = SplitSrc{};  // only the first pass reads the child slots
     int lpre = 0;
@@ -1531,7 +1529,7 @@ void ntt_inverse_dit(const NttBatch& b_in, int k, cudaStream_t s)
     NttBatch b = b_in;
     b.src = SplitSrc{};
     check_batch(b, k);
-    std::vector<int> bits = ntt_pass_bits(k, b.prime[0].fp64 ? kFormDbl : kFormInt);
+    std::vector<int> bits = ntt_pass_bits(k);
     launch_rows(true, b, k, bits.back(), s);
     int lpre = k - bits.back();
     for (int i = (int)bits.size() - 2; i >= 0; i--) {
@@ -1599,10 +1597,6 @@ __global__ void pointwise_mont_kernel(NttBatch B, const uint64_t* __restrict__ o
         const size_t tr = g >> k, i = g & (n - 1);
         const PrimeDev P = pick_prime(B, (int)tr);
         uint64_t* d = B.data + tr * B.stride + i;
-        if (P.fp64) {  // forward outputs |x| <= p: the product is below p^2
-            *d = dstore(dmul_mod(dbits(*d), dbits(other[tr * ostride + i]), P.pd, P.pinv));
-            continue;
-        }
         *d = P.lazy ? mont_mul_c(*d, other[tr * ostride + i], P.p, (uint32_t)(P.p >> 32))
                     : mont_mul(*d, other[tr * ostride + i], P.p, P.pinv_neg);
     }

@@ -198,8 +198,8 @@ double butterfly_ceiling(cudaStream_t s);
 // The same for the FP64 form's butterflies (about nine FP64 instructions each).
 double butterfly_ceiling_dbl(cudaStream_t s);
 
-// Pass split used for length 2^k (for reporting / tests).
-std::vector<int> ntt_pass_bits(int k, int form = kFormInt);
+// Pass split of the whole integer transforms of length 2^k.
+std::vector<int> ntt_pass_bits(int k);
 // Tunable geometry per length and form (row-pass bits 8..13, column tile
 // log2 width 0..6 with 0 = automatic, bits per register round 2..4; the FP64
 // form accepts row bits 11..13 and rounds of 3 or 4 bits, but its row passes are
