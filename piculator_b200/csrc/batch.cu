@@ -155,9 +155,7 @@ static void enqueue_plan(Plan& P, cudaStream_t s)
     if (!P.school.empty()) {
         PIC_CUDA(cudaMemsetAsync(P.counter.get(), 0, sizeof(uint32_t), s));
         const size_t smem = sizeof(uint32_t) * (size_t)P.school_words;
-        if (smem > 48 * 1024)
-            PIC_CUDA(cudaFuncSetAttribute(school_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+        allow_smem(school_persistent_kernel, smem, kSchoolMaxSmem);
         const unsigned grid = (unsigned)std::min<size_t>(P.school.size(), 148 * 8);
         school_persistent_kernel<<<grid, kPSchThreads, smem, s>>>(P.desc.get(), P.dschool.get(),
                                                                  (uint32_t)P.school.size(), P.counter.get());

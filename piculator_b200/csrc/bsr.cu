@@ -603,6 +603,7 @@ __global__ void __launch_bounds__(256) merge_school_kernel(MergeArgs m)
 // warp per parent), 23, 38 and 75 -> 10.8, 10.6, 15.5 and 24.2 ms (the last one's
 // multiply-adds alone: 16.5); one parent a CTA and digits made twice, before and
 // after a scan by shuffles, took 12.5, 17.3, 17.5 and 25.4.
+constexpr size_t kMergeMaxSmem = 200 * 1024;  // of a schoolbook merge
 constexpr int kBlockMergeThreads = 512;
 constexpr int kBlockMergeParents = 8;  // 4 products each: one warp scans their lengths
 
@@ -850,9 +851,8 @@ static bool launch_merge_block(const MergeArgs& m, cudaStream_t s)
     S.G = std::max<uint32_t>(1, std::min<uint32_t>(kBlockMergeParents, 256 / S.rows()));
     S.G = (uint32_t)std::max<size_t>(1, std::min<size_t>(S.G, m.count / (4 * (size_t)ctx().num_sms)));
     const size_t smem = sizeof(uint32_t) * (size_t)S.words();
-    if (smem > 200 * 1024) return false;
-    if (smem > 48 * 1024)
-        PIC_CUDA(cudaFuncSetAttribute(merge_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kMergeMaxSmem) return false;
+    allow_smem(merge_block_kernel, smem, kMergeMaxSmem);
     const uint32_t threads = std::min<uint32_t>(kBlockMergeThreads, (S.G * S.rows() + 31) / 32 * 32);
     merge_block_kernel<<<(unsigned)((m.count + S.G - 1) / S.G), std::max<uint32_t>(threads, 64), smem, s>>>(m, S);
     return true;
@@ -1738,9 +1738,8 @@ static void merge_school(Level& ch, Level& par, cudaStream_t s)
     const size_t words = 2 * ((size_t)m.ccP + m.ccQ + m.ccR) + (m.ccP + m.ccQ) + (m.ccP + m.ccR) +
                          3 * ((size_t)m.ccP + m.ccQ) + (g_kara_min ? 3 * ((size_t)m.ccP + m.ccQ) + 8 : 0);
     const size_t smem = words * sizeof(uint32_t);
-    PIC_REQUIRE(smem <= 200 * 1024, PIC_ERR_INVALID, "schoolbook merge tile too large");
-    if (smem > 48 * 1024)
-        PIC_CUDA(cudaFuncSetAttribute(merge_school_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PIC_REQUIRE(smem <= kMergeMaxSmem, PIC_ERR_INVALID, "schoolbook merge tile too large");
+    allow_smem(merge_school_kernel, smem, kMergeMaxSmem);
     const int threads = cmax <= 16 ? 32 : (cmax <= 64 ? 64 : (cmax <= 256 ? 128 : 256));
     merge_school_kernel<<<(unsigned)par.count, threads, smem, s>>>(m);
     PIC_CHECK_LAUNCH();

@@ -201,6 +201,16 @@ struct TraceSpan {
     ~TraceSpan();
 };
 
+// Before a launch with `smem` bytes of dynamic shared memory, of at most `most` in
+// any call of this kernel: lifts the default limit, which counts the kernel's static
+// shared memory too (under 2 KB here).  The limit is always the same, so launches
+// of other sizes from other threads never find it lowered.
+template <class K>
+inline void allow_smem(K kern, size_t smem, size_t most)
+{
+    if (smem > 46 * 1024) PIC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+}
+
 inline unsigned grid_for(size_t n, unsigned block, unsigned cap = 148u * 32u)
 {
     size_t g = (n + block - 1) / block;

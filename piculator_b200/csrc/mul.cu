@@ -1198,8 +1198,7 @@ void mul_school(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, si
 {
     PIC_REQUIRE(na + nb <= kSchoolMaxWords, PIC_ERR_INVALID, "schoolbook product too long");
     const size_t smem = 4 * (size_t)BlockProduct((uint32_t)na, (uint32_t)nb, kSchThreads).words();
-    if (smem > 48 * 1024)
-        PIC_CUDA(cudaFuncSetAttribute(school_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(school_kernel, smem, kSchoolMaxSmem);
     ProfScope ps(KC_SCHOOL, 4.0 * (double)(2 * (na + nb)), s);
     school_kernel<<<1, kSchThreads, smem, s>>>(z, a, (uint32_t)na, b, (uint32_t)nb, mail ? mail->ref() : MailRef{});
     PIC_CHECK_LAUNCH();

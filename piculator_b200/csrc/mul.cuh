@@ -80,6 +80,9 @@ uint64_t held_transform_reuses();
 void mul_ntt_ref(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s);
 // One CTA per product, column sums in shared memory (na + nb <= kSchoolMax).
 constexpr size_t kSchoolMaxWords = 4096;
+// Shared memory of the largest one (BlockProduct::words(): 513 blocks, one run of
+// 17-word diagonals; shorter ones with more runs take less).
+constexpr size_t kSchoolMaxSmem = 4 * 513 * (8 + 17);
 void mul_school(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s,
                 Mail* mail = nullptr);
 // FP64 FFT product; returns false (and leaves z undefined) when the largest

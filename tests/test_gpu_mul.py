@@ -267,3 +267,33 @@ def test_radix16_row_passes(pic, row_bits):
     finally:
         for k, (r, lw, rb) in saved.items():
             pic.set_ntt_geometry(k, r, lw, rb)
+
+
+def _fresh(code):
+    """Runs code in a process of its own, the library just initialised."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    head = ("import numpy as np\nimport piculator_b200 as P\nfrom oracle.ffi import random_words\nP.init(0)\n"
+            "val = lambda x: int.from_bytes(x.tobytes(), 'little')\n")
+    r = subprocess.run([sys.executable, "-c", head + code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("na,nb,mode", [(48, 3873, "auto"), (48, 3876, "auto"), (1, 3920, "auto"), (3880, 41, "auto"),
+                                        (1960, 1962, "school"), (2048, 2048, "school")])
+def test_first_schoolbook_product_near_48_kb(pic, na, nb, mode):
+    """Sizes whose dynamic shared memory is just under 48 KB and passes it with the
+    kernel's static part, as the first product of a process (no larger one has lifted
+    the limit yet)."""
+    _fresh(f"a, b = random_words(1, {na}), random_words(2, {nb})\n"
+           f"assert val(P.mul_host(a, b, '{mode}')) == val(a) * val(b)\n")
+
+
+@pytest.mark.parametrize("digits", [14_200, 27_240])
+def test_first_block_merge_near_48_kb(pic, digits):
+    """The same for the merges: schoolbook levels up to 1400 words, where a level's
+    tile is between 47 and 48 KB and no level before it is larger."""
+    _fresh(f"P.set_tuning(P.TUNE_BSR_SCHOOL_MAX, 1400)\ngot = P.pi_hex({digits}, P.PI_CHOSEN)[0]\n"
+           f"P.set_tuning(P.TUNE_BSR_SCHOOL_MAX, 300)\nassert got == P.pi_hex({digits}, P.PI_CHOSEN)[0]\n")
