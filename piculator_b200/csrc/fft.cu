@@ -377,17 +377,16 @@ static void fft_launch_rows(bool inv, const FftBatch& b, int k, int lr, cudaStre
         count_launch();
         return;
     }
+    constexpr size_t kFftRowSmem = sizeof(double2) << kFftInnerBits;  // the longest single pass
     const size_t smem = (size_t)rpc * n * sizeof(double2);
     int threads = (rpc * n) / 8;
     if (threads < 32) threads = 32;
     if (threads > 512) threads = 512;
     if (inv) {
-        if (smem > 48 * 1024)
-            PIC_CUDA(cudaFuncSetAttribute(fft_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_smem(fft_rows_kernel<true>, smem, kFftRowSmem);
         fft_rows_kernel<true><<<(unsigned)grid, threads, smem, s>>>(b, k, lr, rpc, T.inner);
     } else {
-        if (smem > 48 * 1024)
-            PIC_CUDA(cudaFuncSetAttribute(fft_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_smem(fft_rows_kernel<false>, smem, kFftRowSmem);
         fft_rows_kernel<false><<<(unsigned)grid, threads, smem, s>>>(b, k, lr, rpc, T.inner);
     }
     PIC_CHECK_LAUNCH();

@@ -297,3 +297,28 @@ def test_first_block_merge_near_48_kb(pic, digits):
     tile is between 47 and 48 KB and no level before it is larger."""
     _fresh(f"P.set_tuning(P.TUNE_BSR_SCHOOL_MAX, 1400)\ngot = P.pi_hex({digits}, P.PI_CHOSEN)[0]\n"
            f"P.set_tuning(P.TUNE_BSR_SCHOOL_MAX, 300)\nassert got == P.pi_hex({digits}, P.PI_CHOSEN)[0]\n")
+
+
+def test_shared_memory_limits_from_several_threads(pic, torch_cuda):
+    """Two lengths of one kernel from two threads: neither lowers the limit between
+    the other's setting it and its launch."""
+    import threading
+    torch = torch_cuda
+    bad: list[str] = []
+
+    def work(k):
+        t = torch.zeros(1 << k, dtype=torch.complex128, device="cuda")
+        torch.cuda.synchronize()
+        try:
+            for _ in range(3000):
+                pic.check(pic.lib().pic_fft_forward(t.data_ptr(), k, None))
+        except pic.PicError as e:
+            bad.append(f"k={k}: {e}")
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in (12, 13, 12, 13)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    pic.synchronize()
+    assert not bad, bad
