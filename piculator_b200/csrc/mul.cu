@@ -1248,7 +1248,10 @@ static double ntt_work(size_t coefs, size_t per_max, bool wrap)
 }
 
 // The FP64 form's cost per butterfly relative to the integer form's, at equal
-// transform length (isolated products of 2^20 .. 2^26 points: 0.83 - 0.90).
+// transform length, as timed on passes launched apart (isolated products of 2^20 ..
+// 2^26 points: 0.83 - 0.90).  With the fused middle passes whole products of 2^20,
+// 2^24 and 2^27 words take 0.79, 0.78 and 0.75 of the integer form's time (2^16:
+// 0.98), so near the line this still favours the integer form.
 constexpr double kDblWorkRatio = 0.87;
 
 int ntt_form_for(size_t pieces_int_a, size_t pieces_int_b, size_t pieces_dbl_a, size_t pieces_dbl_b, bool wrap)

@@ -78,7 +78,7 @@ uint64_t held_transform_reuses();
 // The reference's own layout: 16-bit points in u64, one prime (the
 // reference's prime for k), length 2^k >= 4 (na + nb) (BigFloat.cpp:380-385).
 void mul_ntt_ref(uint32_t* z, const uint32_t* a, size_t na, const uint32_t* b, size_t nb, cudaStream_t s);
-// One CTA per product, column sums in shared memory (na + nb <= kSchoolMax).
+// One CTA per product, in 8 x 8-word register blocks (na + nb <= kSchoolMaxWords).
 constexpr size_t kSchoolMaxWords = 4096;
 // Shared memory of the largest one (BlockProduct::words(): 513 blocks, one run of
 // 17-word diagonals; shorter ones with more runs take less).
