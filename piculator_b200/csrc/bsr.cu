@@ -1151,6 +1151,7 @@ struct WideAdd {
     uint32_t* hd;    // per parent: highest differing word + 1
     uint32_t* agg;   // per (parent, chunk): (G, P)
     uint32_t cpp;    // chunks per parent
+    const uint32_t* group;  // groups of chunks, see carry.cuh
 };
 
 struct WideOp {
@@ -1263,7 +1264,7 @@ __global__ void __launch_bounds__(256) wide_fix_kernel(WideAdd w)
     uint32_t* z = w.Pw + (w.c0 + i) * (size_t)w.cP;
     if (o.sub && c == 0 && threadIdx.x == 0) w.Ps[w.c0 + i] = o.zero ? 1 : ((o.swap ? sb : sa) ? 1 : 0);
     if (o.zero) return;
-    const uint32_t* agg = w.agg + i * (size_t)w.cpp;
+    const CarryAgg agg = CarryAgg{w.agg, w.group}.item(i, w.cpp);
     const uint32_t last = n ? (n - 1) / kWideWPC : 0;
     if (c > last) return;
     const uint32_t cin = chunk_carry_in(agg, c);
@@ -1271,7 +1272,7 @@ __global__ void __launch_bounds__(256) wide_fix_kernel(WideAdd w)
     if (cin) chunk_ripple(z, b0, e, o.sub);
     if (!o.sub) {
         if (c == last && threadIdx.x == 0) {
-            const uint32_t gp = agg[c];
+            const uint32_t gp = agg.chunk[c];
             const uint32_t carry = n ? ((gp & 1u) | ((gp >> 1) & cin)) : 0u;
             if (carry && n < w.cP) z[n] = 1;
             w.Pl[w.c0 + i] = n + carry;
@@ -1598,15 +1599,16 @@ static void signed_sum(const uint32_t* A, const uint32_t* lA, uint32_t cA, const
     ProfScope ps(KC_LINEAR, 12.0 * (double)np * (double)nmax, s);
     const uint32_t cpp = (uint32_t)((nmax + kWideWPC - 1) / kWideWPC);
     if (g_wide_add && np < 2 * 148 && cpp > 1) {
-        DevBuf<uint32_t> hd(np, s), agg(np * cpp, s);
+        DevBuf<uint32_t> hd(np, s), agg(carry_agg_words(np, cpp), s);
         PIC_CUDA(cudaMemsetAsync(hd.get(), 0, 4 * np, s));
         PIC_CUDA(cudaMemsetAsync(par.P.len.get() + p0, 0, 4 * np, s));
         WideAdd w{A, lA, B, lB, cA, cB, cS, p0, par.P.w.get(), par.P.len.get(), par.P.cap, par.sign.get(), hd.get(),
-                  agg.get(), cpp};
+                  agg.get(), cpp, nullptr};
         const unsigned grid = (unsigned)(np * cpp);
         wide_cmp_kernel<<<grid, 256, 0, s>>>(w);
         wide_k1_kernel<<<grid, 256, 0, s>>>(w);
         PIC_CHECK_LAUNCH();
+        w.group = carry_group(agg.get(), np, cpp, s).group;
         wide_fix_kernel<<<grid, 256, 0, s>>>(w);
         PIC_CHECK_LAUNCH();
         count_launch(3);

@@ -10,9 +10,37 @@ namespace cg = cooperative_groups;
 
 namespace pic {
 
+// ---- groups of chunks ---------------------------------------------------------
+__global__ void __launch_bounds__(256) carry_group_kernel(const uint32_t* __restrict__ agg, size_t cpp, size_t groups,
+                                                          uint32_t* __restrict__ out)
+{
+    const size_t item = blockIdx.x / groups, g = blockIdx.x - item * groups;
+    const uint32_t* a = agg + item * cpp;
+    constexpr int IPT = (int)kCarryGroup / 256;
+    const size_t i0 = g * kCarryGroup + (size_t)threadIdx.x * IPT;
+    uint32_t acc = kGPIdentity;
+#pragma unroll
+    for (int u = 0; u < IPT; u++)
+        if (i0 + u < cpp) acc = gp_combine(acc, a[i0 + u]);
+    uint32_t total;
+    block_gp_scan(acc, &total);
+    if (threadIdx.x == 0) out[blockIdx.x] = total;
+}
+
+CarryAgg carry_group(uint32_t* agg, size_t count, size_t cpp, cudaStream_t s)
+{
+    const size_t groups = carry_groups(cpp);
+    if (groups == 0) return CarryAgg{agg, nullptr};
+    uint32_t* out = agg + count * cpp;
+    carry_group_kernel<<<(unsigned)(count * groups), 256, 0, s>>>(agg, cpp, groups, out);
+    PIC_CHECK_LAUNCH();
+    count_launch();
+    return CarryAgg{agg, out};
+}
+
 // ---- K2 ---------------------------------------------------------------------
 __global__ void __launch_bounds__(256) carry_fix_kernel(uint32_t* z, size_t n, size_t wpc,
-                                                        const uint32_t* __restrict__ agg, size_t nctas, MailRef mail)
+                                                        CarryAgg agg, size_t nctas, MailRef mail)
 {
     const size_t c = blockIdx.x;
     const size_t b = c * wpc, e = b + wpc < n ? b + wpc : n;
@@ -23,32 +51,34 @@ __global__ void __launch_bounds__(256) carry_fix_kernel(uint32_t* z, size_t n, s
     }
 }
 
-void carry_fix(uint32_t* z, size_t nwords, size_t words_per_cta, const uint32_t* agg, size_t nctas, cudaStream_t s,
+void carry_fix(uint32_t* z, size_t nwords, size_t words_per_cta, uint32_t* agg, size_t nctas, cudaStream_t s,
                MailRef mail)
 {
     ProfScope ps(KC_CARRY, 4.0 * (double)nctas, s);
-    carry_fix_kernel<<<(unsigned)nctas, 256, 0, s>>>(z, nwords, words_per_cta, agg, nctas, mail);
+    const CarryAgg A = carry_group(agg, 1, nctas, s);
+    carry_fix_kernel<<<(unsigned)nctas, 256, 0, s>>>(z, nwords, words_per_cta, A, nctas, mail);
     PIC_CHECK_LAUNCH();
     count_launch();
 }
 
 __global__ void __launch_bounds__(256) carry_fix_batch_kernel(uint32_t* z, uint32_t zcap,
                                                               const uint32_t* __restrict__ zlen, size_t wpc,
-                                                              const uint32_t* __restrict__ agg, size_t cpp, bool sub)
+                                                              CarryAgg agg, size_t cpp, bool sub)
 {
     const size_t prod = blockIdx.x / cpp, c = blockIdx.x - prod * cpp;
     const size_t n = zlen[prod];
     const size_t b = c * wpc, e = b + wpc < n ? b + wpc : n;
-    if (b >= e || !chunk_carry_in(agg + prod * cpp, c)) return;
+    if (b >= e || !chunk_carry_in(agg.item(prod, cpp), c)) return;
     chunk_ripple(z + prod * (size_t)zcap, b, e, sub);
 }
 
-void carry_fix_batch(uint32_t* z, uint32_t zcap, const uint32_t* zlen, size_t words_per_cta, const uint32_t* agg,
+void carry_fix_batch(uint32_t* z, uint32_t zcap, const uint32_t* zlen, size_t words_per_cta, uint32_t* agg,
                      size_t count, size_t cpp, cudaStream_t s, bool sub)
 {
     if (cpp <= 1) return;  // one CTA per product: no carries between CTAs
     ProfScope ps(KC_CARRY, 4.0 * (double)(count * cpp), s);
-    carry_fix_batch_kernel<<<(unsigned)(count * cpp), 256, 0, s>>>(z, zcap, zlen, words_per_cta, agg, cpp, sub);
+    const CarryAgg A = carry_group(agg, count, cpp, s);
+    carry_fix_batch_kernel<<<(unsigned)(count * cpp), 256, 0, s>>>(z, zcap, zlen, words_per_cta, A, cpp, sub);
     PIC_CHECK_LAUNCH();
     count_launch();
 }
@@ -110,13 +140,13 @@ __device__ __forceinline__ void lin_end(const LinEnd& E, const uint32_t* z, size
 }
 
 // K2 of the linear operations (several CTAs).
-__global__ void __launch_bounds__(kLinThreads) lin_fix_kernel(uint32_t* z, size_t n, const uint32_t* __restrict__ agg,
-                                                              uint32_t nctas, LinEnd E, const uint32_t* a, uint32_t x)
+__global__ void __launch_bounds__(kLinThreads) lin_fix_kernel(uint32_t* z, size_t n, CarryAgg agg, uint32_t nctas,
+                                                              LinEnd E, const uint32_t* a, uint32_t x)
 {
     const size_t c = blockIdx.x;
     const size_t b = c * kLinWPC, e = b + kLinWPC < n ? b + kLinWPC : n;
     const uint32_t cin = chunk_carry_in(agg, c);
-    const uint32_t gp = agg[c];
+    const uint32_t gp = agg.chunk[c];
     if (cin) chunk_ripple(z, b, e, E.kind == kLinSub);
     if (E.kind == kLinMul) E.top_hi = (uint32_t)(((uint64_t)a[n - 1] * x) >> 32);
     lin_end(E, z, b, e, (gp & 1u) | ((gp >> 1) & cin), nctas);
@@ -230,12 +260,13 @@ void lin_set(uint32_t* p, uint32_t lo, uint32_t hi, int n, cudaStream_t s)
 
 static size_t lin_ctas(size_t n) { return (n + kLinWPC - 1) / kLinWPC; }
 
-static void lin_fix(uint32_t* z, size_t n, const uint32_t* agg, size_t nctas, const LinEnd& E, const uint32_t* a,
+static void lin_fix(uint32_t* z, size_t n, uint32_t* agg, size_t nctas, const LinEnd& E, const uint32_t* a,
                     uint32_t x, cudaStream_t s)
 {
     if (nctas <= 1) return;
     ProfScope ps(KC_CARRY, 4.0 * (double)nctas, s);
-    lin_fix_kernel<<<(unsigned)nctas, kLinThreads, 0, s>>>(z, n, agg, (uint32_t)nctas, E, a, x);
+    const CarryAgg A = carry_group(agg, 1, nctas, s);
+    lin_fix_kernel<<<(unsigned)nctas, kLinThreads, 0, s>>>(z, n, A, (uint32_t)nctas, E, a, x);
     PIC_CHECK_LAUNCH();
     count_launch();
 }
@@ -244,7 +275,7 @@ static void addsub(uint32_t* z, size_t TL, const WordView& a, const WordView& b,
                    cudaStream_t s)
 {
     const size_t nctas = lin_ctas(TL);
-    DevBuf<uint32_t> agg(nctas, s);
+    DevBuf<uint32_t> agg(carry_agg_words(1, nctas), s);
     ProfScope ps(KC_LINEAR, 12.0 * (double)TL, s);
     addsub_k1<<<(unsigned)nctas, kLinThreads, 0, s>>>(z, TL, a, b, bot, agg.get(), E);
     PIC_CHECK_LAUNCH();
@@ -455,7 +486,7 @@ uint32_t lin_mul_u32(uint32_t* z, const uint32_t* a, size_t L, uint32_t x)
     }
     const size_t nctas = lin_ctas(L);
     Mail mail(s);
-    DevBuf<uint32_t> agg(nctas, s);
+    DevBuf<uint32_t> agg(carry_agg_words(1, nctas), s);
     LinEnd E{};
     E.kind = kLinMul;
     E.carry_out = z + L;

@@ -16,7 +16,12 @@
 //       1, ripples it through its own words.
 // A chunk passes a carry on only when all its words are all-ones (zero), so
 // the aggregate just below decides almost always; where it does not, the CTA
-// scans all those below it.
+// scans all those below it.  Of more than kCarryDirect chunks a launch between
+// the two makes one (G, P) per kCarryGroup chunks, and a CTA scans those of the
+// groups below and its own group's: scanning every chunk below takes time that
+// grows with the square of a run of all-ones (zero) words, 28 ms of the
+// difference of two equal numbers of 4e8 words where their words take 4; the
+// launch costs 3 us, a scan of as many chunks as the line allows some 25.
 // Against a scan launch and a ripple launch (three in all): division and inverse
 // square root at 300,007 words 9.65 -> 4.17 ms together with the results posted
 // to the host (common.cuh) and the comparison of a difference left on the
@@ -150,17 +155,37 @@ __device__ __forceinline__ bool last_cta(uint32_t* ticket, uint32_t nctas)
     return s_last;
 }
 
-// The carry into chunk c from the (G, P) of chunks 0 .. c - 1 (every thread
-// calls, the same result in each).
-__device__ __forceinline__ uint32_t chunk_carry_in(const uint32_t* __restrict__ agg, size_t c)
+constexpr size_t kCarryDirect = 8192, kCarryGroup = 512;
+
+// Groups of an item of cpp chunks (0: none), and the words its aggregates take:
+// `count` items of cpp chunks, then their groups.
+inline size_t carry_groups(size_t cpp) { return cpp > kCarryDirect ? (cpp + kCarryGroup - 1) / kCarryGroup : 0; }
+inline size_t carry_agg_words(size_t count, size_t cpp) { return count * (cpp + carry_groups(cpp)); }
+
+// The aggregates of one item as K2 reads them.
+struct CarryAgg {
+    const uint32_t* chunk;
+    const uint32_t* group;  // null: none
+    __host__ __device__ CarryAgg item(size_t i, size_t cpp) const
+    {
+        return CarryAgg{chunk + i * cpp, group ? group + i * ((cpp + kCarryGroup - 1) / kCarryGroup) : nullptr};
+    }
+};
+// Makes the groups of `count` items where there are any (agg: carry_agg_words).
+CarryAgg carry_group(uint32_t* agg, size_t count, size_t cpp, cudaStream_t s);
+
+// The carry into chunk c of an item from the (G, P) of chunks 0 .. c - 1 (every
+// thread calls, the same result in each).
+__device__ __forceinline__ uint32_t chunk_carry_in(const CarryAgg& A, size_t c)
 {
     if (c == 0) return 0;
-    const uint32_t below = agg[c - 1];
+    const uint32_t below = A.chunk[c - 1];
     if (!(below & 2u)) return below & 1u;
-    const size_t per = (c + blockDim.x - 1) / blockDim.x;
-    const size_t b = threadIdx.x * per < c ? threadIdx.x * per : c, e = b + per < c ? b + per : c;
+    const size_t ng = A.group ? c / kCarryGroup : 0, c0 = ng * kCarryGroup, n = ng + (c - c0);
+    const size_t per = (n + blockDim.x - 1) / blockDim.x;
+    const size_t b = threadIdx.x * per < n ? threadIdx.x * per : n, e = b + per < n ? b + per : n;
     uint32_t acc = kGPIdentity;
-    for (size_t i = b; i < e; i++) acc = gp_combine(acc, agg[i]);
+    for (size_t i = b; i < e; i++) acc = gp_combine(acc, i < ng ? A.group[i] : A.chunk[c0 + (i - ng)]);
     uint32_t total;
     block_gp_scan(acc, &total);
     return total & 1u;
@@ -186,13 +211,13 @@ __device__ __forceinline__ void chunk_ripple(uint32_t* z, size_t b, size_t e, bo
     if (threadIdx.x == 0 && f < e) z[f] += sub ? 0xffffffffu : 1u;
 }
 
-// K2 (carry.cu).  agg[c] = (G, P) of CTA c, which owns words_per_cta words.
-// mail: receives the top word z[nwords - 1].
-void carry_fix(uint32_t* z, size_t nwords, size_t words_per_cta, const uint32_t* agg, size_t nctas, cudaStream_t s,
+// K2 (carry.cu).  agg[c] = (G, P) of CTA c, which owns words_per_cta words;
+// carry_agg_words(1, nctas) words.  mail: receives the top word z[nwords - 1].
+void carry_fix(uint32_t* z, size_t nwords, size_t words_per_cta, uint32_t* agg, size_t nctas, cudaStream_t s,
                MailRef mail = MailRef{});
 // For batches of products: `count` segments of `cpp` CTAs; product i writes
-// zlen[i] words at z + i * zcap.
-void carry_fix_batch(uint32_t* z, uint32_t zcap, const uint32_t* zlen, size_t words_per_cta, const uint32_t* agg,
+// zlen[i] words at z + i * zcap; agg of carry_agg_words(count, cpp) words.
+void carry_fix_batch(uint32_t* z, uint32_t zcap, const uint32_t* zlen, size_t words_per_cta, uint32_t* agg,
                      size_t count, size_t cpp, cudaStream_t s, bool sub = false);
 
 }  // namespace pic

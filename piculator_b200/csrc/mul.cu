@@ -381,7 +381,7 @@ void coef16_to_words(const uint64_t* c, size_t ncoef, uint64_t scale_mont, uint6
     if (zw == 0) return;
     const size_t nlimbs = (zw + 1) / 2;
     const size_t nctas = (nlimbs + kCvtLPC - 1) / kCvtLPC;
-    DevBuf<uint32_t> agg(nctas, s);
+    DevBuf<uint32_t> agg(carry_agg_words(1, nctas), s);
     ProfScope ps(KC_CRT, 8.0 * (double)ncoef + 4.0 * (double)zw, s);
     coeflimbs_k1<16, NttCoefLoader><<<(unsigned)nctas, kCvtThreads, 0, s>>>(
         NttCoefLoader{c, scale_mont, p, pinv_neg}, ncoef, z, zw, agg.get(), nullptr);
@@ -397,7 +397,7 @@ double fft_coef_to_words(const double2* T, size_t ncoef, double scale, int bits,
     if (zw == 0) return 0.0;
     const size_t nlimbs = (zw + 1) / 2;
     const size_t nctas = (nlimbs + kCvtLPC - 1) / kCvtLPC;
-    DevBuf<uint32_t> agg(nctas, s);
+    DevBuf<uint32_t> agg(carry_agg_words(1, nctas), s);
     DevBuf<unsigned long long> err(1, s);
     PIC_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(unsigned long long), s));
     ProfScope ps(KC_CRT, 16.0 * (double)ncoef + 4.0 * (double)zw, s);
@@ -480,7 +480,7 @@ void ntt3_inverse_to_words(uint64_t* y, int k, size_t ncoef, int depth, uint32_t
     const Crt3Consts C = make_crt3(k, depth);
     const size_t nlimbs = (zw + 1) / 2;
     const size_t nctas = (nlimbs + kCrtLPC - 1) / kCrtLPC;
-    DevBuf<uint32_t> agg(nctas, s);
+    DevBuf<uint32_t> agg(carry_agg_words(1, nctas), s);
     ProfScope ps(KC_CRT, 24.0 * (double)ncoef + 4.0 * (double)zw, s);
     crt3_k1<<<(unsigned)nctas, kCvtThreads, 0, s>>>(y, (size_t)1 << k, ncoef, C, z, zw, agg.get());
     PIC_CHECK_LAUNCH();
@@ -498,7 +498,7 @@ void ntt3_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, size
         for (int q = 0; q < 3; q++) C.off[q] = host_powmod(2, 159, C.p[q]);
     const size_t cpp = (((size_t)zcap + 1) / 2 + kCrtLPC - 1) / kCrtLPC;
     const size_t nctas = count * cpp;
-    DevBuf<uint32_t> agg(nctas, s);
+    DevBuf<uint32_t> agg(carry_agg_words(count, cpp), s);
     {
         ProfScope ps(KC_CRT, (24.0 * (double)ncoef + 4.0 * zcap) * (double)count, s);
         crt3_batch_k1<<<(unsigned)nctas, kCvtThreads, 0, s>>>(y, istride, pstride, ncoef, C, z, zcap, zlen,
@@ -526,6 +526,7 @@ void crt3_to_words_scratch(const uint64_t* y, int k, size_t ncoef, uint32_t* z, 
 {
     const Crt3Consts C = make_crt3(k, 1);
     const size_t nctas = crt3_scratch_ctas(zw);
+    PIC_REQUIRE(carry_groups(nctas) == 0, PIC_ERR_LENGTH, "product too long for the scratch form");
     crt3_k1<<<(unsigned)nctas, kCvtThreads, 0, s>>>(y, (size_t)1 << k, ncoef, C, z, zw, agg);
     PIC_CHECK_LAUNCH();
     count_launch();
@@ -721,7 +722,7 @@ static void mul_ntt3_wrapped(uint32_t* z, const uint32_t* a, size_t na, const ui
     }
     const Crt3Consts C = make_crt3(km, 1);
     const size_t nctas = crt3_scratch_ctas(zw);
-    DevBuf<uint32_t> agg(nctas, s);
+    DevBuf<uint32_t> agg(carry_agg_words(1, nctas), s);
     ProfScope ps(KC_CRT, 24.0 * (double)L + 4.0 * (double)zw, s);
     crt3_k1<<<(unsigned)nctas, kCvtThreads, 0, s>>>(A.get(), ST, L, C, z, zw, agg.get());
     PIC_CHECK_LAUNCH();
@@ -982,7 +983,7 @@ static void crt3d_to_words(const uint64_t* y, size_t pstride, int k, size_t ncoe
 {
     const CrtDConsts C = make_crtd(k, false);
     const size_t nctas = crt3d_ctas(zw);
-    DevBuf<uint32_t> agg(nctas, s);
+    DevBuf<uint32_t> agg(carry_agg_words(1, nctas), s);
     const MailRef m = mail ? mail->ref() : MailRef{};
     ProfScope ps(KC_CRT, 24.0 * (double)ncoef + 4.0 * (double)zw, s);
     auto kern = wrap.tail ? crt3d_k1<true> : crt3d_k1<false>;
@@ -1014,7 +1015,7 @@ void ntt3d_batch_to_words(const uint64_t* y, size_t istride, size_t pstride, siz
     }
     const size_t cpp = crt3d_ctas(zcap);
     const size_t nctas = count * cpp;
-    DevBuf<uint32_t> agg(nctas, s);
+    DevBuf<uint32_t> agg(carry_agg_words(count, cpp), s);
     {
         ProfScope ps(KC_CRT, (24.0 * (double)ncoef + 4.0 * zcap) * (double)count, s);
         auto kern = wrap.tail ? crt3d_batch_k1<true> : crt3d_batch_k1<false>;

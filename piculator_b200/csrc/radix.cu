@@ -117,25 +117,26 @@ __global__ void __launch_bounds__(kDecThreads) dec_sub_k1(uint32_t* __restrict__
 
 // K2: CTAs with a borrow in subtract it from their own words.
 __global__ void __launch_bounds__(256) dec_sub_fix(uint32_t* r, size_t r_stride, size_t n, size_t cpi,
-                                                   const uint32_t* __restrict__ agg)
+                                                   CarryAgg agg)
 {
     const size_t it = blockIdx.x / cpi, c = blockIdx.x - it * cpi;
     const size_t b = c * kDecWPC, e = b + kDecWPC < n ? b + kDecWPC : n;
-    if (chunk_carry_in(agg + it * cpi, c)) chunk_ripple(r + it * r_stride, b, e, true);
+    if (chunk_carry_in(agg.item(it, cpi), c)) chunk_ripple(r + it * r_stride, b, e, true);
 }
 
 static void dec_sub(uint32_t* r, size_t r_stride, const uint32_t* a, size_t a_stride, const uint32_t* b,
                     size_t b_stride, size_t b_words, size_t n, size_t count, cudaStream_t s)
 {
     const size_t cpi = (n + kDecWPC - 1) / kDecWPC;
-    DevBuf<uint32_t> agg(count * cpi, s);
+    DevBuf<uint32_t> agg(carry_agg_words(count, cpi), s);
     ProfScope ps(KC_LINEAR, 12.0 * (double)(count * n), s);
     dec_sub_k1<<<(unsigned)(count * cpi), kDecThreads, 0, s>>>(r, r_stride, a, a_stride, b, b_stride, b_words, n,
                                                               cpi, agg.get());
     PIC_CHECK_LAUNCH();
     count_launch();
     if (cpi == 1) return;
-    dec_sub_fix<<<(unsigned)(count * cpi), 256, 0, s>>>(r, r_stride, n, cpi, agg.get());
+    const CarryAgg A = carry_group(agg.get(), count, cpi, s);
+    dec_sub_fix<<<(unsigned)(count * cpi), 256, 0, s>>>(r, r_stride, n, cpi, A);
     PIC_CHECK_LAUNCH();
     count_launch();
 }

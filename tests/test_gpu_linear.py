@@ -5,6 +5,7 @@ through all of them, against Python integers; and the comparison that orders a
 subtraction, from several threads at once."""
 from __future__ import annotations
 
+import ctypes as C
 import threading
 import time
 
@@ -142,3 +143,63 @@ def test_long_ordered_differences_from_several_threads(pic):
     for t in threads:
         t.join()
     assert not bad
+
+
+CHUNK, DIRECT, GROUP = 2048, 8192, 512  # words of a chunk; chunks scanned directly; chunks of a group
+
+
+@pytest.mark.parametrize("n", [DIRECT * CHUNK, DIRECT * CHUNK + 1, 20_000_003])
+def test_carries_through_groups_of_chunks(pic, n):
+    """More than 8192 chunks: a carry through all of them, through some of them up to
+    or from the edge of a chunk and of a group, and a borrow the same way."""
+    one = pic.DeviceBigFloat.from_u32(1)
+    ones = np.full(n, 0xFFFFFFFF, dtype=np.uint32)
+    got = _num(pic, ones).add(one).to_bf()
+    assert got.words.size == n + 1 and got.words[n] == 1 and not got.words[:n].any()
+    got = got.words
+    got = _num(pic, got).sub(one).to_bf()
+    assert got.words.size == n and np.all(got.words == 0xFFFFFFFF)
+    got = _num(pic, ones).mul_u32(0xFFFFFFFF).to_bf().words  # (B^n - 1)(B - 1)
+    assert got[0] == 1 and np.all(got[1:n] == 0xFFFFFFFF) and got[n] == 0xFFFFFFFE
+    for c in (1, GROUP, GROUP + 1, 3 * GROUP - 1, DIRECT - 1):
+        for q in (c * CHUNK - 1, c * CHUNK):
+            w = ones.copy()
+            w[q] = 7
+            got = _num(pic, w).add(one).to_bf().words  # stops at q
+            assert not got[:q].any() and got[q] == 8 and np.all(got[q + 1:] == 0xFFFFFFFF)
+            w = np.zeros(n, dtype=np.uint32)
+            w[q], w[n - 1] = 7, 5
+            low = np.zeros(2 * CHUNK + 1, dtype=np.uint32)
+            low[0], low[-1] = 1, 1
+            if q > 2 * CHUNK:  # two borrows, the second from a chunk further up
+                got = _num(pic, w).sub(_num(pic, low)).to_bf().words
+                assert np.all(got[:2 * CHUNK] == 0xFFFFFFFF) and got[2 * CHUNK] == 0xFFFFFFFE
+                assert np.all(got[2 * CHUNK + 1:q] == 0xFFFFFFFF) and got[q] == 6 and got[n - 1] == 5
+
+
+def test_long_runs_cost_what_their_words_cost(pic, torch_cuda):
+    """The carries through a run of all-ones or zero words take time in proportion."""
+    torch = torch_cuda
+    n = 400_000_000
+
+    def number(t):
+        out = C.c_void_p()
+        torch.cuda.synchronize()
+        pic.check(pic.lib().pic_bf_from_device(C.byref(out), 1, 0, t.data_ptr(), n, None))
+        return pic.DeviceBigFloat(out.value)
+
+    def cost(x, y):
+        seconds = []
+        for _ in range(5):
+            pic.synchronize()
+            t = time.perf_counter()
+            z = x.sub(y)
+            pic.synchronize()
+            seconds.append(time.perf_counter() - t)
+            del z
+        return sorted(seconds)[2]
+
+    ones = number(torch.full((n,), -1, dtype=torch.int32, device="cuda"))
+    a = torch.randint(1, 1 << 31, (n,), dtype=torch.int32, device="cuda")
+    x, y = number(a), number(a ^ 0x5555)
+    assert cost(ones, ones) < 3 * cost(x, y)  # 7 times before groups

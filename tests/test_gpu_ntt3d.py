@@ -278,3 +278,13 @@ def test_largest_residues_through_three_bit_columns(pic, pa, pb, bits):
             got = pic.mul_host(x, y, "ntt3d")
             assert np.array_equal(got, pic.mul_host(x, y, "ntt3")), p
             assert _int(got) == _int(x) * _int(y), p
+
+
+@pytest.mark.parametrize("mode", ["ntt3d", "ntt3"])
+def test_carry_chain_through_groups_of_chunks(pic, mode):
+    """(B^n - 1)^2 with more than 8192 CTAs' chunks of result words."""
+    n = (1 << 23) + 12_345
+    ones = np.full(n, 0xFFFFFFFF, dtype=np.uint32)
+    z = pic.mul_host(ones, ones, mode)
+    assert z[0] == 1 and not z[1:n].any()
+    assert z[n] == 0xFFFFFFFE and np.all(z[n + 1:] == 0xFFFFFFFF)
